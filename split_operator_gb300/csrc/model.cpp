@@ -262,11 +262,25 @@ static void upload_complex(DeviceBuffer& buf, const std::vector<cplx>& t, int re
   }
 }
 
+// largest magnitude of a table (infinity when a value is not finite)
+static double table_max(const std::vector<cplx>& t) {
+  double m = 0.0;
+  bool ok = true;
+  for (const cplx& v : t) {
+    const double a = v.real() * v.real() + v.imag() * v.imag();
+    ok = ok && a <= 1e300;  // false for NaN
+    m = a > m ? a : m;
+  }
+  return ok ? std::sqrt(m) : HUGE_VAL;
+}
+
 const void* Engine::table_1d(const void* key, uint64_t version, const std::vector<cplx>& t) {
   auto& c = tables_[{key, 0}];
   if (c.buf.ptr && c.version == version) return c.buf.ptr;
   if (c.buf.ptr) flush();  // replacing a table the open pass may reference (a first upload needs no flush)
   upload_complex(c.buf, t, real, stream);
+  c.fx = DeviceBuffer();
+  if (fx) c.max_abs = table_max(t);
   c.version = version;
   return c.buf.ptr;
 }
@@ -295,8 +309,79 @@ const void* Engine::table_nd(const void* key, uint64_t version, const std::vecto
     st[s] = t[li];
   }
   upload_complex(c.buf, st, real, stream);
+  c.fx = DeviceBuffer();
+  if (fx) c.max_abs = table_max(t);
   c.version = version;
   return c.buf.ptr;
+}
+
+Engine::Cached* Engine::phase_table(const void* device_ptr) {
+  for (auto& kv : tables_)
+    if (kv.first.second < 2 && kv.second.buf.ptr == device_ptr) return &kv.second;
+  return nullptr;
+}
+
+const void* Engine::fx_table(Cached& c) {
+  if (c.fx.ptr) return c.fx.ptr;
+  DeviceBuffer b(c.buf.bytes);
+  cuda_check(launch_fx_table(b.ptr, c.buf.ptr, real, (int64_t)(c.buf.bytes / 16), stream), "fixed-point table");
+  // as the uploads: complete before any stream of the engine uses it
+  cuda_check(cudaStreamSynchronize(stream), "fixed-point table sync");
+  c.fx = std::move(b);
+  return c.fx.ptr;
+}
+
+// Twiddles of the fixed-point FFT pair: w 2^62 in two signed digits {re.l, re.h, im.l, im.h},
+// stage-major for radix 16 (forward order, then reversed order), one copy per device and length
+// for the process (entries are held weakly, by the engines that use them).
+const void* Engine::fx_twiddle(size_t n) {
+  static std::mutex mu;
+  static std::map<std::pair<int, size_t>, std::weak_ptr<DeviceBuffer>> cache;
+  auto& mine = fx_twiddles_[n];
+  if (mine) return mine->ptr;
+  int dev = 0;
+  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+  std::lock_guard<std::mutex> lock(mu);
+  auto& slot = cache[{dev, n}];
+  mine = slot.lock();
+  if (mine) return mine->ptr;
+  // (cos, sin) of 2 pi m / n times 2^62 for m = 0 .. n / 8, the other octants by symmetry
+  const long double kTau = 6.283185307179586476925286766559005768L;
+  std::vector<std::pair<int64_t, int64_t>> oct0(n / 8 + 1);
+  for (size_t m = 0; m <= n / 8; ++m) {
+    const long double a = kTau * (long double)m / (long double)n;
+    oct0[m] = {(int64_t)llroundl(ldexpl(cosl(a), 62)), (int64_t)llroundl(ldexpl(sinl(a), 62))};
+  }
+  std::vector<int32_t> st(8 * n, 0);
+  auto put = [](int64_t v, int32_t* d) {
+    if ((int32_t)v == INT32_MIN) ++v;  // the kernels negate digits
+    const int32_t l = (int32_t)v;
+    d[0] = l;
+    d[1] = (int32_t)((v - l) >> 32);
+  };
+  for (size_t e = 0; e < 2 * n; ++e) {
+    const size_t m = (size_t)stage_twiddle_exponent((int64_t)(e % n), (int64_t)n, 16, e >= n) % n;
+    const size_t quad = 4 * m / n, r = m - quad * (n / 4);  // r < n / 4 within quadrant quad
+    int64_t c, s;
+    if (r <= n / 8) {
+      c = oct0[r].first;
+      s = oct0[r].second;
+    } else {
+      c = oct0[n / 4 - r].second;
+      s = oct0[n / 4 - r].first;
+    }
+    for (size_t q = 0; q < quad; ++q) {
+      const int64_t t = c;
+      c = -s;
+      s = t;
+    }
+    put(c, &st[4 * e]);
+    put(-s, &st[4 * e + 2]);  // exp(-2 pi i m / n)
+  }
+  mine = std::make_shared<DeviceBuffer>();
+  upload(*mine, st, stream);
+  slot = mine;
+  return mine->ptr;
 }
 
 // Parity structure of a real n x n matrix (logical M[a][b] = m[a n + b]) within tol of its
@@ -550,11 +635,7 @@ bool Engine::try_launch_tc(const std::vector<DevOp>& ops, int axis, PassParams& 
   g.tiles_per_outer = (int32_t)(g.inner / bn);
   g.tiles = g.outer * g.tiles_per_outer;
   p.g = g;
-  if ((size_t)g.tiles > partials_cap_) {
-    partials_cap_ = (size_t)g.tiles;
-    partials_ = DeviceBuffer(partials_cap_ * kMaxRed * sizeof(double));
-    p.partials = partials_.as<double>();
-  }
+  grow_partials(p);
   static const char* const kTcNames[3] = {"f32 tc3xtf32", "f32 tcbf16x3", "f32 tcbf16x6"};
   std::string name = std::string(kTcNames[tc_mode()]) + (par ? " parity axis" : (pk > 1 ? " packed axis" : " axis")) +
                      std::to_string(axis) + ":";
@@ -680,6 +761,32 @@ void Engine::submit(const Action& a) {
   cur_.push_back(op);
 }
 
+bool Engine::try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p) {
+  double mx[kMaxOps] = {};
+  Cached* tab[kMaxOps] = {};
+  for (size_t i = 0; i < ops.size(); ++i)
+    if (ops[i].kind == OP_DIAGND || ops[i].kind == OP_DIAG1D) {
+      tab[i] = phase_table(ops[i].ptr);
+      if (!tab[i]) return false;
+      mx[i] = tab[i]->max_abs;
+    }
+  if (!fx_pair_plan(p, real, mx)) return false;
+  for (size_t i = 0; i < ops.size(); ++i)
+    if (tab[i]) p.ops[i].ptr = fx_table(*tab[i]);
+  p.twiddle = fx_twiddle((size_t)p.g.n);
+  return true;
+}
+
+// Room for the norm partials of a pass (one entry per reduction and tile).  The buffer it
+// replaces is kept: passes recorded earlier (a batch's, launched later) hold its address.
+void Engine::grow_partials(PassParams& p) {
+  if (p.nred == 0 || (size_t)p.g.tiles <= partials_cap_) return;
+  retired_partials_.push_back(std::move(partials_));
+  partials_cap_ = (size_t)p.g.tiles;
+  partials_ = DeviceBuffer(partials_cap_ * kMaxRed * sizeof(double));
+  p.partials = partials_.as<double>();
+}
+
 void Engine::launch(const std::vector<DevOp>& ops, int axis, bool resident, int repeat) {
   PassParams p{};
   const char* name_tag = "";
@@ -705,7 +812,9 @@ void Engine::launch(const std::vector<DevOp>& ops, int axis, bool resident, int 
   if (fft) p.twiddle = twiddle((size_t)p.g.n);
   pass_choose_buffers(p, fp64);
   if (!fp64 && tc_mode() >= 0 && !resident && try_launch_tc(ops, axis, p)) return;
-  if ((fft_pair || (fp64 && p.g.n > 4096)) && fft_pair_plan(p, real, resident)) {
+  if (fx && !resident && try_launch_fx_pair(ops, p)) {
+    name_tag = " fftpair fx";
+  } else if ((fft_pair || (fp64 && p.g.n > 4096)) && fft_pair_plan(p, real, resident)) {
     name_tag = p.radix == 8 && !fp64 ? " fftpair r8" : " fftpair";
     if (p.radix != (fp64 ? 8 : 16)) p.twiddle = twiddle((size_t)p.g.n, p.radix);  // the table in its stage order
     p.ct = fft_pair_ct ? fft_pair_ct_lgn(p, fp64) : 0;
@@ -714,20 +823,17 @@ void Engine::launch(const std::vector<DevOp>& ops, int axis, bool resident, int 
   if (fp64 && p.g.n > 4096 && !p.fused)
     throw Error(SO_ERR_UNSUPPORTED, "FP64 lanes longer than 4096 points are not supported outside FFT-pair passes "
                                     "([FFT] [point-wise] [FFT] [point-wise] on contiguous power-of-two lanes)");
-  if (!resident && (size_t)p.g.tiles > partials_cap_) {
-    partials_cap_ = (size_t)p.g.tiles;
-    partials_ = DeviceBuffer(partials_cap_ * kMaxRed * sizeof(double));
-    p.partials = partials_.as<double>();
-  }
+  if (!resident) grow_partials(p);
   std::string name = std::string(real == kRealFF ? "ff" : (fp64 ? "f64" : "f32")) + (resident ? " resident" : " sweep") +
                      name_tag + " axis" +
                      std::to_string(axis) + ":";
   for (const DevOp& o : ops) name += std::string(" ") + op_kind_name(o.kind);
   if (recording) {
     // fused FFT pairs: bit 16 of the thread count (their own launch group and kernel)
-    // radix-8 FP32 pairs: bit 19 (their own kernel); fixed-shape FP32 pairs: bit 20
+    // radix-8 FP32 pairs: bit 19 (their own kernel); fixed-shape FP32 pairs: bit 20;
+    // fixed-point pairs: bit 25
     const int threads = p.fused ? (fft_pair_block(p.g) | (1 << 16) | (p.radix == 8 && !fp64 ? 1 << 19 : 0) |
-                                   (p.ct ? 1 << 20 : 0))
+                                   (p.ct ? 1 << 20 : 0) | (p.fx ? 1 << 25 : 0))
                                 : pass_threads(p.g);
     RecordedPass r{resident ? RecordedPass::Resident : RecordedPass::Generic, real, p, {},
                    threads, pass_smem_bytes(p, fp64), name, pass_bytes(ops, p.g)};
@@ -738,8 +844,14 @@ void Engine::launch(const std::vector<DevOp>& ops, int axis, bool resident, int 
     timed_begin(name);
     timed_.back().bytes = pass_bytes(ops, p.g);
   }
-  cuda_check(real == kRealFF ? launch_pass_ff(p, stream) : (fp64 ? launch_pass_f64(p, stream) : launch_pass_f32(p, stream)),
-             "pass launch");
+  if (p.fx)
+    cuda_check(launch_fx_pair(real, p.fx, &p, nullptr, nullptr, 0, p.g.tiles, fft_pair_block(p.g),
+                              pass_smem_bytes(p, true), stream),
+               "pass launch");
+  else
+    cuda_check(real == kRealFF ? launch_pass_ff(p, stream)
+                               : (fp64 ? launch_pass_f64(p, stream) : launch_pass_f32(p, stream)),
+               "pass launch");
   if (timing) timed_end();
 }
 
@@ -1343,6 +1455,8 @@ Propagation::Propagation(WaveFunction& src, so_time_grid time, std::shared_ptr<O
     wf_->eng->fft_pair = !(fp && fp[0] == '0');
     const char* ct = std::getenv("SO_FFT_PAIR_CT");  // "0": FFT pairs keep the general-shape kernel
     wf_->eng->fft_pair_ct = !(ct && ct[0] == '0');
+    const char* fxe = std::getenv("SO_FX");  // "0": FP64 and float-float passes stay in floating point
+    wf_->eng->fx = real != kRealF32 && !(fxe && fxe[0] == '0');
   }
   wf_->last_grid_names = src.last_grid_names;
   wf_->possible_norm_change = src.possible_norm_change;
@@ -1857,6 +1971,7 @@ std::vector<Batch::Group> Batch::build_groups(const std::vector<std::vector<Reco
     g.name = "batched " + std::to_string(v.size()) + "x " + v[0]->name;
     g.n = v[0]->p.g.n;
     if (g.kind == RecordedPass::Generic && ((g.threads >> 20) & 1)) g.ct_lgn = v[0]->p.ct;
+    if (g.kind == RecordedPass::Generic && ((g.threads >> 25) & 1)) g.fx_lgn = v[0]->p.fx;
     std::vector<int64_t> off(v.size() + 1, 0);
     const size_t pb = g.kind == RecordedPass::TensorCore ? tc_params_bytes() : sizeof(PassParams);
     std::vector<unsigned char> params(pb * v.size());
@@ -1968,6 +2083,10 @@ void Batch::run_groups(std::vector<Group>& gs, bool concurrent) {
       cuda_check(launch_angular_tc_batched(g.params.ptr, g.owners.ptr, g.blocks, g.smem, (g.threads >> 17) & 3,
                                            st, (g.threads >> 20) & 3, 1 << ((g.threads >> 23) & 3)),
                  "batched tensor-core pass");
+    else if (g.fx_lgn)
+      cuda_check(launch_fx_pair(g.real, g.fx_lgn, nullptr, g.params.as<PassParams>(), g.offsets.as<int64_t>(), g.count,
+                                g.blocks, g.threads & 0xffff, g.smem, st),
+                 "batched pass");
     else
       cuda_check(launch_pass_batched(g.real, g.sweep, (g.threads >> 16) & 1, g.params.as<PassParams>(),
                                      g.offsets.as<int64_t>(), g.count, g.blocks, g.threads & 0xffff, g.smem, st,

@@ -135,6 +135,7 @@ class Engine {
   int tc_mode() const { return tc_tf32 ? 0 : (tc_bf16 ? 1 : (tc_bf16x6 ? 2 : -1)); }
   bool fft_pair = true;  // FP32 FFT-pair passes run the fused register kernel (SO_FFT_PAIR=0: the general pass)
   bool fft_pair_ct = true;  // ... its fixed-shape form where it applies (SO_FFT_PAIR_CT=0: the general shape)
+  bool fx = false;  // FP64 / float-float passes in 64-bit fixed point where they can (SO_FX=0: floating point)
 
   size_t points() const;
   size_t elem_bytes() const { return fp64 ? 16 : 8; }
@@ -201,6 +202,8 @@ class Engine {
   cudaEvent_t take_event();
   double pass_bytes(const std::vector<DevOp>& ops, const Geometry& g) const;
   DeviceBuffer slots_, partials_, counter_, staging_;
+  std::vector<DeviceBuffer> retired_partials_;
+  void grow_partials(PassParams& p);
   size_t partials_cap_ = 0;
   std::vector<int> free_slots_;
   int next_slot_ = 1;
@@ -208,6 +211,8 @@ class Engine {
     uint64_t version;
     DeviceBuffer buf;
     bool real;
+    double max_abs = 0.0;  // phase tables: the largest magnitude (infinity when one is not finite)
+    DeviceBuffer fx;       // phase tables: fixed-point copy, made at its first use
     int parity = 0;     // float-float: kind of the parity structure, half matrix in half_buf
     DeviceBuffer half_buf;
     // A-operand chunk images of the tensor-core passes, and the same for the parity-split
@@ -225,6 +230,11 @@ class Engine {
   bool try_launch_tc(const std::vector<DevOp>& ops, int axis, PassParams& p);
   static void shared_tc_images(const std::vector<double>& md, int n, int mode, cudaStream_t s,
                                std::shared_ptr<DeviceBuffer>& img, std::shared_ptr<DeviceBuffer>& par, int& kind);
+  bool try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p);
+  Cached* phase_table(const void* device_ptr);           // the cache entry of a phase table
+  const void* fx_table(Cached& c);                       // its fixed-point copy
+  const void* fx_twiddle(size_t n);                      // fixed-point twiddles, shared by the process
+  std::map<size_t, std::shared_ptr<DeviceBuffer>> fx_twiddles_;
   std::map<uint64_t, DeviceBuffer> weights_;
   std::map<std::pair<size_t, int>, DeviceBuffer> twiddles_;  // by (n, stage radix)
   // open pass
@@ -502,6 +512,7 @@ class Batch {
     double bytes;
     int64_t n = 0;  // lane extent of the members' passes (the schedule class)
     int ct_lgn = 0;  // fixed-shape FFT-pair kernel: log2 of the lane extent (0: general shape)
+    int fx_lgn = 0;  // fixed-point FFT-pair kernel: log2 of the lane extent (0: floating point)
   };
   std::vector<Group> build_groups(const std::vector<std::vector<RecordedPass>>& rec, size_t pos);
   std::vector<std::vector<RecordedPass>> cached_rec_;  // the passes the cached groups were built from

@@ -1,0 +1,126 @@
+"""The fixed-point passes of FP64 and float-float states against numpy.
+
+FFT pair [F, K, F^-1, phase]: every power-of-two lane length, tiles that do not divide the lane
+count, lanes of very different magnitude, lanes that are zero or not finite.  numpy's FP64
+transform pair is within 5e-16 of the exact one (relative L2 per lane), the fixed-point pass
+within 4e-16; a float-float result is rounded to 2^-47 per value.  The bounds are twice the sums.
+"""
+import numpy as np
+import pytest
+
+from tests.gpu_common import ensure_built
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"fp64": 2e-15, "float_float": 2e-14}
+
+
+@pytest.fixture(scope="module")
+def so():
+    ensure_built()
+    import split_operator_gb300 as so
+    return so
+
+
+def _lanes(lanes, n, seed):
+    rng = np.random.default_rng(seed)
+    x = np.arange(n)
+    a = rng.standard_normal((lanes, n)) + 1j * rng.standard_normal((lanes, n))
+    # packets, a single point, and magnitudes from 1e-25 to 1e25
+    a[1::4] = np.exp(-((x - 0.4 * n) / (0.03 * n + 1.0)) ** 2 + 0.7j * x)
+    a[2::4] = 0.0
+    a[2::4, n // 3] = 1.0 - 2.0j
+    return a * 10.0 ** rng.integers(-25, 26, (lanes, 1))
+
+
+def _pass(so, a, precision, scale=None):
+    """[FFT, kinetic phase, inverse FFT] (scale None), or with a full-size table of magnitude
+    `scale` before and after it; an identity matrix along the lane axis keeps the table before the
+    transforms in a pass of its own.  Returns (result, reference, the passes' names)."""
+    lanes, n = a.shape
+    lg = so.Grid.new_linear_countable("lane", 0.0, lanes - 1.0, lanes, 0)
+    xg = so.Grid.new_linear_continuos("x", -5.0, 5.0, n, 1)
+    tg = so.TimeGrid(0.01, 100)
+    st = so.OperationStack()
+    t = np.ones((lanes, n), dtype=np.complex128)
+    if scale is not None:
+        t = scale * np.exp(-1j * np.random.default_rng(n).uniform(-3.0, 3.0, (lanes, n)))
+        mt = so.MatrixTransformation(lg, so.Grid.new_linear_countable("same", 0.0, lanes - 1.0, lanes, 0))
+        mt.set_diagonalization_matrix(np.eye(lanes), np.eye(lanes))
+        st.add_transformation(mt, so.NORMAL)
+        ph = so.NDimPropagator()
+        ph.set_operator(t)
+        st.add_propagator(ph)
+    st.add_transformation(so.FFTTransformation(xg, "k"), so.NORMAL)
+    kin = so.kinetic_hamiltonian(xg, 1.0)
+    st.add_propagator(so.one_dim_into_propagator(kin, xg, tg, so.FULL))
+    p = so.Propagation(so.WaveFunction(a, [lg, xg]), tg, st, precision)
+    p.set_timing(True)
+    p.steps(1)
+    with np.errstate(invalid="ignore"):
+        ref = np.fft.ifft(np.fft.fft(a * t, axis=1) * np.exp(-0.01j * kin), axis=1) * t
+    return p.get_array(), ref, " ".join(k[0] for k in p.kernel_times())
+
+
+@pytest.mark.parametrize("precision", ["fp64", "float_float"])
+@pytest.mark.parametrize("n,lanes", [(16, 600), (32, 37), (64, 5), (128, 700), (256, 37), (512, 2), (1024, 9),
+                                     (2048, 37), (4096, 3), (8192, 5)])
+def test_fft_pair_lanes_match_numpy(so, precision, n, lanes):
+    a = _lanes(lanes, n, 7 * n + lanes)
+    got, ref, names = _pass(so, a, precision, 1.0 if lanes <= 37 else None)
+    assert "fftpair fx" in names
+    err = np.linalg.norm(got - ref, axis=1) / np.linalg.norm(ref, axis=1)
+    assert err.max() < TOL[precision], (int(err.argmax()), err.max())
+
+
+@pytest.mark.parametrize("precision", ["fp64", "float_float"])
+@pytest.mark.parametrize("n", [16, 256, 1024, 8192])
+def test_lanes_of_zeros_and_of_nan_stay_apart(so, precision, n):
+    a = _lanes(6, n, n)
+    a[1] = 0.0
+    a[3, n // 2] = complex(np.nan, 0.0)
+    a[4, 1] = complex(0.0, np.inf)
+    got, ref, names = _pass(so, a, precision)
+    assert "fftpair fx" in names
+    assert np.all(got[1] == 0.0)
+    assert np.all(np.isnan(got[3].real)) and np.all(np.isnan(got[4].imag))
+    for l in (0, 2, 5):
+        assert np.linalg.norm(got[l] - ref[l]) < TOL[precision] * np.linalg.norm(ref[l])
+
+
+@pytest.mark.parametrize("scale,fixed", [(1.2, True), (0.6, True), (1.3, False), (3.0, False), (0.3, False)])
+def test_tables_out_of_the_fixed_point_range_keep_floating_point(so, scale, fixed):
+    a = _lanes(4, 1024, 3)
+    got, ref, names = _pass(so, a, "fp64", scale)
+    assert ("fftpair fx" in names) == fixed
+    err = np.linalg.norm(got - ref, axis=1) / np.linalg.norm(ref, axis=1)
+    assert err.max() < TOL["fp64"]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "float_float"])
+def test_batch_of_many_short_lanes_equals_single_runs(so, precision):
+    """512 points x 256 lanes: the fixed-point pass has more tiles than any pass of the general
+    geometry, and the passes recorded before it keep their norm partials."""
+    from split_operator_gb300 import workloads as W
+    sizes = [(512, 256), (1024, 64), (512, 32)]
+
+    def build():
+        return [W.radial_angular_2d(nr=nr, nth=nth, step_no=50, seed=60 + k, r0=52.0, precision=precision)[0]
+                for k, (nr, nth) in enumerate(sizes)]
+
+    alone, members = build(), build()
+    for p in alone:
+        p.steps(6)
+    b = so.Batch(members)
+    b.steps(6)
+    for p, q in zip(alone, members):
+        assert np.array_equal(p.get_array(), q.get_array())
+        assert p.all_losses() == q.all_losses()
+    # the host-to-host call: 4 more steps from the same states
+    ins = [p.get_array() for p in members]
+    outs = [np.empty_like(a) for a in ins]
+    b.steps_host_ptr([a.ctypes.data for a in ins], [a.ctypes.data for a in outs], 4)
+    for p, a, o in zip(alone, ins, outs):
+        p.set_array(a)
+        p.steps(4)
+        assert np.array_equal(p.get_array(), o)
