@@ -1,0 +1,754 @@
+// The lane-matrix pass of FP64 and float-float states on the tensor cores.
+//
+// Replaces, fused into one pass like the FP32 kernel of angular_tc.cu, MatrixTransformation and
+// StateMatrixTransformation for real matrices (matrix_transformation.rs:60-75,
+// state_matrix_transformation.rs:48-73) with the diagonal propagators, masks, scales and norm
+// folds around them.  On the CUDA cores the products were bound by the FP64 pipe (two FMAs per
+// matrix entry and complex value at 1.7 a clock and SM: 592 us for the two-matrix pass of a
+// 4096 x 128 state).  Here they are exact integer products on the tensor cores and everything
+// else is 64-bit fixed point (fx.cuh).
+//
+// Slices (the Ozaki scheme: K. Ozaki, T. Ogita, S. Oishi, S. M. Rump, Numer. Algorithms 59,
+// 2012).  Every B column (a real or imaginary column of the tile) is scaled by a power of two
+// above its largest magnitude and rounded to 55 bits, every A row (a matrix row, on the host)
+// likewise; both are cut into seven signed 8-bit digits, held as FP16 integers of magnitude
+// <= 128.  The digit products of one order r = i + j (A digit i, B digit j) share a weight, so
+// they sum in one FP32 accumulator: (r + 1) K 2^14 <= 2^24 for K = 128 and every r <= 6, so
+// the sums are exact (K = 256: r <= 3; the other orders weigh less than 2^-48).  The 28
+// products of orders 0 .. 6 give the matrix product to 2^-54 of (row maximum x column
+// maximum), a rounding error of FP64's size at the largest terms.
+//
+// A tile is BN complex columns of the inner axis for all n rows (n <= 256), N = 2 BN real
+// columns.  One persistent CTA per SM (seven accumulators of 64 columns fill its tensor memory):
+//   warps 0-15  load the tile, apply the point-wise ops, write the B digits, drain the
+//               accumulators, store, and fold the norms; thread = one matrix row (TMEM lane) and
+//               NB neighbouring complex columns in every phase
+//   warp 16     streams the A digit images (8 KB per 128 rows x 32 K values) through a 64 KB
+//               ring by bulk TMA copies
+//   warp 17     issues tcgen05.mma kind::f16
+// B digits lie N-major in shared memory (eight real columns of one K row are 16 bytes), so a
+// thread writes its four complex columns of a digit with one 16-byte store.
+// Every mbarrier wait is bounded (2 s), as in angular_tc.cu.
+#pragma once
+#include "common.cuh"
+#include "fx.cuh"
+#include "tc_common.cuh"
+
+namespace so {
+
+using namespace fx;
+
+struct FxTcParams {
+  PassParams p;
+  int32_t mat_op[2];  // op indices of the (one or two) lane matrices
+  int32_t nmat;
+  int32_t kp;         // lane extent rounded up to 32: K of the products
+  int32_t error_slot;
+  int32_t slice_axis[2];      // state matrix: the logical axis whose coordinate picks the image (-1: one)
+  const unsigned char* images[2];
+  int64_t slice_stride[2];    // bytes between two coordinates' images
+  uint32_t slice_pre[2], slice_div[2], slice_ext[2];  // the tile's coordinate, as in TcParams
+};
+
+namespace {
+
+constexpr int kFxWork = 512;                 // work threads (warps 0-15)
+constexpr int kFxThreads = kFxWork + 64;     // + warp 16 (TMA) + warp 17 (MMA)
+constexpr int kDigits = 7;
+constexpr uint32_t kRingBytes = 65536;
+constexpr uint32_t kChunkRowBytes = 8192;    // 128 rows x 32 K values of one digit
+constexpr uint64_t kFxWait = 2000000000ull;  // 2 s per wait
+constexpr int kFxTabSlots = 4;               // DIAG1D ops on a non-lane axis per pass
+constexpr int kFxMaxCols = 32;
+
+__host__ __device__ constexpr uint32_t fx_b_bytes(int cols, int kp) { return (uint32_t)(2 * cols * kp * 2); }
+__host__ __device__ constexpr uint32_t fx_tc_smem(int cols, int kp) {
+  return kRingBytes + kDigits * fx_b_bytes(cols, kp) + kMaxRed * kFxWork * 8;
+}
+
+__device__ __forceinline__ void fx_work_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kFxWork) : "memory"); }
+__device__ __forceinline__ bool fx_work_all(bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, 1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)v), "n"(kFxWork)
+      : "memory");
+  return r != 0;
+}
+
+// kind::f16 with FP16 A (K-major) and B (N-major), D = F32
+__host__ __device__ constexpr uint32_t idesc_f16_nmajor(uint32_t m, uint32_t n) {
+  return (1u << 4) | (1u << 16) | ((n >> 3) << 17) | ((m >> 4) << 24);
+}
+
+// columns c .. c + 3 of the seven accumulators (step columns apart), one wait
+__device__ __forceinline__ void tmem_ld4x7(uint32_t taddr, uint32_t step, uint32_t (&r)[28]) {
+#pragma unroll
+  for (int k = 0; k < 7; ++k)
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[4 * k]), "=r"(r[4 * k + 1]), "=r"(r[4 * k + 2]), "=r"(r[4 * k + 3])
+                 : "r"(taddr + (uint32_t)k * step)
+                 : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13])
+               :
+               : "memory");
+  asm volatile(""
+               : "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]),
+                 "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27])
+               :
+               : "memory");
+}
+
+// The seven orders' sums of one value -> the product times 2^-sh of the last order's unit,
+// rounded to nearest (sh = lg K + 1 keeps it below 2^61).  s0 .. s6 are integers below 2^24.
+template <int MH>
+__device__ __forceinline__ i64 combine(int s0, int s1, int s2, int s3, int s4, int s5, int s6, int sh) {
+  i64 hi;
+  if constexpr (MH == 1)
+    hi = mw(s0 * 256 + s1, 65536, (i64)(s2 * 256 + s3));  // K <= 128: both fit 32 bits
+  else
+    hi = mw(s0, 1 << 24, mw(s1, 65536, mw(s2, 256, (i64)s3)));
+  const i64 lo = mw(s4, 65536, mw(s5, 256, (i64)s6));
+  return (hi << (24 - sh)) + (((lo >> (sh - 1)) + 1) >> 1);
+}
+
+// pair (a, b) of 56-bit values: digit j of both as packed FP16 integers
+__device__ __forceinline__ uint32_t digit_pair(const uint32_t (&a)[2], const uint32_t (&b)[2], int j) {
+  const int byte = 6 - j;
+  uint32_t p;
+  if (byte == 6)
+    p = __byte_perm(a[1], b[1], 0x7632);  // the top digit (plus 128) may be 256: a half word
+  else
+    p = __byte_perm(a[byte >> 2], b[byte >> 2], 0x0400 | (byte & 3) | ((4 + (byte & 3)) << 8)) & 0x00ff00ffu;
+  p |= 0x64006400u;  // FP16 1024 + (digit + 128)
+  uint32_t r;
+  asm("sub.f16x2 %0, %1, %2;" : "=r"(r) : "r"(p), "r"(0x64806480u));
+  return r;
+}
+
+// v 2^sh rounded to nearest (-63 <= sh; left shifts stay in range by the caller's bounds)
+__device__ __forceinline__ i64 shift_by(i64 v, int sh) {
+  if (sh >= 0) return v << sh;
+  const int r = sh < -62 ? 62 : -sh;
+  return (((v >> (r - 1)) + 1) >> 1);
+}
+
+__device__ __forceinline__ int bits_of(i64 x, i64 y) {  // |x|, |y| <= 2^bits (0: both zero)
+  const unsigned long long a = (unsigned long long)(x ^ (x >> 63)) | (unsigned long long)(y ^ (y >> 63));
+  return a == 0 ? ((x | y) != 0 ? 1 : 0) : 64 - __clzll((i64)a);
+}
+
+// d 2^k (d >= 0 or NaN), flushing to zero and saturating to infinity
+__device__ __forceinline__ double scale_pow2(double d, int k) {
+  const i64 b = __double_as_longlong(d);
+  const int e = (int)(b >> 52) & 0x7ff;
+  if (e == 0 || e == 0x7ff) return d;
+  if (e + k <= 0) return 0.0;
+  if (e + k >= 0x7ff) return __longlong_as_double(0x7ff0000000000000ll);
+  return __longlong_as_double(b + ((i64)k << 52));
+}
+
+struct FxTabs {
+  int4 colt[kFxTabSlots][kFxMaxCols];   // DIAG1D on a non-lane axis: its factor per tile column
+  double colw[kMaxRed][kFxMaxCols];     // NORM: product of the weights of every non-lane axis
+  int scale_x[kMaxOps];                 // SCALE: factor = digits x 2^scale_x
+  int2 scale_d[kMaxOps];
+  int colx[kFxMaxCols];                 // exponent of the column's values (before row exponents)
+  int cole[2][kFxMaxCols];              // column maxima: biased exponents
+  int coler[kFxMaxCols];                // the same at a ROUND
+  int colb[kFxMaxCols];                 // exponent bound of the column's B operand
+  int nonident[kFxTabSlots];            // the factors of this tile are not all 1
+  int8_t slot[kMaxOps];
+};
+
+__device__ __forceinline__ int64_t fx_coord(const Geometry& g, int a, int64_t o, int64_t i) {
+  int64_t v = i;
+  for (int q = g.ndim - 1; q > g.spos; --q) {
+    if (g.perm[q] == a) return v % g.sshape[q];
+    v /= g.sshape[q];
+  }
+  v = o;
+  for (int q = g.spos - 1; q >= 0; --q) {
+    if (g.perm[q] == a) return v % g.sshape[q];
+    v /= g.sshape[q];
+  }
+  return 0;
+}
+
+__device__ void fx_run_scalar(const PassParams& p, const DevOp& op, const double* totals) {
+  double* s = p.slots;
+  switch (op.kind) {
+    case OP_NORM: {
+      const double v = totals[op.red];
+      s[op.a] = v;
+      if (!isfinite(v) && p.nonfinite_slot >= 0) s[p.nonfinite_slot] = 1.0;
+      break;
+    }
+    case OP_COPY: s[op.a] = s[op.b]; break;
+    case OP_LOSS: s[op.a] += s[op.b] - s[op.c]; break;
+    case OP_SETC: s[op.a] = op.value; break;
+    case OP_RECORD:
+      if (p.record) p.record[op.count] = s[op.a];
+      break;
+    default: break;
+  }
+}
+
+// image block of matrix m for a tile (a state matrix: the one of the tile's coordinate)
+__device__ __forceinline__ const unsigned char* fx_image(const FxTcParams& q, int m, int64_t tile) {
+  const unsigned char* img = q.images[m];
+  if (q.slice_axis[m] >= 0) {
+    uint32_t t = (uint32_t)tile;
+    if (q.slice_pre[m]) t %= q.slice_pre[m];
+    img += (int64_t)((t / q.slice_div[m]) % q.slice_ext[m]) * q.slice_stride[m];
+  }
+  return img;
+}
+
+struct FxTile {
+  const FxTcParams* prm;
+  int64_t tile;
+};
+struct FxResolve {
+  const FxTcParams* one;
+  const FxTcParams* params;
+  const uint2* owners;
+  __device__ __forceinline__ FxTile operator()(int64_t b) const {
+    if (params == nullptr) return {one, b};
+    const uint2 o = __ldg(owners + b);
+    return {params + o.x, (int64_t)o.y};
+  }
+};
+
+// Warp 16, lane 0: the digit images of every tile's matrices, digit by digit, through the ring.
+template <int MH>
+__device__ __noinline__ void fx_producer(FxResolve resolve, int64_t total, uint32_t ring, uint64_t* full,
+                                         uint64_t* empty, volatile int* fail) {
+  using namespace tc;
+  constexpr uint32_t bytes = kChunkRowBytes * MH;
+  constexpr int ns = (int)(kRingBytes / bytes);
+  int s = 0;
+  uint32_t use = 0;
+  int64_t cc = 0;
+  bool ok = true;
+  for (int64_t gt = blockIdx.x; gt < total && ok && !*fail; gt += gridDim.x) {
+    const FxTile r = resolve(gt);
+    const int chunks = kDigits * (r.prm->kp / 32);
+    for (int m = 0; m < r.prm->nmat && ok; ++m) {
+      const unsigned char* img = fx_image(*r.prm, m, r.tile);
+      for (int q = 0; q < chunks; ++q) {
+        if (use > 0 && !mbar_poll(&empty[s], (use - 1) & 1u, kFxWait)) {
+          ok = false;
+          break;
+        }
+        mbar_expect_tx(&full[s], bytes);
+        bulk_g2s(sm_ptr(ring + (uint32_t)s * bytes), img + (size_t)q * bytes, bytes, &full[s]);
+        ++cc;
+        if (++s == ns) {
+          s = 0;
+          ++use;
+        }
+      }
+    }
+  }
+  if (!ok) {
+    *fail = 1;
+    // let the copies in flight land before the CTA lets go of its shared memory
+    for (int64_t c = cc - ns < 0 ? 0 : cc - ns; c < cc; ++c)
+      mbar_poll(&full[(int)(c % ns)], (uint32_t)((c / ns) & 1), kFxWait);
+  }
+}
+
+// Warp 17, lane 0: per matrix, once its B digits are written, the products of A digit i (chunk by
+// chunk) with the B digits j <= 6 - i into accumulator i + j.
+template <int N, int MH>
+__device__ __noinline__ void fx_issuer(FxResolve resolve, int64_t total, uint32_t ring, uint32_t b0, uint64_t* full,
+                                       uint64_t* empty, uint64_t* dbar, uint64_t* bready, uint64_t* quiet,
+                                       uint32_t tmem, volatile int* fail) {
+  using namespace tc;
+  constexpr uint32_t bytes = kChunkRowBytes * MH;
+  constexpr int ns = (int)(kRingBytes / bytes);
+  constexpr uint32_t idesc = idesc_f16_nmajor(128, N);
+  const uint64_t abits = smem_desc_bits(128, 512);
+  int s = 0;
+  uint32_t phase = 0, nready = 0;
+  bool ok = true;
+  for (int64_t gt = blockIdx.x; gt < total && ok; gt += gridDim.x) {
+    const FxTile r = resolve(gt);
+    const int kp = r.prm->kp, nk = kp / 32;
+    // B: K rows of 16 bytes (eight columns), K groups of 8 rows 128 bytes apart, column groups
+    // 16 kp apart, digits 2 N kp apart
+    const uint64_t bbits = smem_desc_bits(128, (uint32_t)(16 * kp));
+    const uint64_t bfirst = smem_desc_at(bbits, b0), bdig = (uint64_t)((2 * N * kp) >> 4);
+    const int nmat = r.prm->nmat;
+    for (int m = 0; m < nmat && ok; ++m) {
+      ok = mbar_poll(bready, nready & 1u, kFxWait);
+      ++nready;
+      tc_fence_after();
+      for (int i = 0; i < kDigits && ok; ++i) {
+        uint64_t bk = bfirst;
+        for (int q = 0; q < nk; ++q) {
+          ok = mbar_poll(&full[s], phase, kFxWait);
+          if (!ok) break;
+          tc_fence_after();
+          uint64_t a = smem_desc_at(abits, ring + (uint32_t)s * bytes);
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks) {
+            for (int h = 0; h < MH; ++h) {
+              uint32_t d = tmem + (uint32_t)(i * MH * N + h * N);
+              uint64_t b = bk;
+              const uint32_t acc = (i | q | ks) != 0 ? 1u : 0u;
+              for (int j = 0; j < kDigits - i; ++j) {
+                mma_bf16(d, a + (uint64_t)(h * (kChunkRowBytes >> 4)), b, idesc, acc);  // types: idesc
+                d += MH * N;
+                b += bdig;
+              }
+            }
+            bk += 256 >> 4;
+            a += 256 >> 4;
+          }
+          mma_commit(&empty[s]);
+          if (++s == ns) {
+            s = 0;
+            phase ^= 1u;
+          }
+        }
+      }
+      if (ok) mma_commit(dbar);
+    }
+  }
+  if (!ok) {
+    *fail = 1;
+    // every MMA already issued completes before the tensor memory is released
+    mma_commit(quiet);
+    mbar_poll(quiet, 0u, kFxWait);
+  }
+}
+
+// The work threads' view of a tile: row j, complex columns c0 .. c0 + NB - 1.
+template <int NB, bool FF>
+struct FxWork {
+  cx w[NB];
+  int rowx;    // exponent of this row's values on top of their column's
+  int xs;      // exponent from SCALE ops, of the whole tile
+  int j, c0, ncols;
+  bool row_ok;
+
+  // point-wise ops [ob, oe)
+  __device__ __forceinline__ void apply(const PassParams& p, FxTabs& T, int ob, int oe, int64_t ix0, double* acc) {
+    const Geometry& g = p.g;
+    for (int oi = ob; oi < oe; ++oi) {
+      const DevOp& op = p.ops[oi];
+      switch (op.kind) {
+        case OP_DIAGND: {
+          const int4* t = reinterpret_cast<const int4*>(op.ptr) + ix0;
+          if (row_ok) {
+#pragma unroll
+            for (int u = 0; u < NB; ++u)
+              if (c0 + u < ncols) w[u] = cmul<0>(w[u], __ldg(t + u));
+          }
+          break;
+        }
+        case OP_DIAG1D: {
+          if (op.axis == g.sweep_axis) {
+            if (row_ok) {
+              const int4 t = __ldg(reinterpret_cast<const int4*>(op.ptr) + j);
+#pragma unroll
+              for (int u = 0; u < NB; ++u) w[u] = cmul<0>(w[u], t);
+            }
+          } else if (T.nonident[T.slot[oi]]) {
+#pragma unroll
+            for (int u = 0; u < NB; ++u) w[u] = cmul<0>(w[u], T.colt[T.slot[oi]][c0 + u]);
+          }
+          break;
+        }
+        case OP_SCALE: {
+          const int2 d = T.scale_d[oi];
+#pragma unroll
+          for (int u = 0; u < NB; ++u) w[u] = cmul<0>(w[u], int4{d.x, d.y, 0, 0});
+          xs += T.scale_x[oi];
+          break;
+        }
+        case OP_NORM: {
+          // squares of the values moved up to 61 bits, in units of 2^64
+          unsigned long long m = 0;
+#pragma unroll
+          for (int u = 0; u < NB; ++u)
+            m |= (unsigned long long)(w[u].x ^ (w[u].x >> 63)) | (unsigned long long)(w[u].y ^ (w[u].y >> 63));
+          const int lz = __clzll((i64)m), s = lz > 3 ? (lz < 60 ? lz - 3 : 57) : 0;
+          double sum = 0.0;
+#pragma unroll
+          for (int u = 0; u < NB; ++u) {
+            const dig a = split(w[u].x << s), b = split(w[u].y << s);
+            const i64 q = mw(a.h, a.h, (mw(a.h, a.l, 1ll << 30)) >> 31) + mw(b.h, b.h, (mw(b.h, b.l, 1ll << 30)) >> 31);
+            const int x = T.colx[c0 + u];
+            const double v = x == kPoison ? __longlong_as_double(0x7ff8000000000000ll)
+                                          : scale_pow2((double)q * T.colw[op.red][c0 + u], 2 * x);
+            sum += c0 + u < ncols ? v : 0.0;
+          }
+          if (row_ok)
+            acc[op.red * kFxWork + threadIdx.x] +=
+                scale_pow2(sum, 64 + 2 * (rowx + xs - s)) * __ldg(op.w[g.sweep_axis] + j);
+          break;
+        }
+        case OP_ROUND: {
+          cx raw[NB];
+          int mx[NB];
+#pragma unroll
+          for (int u = 0; u < NB; ++u) {
+            const int x = T.colx[c0 + u];
+            const bool ok = row_ok && c0 + u < ncols && x != kPoison;
+            const int e = x + rowx + xs;
+            raw[u] = {ok ? fx_to_raw<FF>(w[u].x, e) : 0, ok ? fx_to_raw<FF>(w[u].y, e) : 0};
+            mx[u] = __reduce_max_sync(0xffffffffu, max(raw_exp<FF>(raw[u].x), raw_exp<FF>(raw[u].y)));
+          }
+          if (threadIdx.x < 4 * NB) T.coler[threadIdx.x] = 0;
+          fx_work_sync();
+#pragma unroll
+          for (int u = 0; u < NB; ++u)
+            if ((threadIdx.x & 31) == u) atomicMax(&T.coler[c0 + u], mx[u]);
+          fx_work_sync();
+          if (threadIdx.x < 4 * NB) {
+            const int e = T.coler[threadIdx.x];
+            if (e == 2047) T.colx[threadIdx.x] = kPoison;
+            if (T.colx[threadIdx.x] != kPoison) T.colx[threadIdx.x] = max(e, 1) - 1022 - 60;
+          }
+#pragma unroll
+          for (int u = 0; u < NB; ++u) {
+            const int e = T.coler[c0 + u];
+            const bool live = e != 2047 && e != 0;
+            w[u] = {live ? raw_to_fx<FF>(raw[u].x, e - 1022) : 0, live ? raw_to_fx<FF>(raw[u].y, e - 1022) : 0};
+          }
+          rowx = 0;
+          xs = 0;
+          fx_work_sync();
+          break;
+        }
+        default:
+          break;
+      }
+    }
+  }
+  static constexpr int kPoison = 1 << 24;  // colx of a column with a value that is not finite
+
+  // B digits of the values, K row j: v = value 2^(55 - colb) as seven digits
+  __device__ __forceinline__ void write_operand(const FxTabs& T, unsigned char* B, int kp, uint32_t bbytes) {
+    if (j >= kp) return;
+#pragma unroll
+    for (int u4 = 0; u4 < NB; u4 += 4) {
+      constexpr int kU = NB < 4 ? NB : 4;
+      uint32_t re[kU][2], im[kU][2];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int c = c0 + u4 + u;
+        const int x = T.colx[c];
+        const int sh = (x == kPoison ? 0 : x) + rowx + xs + 55 - T.colb[c];
+        const i64 a = shift_by(w[u4 + u].x, sh) + 0x0080808080808080ll;
+        const i64 b = shift_by(w[u4 + u].y, sh) + 0x0080808080808080ll;
+        re[u][0] = (uint32_t)a;
+        re[u][1] = (uint32_t)(a >> 32);
+        im[u][0] = (uint32_t)b;
+        im[u][1] = (uint32_t)(b >> 32);
+      }
+      // complex column c: real columns 2 c, 2 c + 1; column group (2 c) / 8
+      unsigned char* dst = B + (uint32_t)((c0 + u4) >> 2) * (uint32_t)(16 * kp) + (uint32_t)(j >> 3) * 128u +
+                           (uint32_t)(j & 7) * 16u + (uint32_t)((c0 + u4) & 3) * 4u;
+#pragma unroll
+      for (int d = 0; d < kDigits; ++d) {
+        uint32_t v[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) v[u] = digit_pair(re[u], im[u], d);
+        if constexpr (kU == 4)
+          *reinterpret_cast<uint4*>(dst + (uint32_t)d * bbytes) = make_uint4(v[0], v[1], v[2], v[3]);
+        else
+          *reinterpret_cast<uint2*>(dst + (uint32_t)d * bbytes) = make_uint2(v[0], v[1]);
+      }
+    }
+  }
+};
+
+template <int NB, int MH, bool FF>
+__global__ void __launch_bounds__(kFxThreads, 1)
+    fx_angular_kernel(const __grid_constant__ FxTcParams one, const FxTcParams* __restrict__ params,
+                      const uint2* __restrict__ owners, const int64_t total) {
+  using namespace tc;
+  constexpr int kGroups = MH == 1 ? 4 : 2;     // column groups of the work warps
+  constexpr int BN = NB * kGroups, N = 2 * BN;
+  constexpr int kRing = (int)(kRingBytes / (kChunkRowBytes * MH));
+  using Work = FxWork<NB, FF>;
+  extern __shared__ __align__(1024) unsigned char sm[];
+  __shared__ __align__(16) FxTcParams tp;
+  __shared__ __align__(16) FxTabs T;
+  __shared__ __align__(8) uint64_t bars[2 * 8 + 3];
+  __shared__ uint32_t tmem_s;
+  __shared__ double totals[kMaxRed];
+  __shared__ volatile int s_fail;
+  __shared__ int s_bad;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (blockIdx.x >= total) return;
+  const FxResolve resolve{&one, params, owners};
+  uint64_t *full = bars, *empty = bars + kRing, *dbar = bars + 2 * kRing, *bready = dbar + 1, *quiet = dbar + 2;
+  if (tid == 0) {
+    for (int k = 0; k < 2 * kRing; ++k) mbar_init(bars + k, 1);
+    mbar_init(dbar, 1);
+    mbar_init(bready, kFxWork);
+    mbar_init(quiet, 1);
+    fence_mbar_init();
+    s_fail = 0;
+    s_bad = 0;
+  }
+  if (warp == 0) tmem_alloc(&tmem_s, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_s;
+  const uint32_t ring = smem_u32(sm);
+  unsigned char* B = sm + kRingBytes;
+
+  if (warp == kFxWork / 32) {
+    if (lane == 0) fx_producer<MH>(resolve, total, ring, full, empty, &s_fail);
+  } else if (warp == kFxWork / 32 + 1) {
+    if (lane == 0)
+      fx_issuer<N, MH>(resolve, total, ring, ring + kRingBytes, full, empty, dbar, bready, quiet, tmem, &s_fail);
+  } else {
+    const int quad = warp & 3, grp = warp >> 2;
+    Work W;
+    W.j = (MH == 2 ? 128 * (grp >> 1) : 0) + 32 * quad + lane;
+    W.c0 = NB * (MH == 2 ? (grp & 1) : grp);
+    // this thread's accumulator columns: half (MH = 2) grp >> 1, real columns 2 c0 ..
+    const uint32_t tcol = tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)((MH == 2 ? (grp >> 1) * N : 0) + 2 * W.c0);
+    uint32_t drains = 0;
+    const FxTcParams* cur = nullptr;
+    for (int64_t gt = blockIdx.x; gt < total; gt += gridDim.x) {
+      const FxTile r = resolve(gt);
+      if (r.prm != cur) {
+        for (int k = tid; k < (int)(sizeof(FxTcParams) / 4); k += kFxWork)
+          reinterpret_cast<uint32_t*>(&tp)[k] = reinterpret_cast<const uint32_t*>(r.prm)[k];
+        cur = r.prm;
+        fx_work_sync();
+      }
+      const PassParams& p = tp.p;
+      const Geometry& g = p.g;
+      const int n = (int)g.n, kp = tp.kp;
+      const uint32_t bbytes = fx_b_bytes(BN, kp);
+      // products are drained with 2^-sh of their last bit: |product| <= 2^61
+      const int sh = kp <= 32 ? 6 : (kp <= 64 ? 7 : (kp <= 128 ? 8 : 9));
+      double* acc = reinterpret_cast<double*>(sm + kRingBytes + kDigits * bbytes);
+      const int64_t o = r.tile / g.tiles_per_outer;
+      const int64_t i0 = (r.tile - o * g.tiles_per_outer) * BN;
+      const int64_t left = g.inner - i0;
+      W.ncols = left < BN ? (int)left : BN;
+      W.row_ok = W.j < n;
+      W.xs = 0;
+      W.rowx = 0;
+      const int64_t ix0 = o * g.n * g.inner + (int64_t)W.j * g.inner + i0 + W.c0;
+      longlong2* psi = reinterpret_cast<longlong2*>(p.psi) + ix0;
+
+      // the tile's values
+      cx raw[NB];
+#pragma unroll
+      for (int u = 0; u < NB; ++u) {
+        const bool ok = W.row_ok && W.c0 + u < W.ncols;
+        const longlong2 x = ok ? psi[u] : longlong2{0, 0};
+        raw[u] = {x.x, x.y};
+      }
+      // per-tile tables
+      if (tid < 2 * kFxMaxCols) T.cole[tid >> 5][tid & 31] = 0;
+      if (tid < kFxTabSlots) T.nonident[tid] = 0;
+      if (tid < p.nops) {
+        int k = 0;
+        for (int q = 0; q < tid; ++q) k += p.ops[q].kind == OP_DIAG1D && p.ops[q].axis != g.sweep_axis;
+        T.slot[tid] = (int8_t)k;
+        if (p.ops[tid].kind == OP_SCALE) {
+          // sqrt(target / norm) = m 2^x, m in [1/2, 1): digits of m 2^62
+          const double f = sqrt(__ldcg(p.slots + p.ops[tid].b) / __ldcg(p.slots + p.ops[tid].c));
+          int x = 0;
+          const double m = frexp(f, &x);
+          i64 v = isfinite(f) ? __double2ll_rn(ldexp(m, 62)) : 0;
+          if ((int)v == (int)0x80000000) ++v;
+          const dig d = split(v);
+          T.scale_d[tid] = {d.l, d.h};
+          T.scale_x[tid] = x;
+          if (!isfinite(f)) s_bad = 1;  // the whole tile becomes NaN
+        }
+      }
+      for (int k = 0; k < p.nred; ++k) acc[k * kFxWork + tid] = 0.0;
+      fx_work_sync();
+      for (int idx = tid; idx < p.nops * BN; idx += kFxWork) {
+        const int oi = idx / BN, c = idx - oi * BN;
+        const DevOp& op = p.ops[oi];
+        const int64_t i = i0 + (c < W.ncols ? c : 0);
+        if (op.kind == OP_NORM) {
+          double wt = 1.0;
+          for (int a = 0; a < g.ndim; ++a)
+            if (a != g.sweep_axis) wt *= __ldg(op.w[a] + fx_coord(g, a, o, i));
+          T.colw[op.red][c] = wt;
+        } else if (op.kind == OP_DIAG1D && op.axis != g.sweep_axis) {
+          const int4 t = __ldg(reinterpret_cast<const int4*>(op.ptr) + fx_coord(g, op.axis, o, i));
+          T.colt[T.slot[oi]][c] = t;
+          if (t.x != 0 || t.y != (1 << 30) || t.z != 0 || t.w != 0) T.nonident[T.slot[oi]] = 1;
+        }
+      }
+      // column exponents
+#pragma unroll
+      for (int u = 0; u < NB; ++u) {
+        const int m = __reduce_max_sync(0xffffffffu, max(raw_exp<FF>(raw[u].x), raw_exp<FF>(raw[u].y)));
+        if (lane == u) atomicMax(&T.cole[0][W.c0 + u], m);
+      }
+      fx_work_sync();
+      if (tid < BN) {
+        const int e = T.cole[0][tid];
+        T.colx[tid] = e == 2047 || s_bad ? Work::kPoison : max(e, 1) - 1022 - 60;
+        T.colb[tid] = max(e, 1) - 1022;
+      }
+#pragma unroll
+      for (int u = 0; u < NB; ++u) {
+        const int e = T.cole[0][W.c0 + u];
+        const bool live = e != 2047 && e != 0 && !s_bad;
+        W.w[u] = {live ? raw_to_fx<FF>(raw[u].x, e - 1022) : 0, live ? raw_to_fx<FF>(raw[u].y, e - 1022) : 0};
+      }
+      fx_work_sync();  // the exponents and tables are complete
+      bool ok = true;
+      for (int m = -1; m < tp.nmat && ok; ++m) {
+        if (m >= 0) {
+          // drain matrix m
+          ok = fx_work_all(mbar_wait(dbar, drains & 1u, kFxWait));
+          if (!ok) break;
+          ++drains;
+          tc_fence_after();
+          const unsigned char* img = fx_image(tp, m, r.tile);
+          W.rowx = __ldg(reinterpret_cast<const int*>(img + (size_t)kDigits * (kp / 32) * kChunkRowBytes * MH) + W.j);
+          W.xs = 0;
+          if (tid < BN) {
+            T.colx[tid] = T.colx[tid] == Work::kPoison ? Work::kPoison : T.colb[tid] + sh - 62;
+            T.cole[0][tid] = 0;
+          }
+#pragma unroll
+          for (int u = 0; u < NB; u += 2) {
+            uint32_t rg[28];
+            tmem_ld4x7(tcol + 2u * u, (uint32_t)(MH * N), rg);
+            float mx = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 28; ++k) mx = fmaxf(mx, fabsf(__uint_as_float(rg[k])));
+            int v[28];
+            if (mx <= 4194304.0f) {
+              // |sum| <= 2^22: the FP32 addition of 1.5 2^23 leaves the integer in the low bits
+#pragma unroll
+              for (int k = 0; k < 28; ++k)
+                v[k] = __float_as_int(__fadd_rn(__uint_as_float(rg[k]), 12582912.0f)) - 0x4B400000;
+            } else {
+#pragma unroll
+              for (int k = 0; k < 28; ++k) v[k] = __float2int_rn(__uint_as_float(rg[k]));
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              W.w[u + q].x = combine<MH>(v[2 * q], v[4 + 2 * q], v[8 + 2 * q], v[12 + 2 * q], v[16 + 2 * q],
+                                         v[20 + 2 * q], v[24 + 2 * q], sh);
+              W.w[u + q].y = combine<MH>(v[2 * q + 1], v[5 + 2 * q], v[9 + 2 * q], v[13 + 2 * q], v[17 + 2 * q],
+                                         v[21 + 2 * q], v[25 + 2 * q], sh);
+            }
+          }
+          tc_fence_before();
+          fx_work_sync();  // colx is complete
+        }
+        const int ob = m < 0 ? 0 : tp.mat_op[m] + 1;
+        const int oe = m + 1 < tp.nmat ? tp.mat_op[m + 1] : p.nops;
+        W.apply(p, T, ob, oe, ix0, acc);
+        if (m + 1 < tp.nmat) {
+          if (m >= 0 || oe > 0) {
+            // the operand's column maxima
+            int* ce = T.cole[m < 0 ? 1 : 0];  // set 0 was cleared with the drain
+#pragma unroll
+            for (int u = 0; u < NB; ++u) {
+              const int b = W.row_ok ? bits_of(W.w[u].x, W.w[u].y) : 0;
+              const int e = b ? b + W.rowx + 8192 : 0;
+              const int mx = __reduce_max_sync(0xffffffffu, e);
+              if (lane == u) atomicMax(ce + W.c0 + u, mx);
+            }
+            fx_work_sync();
+            if (tid < BN) {
+              const int e = ce[tid], x = T.colx[tid];
+              T.colb[tid] = (e ? e - 8192 : 0) + (x == Work::kPoison ? 0 : x) + W.xs;
+            }
+            fx_work_sync();
+          }
+          W.write_operand(T, B, kp, bbytes);
+          fence_proxy_async();
+          mbar_arrive(bready);
+        }
+      }
+      if (!ok) {
+        if (tid == 0) s_fail = 1;
+        break;
+      }
+      // store
+#pragma unroll
+      for (int u = 0; u < NB; ++u) {
+        if (!(W.row_ok && W.c0 + u < W.ncols)) continue;
+        const int x = T.colx[W.c0 + u];
+        const int e = x + W.rowx + W.xs;
+        longlong2 v{fx_to_raw<FF>(W.w[u].x, e), fx_to_raw<FF>(W.w[u].y, e)};
+        if (x == Work::kPoison) v = {raw_nan<FF>(), raw_nan<FF>()};
+        psi[u] = v;
+      }
+      // norm partials and the pass ticket
+      fx_work_sync();
+      if (warp < p.nred) {
+        double a = 0.0;
+#pragma unroll
+        for (int k = 0; k < kFxWork / 32; ++k) a += acc[warp * kFxWork + lane + 32 * k];
+#pragma unroll
+        for (int o2 = 16; o2 > 0; o2 >>= 1) a += __shfl_down_sync(0xffffffffu, a, o2);
+        if (lane == 0) {
+          p.partials[(int64_t)warp * g.tiles + r.tile] = a;
+          __threadfence();
+        }
+      }
+      fx_work_sync();
+      if (warp == 0) {
+        unsigned int last = 0;
+        if (lane == 0) {
+          __threadfence();
+          last = atomicAdd(p.counter, 1u) == (unsigned int)(g.tiles - 1) ? 1u : 0u;
+        }
+        last = __shfl_sync(0xffffffffu, last, 0);
+        if (last) {
+          __threadfence();
+          for (int k = 0; k < p.nred; ++k) {
+            double a = 0.0;
+            for (int64_t b = lane; b < g.tiles; b += 32) a += __ldcg(p.partials + (int64_t)k * g.tiles + b);
+#pragma unroll
+            for (int o2 = 16; o2 > 0; o2 >>= 1) a += __shfl_down_sync(0xffffffffu, a, o2);
+            if (lane == 0) totals[k] = a;
+          }
+          __syncwarp();
+          if (lane == 0) {
+            for (int oi = 0; oi < p.nops; ++oi) fx_run_scalar(p, p.ops[oi], totals);
+            __threadfence();
+            *p.counter = 0u;
+          }
+        }
+      }
+      if (tid == 0) s_bad = 0;
+      fx_work_sync();  // the tables and the pass copy are free for the next tile
+    }
+  }
+  __syncthreads();
+  if (tid == 0 && s_fail) {
+    const FxTcParams* f0 = resolve(blockIdx.x).prm;  // the pass of the first tile records the failure
+    if (f0->error_slot >= 0) f0->p.slots[f0->error_slot] = 1.0;
+  }
+  // teardown: every MMA has completed (drained, or waited on by the MMA warp)
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 512);
+}
+
+}  // namespace
+}  // namespace so

@@ -41,7 +41,9 @@ enum OpKind : int32_t {
   OP_SCALE = 9,      // psi *= sqrt(slot[b] / slot[c])
   OP_SETC = 10,      // slot[a] = value
   OP_RECORD = 11,    // record[count] = slot[a]
-  OP_DOT = 12        // slot[a] + i slot[b] = sum psi conj(other) prod w  (other = ptr, same layout)
+  OP_DOT = 12,       // slot[a] + i slot[b] = sum psi conj(other) prod w  (other = ptr, same layout)
+  OP_ROUND = 13      // end of a step inside a pass: psi as it would be stored and loaded again (fixed-point
+                     // passes of FP64 states, so that a run split here gives the same bits; else nothing)
 };
 
 struct DevOp {
@@ -185,6 +187,20 @@ cudaError_t launch_fx_pair(int real, int lgn, const PassParams* one, const PassP
                            cudaStream_t s);
 // a device table in the state precision as fixed-point factors (16 bytes a value as well)
 cudaError_t launch_fx_table(void* dst, const void* src, int real, int64_t n, cudaStream_t s);
+
+// Lane-matrix passes of FP64 and float-float states on the tensor cores (angular_fx.cu): real
+// matrices of 16 to 256 points, at most two per pass.  The plan sets the tiling (*cols complex
+// columns per tile); the pass's tables are then the fixed-point ones.
+bool fx_angular_plan(PassParams& p, const DevOp* ops, int nops, const double* table_max, int* cols);
+size_t fx_angular_image_bytes(int n);
+bool fx_angular_image(const double* m, int n, unsigned char* out);  // false: not finite, or sparse
+size_t fx_angular_params_bytes();
+void fx_angular_params(const PassParams& p, const int* mat_op, int nmat, const unsigned char* const* images,
+                       const int* slice_axis, int error_slot, void* out);
+// one: the parameters of a single pass (host); or the batched form (params_dev, owners_dev)
+cudaError_t launch_fx_angular(int real, int n, int cols, const void* one, const void* params_dev, const void* owners_dev,
+                              int64_t tiles, cudaStream_t s);
+int64_t fx_angular_grid(int64_t tiles);  // persistent CTAs of a launch
 
 // Host launchers (lane_sweep.cu)
 cudaError_t launch_pass_f64(const PassParams& p, cudaStream_t s);

@@ -270,17 +270,20 @@ __device__ __forceinline__ i64 fx_to_f64(i64 v, int x) {
   return (i64)(b | ((unsigned long long)(uint32_t)s << 63));
 }
 // v 2^x -> the hi + lo FP32 pair as a raw half
-__device__ __forceinline__ i64 fx_to_ff(i64 v, int x) {
+__device__ __forceinline__ i64 fx_to_ff(i64 v0, int x) {
+  // moved up to 62 bits first: small values keep all of theirs
+  const int s = __clzll(v0 ^ (v0 >> 63)) - 2;  // at least -1 (|v0| <= 2^63), 62 for zero
+  const i64 v = s >= 0 ? v0 << s : v0 >> 1;
   const int h = (int)(v >> 32);
   float fh = __int2float_rn(h);
   const i64 rem = v - ((i64)__float2int_rn(fh) << 32);
   // fh counts 2^32 units; the remainder, below 2^38, in units of 2^8
   float fl = __int2float_rn((int)((rem + 128) >> 8)) * 0x1p-24f;
-  const float s = __fadd_rn(fh, fl);
-  fl = __fsub_rn(fl, __fsub_rn(s, fh));
-  fh = s;
-  // times 2^(x + 32) in two exact steps
-  int q = x + 32;
+  const float t = __fadd_rn(fh, fl);
+  fl = __fsub_rn(fl, __fsub_rn(t, fh));
+  fh = t;
+  // times 2^(x - s + 32) in two exact steps
+  int q = x - s + 32;
   q = q < -250 ? -250 : (q > 250 ? 250 : q);
   const int q1 = q / 2, q2 = q - q1;
   const float f1 = __int_as_float((127 + q1) << 23), f2 = __int_as_float((127 + q2) << 23);

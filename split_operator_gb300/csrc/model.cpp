@@ -80,7 +80,9 @@ void ScalarState::set(size_t i, double v) {
 
 // ----------------------------------------------------------------------- Engine
 const char* op_kind_name(int k);
-static bool is_scalar_kind(int k) { return k == OP_COPY || k == OP_LOSS || k == OP_SETC || k == OP_RECORD; }
+static bool is_scalar_kind(int k) {
+  return k == OP_COPY || k == OP_LOSS || k == OP_SETC || k == OP_RECORD || k == OP_ROUND;
+}
 
 Engine::Engine(const std::vector<size_t>& shp, const std::vector<int>& prm, int rl)
     : real(rl), fp64(rl != kRealF32), shape(shp), perm(prm) {
@@ -441,6 +443,9 @@ const void* Engine::matrices(const void* key, uint64_t version, const std::vecto
   c.version = version;
   c.real = real;
   c.parity = 0;
+  fx_images_.erase(c.buf.ptr);
+  if (c.half_buf.ptr) fx_images_.erase(c.half_buf.ptr);
+  if (fx && real && n >= 16 && n <= 256) fx_images(c.buf.ptr, m, n, count);
   if (this->real == kRealFF && real && count == 1) {
     // float-float Legendre pairs: the half matrix of the parity form, each entry the mean of
     // the two it stands for (the structure holds to ~1e-14 of the largest entry: the nodes'
@@ -460,6 +465,9 @@ const void* Engine::matrices(const void* key, uint64_t version, const std::vecto
         }
       upload(c.half_buf, v, stream);
       c.parity = kind;
+      // the pass is known by the half matrix's address then
+      auto img = fx_images_.find(c.buf.ptr);
+      if (img != fx_images_.end()) fx_images_[c.half_buf.ptr] = img->second;
       if (parity) {
         *parity = kind;
         return c.half_buf.ptr;
@@ -741,10 +749,10 @@ void Engine::submit(const Action& a) {
   }
   const int need = k == OP_NORM ? 1 : (k == OP_DOT ? 2 : 0);
   if ((int)cur_.size() >= kMaxOps || cur_red_ + need > kMaxRed) flush();
-  if (k == OP_MAT && tc_mode() >= 0) {
-    // the tensor-core pass holds at most two lane-matrix products
+  if ((k == OP_MAT && tc_mode() >= 0) || ((k == OP_MAT || k == OP_MAT_SLICE) && fx)) {
+    // the tensor-core passes hold at most two lane-matrix products
     int mats = 0;
-    for (const DevOp& o : cur_) mats += o.kind == OP_MAT;
+    for (const DevOp& o : cur_) mats += o.kind == OP_MAT || (fx && o.kind == OP_MAT_SLICE);
     if (mats >= 2) flush();
   }
   if (a.lane_axis >= 0) cur_axis_ = a.lane_axis;
@@ -759,6 +767,87 @@ void Engine::submit(const Action& a) {
     cur_written_.push_back(op.b);
   }
   cur_.push_back(op);
+}
+
+// Digit images of `count` real n x n matrices for the fixed-point lane-matrix pass, one copy per
+// value for the process (entries are held weakly by the engines that use them, like the FP32
+// images above).  Sparse matrices and ones with a value that is not finite get none.
+void Engine::fx_images(const void* matrix, const std::vector<cplx>& m, size_t n, size_t count) {
+  struct Entry {
+    int device;
+    size_t n;
+    std::vector<double> m;
+    std::weak_ptr<DeviceBuffer> img;
+  };
+  static std::mutex mu;
+  static std::vector<Entry> cache;
+  std::vector<double> md(m.size());
+  for (size_t i = 0; i < m.size(); ++i) md[i] = m[i].real();
+  int dev = 0;
+  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+  std::lock_guard<std::mutex> lock(mu);
+  cache.erase(std::remove_if(cache.begin(), cache.end(), [](const Entry& e) { return e.img.expired(); }), cache.end());
+  for (const Entry& e : cache)
+    if (e.device == dev && e.n == n && e.m == md)
+      if (auto img = e.img.lock()) {
+        fx_images_[matrix] = img;
+        return;
+      }
+  const size_t b = fx_angular_image_bytes((int)n);
+  std::vector<unsigned char> h(b * count);
+  for (size_t i = 0; i < count; ++i)
+    if (!fx_angular_image(md.data() + i * n * n, (int)n, h.data() + i * b)) return;
+  auto img = std::make_shared<DeviceBuffer>();
+  upload(*img, h, stream);
+  fx_images_[matrix] = img;
+  cache.push_back(Entry{dev, n, std::move(md), img});
+}
+
+bool Engine::try_launch_fx_tc(const std::vector<DevOp>& ops, int axis, PassParams& p) {
+  double mx[kMaxOps] = {};
+  Cached* tab[kMaxOps] = {};
+  int mats[2] = {0, 0}, slices[2] = {-1, -1}, nmat = 0;
+  const unsigned char* images[2] = {nullptr, nullptr};
+  for (size_t i = 0; i < ops.size(); ++i) {
+    const DevOp& op = ops[i];
+    if (op.kind == OP_DIAGND || op.kind == OP_DIAG1D) {
+      tab[i] = phase_table(op.ptr);
+      if (!tab[i]) return false;
+      mx[i] = tab[i]->max_abs;
+    } else if (op.kind == OP_MAT || op.kind == OP_MAT_SLICE) {
+      auto it = fx_images_.find(op.ptr);
+      if (nmat == 2 || !(op.flags & 1) || it == fx_images_.end()) return false;
+      images[nmat] = it->second->as<unsigned char>();
+      slices[nmat] = op.kind == OP_MAT_SLICE ? op.axis : -1;
+      mats[nmat++] = (int)i;
+    }
+  }
+  int cols = 0;
+  PassParams q = p;
+  if (nmat == 0 || !fx_angular_plan(q, ops.data(), (int)ops.size(), mx, &cols)) return false;
+  p = q;
+  for (size_t i = 0; i < ops.size(); ++i)
+    if (tab[i]) p.ops[i].ptr = fx_table(*tab[i]);
+  grow_partials(p);
+  const Geometry& g = p.g;
+  std::string name = std::string(real == kRealFF ? "ff" : "f64") + " tcfx axis" + std::to_string(axis) + ":";
+  for (const DevOp& o : ops) name += std::string(" ") + op_kind_name(o.kind);
+  std::vector<unsigned char> prm(fx_angular_params_bytes());
+  fx_angular_params(p, mats, nmat, images, slices, timeout_slot, prm.data());
+  if (recording) {
+    // threads: the lane extent and the tile's columns (one batched launch serves one of each)
+    recording->push_back(RecordedPass{RecordedPass::TensorCore, real, p, std::move(prm), (int)g.n | (cols << 16), 0,
+                                      name, pass_bytes(ops, g)});
+    return true;
+  }
+  if (timing) {
+    timed_begin(name);
+    timed_.back().bytes = pass_bytes(ops, g);
+  }
+  cuda_check(launch_fx_angular(real, (int)g.n, cols, prm.data(), nullptr, nullptr, g.tiles, stream),
+             "lane-matrix pass launch");
+  if (timing) timed_end();
+  return true;
 }
 
 bool Engine::try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p) {
@@ -812,6 +901,7 @@ void Engine::launch(const std::vector<DevOp>& ops, int axis, bool resident, int 
   if (fft) p.twiddle = twiddle((size_t)p.g.n);
   pass_choose_buffers(p, fp64);
   if (!fp64 && tc_mode() >= 0 && !resident && try_launch_tc(ops, axis, p)) return;
+  if (fx && !resident && try_launch_fx_tc(ops, axis, p)) return;
   if (fx && !resident && try_launch_fx_pair(ops, p)) {
     name_tag = " fftpair fx";
   } else if ((fft_pair || (fp64 && p.g.n > 4096)) && fft_pair_plan(p, real, resident)) {
@@ -919,8 +1009,25 @@ std::string Engine::collect_timing() {
   return out;
 }
 
+void Engine::step_end() {
+  if (!fx || real != kRealF64 || cur_.empty() || cur_.back().kind == OP_ROUND) return;
+  if ((int)cur_.size() >= kMaxOps) {
+    flush();
+    return;
+  }
+  DevOp r{};
+  r.kind = OP_ROUND;
+  cur_.push_back(r);
+}
+
 void Engine::flush() {
-  if (cur_.empty()) return;
+  while (!cur_.empty() && cur_.back().kind == OP_ROUND) cur_.pop_back();  // the pass ends with the step
+  if (cur_.empty()) {
+    cur_axis_ = -1;
+    cur_red_ = 0;
+    cur_written_.clear();
+    return;
+  }
   std::vector<DevOp> ops;
   ops.swap(cur_);
   const int axis = cur_axis_ >= 0 ? cur_axis_ : perm.back();
@@ -1535,7 +1642,10 @@ void Propagation::steps(uint64_t n) {
   steps_done_ += n;
   if (!e.resident_capable()) {
     Emitter em{&e};
-    for (uint64_t i = 0; i < n; ++i) step(em);
+    for (uint64_t i = 0; i < n; ++i) {
+      step(em);
+      e.step_end();
+    }
     e.flush();
     return;
   }
@@ -1878,7 +1988,10 @@ std::vector<RecordedPass> Propagation::record_steps(uint64_t n) {
   e.recording = &out;
   try {
     Emitter em{&e};
-    for (uint64_t i = 0; i < n; ++i) step(em);
+    for (uint64_t i = 0; i < n; ++i) {
+      step(em);
+      e.step_end();
+    }
     e.flush();
   } catch (...) {
     e.recording = nullptr;
@@ -1973,7 +2086,9 @@ std::vector<Batch::Group> Batch::build_groups(const std::vector<std::vector<Reco
     if (g.kind == RecordedPass::Generic && ((g.threads >> 20) & 1)) g.ct_lgn = v[0]->p.ct;
     if (g.kind == RecordedPass::Generic && ((g.threads >> 25) & 1)) g.fx_lgn = v[0]->p.fx;
     std::vector<int64_t> off(v.size() + 1, 0);
-    const size_t pb = g.kind == RecordedPass::TensorCore ? tc_params_bytes() : sizeof(PassParams);
+    const bool fxtc = g.kind == RecordedPass::TensorCore && g.real != kRealF32;
+    const size_t pb = fxtc ? fx_angular_params_bytes()
+                           : (g.kind == RecordedPass::TensorCore ? tc_params_bytes() : sizeof(PassParams));
     std::vector<unsigned char> params(pb * v.size());
     // SO_TC_TRACE_BATCH=<file>: per-tile phase timestamps of every member's tensor-core pass
     // (the last launch of each cached group), written when the batch is destroyed
@@ -1985,7 +2100,7 @@ std::vector<Batch::Group> Batch::build_groups(const std::vector<std::vector<Reco
       g.sweep = g.sweep && v[i]->p.sweep;
       if (g.kind == RecordedPass::TensorCore) {
         std::memcpy(params.data() + i * pb, v[i]->tcp.data(), pb);
-        if (trace_path) {
+        if (trace_path && !fxtc) {
           TraceBuf tb;
           tb.tiles = v[i]->p.g.tiles;
           tb.name = v[i]->name + " n=" + std::to_string(v[i]->p.g.n) + " member " + std::to_string(i);
@@ -2014,11 +2129,11 @@ std::vector<Batch::Group> Batch::build_groups(const std::vector<std::vector<Reco
           own[(size_t)t * 2] = (uint32_t)i;
           own[(size_t)t * 2 + 1] = (uint32_t)(t - off[i]);
         }
-      if ((g.threads >> 22) & 1) {
+      if (fxtc || ((g.threads >> 22) & 1)) {
         // blocked: CTA k (positions k, k + G, k + 2G, ...) takes one run of consecutive tiles,
         // mostly of one member (one pass description, neighbouring columns)
-        const int64_t G = angular_tc_grid(g.blocks, (g.threads >> 20) & 3), base = g.blocks / G,
-                      rem = g.blocks % G;
+        const int64_t G = fxtc ? fx_angular_grid(g.blocks) : angular_tc_grid(g.blocks, (g.threads >> 20) & 3),
+                      base = g.blocks / G, rem = g.blocks % G;
         std::vector<uint32_t> blk(own.size());
         for (int64_t b = 0; b < g.blocks; ++b) {
           const int64_t k = b % G, i = b / G;
@@ -2067,7 +2182,7 @@ void Batch::run_groups(std::vector<Group>& gs, bool concurrent) {
     if (timing_) {
       t.name = g.name;
       t.bytes = g.bytes;
-      if (g.kind == RecordedPass::TensorCore) {
+      if (g.kind == RecordedPass::TensorCore && g.real == kRealF32) {
         t.cls_kind = 1;
         t.cls_mode = (g.threads >> 17) & 3;
       } else if ((g.threads >> 16) & 1) {
@@ -2079,7 +2194,11 @@ void Batch::run_groups(std::vector<Group>& gs, bool concurrent) {
       cuda_check(cudaEventCreate(&t.b), "event");
       cuda_check(cudaEventRecord(t.a, stream_), "event record");
     }
-    if (g.kind == RecordedPass::TensorCore)
+    if (g.kind == RecordedPass::TensorCore && g.real != kRealF32)
+      cuda_check(launch_fx_angular(g.real, g.threads & 0xffff, g.threads >> 16, nullptr, g.params.ptr, g.owners.ptr,
+                                   g.blocks, st),
+                 "batched lane-matrix pass");
+    else if (g.kind == RecordedPass::TensorCore)
       cuda_check(launch_angular_tc_batched(g.params.ptr, g.owners.ptr, g.blocks, g.smem, (g.threads >> 17) & 3,
                                            st, (g.threads >> 20) & 3, 1 << ((g.threads >> 23) & 3)),
                  "batched tensor-core pass");
@@ -2414,7 +2533,7 @@ std::string Batch::tune(const std::string& cache_path, int trial_steps) {
   std::map<std::tuple<int, int64_t, int>, std::vector<std::pair<int, int>>> cands;
   for (Propagation* p : props_)
     for (const RecordedPass& r : p->record_steps(2)) {
-      if (r.kind == RecordedPass::TensorCore) {
+      if (r.kind == RecordedPass::TensorCore && r.real == kRealF32) {
         const int mode = (r.threads >> 17) & 3;
         // (CTAs per SM, blocked order); the first candidate is the built-in default
         cands[{1, r.p.g.n, mode}] = {{2, 1}, {2, 0}, {1, 1}, {1, 0}};
@@ -2544,6 +2663,7 @@ const char* op_kind_name(int k) {
     case OP_SETC: return "setc";
     case OP_RECORD: return "record";
     case OP_DOT: return "dot";
+    case OP_ROUND: return "round";
   }
   return "?";
 }

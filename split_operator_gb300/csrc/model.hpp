@@ -161,6 +161,7 @@ class Engine {
 
   // pass building
   void submit(const Action& a);
+  void step_end();  // marks the end of a step in the open pass (OP_ROUND)
   void flush();
   void run_resident(const std::vector<Action>& prog, int repeat);
   void sync();
@@ -231,6 +232,9 @@ class Engine {
   static void shared_tc_images(const std::vector<double>& md, int n, int mode, cudaStream_t s,
                                std::shared_ptr<DeviceBuffer>& img, std::shared_ptr<DeviceBuffer>& par, int& kind);
   bool try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p);
+  bool try_launch_fx_tc(const std::vector<DevOp>& ops, int axis, PassParams& p);
+  void fx_images(const void* matrix, const std::vector<cplx>& m, size_t n, size_t count);
+  std::map<const void*, std::shared_ptr<DeviceBuffer>> fx_images_;  // digit images by device matrix
   Cached* phase_table(const void* device_ptr);           // the cache entry of a phase table
   const void* fx_table(Cached& c);                       // its fixed-point copy
   const void* fx_twiddle(size_t n);                      // fixed-point twiddles, shared by the process

@@ -124,3 +124,104 @@ def test_batch_of_many_short_lanes_equals_single_runs(so, precision):
         p.set_array(a)
         p.steps(4)
         assert np.array_equal(p.get_array(), o)
+
+
+# ---- lane matrices on the tensor cores
+def _legendre(n):
+    x, w = np.polynomial.legendre.leggauss(n)
+    v = np.stack([np.sqrt(l + 0.5) * np.polynomial.legendre.Legendre.basis(l)(x) for l in range(n)])
+    return v * w[None, :], v.T.copy()
+
+
+def _matrix_pass(so, a, t, tinv, ph, precision):
+    """[T, phase, T^-1] along axis 0: (result, reference in long double, the passes' names)."""
+    n, nr = a.shape
+    pg = so.Grid.new_linear_countable("p", 0.0, n - 1.0, n, 0)
+    rg = so.Grid.new_linear_continuos("r", 0.0, 5.0, nr, 1)
+    st = so.OperationStack()
+    mt = so.MatrixTransformation(pg, so.Grid.new_linear_countable("l", 0.0, n - 1.0, n, 0))
+    mt.set_diagonalization_matrix(t, tinv)
+    st.add_transformation(mt, so.NORMAL)
+    pd = so.NDimPropagator()
+    pd.set_operator(ph)
+    st.add_propagator(pd)
+    p = so.Propagation(so.WaveFunction(a, [pg, rg]), so.TimeGrid(0.01, 100), st, precision)
+    p.set_timing(True)
+    p.steps(1)
+
+    def mul(m, z):
+        m = m.real.astype(np.longdouble)
+        return m @ z.real.astype(np.longdouble) + 1j * (m @ z.imag.astype(np.longdouble))
+
+    with np.errstate(invalid="ignore"):
+        ref = mul(tinv, mul(t, a.astype(np.clongdouble)) * ph)
+    return p.get_array(), ref, " ".join(k[0] for k in p.kernel_times())
+
+
+# FP64 sums of n products are within sqrt(n) roundings, the exact sums of 55-bit operands within a
+# few: both transforms and the phase stay below 16 roundings (2^-53) of the column; a float-float
+# result adds its own 2^-48 per value, grown by the inverse matrix's condition on a column of few l
+MAT_TOL = {"fp64": 2e-15, "float_float": 8e-14}
+
+
+@pytest.mark.parametrize("precision", ["fp64", "float_float"])
+@pytest.mark.parametrize("n,nr", [(16, 8), (17, 5), (31, 700), (32, 1216), (33, 64), (64, 7), (100, 2433), (128, 33),
+                                  (129, 40), (160, 9), (255, 17), (256, 2448)])
+def test_lane_matrices_match_long_double(so, precision, n, nr):
+    rng = np.random.default_rng(n + nr)
+    t, tinv = _legendre(n)
+    a = rng.standard_normal((n, nr)) + 1j * rng.standard_normal((n, nr))
+    a[:, 1::3] = tinv[:, :5] @ a[:5, 1::3]           # few l
+    a[:, 2::3] = a[:1, 2::3]                          # constant along the lane
+    a *= 10.0 ** rng.integers(-25, 25, (1, nr))
+    a[:, nr // 2] = 0.0
+    a = a.real.astype(np.float32) + 1j * a.imag.astype(np.float32) if precision == "float_float" else a
+    ph = np.exp(1j * rng.uniform(0.0, 6.0, (n, nr)))
+    got, ref, names = _matrix_pass(so, a.astype(np.complex128), t, tinv, ph, precision)
+    assert "tcfx" in names
+    assert np.all(got[:, nr // 2] == 0.0)
+    live = np.arange(nr) != nr // 2
+    err = (np.linalg.norm((got - ref).astype(np.complex128), axis=0)[live] /
+           np.linalg.norm(ref.astype(np.complex128), axis=0)[live])
+    assert err.max() < MAT_TOL[precision], err.max()
+
+
+def test_columns_that_are_not_finite_stay_apart(so):
+    rng = np.random.default_rng(3)
+    n, nr = 64, 50
+    t, tinv = _legendre(n)
+    a = rng.standard_normal((n, nr)) + 1j * rng.standard_normal((n, nr))
+    a[5, 7] = complex(np.nan, 1.0)
+    a[60, 31] = complex(0.0, np.inf)
+    got, ref, names = _matrix_pass(so, a, t, tinv, np.ones((n, nr)), "fp64")
+    assert "tcfx" in names
+    bad = np.zeros(nr, dtype=bool)
+    bad[[7, 31]] = True
+    assert np.all(np.isnan(got[:, bad].real))
+    err = np.linalg.norm((got - ref).astype(np.complex128)[:, ~bad], axis=0)
+    assert np.all(err < MAT_TOL["fp64"] * np.linalg.norm(ref.astype(np.complex128)[:, ~bad], axis=0))
+
+
+@pytest.mark.parametrize("kind", ["identity", "blocks", "complex", "large_table"])
+def test_other_matrices_and_tables_keep_floating_point(so, kind):
+    rng = np.random.default_rng(5)
+    n, nr = 32, 40
+    t, tinv = _legendre(n)
+    ph = np.exp(1j * rng.uniform(0.0, 6.0, (n, nr)))
+    a = rng.standard_normal((n, nr)) + 1j * rng.standard_normal((n, nr))
+    if kind == "identity":
+        t = tinv = np.eye(n)
+        a[::2] *= 1e-30
+    elif kind == "blocks":
+        t = np.kron(np.eye(4), rng.standard_normal((8, 8)))
+        tinv = t.T.copy()
+    elif kind == "complex":
+        t = t + 0.1j * t
+    else:
+        ph = 40.0 * ph
+    got, ref, names = _matrix_pass(so, a, t.real if kind != "complex" else t, tinv, ph, "fp64")
+    assert "tcfx" not in names
+    if kind == "complex":
+        ref = ref * (1.0 + 0.1j)
+    err = np.abs(got - ref.astype(np.complex128))
+    assert np.all(err <= 1e-13 * np.abs(ref).max(axis=1, keepdims=True))
