@@ -96,6 +96,9 @@ struct PassParams {
   int32_t radix;                // fused: radix of the Stockham stages (16 or 8; the twiddle table's order)
   int32_t ct;                   // fused FP32: log2 n of the fixed-shape kernel (0: the general-shape kernel)
   int32_t fx;                   // fused FP64 / float-float: log2 n of the fixed-point kernel (0: floating point)
+  int32_t fx_chirp, fx_g;       // ... lengths that are no power of two: fx is log2 of the inner transforms'
+                                // length M, and the filter in aux is scaled by 2^-fx_g
+  const void* aux;              // ... chirp (n factors) and filter spectrum (M factors)
   DevOp ops[kMaxOps];
 };
 
@@ -174,17 +177,18 @@ bool schedules_from_json(const std::string& text);
 // fft_pair_plan checks the pass and sets its tiling (lanes per tile, tiles) and p.fused.
 bool fft_pair_plan(PassParams& p, int real, bool resident);
 int fft_pair_threads(const Geometry& g);  // the default threads per CTA
-int fft_pair_block(const Geometry& g);    // threads per CTA of a planned pass (lanes per tile x n / 16)
+int fft_pair_block(const PassParams& p);  // threads per CTA of a planned pass (lanes per tile x n / 16)
 
-// The same pass of FP64 and float-float states in 64-bit fixed point (fx_fft.cu), n = 16 .. 8192:
-// a forward transform, then an inverse one, with tables whose largest magnitudes (table_max,
+// The same pass of FP64 and float-float states in 64-bit fixed point (fx_fft.cu), powers of two
+// from 16 to 8192 and other lengths from 17 to 4096 (p.fx_chirp): a forward transform, then an inverse one, with tables whose largest magnitudes (table_max,
 // per op) fx.cuh's bounds allow.  Sets the tiling and p.fx; the ops' tables and p.twiddle are
 // then the fixed-point ones.
 bool fx_pair_plan(PassParams& p, int real, const double* table_max);
 // one pass (one != nullptr) or a batched launch
-cudaError_t launch_fx_pair(int real, int lgn, const PassParams* one, const PassParams* params_dev,
+cudaError_t launch_fx_pair(int real, bool chirp, int lgn, const PassParams* one, const PassParams* params_dev,
                            const int64_t* offsets_dev, int count, int64_t blocks, int threads, size_t smem,
                            cudaStream_t s);
+int fx_pair_out(int lgm);  // exponent gained by a pair of inner transforms (values in at 2^60)
 // a device table in the state precision as fixed-point factors (16 bytes a value as well)
 cudaError_t launch_fx_table(void* dst, const void* src, int real, int64_t n, cudaStream_t s);
 

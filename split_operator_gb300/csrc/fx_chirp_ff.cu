@@ -1,0 +1,11 @@
+// Fixed-point FFT pair of other lengths (fx_pair.cuh), float-float states: a translation unit of its own.
+#include "fx_pair.cuh"
+
+namespace so {
+
+cudaError_t launch_fx_chirp_ff(int lgn, const PassParams* one, const PassParams* params, const int64_t* offsets,
+                            int count, int64_t blocks, int threads, size_t smem, cudaStream_t s) {
+  return launch_any<true, true>(lgn, one, params, offsets, count, blocks, threads, smem, s);
+}
+
+}  // namespace so

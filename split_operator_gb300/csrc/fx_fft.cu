@@ -3,9 +3,13 @@
 
 namespace so {
 
-// fx_fft_ff.cu
+// the other kernels, each set in a translation unit of its own (they compile side by side)
 cudaError_t launch_fx_pair_ff(int lgn, const PassParams* one, const PassParams* params, const int64_t* offsets,
                               int count, int64_t blocks, int threads, size_t smem, cudaStream_t s);
+cudaError_t launch_fx_chirp(int lgn, const PassParams* one, const PassParams* params, const int64_t* offsets,
+                            int count, int64_t blocks, int threads, size_t smem, cudaStream_t s);
+cudaError_t launch_fx_chirp_ff(int lgn, const PassParams* one, const PassParams* params, const int64_t* offsets,
+                               int count, int64_t blocks, int threads, size_t smem, cudaStream_t s);
 
 namespace {
 
@@ -32,7 +36,9 @@ __global__ void fx_table_kernel(int4* dst, const longlong2* src, int64_t n) {
 
 bool fx_pair_plan(PassParams& p, int real, const double* table_max) {
   Geometry& g = p.g;
-  if (real == kRealF32 || g.inner != 1 || !stage_twiddles(g.n) || g.n > 8192) return false;
+  // powers of two from 16 to 8192 points; other lengths through transforms of M >= 2 n - 1 points
+  const bool pow2 = (g.n & (g.n - 1)) == 0;
+  if (real == kRealF32 || g.inner != 1 || g.n < 16 || g.n > (pow2 ? 8192 : 4096)) return false;
   if (p.nops < 2 || p.ops[0].kind != OP_FFT || p.ops[0].dir != -1) return false;
   int ffts = 0;
   double prod = 1.0;
@@ -50,27 +56,37 @@ bool fx_pair_plan(PassParams& p, int real, const double* table_max) {
   }
   if (ffts != 2 || !(prod <= kMaxProduct)) return false;
   int lg = 0;
-  while ((int64_t)1 << lg < g.n) ++lg;
+  while ((int64_t)1 << lg < (pow2 ? g.n : 2 * g.n - 1)) ++lg;
+  const int64_t m = (int64_t)1 << lg;
   // 256 threads a CTA (512 for 8192 points), fewer while the tiles do not fill the SMs twice
-  int T = g.n >= 8192 ? 512 : 256;
-  const int least = g.n / kV > 32 ? (int)(g.n / kV) : 32;
-  while (T > least && (g.outer * g.n + (int64_t)kV * T - 1) / ((int64_t)kV * T) < 304) T /= 2;
-  const int64_t L = (int64_t)kV * T / g.n;
+  int T = m >= 8192 ? 512 : 256;
+  const int least = m / kV > 32 ? (int)(m / kV) : 32;
+  while (T > least && (g.outer * m + (int64_t)kV * T - 1) / ((int64_t)kV * T) < 304) T /= 2;
+  const int64_t L = (int64_t)kV * T / m;
   g.lanes_per_tile = (int32_t)L;
   g.tiles_per_outer = 1;
   g.tiles = (g.outer + L - 1) / L;
-  g.lane_stride = (int32_t)(g.n + g.n / 16 + 1);
+  g.lane_stride = (int32_t)(m + m / 16 + 1);
+  p.fx_chirp = pow2 ? 0 : 1;
   p.fused = 1;
   p.radix = 16;
   p.fx = lg;
   return true;
 }
 
-cudaError_t launch_fx_pair(int real, int lgn, const PassParams* one, const PassParams* params_dev,
+int fx_pair_out(int lgm) {
+  const int rl = lgm - 4 * ((lgm + 3) / 4 - 1);
+  return 60 + rl + 2 - 2 * ((rl + 1) / 2);  // Shape::kOut
+}
+
+cudaError_t launch_fx_pair(int real, bool chirp, int lgn, const PassParams* one, const PassParams* params_dev,
                            const int64_t* offsets_dev, int count, int64_t blocks, int threads, size_t smem,
                            cudaStream_t s) {
+  if (chirp)
+    return real == kRealFF ? launch_fx_chirp_ff(lgn, one, params_dev, offsets_dev, count, blocks, threads, smem, s)
+                           : launch_fx_chirp(lgn, one, params_dev, offsets_dev, count, blocks, threads, smem, s);
   return real == kRealFF ? launch_fx_pair_ff(lgn, one, params_dev, offsets_dev, count, blocks, threads, smem, s)
-                         : launch_any<false>(lgn, one, params_dev, offsets_dev, count, blocks, threads, smem, s);
+                         : launch_any<false, false>(lgn, one, params_dev, offsets_dev, count, blocks, threads, smem, s);
 }
 
 cudaError_t launch_fx_table(void* dst, const void* src, int real, int64_t n, cudaStream_t s) {

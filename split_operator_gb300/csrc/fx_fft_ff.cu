@@ -6,7 +6,7 @@ namespace so {
 
 cudaError_t launch_fx_pair_ff(int lgn, const PassParams* one, const PassParams* params, const int64_t* offsets,
                               int count, int64_t blocks, int threads, size_t smem, cudaStream_t s) {
-  return launch_any<true>(lgn, one, params, offsets, count, blocks, threads, smem, s);
+  return launch_any<true, false>(lgn, one, params, offsets, count, blocks, threads, smem, s);
 }
 
 }  // namespace so

@@ -248,14 +248,117 @@ __device__ __forceinline__ void fx_pair_tile(const PassParams& pp, int64_t tile)
   }
 }
 
+// Lanes of other lengths, n <= M / 2 points with M = 2^LGM, by Bluestein's algorithm (L. Bluestein,
+// "A linear filtering approach to the computation of the discrete Fourier transform", IEEE
+// Trans. Audio Electroacoust. 18, 1970): with w_j = exp(-i pi j^2 / n), the transform of x is
+// w_k times the convolution of x_j w_j with conj w, a pair of transforms of M points around a
+// product with the filter's spectrum G.  The closing w_k of the forward transform and the
+// opening conj w_k of the inverse one cancel in the pair, and the inverse filter is conj G.
+// (A direct sum in FP64 took 5.8 ms for 45 lanes of 1000 points.)
+// pp.aux: the chirp w (n entries), then G 2^-pp.fx_g (M entries, natural order, magnitudes <= 1).
+template <int LGM, bool FF>
+__device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile) {
+  using Sh = Shape<LGM>;
+  constexpr int kM = Sh::kN, kNb = kM / 16, kLgNb = LGM - 4;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ NormPart part[16];
+  cx* buf = reinterpret_cast<cx*>(smem_raw);
+  const Geometry& g = pp.g;
+  const int n = (int)g.n;
+  const int64_t lane0 = tile * g.lanes_per_tile;
+  const int64_t rem = g.outer - lane0;
+  const int nl = rem < g.lanes_per_tile ? (int)rem : g.lanes_per_tile;
+  longlong2* psi = reinterpret_cast<longlong2*>(pp.psi) + lane0 * n;
+  const int4* tw = reinterpret_cast<const int4*>(pp.twiddle);
+  const int4* chirp = reinterpret_cast<const int4*>(pp.aux);
+  const int4* gt = chirp + n;
+  const int t = threadIdx.x, T = blockDim.x;
+  cx v[kV];
+  // value r: point i0 + r M / 16 of lane l0 (the layout of the outer radix-16 stages)
+  const int l0 = t >> kLgNb, i0 = t & (kNb - 1);
+  const bool ok0 = l0 < nl;
+#pragma unroll
+  for (int r = 0; r < 16; ++r) {
+    const int j = i0 + r * kNb;
+    const longlong2 x = ok0 && j < n ? psi[l0 * n + j] : longlong2{0, 0};
+    v[r] = {x.x, x.y};
+  }
+  const int e = lane_exponent<LGM, FF>(v, part);
+#pragma unroll
+  for (int r = 0; r < 16; ++r) {
+    const int j = i0 + r * kNb;
+    v[r].x = e == kNonFinite || e == kZero ? 0 : raw_to_fx<FF>(v[r].x, e);
+    v[r].y = e == kNonFinite || e == kZero ? 0 : raw_to_fx<FF>(v[r].y, e);
+    if (j < n) v[r] = cmul<0>(v[r], __ldg(chirp + j));
+  }
+  int f1 = 1;
+  while (f1 < pp.nops && pp.ops[f1].kind != OP_FFT) ++f1;
+  // (one copy of the transforms' code serves both halves)
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+    transform<LGM, false, 0, -1>(v, buf, tw);
+    // the filter on the outputs of the closing stage (value j RS + q: point k + q P)
+    constexpr int RS = Sh::kRl, kP = kM / RS;
+#pragma unroll
+    for (int j = 0; j < kV / RS; ++j) {
+      const int k = (t + j * T) & (kP - 1);
+#pragma unroll
+      for (int q = 0; q < RS; ++q) {
+        int4 w = __ldg(gt + k + q * kP);
+        if (half) {
+          w.z = -w.z;
+          w.w = -w.w;
+        }
+        v[j * RS + q] = cmul<Sh::kSh>(v[j * RS + q], w);
+      }
+    }
+    transform<LGM, true, 0, 1>(v, buf, tw);
+    // the n points of the transform, and the ops up to the next one
+    const int ob = half ? f1 + 1 : 1, oe = half ? pp.nops : f1;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      const int j = i0 + r * kNb;
+      if (j >= n || !ok0) {
+        v[r] = {0, 0};
+        continue;
+      }
+      if (half) {
+        int4 w = __ldg(chirp + j);
+        w.z = -w.z;
+        w.w = -w.w;
+        v[r] = cmul<0>(v[r], w);
+      }
+      for (int oi = ob; oi < oe; ++oi) {
+        const DevOp& op = pp.ops[oi];
+        const int4* tab = reinterpret_cast<const int4*>(op.ptr) + (op.kind == OP_DIAGND ? (lane0 + l0) * n : 0);
+        v[r] = cmul<0>(v[r], __ldg(tab + j));
+      }
+    }
+  }
+  if (ok0) {
+    const int x = e - (2 * Sh::kOut - 2 * pp.fx_g - 60);
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      const int j = i0 + r * kNb;
+      if (j >= n) continue;
+      longlong2 o{fx_to_raw<FF>(v[r].x, x), fx_to_raw<FF>(v[r].y, x)};
+      if (e == kNonFinite) o = {raw_nan<FF>(), raw_nan<FF>()};
+      psi[l0 * n + j] = o;
+    }
+  }
+}
+
 // one pass (params == nullptr: `one`), or many propagations' passes in one launch: block b
 // runs tile (b - offsets[i]) of params[i], offsets[i] <= b < offsets[i + 1]
-template <int LGN, bool FF>
+template <int LGN, bool FF, bool CHIRP>
 __global__ void __launch_bounds__(Shape<LGN>::kThreads, LGN >= 13 ? 1 : 2)
     fx_pair_kernel(const __grid_constant__ PassParams one, const PassParams* __restrict__ params,
                    const int64_t* __restrict__ offsets, int count) {
   if (params == nullptr) {
-    fx_pair_tile<LGN, FF>(one, blockIdx.x);
+    if constexpr (CHIRP)
+      fx_chirp_tile<LGN, FF>(one, blockIdx.x);
+    else
+      fx_pair_tile<LGN, FF>(one, blockIdx.x);
     return;
   }
   const int64_t b = blockIdx.x;
@@ -267,14 +370,17 @@ __global__ void __launch_bounds__(Shape<LGN>::kThreads, LGN >= 13 ? 1 : 2)
     else
       hi = mid - 1;
   }
-  fx_pair_tile<LGN, FF>(params[lo], b - offsets[lo]);
+  if constexpr (CHIRP)
+    fx_chirp_tile<LGN, FF>(params[lo], b - offsets[lo]);
+  else
+    fx_pair_tile<LGN, FF>(params[lo], b - offsets[lo]);
 }
 
-template <int LGN, bool FF>
+template <int LGN, bool FF, bool CHIRP>
 cudaError_t launch_lgn(const PassParams* one, const PassParams* params, const int64_t* offsets, int count,
                        int64_t blocks, int threads, size_t smem, cudaStream_t s) {
   static bool done = false;
-  auto kern = fx_pair_kernel<LGN, FF>;
+  auto kern = fx_pair_kernel<LGN, FF, CHIRP>;
   if (!done) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     if (e != cudaSuccess) return e;
@@ -287,20 +393,25 @@ cudaError_t launch_lgn(const PassParams* one, const PassParams* params, const in
   return cudaGetLastError();
 }
 
-template <bool FF>
+// lgn: log2 of the lane length (CHIRP: of M)
+template <bool FF, bool CHIRP>
 cudaError_t launch_any(int lgn, const PassParams* one, const PassParams* params, const int64_t* offsets, int count,
                        int64_t blocks, int threads, size_t smem, cudaStream_t s) {
   switch (lgn) {
-    case 4: return launch_lgn<4, FF>(one, params, offsets, count, blocks, threads, smem, s);
-    case 5: return launch_lgn<5, FF>(one, params, offsets, count, blocks, threads, smem, s);
-    case 6: return launch_lgn<6, FF>(one, params, offsets, count, blocks, threads, smem, s);
-    case 7: return launch_lgn<7, FF>(one, params, offsets, count, blocks, threads, smem, s);
-    case 8: return launch_lgn<8, FF>(one, params, offsets, count, blocks, threads, smem, s);
-    case 9: return launch_lgn<9, FF>(one, params, offsets, count, blocks, threads, smem, s);
-    case 10: return launch_lgn<10, FF>(one, params, offsets, count, blocks, threads, smem, s);
-    case 11: return launch_lgn<11, FF>(one, params, offsets, count, blocks, threads, smem, s);
-    case 12: return launch_lgn<12, FF>(one, params, offsets, count, blocks, threads, smem, s);
-    case 13: return launch_lgn<13, FF>(one, params, offsets, count, blocks, threads, smem, s);
+    case 4:
+      if constexpr (!CHIRP) return launch_lgn<4, FF, CHIRP>(one, params, offsets, count, blocks, threads, smem, s);
+      return cudaErrorInvalidValue;
+    case 5:
+      if constexpr (!CHIRP) return launch_lgn<5, FF, CHIRP>(one, params, offsets, count, blocks, threads, smem, s);
+      return cudaErrorInvalidValue;
+    case 6: return launch_lgn<6, FF, CHIRP>(one, params, offsets, count, blocks, threads, smem, s);
+    case 7: return launch_lgn<7, FF, CHIRP>(one, params, offsets, count, blocks, threads, smem, s);
+    case 8: return launch_lgn<8, FF, CHIRP>(one, params, offsets, count, blocks, threads, smem, s);
+    case 9: return launch_lgn<9, FF, CHIRP>(one, params, offsets, count, blocks, threads, smem, s);
+    case 10: return launch_lgn<10, FF, CHIRP>(one, params, offsets, count, blocks, threads, smem, s);
+    case 11: return launch_lgn<11, FF, CHIRP>(one, params, offsets, count, blocks, threads, smem, s);
+    case 12: return launch_lgn<12, FF, CHIRP>(one, params, offsets, count, blocks, threads, smem, s);
+    case 13: return launch_lgn<13, FF, CHIRP>(one, params, offsets, count, blocks, threads, smem, s);
     default: return cudaErrorInvalidValue;
   }
 }

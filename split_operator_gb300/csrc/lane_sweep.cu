@@ -1262,7 +1262,7 @@ static cudaError_t launch_pair_ct(const PassParams& p, cudaStream_t s) {
   static bool done = false;
   cudaError_t e = configure_once(fft_pair_kernel_ct<LGN>, done);
   if (e != cudaSuccess) return e;
-  fft_pair_kernel_ct<LGN><<<(unsigned)p.g.tiles, fft_pair_block(p.g), fft_pair_smem(p.g, false), s>>>(p);
+  fft_pair_kernel_ct<LGN><<<(unsigned)p.g.tiles, fft_pair_block(p), fft_pair_smem(p.g, false), s>>>(p);
   return cudaGetLastError();
 }
 
@@ -1301,7 +1301,9 @@ static cudaError_t launch_pair_batched_ct_any(int lgn, const PassParams* params_
 
 int fft_pair_threads(const Geometry& g) { return g.n >= 8192 ? 512 : 256; }
 
-int fft_pair_block(const Geometry& g) { return (int)((int64_t)g.lanes_per_tile * g.n / kPairV); }
+int fft_pair_block(const PassParams& p) {
+  return (int)((int64_t)p.g.lanes_per_tile * (p.fx ? (int64_t)1 << p.fx : p.g.n) / kPairV);
+}
 
 bool fft_pair_plan(PassParams& p, int real, bool resident) {
   Geometry& g = p.g;
@@ -1504,7 +1506,7 @@ cudaError_t launch_pass_f64(const PassParams& p, cudaStream_t s) {
     }
     const size_t smem = fft_pair_smem(p.g, true);
     if (smem > 220 * 1024) return cudaErrorInvalidValue;
-    fft_pair_kernel_f64<<<(unsigned)p.g.tiles, fft_pair_block(p.g), smem, s>>>(p);
+    fft_pair_kernel_f64<<<(unsigned)p.g.tiles, fft_pair_block(p), smem, s>>>(p);
     count_launch();
     return cudaGetLastError();
   }
@@ -1520,7 +1522,7 @@ cudaError_t launch_pass_ff(const PassParams& p, cudaStream_t s) {
     }
     const size_t smem = fft_pair_smem(p.g, true);
     if (smem > 220 * 1024) return cudaErrorInvalidValue;
-    fft_pair_kernel_ff<<<(unsigned)p.g.tiles, fft_pair_block(p.g), smem, s>>>(p);
+    fft_pair_kernel_ff<<<(unsigned)p.g.tiles, fft_pair_block(p), smem, s>>>(p);
     count_launch();
     return cudaGetLastError();
   }
@@ -1544,9 +1546,9 @@ cudaError_t launch_pass_f32(const PassParams& p, cudaStream_t s) {
       return e;
     }
     if (r8)
-      fft_pair_kernel_r8<<<(unsigned)p.g.tiles, fft_pair_block(p.g), smem, s>>>(p);
+      fft_pair_kernel_r8<<<(unsigned)p.g.tiles, fft_pair_block(p), smem, s>>>(p);
     else
-      fft_pair_kernel<<<(unsigned)p.g.tiles, fft_pair_block(p.g), smem, s>>>(p);
+      fft_pair_kernel<<<(unsigned)p.g.tiles, fft_pair_block(p), smem, s>>>(p);
     count_launch();
     return cudaGetLastError();
   }

@@ -333,57 +333,129 @@ const void* Engine::fx_table(Cached& c) {
   return c.fx.ptr;
 }
 
-// Twiddles of the fixed-point FFT pair: w 2^62 in two signed digits {re.l, re.h, im.l, im.h},
-// stage-major for radix 16 (forward order, then reversed order), one copy per device and length
-// for the process (entries are held weakly, by the engines that use them).
-const void* Engine::fx_twiddle(size_t n) {
-  static std::mutex mu;
-  static std::map<std::pair<int, size_t>, std::weak_ptr<DeviceBuffer>> cache;
-  auto& mine = fx_twiddles_[n];
-  if (mine) return mine->ptr;
-  int dev = 0;
-  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-  std::lock_guard<std::mutex> lock(mu);
-  auto& slot = cache[{dev, n}];
-  mine = slot.lock();
-  if (mine) return mine->ptr;
-  // (cos, sin) of 2 pi m / n times 2^62 for m = 0 .. n / 8, the other octants by symmetry
-  const long double kTau = 6.283185307179586476925286766559005768L;
-  std::vector<std::pair<int64_t, int64_t>> oct0(n / 8 + 1);
-  for (size_t m = 0; m <= n / 8; ++m) {
-    const long double a = kTau * (long double)m / (long double)n;
-    oct0[m] = {(int64_t)llroundl(ldexpl(cosl(a), 62)), (int64_t)llroundl(ldexpl(sinl(a), 62))};
-  }
-  std::vector<int32_t> st(8 * n, 0);
-  auto put = [](int64_t v, int32_t* d) {
-    if ((int32_t)v == INT32_MIN) ++v;  // the kernels negate digits
-    const int32_t l = (int32_t)v;
-    d[0] = l;
-    d[1] = (int32_t)((v - l) >> 32);
-  };
-  for (size_t e = 0; e < 2 * n; ++e) {
-    const size_t m = (size_t)stage_twiddle_exponent((int64_t)(e % n), (int64_t)n, 16, e >= n) % n;
-    const size_t quad = 4 * m / n, r = m - quad * (n / 4);  // r < n / 4 within quadrant quad
-    int64_t c, s;
-    if (r <= n / 8) {
-      c = oct0[r].first;
-      s = oct0[r].second;
-    } else {
-      c = oct0[n / 4 - r].second;
-      s = oct0[n / 4 - r].first;
+// Factor w 2^62 in two signed digits (fx.cuh).
+static void fx_put(int64_t v, int32_t* d) {
+  if ((int32_t)v == INT32_MIN) ++v;  // the kernels negate digits
+  const int32_t l = (int32_t)v;
+  d[0] = l;
+  d[1] = (int32_t)((v - l) >> 32);
+}
+
+// (cos, sin) of 2 pi m / n for any m, to long double's precision, from one octant
+namespace {
+struct Circle {
+  size_t n8;  // steps of the circle, a multiple of 8
+  std::vector<std::pair<long double, long double>> oct;
+  explicit Circle(size_t steps) : n8(steps), oct(steps / 8 + 1) {
+    const long double tau = 6.283185307179586476925286766559005768L;
+    for (size_t m = 0; m <= n8 / 8; ++m) {
+      const long double a = tau * (long double)m / (long double)n8;
+      oct[m] = {cosl(a), sinl(a)};
     }
+  }
+  std::pair<long double, long double> at(size_t m) const {
+    m %= n8;
+    const size_t quad = 4 * m / n8, r = m - quad * (n8 / 4);
+    long double c = r <= n8 / 8 ? oct[r].first : oct[n8 / 4 - r].second;
+    long double s = r <= n8 / 8 ? oct[r].second : oct[n8 / 4 - r].first;
     for (size_t q = 0; q < quad; ++q) {
-      const int64_t t = c;
+      const long double t = c;
       c = -s;
       s = t;
     }
-    put(c, &st[4 * e]);
-    put(-s, &st[4 * e + 2]);  // exp(-2 pi i m / n)
+    return {c, s};
   }
-  mine = std::make_shared<DeviceBuffer>();
-  upload(*mine, st, stream);
-  slot = mine;
-  return mine->ptr;
+};
+int64_t fx_of(long double v) { return (int64_t)llroundl(ldexpl(v, 62)); }
+}  // namespace
+
+// Factors the fixed-point FFT pairs share, one copy per device, kind and length for the process
+// (held weakly, by the engines that use them).
+std::shared_ptr<FxFactors> Engine::fx_shared(int kind, size_t n, const std::function<FxHost()>& make) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, int, size_t>, std::weak_ptr<FxFactors>> cache;
+  auto& mine = fx_factors_[{kind, n}];
+  if (mine) return mine;
+  int dev = 0;
+  cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+  std::lock_guard<std::mutex> lock(mu);
+  auto& slot = cache[{dev, kind, n}];
+  mine = slot.lock();
+  if (mine) return mine;
+  const FxHost h = make();
+  auto f = std::make_shared<FxFactors>();
+  upload(f->buf, h.words, stream);
+  f->g = h.g;
+  slot = mine = f;
+  return mine;
+}
+
+// Twiddles, stage-major for radix 16 (forward order, then reversed order).
+const void* Engine::fx_twiddle(size_t n) {
+  return fx_shared(0, n, [n] {
+    const Circle circ(n);
+    FxHost h;
+    h.words.assign(8 * n, 0);
+    for (size_t e = 0; e < 2 * n; ++e) {
+      const auto w = circ.at((size_t)stage_twiddle_exponent((int64_t)(e % n), (int64_t)n, 16, e >= n));
+      fx_put(fx_of(w.first), &h.words[4 * e]);
+      fx_put(fx_of(-w.second), &h.words[4 * e + 2]);  // exp(-2 pi i m / n)
+    }
+    return h;
+  })->buf.ptr;
+}
+
+// Chirp w_j = exp(-i pi j^2 / n) and the spectrum of the filter conj w (length M, times 2^-g and
+// 1 / sqrt n: a unitary transform) of lanes whose length is no power of two.
+const FxFactors& Engine::fx_chirp(size_t n, int lgm) {
+  return *fx_shared(1, n, [n, lgm] {
+    using C = std::complex<long double>;
+    const size_t M = (size_t)1 << lgm;
+    const Circle circ(8 * n);  // pi j^2 / n = 2 pi (4 j^2) / (8 n)
+    auto chirp = [&](size_t j) { return circ.at(4 * ((j * j) % (2 * n))); };
+    FxHost h;
+    h.words.assign(4 * (n + M), 0);
+    std::vector<C> b(M, C(0, 0));
+    for (size_t j = 0; j < n; ++j) {
+      const auto w = chirp(j);
+      fx_put(fx_of(w.first), &h.words[4 * j]);
+      fx_put(fx_of(-w.second), &h.words[4 * j + 2]);
+      b[j] = C(w.first, w.second);
+      if (j) b[M - j] = b[j];
+    }
+    // in-place radix-2 transform, natural order in, natural order out
+    for (size_t i = 1, j = 0; i < M; ++i) {
+      size_t bit = M >> 1;
+      for (; j & bit; bit >>= 1) j ^= bit;
+      j ^= bit;
+      if (i < j) std::swap(b[i], b[j]);
+    }
+    const Circle cm(M);
+    for (size_t len = 2; len <= M; len <<= 1)
+      for (size_t k = 0; k < len / 2; ++k) {
+        const auto w = cm.at(k * (M / len));
+        const C f(w.first, -w.second);
+        for (size_t i = k; i < M; i += len) {
+          const C u = b[i], v = b[i + len / 2] * f;
+          b[i] = u + v;
+          b[i + len / 2] = u - v;
+        }
+      }
+    long double mx = 0.0L;
+    const long double rn = 1.0L / sqrtl((long double)n);
+    for (C& v : b) {
+      v *= rn;
+      mx = std::max(mx, std::abs(v));
+    }
+    // magnitudes at most 1, and the values after a pair back at 2^60 or below
+    h.g = fx_pair_out(lgm) - 60;
+    while (ldexpl(mx, -h.g) > 1.0L) ++h.g;
+    for (size_t k = 0; k < M; ++k) {
+      fx_put(fx_of(ldexpl(b[k].real(), -h.g)), &h.words[4 * (n + k)]);
+      fx_put(fx_of(ldexpl(b[k].imag(), -h.g)), &h.words[4 * (n + k) + 2]);
+    }
+    return h;
+  });
 }
 
 // Parity structure of a real n x n matrix (logical M[a][b] = m[a n + b]) within tol of its
@@ -862,7 +934,12 @@ bool Engine::try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p) {
   if (!fx_pair_plan(p, real, mx)) return false;
   for (size_t i = 0; i < ops.size(); ++i)
     if (tab[i]) p.ops[i].ptr = fx_table(*tab[i]);
-  p.twiddle = fx_twiddle((size_t)p.g.n);
+  p.twiddle = fx_twiddle((size_t)1 << p.fx);
+  if (p.fx_chirp) {
+    const FxFactors& f = fx_chirp((size_t)p.g.n, p.fx);
+    p.aux = f.buf.ptr;
+    p.fx_g = f.g;
+  }
   return true;
 }
 
@@ -921,9 +998,9 @@ void Engine::launch(const std::vector<DevOp>& ops, int axis, bool resident, int 
   if (recording) {
     // fused FFT pairs: bit 16 of the thread count (their own launch group and kernel)
     // radix-8 FP32 pairs: bit 19 (their own kernel); fixed-shape FP32 pairs: bit 20;
-    // fixed-point pairs: bit 25
-    const int threads = p.fused ? (fft_pair_block(p.g) | (1 << 16) | (p.radix == 8 && !fp64 ? 1 << 19 : 0) |
-                                   (p.ct ? 1 << 20 : 0) | (p.fx ? 1 << 25 : 0))
+    // fixed-point pairs: bit 25 (lengths that are no power of two: and bit 26)
+    const int threads = p.fused ? (fft_pair_block(p) | (1 << 16) | (p.radix == 8 && !fp64 ? 1 << 19 : 0) |
+                                   (p.ct ? 1 << 20 : 0) | (p.fx ? 1 << 25 : 0) | (p.fx_chirp ? 1 << 26 : 0))
                                 : pass_threads(p.g);
     RecordedPass r{resident ? RecordedPass::Resident : RecordedPass::Generic, real, p, {},
                    threads, pass_smem_bytes(p, fp64), name, pass_bytes(ops, p.g)};
@@ -935,7 +1012,7 @@ void Engine::launch(const std::vector<DevOp>& ops, int axis, bool resident, int 
     timed_.back().bytes = pass_bytes(ops, p.g);
   }
   if (p.fx)
-    cuda_check(launch_fx_pair(real, p.fx, &p, nullptr, nullptr, 0, p.g.tiles, fft_pair_block(p.g),
+    cuda_check(launch_fx_pair(real, p.fx_chirp, p.fx, &p, nullptr, nullptr, 0, p.g.tiles, fft_pair_block(p),
                               pass_smem_bytes(p, true), stream),
                "pass launch");
   else
@@ -2203,7 +2280,7 @@ void Batch::run_groups(std::vector<Group>& gs, bool concurrent) {
                                            st, (g.threads >> 20) & 3, 1 << ((g.threads >> 23) & 3)),
                  "batched tensor-core pass");
     else if (g.fx_lgn)
-      cuda_check(launch_fx_pair(g.real, g.fx_lgn, nullptr, g.params.as<PassParams>(), g.offsets.as<int64_t>(), g.count,
+      cuda_check(launch_fx_pair(g.real, (g.threads >> 26) & 1, g.fx_lgn, nullptr, g.params.as<PassParams>(), g.offsets.as<int64_t>(), g.count,
                                 g.blocks, g.threads & 0xffff, g.smem, st),
                  "batched pass");
     else

@@ -75,6 +75,16 @@ struct DeviceBuffer {
   T* as() const { return reinterpret_cast<T*>(ptr); }
 };
 
+// Factors of the fixed-point FFT pairs: device digits, and the filter's scale (2^-g).
+struct FxFactors {
+  DeviceBuffer buf;
+  int g = 0;
+};
+struct FxHost {
+  std::vector<int32_t> words;
+  int g = 0;
+};
+
 class Engine;
 
 // Scalars of an operator (loss, current norm, leak norm) that live in device
@@ -237,8 +247,11 @@ class Engine {
   std::map<const void*, std::shared_ptr<DeviceBuffer>> fx_images_;  // digit images by device matrix
   Cached* phase_table(const void* device_ptr);           // the cache entry of a phase table
   const void* fx_table(Cached& c);                       // its fixed-point copy
-  const void* fx_twiddle(size_t n);                      // fixed-point twiddles, shared by the process
-  std::map<size_t, std::shared_ptr<DeviceBuffer>> fx_twiddles_;
+  // fixed-point factors shared by the process: twiddles of n points, chirp and filter of n points
+  std::shared_ptr<FxFactors> fx_shared(int kind, size_t n, const std::function<FxHost()>& make);
+  const void* fx_twiddle(size_t n);
+  const FxFactors& fx_chirp(size_t n, int lgm);
+  std::map<std::pair<int, size_t>, std::shared_ptr<FxFactors>> fx_factors_;
   std::map<uint64_t, DeviceBuffer> weights_;
   std::map<std::pair<size_t, int>, DeviceBuffer> twiddles_;  // by (n, stage radix)
   // open pass

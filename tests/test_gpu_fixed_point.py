@@ -225,3 +225,19 @@ def test_other_matrices_and_tables_keep_floating_point(so, kind):
         ref = ref * (1.0 + 0.1j)
     err = np.abs(got - ref.astype(np.complex128))
     assert np.all(err <= 1e-13 * np.abs(ref).max(axis=1, keepdims=True))
+
+
+# Lengths that are no power of two: two pairs of inner transforms of M points, each within 4e-16 at
+# the filter's two bits of headroom, against numpy's own 1e-15 there
+@pytest.mark.parametrize("precision,tol", [("fp64", 4e-15), ("float_float", 2e-14)])
+@pytest.mark.parametrize("n,lanes", [(18, 300), (20, 3), (34, 37), (100, 5), (300, 96), (510, 4), (514, 3), (1000, 45),
+                                     (2050, 2), (4094, 3)])
+def test_fft_pair_of_other_lengths_matches_numpy(so, precision, tol, n, lanes):
+    a = _lanes(lanes, n, 11 * n + lanes)
+    a[lanes // 2] = 0.0
+    got, ref, names = _pass(so, a, precision)
+    assert "fftpair fx" in names
+    assert np.all(got[lanes // 2] == 0.0)
+    live = np.arange(lanes) != lanes // 2
+    err = np.linalg.norm(got - ref, axis=1)[live] / np.linalg.norm(ref, axis=1)[live]
+    assert err.max() < tol, (int(err.argmax()), err.max())
