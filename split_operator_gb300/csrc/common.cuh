@@ -188,7 +188,10 @@ bool fx_pair_plan(PassParams& p, int real, const double* table_max);
 cudaError_t launch_fx_pair(int real, bool chirp, int lgn, const PassParams* one, const PassParams* params_dev,
                            const int64_t* offsets_dev, int count, int64_t blocks, int threads, size_t smem,
                            cudaStream_t s);
-int fx_pair_out(int lgm);  // exponent gained by a pair of inner transforms (values in at 2^60)
+// Resident 1-D steps of FP64 and float-float states in fixed point (fx_line.cu): one transform pair
+// per repetition.  Sets p.fx and p.fx_chirp; tables and twiddles (radix 4) are then fixed point.
+bool fx_line_plan(PassParams& p, int real, const double* table_max);
+cudaError_t launch_fx_line(int real, const PassParams& p, cudaStream_t s);
 // a device table in the state precision as fixed-point factors (16 bytes a value as well)
 cudaError_t launch_fx_table(void* dst, const void* src, int real, int64_t n, cudaStream_t s);
 

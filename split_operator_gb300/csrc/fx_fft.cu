@@ -74,11 +74,6 @@ bool fx_pair_plan(PassParams& p, int real, const double* table_max) {
   return true;
 }
 
-int fx_pair_out(int lgm) {
-  const int rl = lgm - 4 * ((lgm + 3) / 4 - 1);
-  return 60 + rl + 2 - 2 * ((rl + 1) / 2);  // Shape::kOut
-}
-
 cudaError_t launch_fx_pair(int real, bool chirp, int lgn, const PassParams* one, const PassParams* params_dev,
                            const int64_t* offsets_dev, int count, int64_t blocks, int threads, size_t smem,
                            cudaStream_t s) {

@@ -11,8 +11,7 @@
 // global memory.  The unitary scaling sits in the products (w 2^62 times v is v w / 4, the
 // factor of a radix-16 stage) and in the exponent the lane leaves with.
 #pragma once
-#include "common.cuh"
-#include "fx.cuh"
+#include "fx_stage.cuh"
 
 namespace so {
 
@@ -21,94 +20,7 @@ using namespace fx;
 namespace {
 
 constexpr int kV = 16;  // values per thread
-
-template <int LGN>
-struct Shape {
-  static constexpr int kN = 1 << LGN;
-  static constexpr int kS = (LGN + 3) / 4;                   // radix-16 stages, the last one kRl
-  static constexpr int kLgRl = LGN - 4 * (kS - 1);           // closing radix 2, 4, 8 or 16
-  static constexpr int kRl = 1 << kLgRl;
-  static constexpr int kSh = (kLgRl + 1) / 2;                // its scaling: 2^-kSh
-  static constexpr int kLs = kN + kN / 16 + 1;               // padded lane stride
-  // exponent of the pass: values are loaded as x 2^(60 - e) and leave as x 2^(kOut - e)
-  static constexpr int kOut = 60 + kLgRl + 2 - 2 * kSh;
-  static constexpr int kThreads = kN >= 8192 ? 512 : 256;    // most threads of a CTA
-  __host__ __device__ static constexpr int rs(bool rev, int s) {
-    return rev ? (s == 0 ? kRl : 16) : (s + 1 < kS ? 16 : kRl);
-  }
-  __host__ __device__ static constexpr int span(bool rev, int s) {
-    return s == 0 ? 1 : span(rev, s - 1) * rs(rev, s - 1);
-  }
-  // first entry of stage s in the stage-major twiddle table (reversed order: from entry n)
-  __host__ __device__ static constexpr int twoff(bool rev, int s) {
-    return s == 0 ? (rev ? kN : 0)
-                  : twoff(rev, s - 1) + (span(rev, s - 1) > 1 ? (rs(rev, s - 1) - 1) * span(rev, s - 1) : 0);
-  }
-};
-__host__ __device__ constexpr int lg2(int x) { return x <= 1 ? 0 : 1 + lg2(x / 2); }
-
-// One stage of radix RS, span P, twiddles from entry OFF; IN: 0 registers, 1 shared memory;
-// OUT: 0 registers, 1 shared memory.  SC: the stage scales by 2^-SC (in its products).
-template <int LGN, int RS, int P, int OFF, bool IN, bool OUT, int DIR, int SC>
-__device__ __forceinline__ void stage(cx (&v)[kV], cx* buf, const int4* __restrict__ tw) {
-  constexpr int kN = 1 << LGN, kNb = kN / RS, kLgNb = LGN - lg2(RS), kLs = Shape<LGN>::kLs;
-  const int t = threadIdx.x, T = blockDim.x;
-  if constexpr (IN) {
-#pragma unroll
-    for (int j = 0; j < kV / RS; ++j) {
-      const int b = t + j * T, l = b >> kLgNb, i = b & (kNb - 1);
-      const cx* src = buf + l * kLs + i + (i >> 4);
-#pragma unroll
-      for (int r = 0; r < RS; ++r) {
-        // element i + r nb: its padding splits as (i >> 4) + (r nb >> 4) when nb is a multiple of 16
-        v[j * RS + r] = kNb % 16 == 0 ? src[r * kNb + ((r * kNb) >> 4)]
-                                      : buf[l * kLs + i + r * kNb + ((i + r * kNb) >> 4)];
-      }
-    }
-    __syncthreads();  // every read of the stage before any write (in place)
-  }
-#pragma unroll
-  for (int j = 0; j < kV / RS; ++j) {
-    if constexpr (P > 1) {
-      // k = i & (P - 1) = b & (P - 1) (P divides nb)
-      const int4* w = tw + OFF + ((t + j * T) & (P - 1));
-      v[j * RS] = shift_down<SC>(v[j * RS]);
-#pragma unroll
-      for (int r = 1; r < RS; ++r) {
-        int4 wv = __ldg(w + (r - 1) * P);
-        if (DIR > 0) {
-          wv.z = -wv.z;
-          wv.w = -wv.w;
-        }
-        v[j * RS + r] = cmul<SC>(v[j * RS + r], wv);
-      }
-    }
-    dft_r<RS, DIR>(&v[j * RS]);
-  }
-  if constexpr (OUT) {
-#pragma unroll
-    for (int j = 0; j < kV / RS; ++j) {
-      const int b = t + j * T, l = b >> kLgNb, i = b & (kNb - 1), k = i & (P - 1);
-      const int base = (i - k) * RS + k;
-#pragma unroll
-      for (int q = 0; q < RS; ++q) {
-        const int x = base + q * P;
-        buf[l * kLs + x + (x >> 4)] = v[j * RS + q];
-      }
-    }
-    __syncthreads();
-  }
-}
-
-template <int LGN, bool REV, int S, int DIR>
-__device__ __forceinline__ void transform(cx (&v)[kV], cx* buf, const int4* tw) {
-  using Sh = Shape<LGN>;
-  constexpr int rs = Sh::rs(REV, S), p = Sh::span(REV, S);
-  // a closing stage of the forward order scales by 2^-kSh, every other stage with twiddles by 1/4
-  constexpr int sc = (!REV && S + 1 == Sh::kS) ? Sh::kSh : 2;
-  stage<LGN, rs, p, Sh::twoff(REV, S), (S > 0), (S + 1 < Sh::kS), DIR, sc>(v, buf, tw);
-  if constexpr (S + 1 < Sh::kS) transform<LGN, REV, S + 1, DIR>(v, buf, tw);
-}
+__host__ __device__ constexpr int pair_threads(int lgn) { return lgn >= 13 ? 512 : 256; }  // most threads of a CTA
 
 // point-wise ops [ob, oe) on the outputs of a last stage of radix RS (span P = n / RS): value
 // j RS + q sits at lane b >> lg P, point k + q P; the first one scales by 2^-SC
@@ -144,61 +56,9 @@ __device__ __forceinline__ void pointwise(cx (&v)[kV], const PassParams& pp, int
   }
 }
 
-// Lane norm bounds.  A thread's 16 values lie in one lane (lane = t >> lg(n / 16)).  Returns e
-// with |lane|_2 <= 2^e, kNonFinite for a lane with a value that is not finite, kZero for one of
-// zeros and subnormals (which becomes zero).  part: one entry per warp.
-struct NormPart {
-  int ref;
-  uint32_t sum;  // sum |x|^2 2^(2 (1023 - ref)) in units of 2^-12, rounded up
-};
-constexpr int kNonFinite = 1 << 20, kZero = -(1 << 20);
-template <int LGN, bool FF>
-__device__ __forceinline__ int lane_exponent(const cx (&raw)[kV], NormPart* part) {
-  constexpr int kTpl = (1 << LGN) / 16;  // threads per lane
-  const int t = threadIdx.x, lane = t & 31;
-  int m = 0;
-#pragma unroll
-  for (int e = 0; e < kV; ++e) m = max(m, max(raw_exp<FF>(raw[e].x), raw_exp<FF>(raw[e].y)));
-  constexpr int kG = kTpl < 32 ? kTpl : 32;
-  const unsigned mask = kG == 32 ? 0xffffffffu : ((1u << (kG & 31)) - 1u) << (lane & ~(kG - 1));
-  m = __reduce_max_sync(mask, m);
-  int ref = max(m, 1);
-  float s = 0.0f;
-#pragma unroll
-  for (int e = 0; e < kV; ++e) {
-    const float x = raw_rel<FF>(raw[e].x, ref), y = raw_rel<FF>(raw[e].y, ref);
-    s = fmaf(x, x, fmaf(y, y, s));
-  }
-  // (a lane with a value that is not finite: s may be infinite, the conversion saturates)
-  uint32_t q = __reduce_add_sync(mask, (uint32_t)min((int)__float2int_ru(s * 4096.0f), 1 << 20));
-  float tot = (float)q;
-  if constexpr (kTpl > 32) {
-    constexpr int kW = kTpl / 32;  // warps per lane
-    const int w = t >> 5, w0 = w & ~(kW - 1);
-    if (lane == 0) part[w] = {m, q};
-    __syncthreads();
-    m = 0;
-#pragma unroll
-    for (int i = 0; i < kW; ++i) m = max(m, part[w0 + i].ref);
-    ref = max(m, 1);
-    tot = 0.0f;
-#pragma unroll
-    for (int i = 0; i < kW; ++i) {
-      const int d = ref - max(part[w0 + i].ref, 1);
-      tot = fmaf((float)part[w0 + i].sum, d < 60 ? __int_as_float((127 - 2 * d) << 23) : 0.0f, tot);
-    }
-    tot += 1.0f;  // the terms cut off above, in units of 2^-12 of the largest value's square
-  }
-  if (m == 2047) return kNonFinite;
-  if (m == 0) return kZero;
-  // |lane|^2 <= tot (1 + 2^-15) 2^-12 2^(2 (ref - 1023)): e = the least integer with 4^e above
-  const int ex = (__float_as_int(fmaf(tot, 0x1p-15f, tot)) >> 23) - 127 - 12;  // tot < 2^(ex + 1)
-  return (ref - 1023) + ((ex + 2) >> 1);
-}
-
 template <int LGN, bool FF>
 __device__ __forceinline__ void fx_pair_tile(const PassParams& pp, int64_t tile) {
-  using Sh = Shape<LGN>;
+  using Sh = Shape<LGN, kV>;
   constexpr int kN = Sh::kN, kNb = kN / 16, kLgNb = LGN - 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ NormPart part[16];
@@ -222,7 +82,7 @@ __device__ __forceinline__ void fx_pair_tile(const PassParams& pp, int64_t tile)
       v[r] = {x.x, x.y};
     }
   }
-  const int e = lane_exponent<LGN, FF>(v, part);
+  const int e = lane_exponent<LGN, kV, FF>(v, part);
 #pragma unroll
   for (int r = 0; r < 16; ++r) {
     v[r].x = e == kNonFinite || e == kZero ? 0 : raw_to_fx<FF>(v[r].x, e);
@@ -230,9 +90,9 @@ __device__ __forceinline__ void fx_pair_tile(const PassParams& pp, int64_t tile)
   }
   int f1 = 1;
   while (f1 < pp.nops && pp.ops[f1].kind != OP_FFT) ++f1;
-  transform<LGN, false, 0, -1>(v, buf, tw);
-  pointwise<LGN, Sh::kRl, Sh::kSh>(v, pp, 1, f1, lane0, nl);
-  transform<LGN, true, 0, 1>(v, buf, tw);
+  transform<LGN, kV, false, 0, -1>(v, buf, tw);
+  pointwise<LGN, Sh::kRl, Sh::kMid>(v, pp, 1, f1, lane0, nl);
+  transform<LGN, kV, true, 0, 1>(v, buf, tw);
   pointwise<LGN, Sh::rs(true, Sh::kS - 1), 0>(v, pp, f1 + 1, pp.nops, lane0, nl);
   // the last stage's outputs have the first stage's layout (radix 16, or the only stage):
   // the same lane, points k + q n / 16
@@ -258,7 +118,7 @@ __device__ __forceinline__ void fx_pair_tile(const PassParams& pp, int64_t tile)
 // pp.aux: the chirp w (n entries), then G 2^-pp.fx_g (M entries, natural order, magnitudes <= 1).
 template <int LGM, bool FF>
 __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile) {
-  using Sh = Shape<LGM>;
+  using Sh = Shape<LGM, kV>;
   constexpr int kM = Sh::kN, kNb = kM / 16, kLgNb = LGM - 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ NormPart part[16];
@@ -283,7 +143,7 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
     const longlong2 x = ok0 && j < n ? psi[l0 * n + j] : longlong2{0, 0};
     v[r] = {x.x, x.y};
   }
-  const int e = lane_exponent<LGM, FF>(v, part);
+  const int e = lane_exponent<LGM, kV, FF>(v, part);
 #pragma unroll
   for (int r = 0; r < 16; ++r) {
     const int j = i0 + r * kNb;
@@ -296,7 +156,7 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
   // (one copy of the transforms' code serves both halves)
 #pragma unroll 1
   for (int half = 0; half < 2; ++half) {
-    transform<LGM, false, 0, -1>(v, buf, tw);
+    transform<LGM, kV, false, 0, -1>(v, buf, tw);
     // the filter on the outputs of the closing stage (value j RS + q: point k + q P)
     constexpr int RS = Sh::kRl, kP = kM / RS;
 #pragma unroll
@@ -309,10 +169,10 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
           w.z = -w.z;
           w.w = -w.w;
         }
-        v[j * RS + q] = cmul<Sh::kSh>(v[j * RS + q], w);
+        v[j * RS + q] = cmul<Sh::kMid>(v[j * RS + q], w);
       }
     }
-    transform<LGM, true, 0, 1>(v, buf, tw);
+    transform<LGM, kV, true, 0, 1>(v, buf, tw);
     // the n points of the transform, and the ops up to the next one
     const int ob = half ? f1 + 1 : 1, oe = half ? pp.nops : f1;
 #pragma unroll
@@ -351,7 +211,7 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
 // one pass (params == nullptr: `one`), or many propagations' passes in one launch: block b
 // runs tile (b - offsets[i]) of params[i], offsets[i] <= b < offsets[i + 1]
 template <int LGN, bool FF, bool CHIRP>
-__global__ void __launch_bounds__(Shape<LGN>::kThreads, LGN >= 13 ? 1 : 2)
+__global__ void __launch_bounds__(pair_threads(LGN), LGN >= 13 ? 1 : 2)
     fx_pair_kernel(const __grid_constant__ PassParams one, const PassParams* __restrict__ params,
                    const int64_t* __restrict__ offsets, int count) {
   if (params == nullptr) {
@@ -386,7 +246,7 @@ cudaError_t launch_lgn(const PassParams* one, const PassParams* params, const in
     if (e != cudaSuccess) return e;
     done = true;
   }
-  if (smem > 220 * 1024 || threads > Shape<LGN>::kThreads) return cudaErrorInvalidValue;
+  if (smem > 220 * 1024 || threads > pair_threads(LGN)) return cudaErrorInvalidValue;
   static const PassParams none{};
   kern<<<(unsigned)blocks, threads, smem, s>>>(one ? *one : none, params, offsets, count);
   count_launch();

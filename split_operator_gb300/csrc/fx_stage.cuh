@@ -1,0 +1,158 @@
+// Fixed-point transforms (fx.cuh) of power-of-two lanes held in registers, KV values per thread,
+// exchanged in place in one shared buffer; and the norm bound a lane is scaled by.
+#pragma once
+#include "common.cuh"
+#include "fx.cuh"
+
+namespace so {
+
+using namespace fx;
+
+namespace {
+
+__host__ __device__ constexpr int lg2(int x) { return x <= 1 ? 0 : 1 + lg2(x / 2); }
+
+// A power-of-two transform of 2^LGN points with KV values per thread (16 or 4) and radix-KV stages.
+// Values come in at 2^60 of the lane's norm bound or below; the first stage is unscaled, a stage
+// with twiddles scales by the square root of its radix or a little more in its products.
+template <int LGN, int KV>
+struct Shape {
+  static constexpr int kN = 1 << LGN, kLgV = lg2(KV);
+  static constexpr int kS = (LGN + kLgV - 1) / kLgV;         // radix-KV stages, the last one kRl
+  static constexpr int kLgRl = LGN - kLgV * (kS - 1);        // closing radix (2 .. KV)
+  static constexpr int kRl = 1 << kLgRl;
+  static constexpr int kSc = kLgV / 2;                       // scaling of a full stage: 2^-kSc
+  static constexpr int kSh = (kLgRl + 1) / 2;                // of the closing stage of the forward order
+  static constexpr int kMid = kLgRl / 2;                     // of the factors between a pair's transforms
+  static constexpr int kPad = KV == 16 ? 4 : 3;              // one padding element every 2^kPad
+  static constexpr int kLs = kN + (kN >> kPad) + 1;          // padded lane stride
+  static constexpr int kOut = 60 + kSc;                      // exponent after a pair: x 2^(kOut - e)
+  __host__ __device__ static constexpr int rs(bool rev, int s) {
+    return rev ? (s == 0 ? kRl : KV) : (s + 1 < kS ? KV : kRl);
+  }
+  __host__ __device__ static constexpr int span(bool rev, int s) {
+    return s == 0 ? 1 : span(rev, s - 1) * rs(rev, s - 1);
+  }
+  // first entry of stage s in the stage-major twiddle table (reversed order: from entry n)
+  __host__ __device__ static constexpr int twoff(bool rev, int s) {
+    return s == 0 ? (rev ? kN : 0)
+                  : twoff(rev, s - 1) + (span(rev, s - 1) > 1 ? (rs(rev, s - 1) - 1) * span(rev, s - 1) : 0);
+  }
+};
+
+// One stage of radix RS, span P, twiddles from entry OFF; IN: 0 registers, 1 shared memory;
+// OUT: 0 registers, 1 shared memory.  SC: the stage scales by 2^-SC (in its products).
+template <int LGN, int KV, int RS, int P, int OFF, bool IN, bool OUT, int DIR, int SC>
+__device__ __forceinline__ void stage(cx (&v)[KV], cx* buf, const int4* __restrict__ tw) {
+  constexpr int kN = 1 << LGN, kNb = kN / RS, kLgNb = LGN - lg2(RS), kLs = Shape<LGN, KV>::kLs, kPad = Shape<LGN, KV>::kPad;
+  const int t = threadIdx.x, T = blockDim.x;
+  if constexpr (IN) {
+#pragma unroll
+    for (int j = 0; j < KV / RS; ++j) {
+      const int b = t + j * T, l = b >> kLgNb, i = b & (kNb - 1);
+      const cx* src = buf + l * kLs + i + (i >> kPad);
+#pragma unroll
+      for (int r = 0; r < RS; ++r) {
+        // element i + r nb: its padding splits into those of i and r nb when nb is a multiple of 2^kPad
+        v[j * RS + r] = kNb % (1 << kPad) == 0 ? src[r * kNb + ((r * kNb) >> kPad)]
+                                               : buf[l * kLs + i + r * kNb + ((i + r * kNb) >> kPad)];
+      }
+    }
+    __syncthreads();  // every read of the stage before any write (in place)
+  }
+#pragma unroll
+  for (int j = 0; j < KV / RS; ++j) {
+    if constexpr (P > 1) {
+      // k = i & (P - 1) = b & (P - 1) (P divides nb)
+      const int4* w = tw + OFF + ((t + j * T) & (P - 1));
+      v[j * RS] = shift_down<SC>(v[j * RS]);
+#pragma unroll
+      for (int r = 1; r < RS; ++r) {
+        int4 wv = __ldg(w + (r - 1) * P);
+        if (DIR > 0) {
+          wv.z = -wv.z;
+          wv.w = -wv.w;
+        }
+        v[j * RS + r] = cmul<SC>(v[j * RS + r], wv);
+      }
+    }
+    dft_r<RS, DIR>(&v[j * RS]);
+  }
+  if constexpr (OUT) {
+#pragma unroll
+    for (int j = 0; j < KV / RS; ++j) {
+      const int b = t + j * T, l = b >> kLgNb, i = b & (kNb - 1), k = i & (P - 1);
+      const int base = (i - k) * RS + k;
+#pragma unroll
+      for (int q = 0; q < RS; ++q) {
+        const int x = base + q * P;
+        buf[l * kLs + x + (x >> kPad)] = v[j * RS + q];
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <int LGN, int KV, bool REV, int S, int DIR>
+__device__ __forceinline__ void transform(cx (&v)[KV], cx* buf, const int4* tw) {
+  using Sh = Shape<LGN, KV>;
+  constexpr int rs = Sh::rs(REV, S), p = Sh::span(REV, S);
+  constexpr int sc = (!REV && S + 1 == Sh::kS) ? Sh::kSh : Sh::kSc;
+  stage<LGN, KV, rs, p, Sh::twoff(REV, S), (S > 0), (S + 1 < Sh::kS), DIR, sc>(v, buf, tw);
+  if constexpr (S + 1 < Sh::kS) transform<LGN, KV, REV, S + 1, DIR>(v, buf, tw);
+}
+
+// Lane norm bounds.  A thread's KV values lie in one lane (lane = t >> lg(n / KV)).  Returns e
+// with |lane|_2 <= 2^e, kNonFinite for a lane with a value that is not finite, kZero for one of
+// zeros and subnormals (which becomes zero).  part: one entry per warp.
+struct NormPart {
+  int ref;
+  uint32_t sum;  // sum |x|^2 2^(2 (1023 - ref)) in units of 2^-12, rounded up
+};
+constexpr int kNonFinite = 1 << 20, kZero = -(1 << 20);
+template <int LGN, int KV, bool FF>
+__device__ __forceinline__ int lane_exponent(const cx (&raw)[KV], NormPart* part) {
+  constexpr int kTpl = (1 << LGN) / KV;  // threads per lane
+  const int t = threadIdx.x, lane = t & 31;
+  int m = 0;
+#pragma unroll
+  for (int e = 0; e < KV; ++e) m = max(m, max(raw_exp<FF>(raw[e].x), raw_exp<FF>(raw[e].y)));
+  constexpr int kG = kTpl < 32 ? kTpl : 32;
+  const unsigned mask = kG == 32 ? 0xffffffffu : ((1u << (kG & 31)) - 1u) << (lane & ~(kG - 1));
+  m = __reduce_max_sync(mask, m);
+  int ref = max(m, 1);
+  float s = 0.0f;
+#pragma unroll
+  for (int e = 0; e < KV; ++e) {
+    const float x = raw_rel<FF>(raw[e].x, ref), y = raw_rel<FF>(raw[e].y, ref);
+    s = fmaf(x, x, fmaf(y, y, s));
+  }
+  // (a lane with a value that is not finite: s may be infinite, the conversion saturates)
+  uint32_t q = __reduce_add_sync(mask, (uint32_t)min((int)__float2int_ru(s * 4096.0f), 1 << 20));
+  float tot = (float)q;
+  if constexpr (kTpl > 32) {
+    constexpr int kW = kTpl / 32;  // warps per lane
+    const int w = t >> 5, w0 = w & ~(kW - 1);
+    if (lane == 0) part[w] = {m, q};
+    __syncthreads();
+    m = 0;
+#pragma unroll
+    for (int i = 0; i < kW; ++i) m = max(m, part[w0 + i].ref);
+    ref = max(m, 1);
+    tot = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kW; ++i) {
+      const int d = ref - max(part[w0 + i].ref, 1);
+      tot = fmaf((float)part[w0 + i].sum, d < 60 ? __int_as_float((127 - 2 * d) << 23) : 0.0f, tot);
+    }
+    tot += 1.0f;  // the terms cut off above, in units of 2^-12 of the largest value's square
+  }
+  if (m == 2047) return kNonFinite;
+  if (m == 0) return kZero;
+  // |lane|^2 <= tot (1 + 2^-15) 2^-12 2^(2 (ref - 1023)): e = the least integer with 4^e above
+  const int ex = (__float_as_int(fmaf(tot, 0x1p-15f, tot)) >> 23) - 127 - 12;  // tot < 2^(ex + 1)
+  return (ref - 1023) + ((ex + 2) >> 1);
+}
+
+}  // namespace
+}  // namespace so

@@ -390,14 +390,14 @@ std::shared_ptr<FxFactors> Engine::fx_shared(int kind, size_t n, const std::func
   return mine;
 }
 
-// Twiddles, stage-major for radix 16 (forward order, then reversed order).
-const void* Engine::fx_twiddle(size_t n) {
-  return fx_shared(0, n, [n] {
+// Twiddles, stage-major (forward order, then reversed order).
+const void* Engine::fx_twiddle(size_t n, int radix) {
+  return fx_shared(radix, n, [n, radix] {
     const Circle circ(n);
     FxHost h;
     h.words.assign(8 * n, 0);
     for (size_t e = 0; e < 2 * n; ++e) {
-      const auto w = circ.at((size_t)stage_twiddle_exponent((int64_t)(e % n), (int64_t)n, 16, e >= n));
+      const auto w = circ.at((size_t)stage_twiddle_exponent((int64_t)(e % n), (int64_t)n, radix, e >= n));
       fx_put(fx_of(w.first), &h.words[4 * e]);
       fx_put(fx_of(-w.second), &h.words[4 * e + 2]);  // exp(-2 pi i m / n)
     }
@@ -447,8 +447,8 @@ const FxFactors& Engine::fx_chirp(size_t n, int lgm) {
       v *= rn;
       mx = std::max(mx, std::abs(v));
     }
-    // magnitudes at most 1, and the values after a pair back at 2^60 or below
-    h.g = fx_pair_out(lgm) - 60;
+    // magnitudes at most 1, and the values after a pair (2^62 in all) back at 2^60 or below
+    h.g = 2;
     while (ldexpl(mx, -h.g) > 1.0L) ++h.g;
     for (size_t k = 0; k < M; ++k) {
       fx_put(fx_of(ldexpl(b[k].real(), -h.g)), &h.words[4 * (n + k)]);
@@ -922,7 +922,8 @@ bool Engine::try_launch_fx_tc(const std::vector<DevOp>& ops, int axis, PassParam
   return true;
 }
 
-bool Engine::try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p) {
+// The fixed-point form of an FFT pair, or of a resident 1-D program.
+bool Engine::try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p, bool resident) {
   double mx[kMaxOps] = {};
   Cached* tab[kMaxOps] = {};
   for (size_t i = 0; i < ops.size(); ++i)
@@ -931,10 +932,10 @@ bool Engine::try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p) {
       if (!tab[i]) return false;
       mx[i] = tab[i]->max_abs;
     }
-  if (!fx_pair_plan(p, real, mx)) return false;
+  if (!(resident ? fx_line_plan(p, real, mx) : fx_pair_plan(p, real, mx))) return false;
   for (size_t i = 0; i < ops.size(); ++i)
     if (tab[i]) p.ops[i].ptr = fx_table(*tab[i]);
-  p.twiddle = fx_twiddle((size_t)1 << p.fx);
+  p.twiddle = fx_twiddle((size_t)1 << p.fx, resident ? 4 : 16);
   if (p.fx_chirp) {
     const FxFactors& f = fx_chirp((size_t)p.g.n, p.fx);
     p.aux = f.buf.ptr;
@@ -979,8 +980,8 @@ void Engine::launch(const std::vector<DevOp>& ops, int axis, bool resident, int 
   pass_choose_buffers(p, fp64);
   if (!fp64 && tc_mode() >= 0 && !resident && try_launch_tc(ops, axis, p)) return;
   if (fx && !resident && try_launch_fx_tc(ops, axis, p)) return;
-  if (fx && !resident && try_launch_fx_pair(ops, p)) {
-    name_tag = " fftpair fx";
+  if (fx && !(resident && recording) && try_launch_fx_pair(ops, p, resident)) {
+    name_tag = resident ? " fx" : " fftpair fx";
   } else if ((fft_pair || (fp64 && p.g.n > 4096)) && fft_pair_plan(p, real, resident)) {
     name_tag = p.radix == 8 && !fp64 ? " fftpair r8" : " fftpair";
     if (p.radix != (fp64 ? 8 : 16)) p.twiddle = twiddle((size_t)p.g.n, p.radix);  // the table in its stage order
@@ -1011,7 +1012,9 @@ void Engine::launch(const std::vector<DevOp>& ops, int axis, bool resident, int 
     timed_begin(name);
     timed_.back().bytes = pass_bytes(ops, p.g);
   }
-  if (p.fx)
+  if (p.fx && resident)
+    cuda_check(launch_fx_line(real, p, stream), "pass launch");
+  else if (p.fx)
     cuda_check(launch_fx_pair(real, p.fx_chirp, p.fx, &p, nullptr, nullptr, 0, p.g.tiles, fft_pair_block(p),
                               pass_smem_bytes(p, true), stream),
                "pass launch");

@@ -241,7 +241,7 @@ class Engine {
   bool try_launch_tc(const std::vector<DevOp>& ops, int axis, PassParams& p);
   static void shared_tc_images(const std::vector<double>& md, int n, int mode, cudaStream_t s,
                                std::shared_ptr<DeviceBuffer>& img, std::shared_ptr<DeviceBuffer>& par, int& kind);
-  bool try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p);
+  bool try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p, bool resident);
   bool try_launch_fx_tc(const std::vector<DevOp>& ops, int axis, PassParams& p);
   void fx_images(const void* matrix, const std::vector<cplx>& m, size_t n, size_t count);
   std::map<const void*, std::shared_ptr<DeviceBuffer>> fx_images_;  // digit images by device matrix
@@ -249,7 +249,7 @@ class Engine {
   const void* fx_table(Cached& c);                       // its fixed-point copy
   // fixed-point factors shared by the process: twiddles of n points, chirp and filter of n points
   std::shared_ptr<FxFactors> fx_shared(int kind, size_t n, const std::function<FxHost()>& make);
-  const void* fx_twiddle(size_t n);
+  const void* fx_twiddle(size_t n, int radix);
   const FxFactors& fx_chirp(size_t n, int lgm);
   std::map<std::pair<int, size_t>, std::shared_ptr<FxFactors>> fx_factors_;
   std::map<uint64_t, DeviceBuffer> weights_;

@@ -241,3 +241,75 @@ def test_fft_pair_of_other_lengths_matches_numpy(so, precision, tol, n, lanes):
     live = np.arange(lanes) != lanes // 2
     err = np.linalg.norm(got - ref, axis=1)[live] / np.linalg.norm(ref, axis=1)[live]
     assert err.max() < tol, (int(err.argmax()), err.max())
+
+
+# ---- resident 1-D propagations
+def _line(lib, n, im, x0=0.3, loss=True):
+    half = 20.0 * np.sqrt(n / 1024.0)
+    grid = lib.Grid.new_linear_continuos("space", -half, half, n, 0)
+    x = np.asarray(grid.nodes)
+    psi = np.exp(-((x - x0 * half) / 1.7) ** 2 - 0.6j * x)
+    wf = lib.WaveFunction(psi.astype(np.complex128), [grid])
+    wf.normalize(1.0)
+    tg = lib.TimeGrid(0.01, 10 ** 6, im)
+    leak = lib.LeakControl()
+    if loss:
+        leak.add_loss_checker("leak control" if not hasattr(lib, "LossChecker") else lib.LossChecker("leak control"))
+    st = lib.OperationStack()
+    st.add_control(leak, lib.FIRST_HALF | lib.SECOND_HALF)
+    st.add_propagator(lib.one_dim_into_propagator(0.5 * x * x, grid, tg, lib.HALF))
+    st.add_transformation(lib.FFTTransformation(grid, "momentum"), lib.NORMAL)
+    st.add_propagator(lib.one_dim_into_propagator(lib.kinetic_hamiltonian(grid, 1.0), grid, tg, lib.FULL))
+    return wf, tg, st
+
+
+# 30 steps of numpy's FP64 (5e-16 a step, growing as its square root at best) against as many
+# fixed-point steps; the bound is the parity tests' 1e-12 over 30 steps in proportion
+# (In imaginary time the packet at x0 decays against the well's centre by e^(-30 dt x0^2 / 2):
+# from 2046 points on the rounding noise at the centre, amplified by that, is all that differs.)
+@pytest.mark.parametrize("precision,tol", [("fp64", 3e-14), ("float_float", 3e-13)])
+@pytest.mark.parametrize("n,im", [(n, False) for n in (16, 18, 32, 34, 64, 100, 128, 256, 500, 512, 1000, 1024, 2046,
+                                                       2048, 4096)] +
+                         [(n, True) for n in (16, 18, 32, 34, 64, 100, 128, 256, 500, 512, 1000, 1024)])
+def test_resident_lines_match_the_oracle(so, precision, tol, n, im):
+    from oracle import split_operator_oracle as O
+    wf, tg, st = _line(so, n, im)
+    owf, otg, ost = _line(O, n, im)
+    p = so.Propagation(wf, tg, st, precision)
+    q = O.Propagation(owf, otg, ost)
+    p.set_timing(True)
+    p.steps(30)
+    q.propagate(30)
+    assert "resident fx" in " ".join(k[0] for k in p.kernel_times())
+    a, b = p.get_array(), q.wave_function.array
+    assert np.linalg.norm(a - b) < tol * np.linalg.norm(b)
+    assert abs(p.norm() - q.wave_function.norm()) < tol
+    assert abs(p.all_losses()[0] - q.all_losses()[0][1]) < 30 * tol
+
+
+@pytest.mark.parametrize("n", [256, 500, 2048])
+def test_resident_lines_do_not_depend_on_the_split(so, n):
+    wf, tg, st = _line(so, n, True)
+    whole = so.Propagation(wf, tg, st, "fp64")
+    whole.steps(23)
+    wf2, tg2, st2 = _line(so, n, True)
+    parts = so.Propagation(wf2, tg2, st2, "fp64")
+    for k in (1, 7, 2, 13):
+        parts.steps(k)
+    np.testing.assert_array_equal(parts.get_array(), whole.get_array())
+    assert parts.all_losses() == whole.all_losses()
+    assert parts.norm() == whole.norm()
+
+
+@pytest.mark.parametrize("n", [64, 500])
+def test_resident_line_with_nan_or_zero(so, n):
+    wf, tg, st = _line(so, n, False)
+    p = so.Propagation(wf, tg, st, "fp64")
+    a = p.get_array()
+    a[3] = complex(np.nan, 0.0)
+    p.set_array(a)
+    p.steps(3)
+    assert np.all(np.isnan(p.get_array().real))
+    from split_operator_gb300._lib import SplitOperatorError
+    with pytest.raises(SplitOperatorError):
+        p.synchronize()
