@@ -6,6 +6,7 @@
 // The three products run on the tensor cores (tcgen05.mma kind::f16, accumulators in
 // TMEM) with FP32 activations and gradients split into two BF16 parts.  Every product and
 // sum runs in a fixed order, so training is deterministic.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -25,200 +26,403 @@ void set_last_error(const char* msg);
 
 namespace {
 
-template <typename T>
-__device__ __forceinline__ float to_f(T v);
-template <>
-__device__ __forceinline__ float to_f<float>(float v) {
-  return v;
-}
-template <>
-__device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) {
-  return __bfloat162float(v);
+// ---- operands
+// Every product's operand is a bf16 matrix (or a hi + lo pair of them: x = bf16(x) + bf16(x -
+// bf16(x)), 16 significant bits together) in one tiled layout: blocks of 128 rows x 64
+// columns (16 KB), row block by row block, each block in core matrices of 8 rows x 8 columns
+// (128 bytes), a row group's eight core matrices after one another.  A core matrix serves as
+// K-major (rows = M or N, columns = K) and, transposed by the tensor core, as MN-major
+// operand (rows = K), so activations, gradients and weights are stored once and read by every
+// product they enter, by bulk TMA copies of whole blocks, half blocks or row groups.
+// Rows and columns are padded to multiples of 128 with zeros.
+constexpr int kPadTo = 128;
+constexpr uint32_t kBlockBytes = 16384, kGroupBytes = 1024;  // 128 x 64 block; 8 rows x 64 columns
+
+int padded(int n) { return (n + kPadTo - 1) / kPadTo * kPadTo; }
+
+// byte offset of element (r, c) of a matrix with `cols` (padded) columns
+__host__ __device__ __forceinline__ size_t tiled(int64_t r, int c, int cols) {
+  return ((size_t)(r >> 7) * (size_t)(cols >> 6) + (size_t)(c >> 6)) * kBlockBytes + (size_t)((r & 127) >> 3) * kGroupBytes +
+         (size_t)((c & 63) >> 3) * 128 + (size_t)(r & 7) * 16 + (size_t)(c & 7) * 2;
 }
 
-// ---- tensor-core GEMM (tcgen05.mma kind::f16, BF16 operands, FP32 accumulation in TMEM)
-// C[m][n] = sum_k A(m, k) B(n, k) over a 128 x 128 tile per CTA, K in chunks of 16.  The
-// 128 threads stage each chunk into shared memory in the K-major core-matrix layout (8 rows
-// x 16 bytes per core matrix, K core matrices 128 B apart, row groups 256 B apart), which
-// also does the transposes the backward products need (A and B are read through strides).
-// FP32 operands are split x = bf16(x) + bf16(x - bf16(x)) (16 significant bits together);
-// the BF16 weights are exact as they are.  Products: hi hi + lo hi (B exact) or
-// hi hi + hi lo + lo hi (both split); the remaining lo lo term is 2^-16 of the result.
-// Two shared-memory stages: thread 0 issues a chunk's MMAs and commits them to the stage's
-// mbarrier, which the threads wait on (bounded) before they overwrite that stage.
-constexpr int kGm = 128, kGn = 128, kGk = 16;
-constexpr uint32_t kGStage = 4u * kGm * kGk * 2u;  // A hi, A lo, B hi, B lo: 4 KB each
-constexpr uint64_t kGWait = 2000000000ull;         // 2 s
+// eight consecutive columns of one row as bf16 hi and lo parts (c a multiple of 8)
+__device__ __forceinline__ void store_split8(unsigned char* hi, unsigned char* lo, size_t off, const float* x) {
+  uint32_t h[4], l[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    uint16_t h0, l0, h1, l1;
+    tc::split_bf16(x[2 * k], h0, l0);
+    tc::split_bf16(x[2 * k + 1], h1, l1);
+    h[k] = h0 | (uint32_t)h1 << 16;
+    l[k] = l0 | (uint32_t)l1 << 16;
+  }
+  *reinterpret_cast<uint4*>(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
+  *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
+}
 
-struct GemmOperand {
-  const void* p;
-  int64_t s_row, s_k;  // element strides: A(m, k) = p[m s_row + k s_k] (B(n, k) likewise)
-  int bf16;            // 1: BF16 values (used as they are); 0: FP32 (split into hi + lo)
+struct Operand {
+  const unsigned char *hi, *lo;  // lo: nullptr for exact bf16 values (weights)
+  int cols;                      // padded columns
 };
 
-// byte offset of element (row r, k) in a 128 x 16 chunk image
-__device__ __forceinline__ uint32_t gemm_off(int r, int k) {
-  return (uint32_t)(r >> 3) * 256u + (uint32_t)(k >> 3) * 128u + (uint32_t)(r & 7) * 16u + (uint32_t)(k & 7) * 2u;
+// ---- tensor-core product C[m][n] = sum_k A(m, k) B(n, k) on tiles of 128 x 64, K in chunks of 64
+// AMN / BMN: the operand's rows are K (MN-major) instead of M / N.  Warp 4 streams the chunks
+// through shared-memory stages by bulk copies, warp 5 issues hi hi + lo hi (+ hi lo when B
+// is split; the lo lo term is 2^-16 of the result) per K step of 16 into one FP32 accumulator
+// (K is not split over CTAs: the tensor core truncates as it accumulates, so the order of the
+// sums is part of the result, and Adam makes a whole step of a gradient that is all rounding),
+// warps 0-3 run the epilogue (thread = one row, 64 columns).  Two CTAs per SM: one's epilogue
+// runs beside the other's products.  Staging FP32 operands element by element in one thread per
+// row, as this kernel did before, took 4.3 ms for a training step of 1024 x (5, 256, 256, 256,
+// 4096).
+enum Epilogue {
+  EPI_RAW,     // C in FP32 (row-major, padded)
+  EPI_HIDDEN,  // bias, tanh: FP32 activation and its bf16 parts
+  EPI_LOSS,    // bias, squared error: the gradient in FP32 and bf16 parts, loss partials
+  EPI_OUT      // bias: FP32 output (row-major, unpadded)
+};
+struct GemmArgs {
+  Operand a, b;
+  int chunks;            // K / 64
+  float* c;              // EPI_RAW: product; EPI_HIDDEN: activation; EPI_LOSS: gradient; EPI_OUT: output
+  int rows, cols;        // valid extent of C (EPI_LOSS, EPI_OUT, EPI_HIDDEN)
+  int ldc;               // padded columns of C
+  const float* bias;
+  unsigned char *hi, *lo;  // bf16 parts written (tiled, ldc columns)
+  const float* target;     // EPI_LOSS: row-major, `cols` columns
+  float scale;             // EPI_LOSS: 2 / (rows cols)
+  double* loss;            // EPI_LOSS: one partial per CTA
+  int* err;
+};
+constexpr uint64_t kGWait = 2000000000ull;  // 2 s
+constexpr int kGThreads = 192;
+
+// Shared-memory stages: two (and two CTAs per SM) where K is short and there are many tiles; the
+// products of the backward pass have few tiles and a long K, and hide a chunk's latency behind
+// the chunks after it (dX of the 4096-wide layer, 32 tiles of 64 chunks).
+__host__ __device__ constexpr int gemm_stages(bool bsplit, int epi) { return epi != EPI_RAW ? 2 : (bsplit ? 4 : 5); }
+__host__ __device__ constexpr uint32_t gemm_stage_bytes(bool bsplit) {
+  return 2 * kBlockBytes + (bsplit ? 2u : 1u) * (kBlockBytes / 2);
 }
 
-// row r of a chunk (16 K values) of one operand into its hi / lo images
-__device__ __forceinline__ void gemm_stage_row(const GemmOperand& o, int64_t row, int64_t rows, int64_t k0, int K,
-                                               int r, unsigned char* hi, unsigned char* lo) {
-  uint32_t h[8], l[8];
-#pragma unroll
-  for (int k = 0; k < kGk; ++k) {
-    float x = 0.0f;
-    if (row < rows && k0 + k < K) {
-      const int64_t e = row * o.s_row + (k0 + k) * o.s_k;
-      x = o.bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(o.p)[e])
-                 : reinterpret_cast<const float*>(o.p)[e];
-    }
-    uint16_t xh, xl;
-    tc::split_bf16(x, xh, xl);  // exact for a BF16 value: xl = 0
-    if (k & 1) {
-      h[k >> 1] |= (uint32_t)xh << 16;
-      l[k >> 1] |= (uint32_t)xl << 16;
-    } else {
-      h[k >> 1] = xh;
-      l[k >> 1] = xl;
-    }
-  }
-  // two 16-byte core-matrix rows (K 0-7 and 8-15) per image
-  *reinterpret_cast<uint4*>(hi + gemm_off(r, 0)) = make_uint4(h[0], h[1], h[2], h[3]);
-  *reinterpret_cast<uint4*>(hi + gemm_off(r, 8)) = make_uint4(h[4], h[5], h[6], h[7]);
-  *reinterpret_cast<uint4*>(lo + gemm_off(r, 0)) = make_uint4(l[0], l[1], l[2], l[3]);
-  *reinterpret_cast<uint4*>(lo + gemm_off(r, 8)) = make_uint4(l[4], l[5], l[6], l[7]);
-}
-
-__global__ void __launch_bounds__(128) tc_gemm_kernel(int M, int N, int K, GemmOperand A, GemmOperand B,
-                                                      float* __restrict__ C, int64_t ldc, int* err) {
+template <bool AMN, bool BMN, bool BSPLIT, int EPI>
+__global__ void __launch_bounds__(kGThreads, EPI == EPI_RAW ? 1 : 2) gemm_kernel(const __grid_constant__ GemmArgs g) {
   using namespace tc;
-  __shared__ __align__(1024) unsigned char sm[2 * kGStage];
-  __shared__ __align__(8) uint64_t done[3];  // per stage: its MMAs completed; [2]: all MMAs
+  constexpr uint32_t kB = BSPLIT ? 2 : 1, kStage = gemm_stage_bytes(BSPLIT);
+  constexpr int kNs = gemm_stages(BSPLIT, EPI);
+  extern __shared__ __align__(1024) unsigned char sm[];
+  __shared__ __align__(8) uint64_t full[kNs], empty[kNs], done;
   __shared__ uint32_t tmem_s;
+  __shared__ double wloss[4];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int64_t m0 = (int64_t)blockIdx.y * kGm, n0 = (int64_t)blockIdx.x * kGn;
+  const int nt = blockIdx.x, mt = blockIdx.y;
+  const int c1 = g.chunks;
   if (tid == 0) {
-    for (int i = 0; i < 3; ++i) mbar_init(&done[i], 1);
+    for (int i = 0; i < kNs; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    mbar_init(&done, 1);
     fence_mbar_init();
   }
-  if (warp == 0) tmem_alloc(&tmem_s, kGn);
+  if (warp == 0) tmem_alloc(&tmem_s, 64);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_s;
-  const uint32_t idesc = idesc_bf16(kGm, kGn);
-  const bool bsplit = !B.bf16, asplit = !A.bf16;
-  const int nk = (K + kGk - 1) / kGk;
   bool ok = true;
-  for (int c = 0; c < nk; ++c) {
-    const int s = c & 1;
-    unsigned char* st = sm + (uint32_t)s * kGStage;
-    // the MMAs that read this stage two chunks ago have completed
-    if (c >= 2) ok = ok && mbar_wait(&done[s], (uint32_t)((c / 2 - 1) & 1), kGWait);
-    gemm_stage_row(A, m0 + tid, M, (int64_t)c * kGk, K, tid, st, st + 4096);
-    gemm_stage_row(B, n0 + tid, N, (int64_t)c * kGk, K, tid, st + 8192, st + 12288);
-    fence_proxy_async();
-    __syncthreads();
-    if (tid == 0) {
-      tc_fence_after();
-      const uint32_t a = smem_u32(st);
-      const uint64_t ah = smem_desc_at(smem_desc_bits(128, 256), a), al = smem_desc_at(smem_desc_bits(128, 256), a + 4096);
-      const uint64_t bh = smem_desc_at(smem_desc_bits(128, 256), a + 8192),
-                     bl = smem_desc_at(smem_desc_bits(128, 256), a + 12288);
-      mma_bf16(tmem, ah, bh, idesc, c > 0 ? 1u : 0u);
-      if (asplit) mma_bf16(tmem, al, bh, idesc, 1u);
-      if (bsplit) mma_bf16(tmem, ah, bl, idesc, 1u);
-      mma_commit(&done[s]);
+  if (warp == 4) {
+    // the whole warp issues a chunk's copies: up to 32 row groups of A, the tiles of B
+    int c = 0;
+    for (; c < c1 && ok; ++c) {
+      const int s = c % kNs, use = c / kNs;
+      if (use > 0) ok = mbar_wait(&empty[s], (use - 1) & 1u, kGWait);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      unsigned char* st = sm + (uint32_t)s * kStage;
+      if (lane == 0) mbar_expect_tx(&full[s], kStage);
+      __syncwarp();
+      if constexpr (!AMN) {
+        if (lane < 2)
+          bulk_g2s(st + (uint32_t)lane * kBlockBytes,
+                   (lane ? g.a.lo : g.a.hi) + ((size_t)mt * (g.a.cols >> 6) + c) * kBlockBytes, kBlockBytes, &full[s]);
+      } else {
+        // 64 rows (K) of two column blocks (M = 128), row group by row group side by side
+        const int q = lane >> 4, r = (lane >> 1) & 7, blk = lane & 1;
+        const unsigned char* src = (q ? g.a.lo : g.a.hi) +
+                                   ((size_t)(c >> 1) * (g.a.cols >> 6) + 2 * mt + blk) * kBlockBytes +
+                                   (size_t)((c & 1) * 8 + r) * kGroupBytes;
+        bulk_g2s(st + (uint32_t)q * kBlockBytes + r * 2048 + blk * 1024, src, kGroupBytes, &full[s]);
+      }
+      if (lane < (int)kB) {
+        const unsigned char* src = lane ? g.b.lo : g.b.hi;
+        const size_t blk = BMN ? (size_t)(c >> 1) * (g.b.cols >> 6) + nt : (size_t)(nt >> 1) * (g.b.cols >> 6) + c;
+        bulk_g2s(st + 2 * kBlockBytes + (uint32_t)lane * (kBlockBytes / 2),
+                 src + blk * kBlockBytes + (size_t)((BMN ? c : nt) & 1) * (kBlockBytes / 2), kBlockBytes / 2, &full[s]);
+      }
     }
-  }
-  if (tid == 0) mma_commit(&done[2]);
-  ok = mbar_wait(&done[2], 0u, kGWait) && ok;
-  tc_fence_after();
-  if (!__syncthreads_and(ok)) {
-    if (tid == 0) atomicExch(err, 1);
-  } else {
-    // TMEM lane = row m0 + 32 warp + lane, 32 columns per load
-    const int64_t m = m0 + 32 * warp + lane;
-    for (int cb = 0; cb < kGn; cb += 32) {
-      float v[32];
-      tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)cb, v);
-      if (m < M)
+    if (!ok && lane == 0)  // let the copies in flight land before the CTA lets go of its shared memory
+      for (int k = c < kNs ? 0 : c - kNs; k < c; ++k) mbar_poll(&full[k % kNs], (k / kNs) & 1u, kGWait);
+  } else if (warp == 5) {
+    if (lane == 0) {
+      const uint32_t base = smem_u32(sm);
+      constexpr uint32_t idesc = idesc_bf16(128, 64) | (AMN ? 1u << 15 : 0u) | (BMN ? 1u << 16 : 0u);
+      // (K-group stride, M/N-group stride) of each form, and the step of 16 K values
+      const uint64_t abits = AMN ? smem_desc_bits(2048, 128) : smem_desc_bits(128, 1024);
+      const uint64_t bbits = BMN ? smem_desc_bits(1024, 128) : smem_desc_bits(128, 1024);
+      constexpr uint32_t astep = AMN ? 4096 : 256, bstep = BMN ? 2048 : 256;
+      for (int c = 0; c < c1 && ok; ++c) {
+        const int s = c % kNs, use = c / kNs;
+        ok = mbar_poll(&full[s], use & 1u, kGWait);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t st = base + (uint32_t)s * kStage;
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (n0 + cb + j < N) C[m * ldc + n0 + cb + j] = v[j];
+        for (int k = 0; k < 4; ++k) {
+          const uint64_t ah = smem_desc_at(abits, st + k * astep), al = smem_desc_at(abits, st + kBlockBytes + k * astep);
+          const uint64_t bh = smem_desc_at(bbits, st + 2 * kBlockBytes + k * bstep);
+          mma_bf16(tmem, ah, bh, idesc, c > 0 || k > 0 ? 1u : 0u);
+          mma_bf16(tmem, al, bh, idesc, 1u);
+          if constexpr (BSPLIT)
+            mma_bf16(tmem, ah, smem_desc_at(bbits, st + 2 * kBlockBytes + kBlockBytes / 2 + k * bstep), idesc, 1u);
+        }
+        mma_commit(&empty[s]);
+      }
+      mma_commit(&done);  // (after a failed wait: everything issued so far)
+      if (!ok) mbar_poll(&done, 0u, kGWait);
+    }
+  } else {
+    ok = mbar_wait(&done, 0u, kGWait);
+    tc_fence_after();
+  }
+  if (!__syncthreads_and(ok)) {
+    if (tid == 0) atomicExch(g.err, 1);
+  } else if (warp < 4) {
+    const int64_t row = (int64_t)mt * 128 + 32 * warp + lane;
+    const int n0 = nt * 64;
+    float v[64];
+    tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16), v);
+    tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + 32u, v + 32);
+    if constexpr (EPI == EPI_RAW) {
+      float* dst = g.c + row * g.ldc + n0;
+#pragma unroll
+      for (int k = 0; k < 64; k += 4) *reinterpret_cast<float4*>(dst + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    } else if constexpr (EPI == EPI_OUT) {
+      if (row < g.rows)
+        for (int k = 0; k < 64; ++k)
+          if (n0 + k < g.cols) g.c[row * g.cols + n0 + k] = v[k] + __ldg(g.bias + n0 + k);
+    } else if constexpr (EPI == EPI_HIDDEN) {
+      const bool live = row < g.rows;
+#pragma unroll
+      for (int k = 0; k < 64; ++k)
+        v[k] = live && n0 + k < g.cols ? tanhf(v[k] + __ldg(g.bias + n0 + k)) : 0.0f;
+#pragma unroll
+      for (int k = 0; k < 64; k += 8) {
+        float* dst = g.c + row * g.ldc + n0 + k;
+        *reinterpret_cast<float4*>(dst) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+        *reinterpret_cast<float4*>(dst + 4) = make_float4(v[k + 4], v[k + 5], v[k + 6], v[k + 7]);
+        store_split8(g.hi, g.lo, tiled(row, n0 + k, g.ldc), v + k);
+      }
+    } else {
+      // d = y - t, its square summed in float-float (two-sum, exact products), the gradient 2 d / n
+      const bool live = row < g.rows;
+      const float* tr = g.target + (live ? row : 0) * g.cols + n0;
+      const bool vec = (g.cols & 3) == 0;
+      float s = 0.0f, e = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 64; k += 4) {
+        float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (live && vec && n0 + k < g.cols) {
+          const float4 q = __ldg(reinterpret_cast<const float4*>(tr + k));
+          t[0] = q.x;
+          t[1] = q.y;
+          t[2] = q.z;
+          t[3] = q.w;
+        } else if (live) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (n0 + k + u < g.cols) t[u] = __ldg(tr + k + u);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const bool in = live && n0 + k + u < g.cols;
+          const float y = v[k + u] + (in ? __ldg(g.bias + n0 + k + u) : 0.0f);
+          const float d = in ? y - t[u] : 0.0f;
+          const float p = __fmul_rn(d, d), pe = __fmaf_rn(d, d, -p);
+          const float q = __fadd_rn(s, p), bb = __fsub_rn(q, s);
+          e = __fadd_rn(e, __fadd_rn(pe, __fadd_rn(__fsub_rn(s, __fsub_rn(q, bb)), __fsub_rn(p, bb))));
+          s = q;
+          v[k + u] = g.scale * d;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 64; k += 8) {
+        float* dst = g.c + row * g.ldc + n0 + k;
+        *reinterpret_cast<float4*>(dst) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+        *reinterpret_cast<float4*>(dst + 4) = make_float4(v[k + 4], v[k + 5], v[k + 6], v[k + 7]);
+        store_split8(g.hi, g.lo, tiled(row, n0 + k, g.ldc), v + k);
+      }
+      double l = (double)s + (double)e;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
+      if (lane == 0) wloss[warp] = l;
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, kGn);
+  if constexpr (EPI == EPI_LOSS) {
+    if (tid == 0) g.loss[blockIdx.y * gridDim.x + blockIdx.x] = (wloss[0] + wloss[1]) + (wloss[2] + wloss[3]);
+  }
+  if (warp == 0) tmem_dealloc(tmem, 64);
 }
 
-// C (M x N, row stride ldc) = A B^T through the tensor-core kernel
-void tc_gemm(int M, int N, int K, GemmOperand A, GemmOperand B, float* C, int64_t ldc, int* err, cudaStream_t s) {
-  dim3 grid((N + kGn - 1) / kGn, (M + kGm - 1) / kGm);
-  tc_gemm_kernel<<<grid, 128, 0, s>>>(M, N, K, A, B, C, ldc, err);
+template <bool AMN, bool BMN, bool BSPLIT, int EPI>
+void launch_gemm(dim3 grid, const GemmArgs& g, cudaStream_t s) {
+  constexpr size_t smem = (size_t)gemm_stages(BSPLIT, EPI) * gemm_stage_bytes(BSPLIT);
+  static bool done = false;
+  auto kern = gemm_kernel<AMN, BMN, BSPLIT, EPI>;
+  if (!done) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    done = true;
+  }
+  kern<<<grid, kGThreads, smem, s>>>(g);
   count_launch();
 }
 
-__global__ void bias_act_kernel(float* Z, const float* b, int rows, int cols, int act) {
-  const int64_t n = (int64_t)rows * cols;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    float v = Z[i] + b[i % cols];
-    Z[i] = act ? tanhf(v) : v;
+// dZ = dX (1 - y^2) of a tanh layer, in place, and its bf16 parts; a thread: one row, 8 columns
+__global__ void __launch_bounds__(256) tanh_back_kernel(float* dx, const float* act, unsigned char* hi,
+                                                        unsigned char* lo, int ld) {
+  const int64_t row = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3);
+  const int c = blockIdx.y * 64 + (threadIdx.x & 7) * 8;
+  const int64_t at = row * ld + c;
+  float v[8];
+#pragma unroll
+  for (int k = 0; k < 8; k += 4) {
+    const float4 q = *reinterpret_cast<const float4*>(dx + at + k);
+    const float4 y = *reinterpret_cast<const float4*>(act + at + k);
+    v[k] = q.x * (1.0f - y.x * y.x);
+    v[k + 1] = q.y * (1.0f - y.y * y.y);
+    v[k + 2] = q.z * (1.0f - y.z * y.z);
+    v[k + 3] = q.w * (1.0f - y.w * y.w);
+    *reinterpret_cast<float4*>(dx + at + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
   }
+  store_split8(hi, lo, tiled(row, c, ld), v);
 }
 
-// dY = 2 (Y - T) / (rows * cols); loss partials per block (fixed order)
-__global__ void mse_grad_kernel(const float* Y, const float* T, float* dY, int rows, int cols, double* partial) {
-  __shared__ double sh[256];
-  const int64_t n = (int64_t)rows * cols;
-  const float sc = 2.0f / (float)n;
-  double acc = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float d = Y[i] - T[i];
-    dY[i] = sc * d;
-    acc += (double)d * d;
+// db[c] = sum_r dZ[r][c], rows in order: 256 threads bring 128 rows of 32 columns at a time into
+// shared memory (the next ones are on their way meanwhile), one warp adds them up.  (One thread
+// per column reading 64 rows ahead from global memory took 34 us for 1024 x 4096.)
+__global__ void __launch_bounds__(256) colsum_kernel(const float* dz, float* db, int rows, int ld) {
+  __shared__ float sh[2][128][33];
+  const int c = threadIdx.x & 31, r = threadIdx.x >> 5, col = blockIdx.x * 32 + c;
+  float v[16], s = 0.0f;
+  auto fetch = [&](int r0) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = r0 + r + 8 * k < rows ? dz[(int64_t)(r0 + r + 8 * k) * ld + col] : 0.0f;
+  };
+  fetch(0);
+  for (int r0 = 0, b = 0; r0 < rows; r0 += 128, b ^= 1) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) sh[b][r + 8 * k][c] = v[k];
+    __syncthreads();
+    if (r0 + 128 < rows) fetch(r0 + 128);
+    if (r == 0) {
+#pragma unroll 16
+      for (int k = 0; k < 128; ++k) s += sh[b][k][c];  // (the zeros past the last row change nothing)
+    }
   }
-  sh[threadIdx.x] = acc;
+  if (r == 0) db[col] = s;
+}
+
+// loss of a step: the CTAs' partials in a fixed order, over the number of outputs
+__global__ void loss_kernel(const double* part, int count, double inv, double* out) {
+  __shared__ double sh[256];
+  double a = 0.0;
+  for (int i = threadIdx.x; i < count; i += 256) a += part[i];
+  sh[threadIdx.x] = a;
   __syncthreads();
   for (int s = 128; s > 0; s >>= 1) {
     if ((int)threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
     __syncthreads();
   }
-  if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
+  if (threadIdx.x == 0) *out = sh[0] * inv;
 }
 
-// dZ = dY * (1 - y^2) for tanh layers (in place)
-__global__ void tanh_back_kernel(float* dY, const float* Y, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    dY[i] *= 1.0f - Y[i] * Y[i];
-}
-
-// db[c] = sum_r dZ[r][c] (one thread per column, fixed order)
-__global__ void colsum_kernel(const float* dZ, float* db, int rows, int cols) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float s = 0.f;
-  for (int r = 0; r < rows; ++r) s += dZ[(size_t)r * cols + c];
-  db[c] = s;
-}
-
-__global__ void adam_kernel(float* w, const float* g, float* m, float* v, int64_t n, float lr, float b1, float b2,
-                            float eps, float c1, float c2) {
+// FP32 rows (row-major) into bf16 parts
+__global__ void split_kernel(const float* src, int rows, int cols, unsigned char* hi, unsigned char* lo, int ld) {
+  const int64_t n = (int64_t)((rows + kPadTo - 1) / kPadTo * kPadTo) * (ld / 8);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    const int64_t r = i / (ld / 8);
+    const int c = (int)(i - r * (ld / 8)) * 8;
+    float x[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = r < rows && c + k < cols ? src[r * cols + c + k] : 0.0f;
+    store_split8(hi, lo, tiled(r, c, ld), x);
   }
 }
 
-__global__ void to_bf16_kernel(const float* src, __nv_bfloat16* dst, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    dst[i] = __float2bfloat16_rn(src[i]);
+// Parameters of every layer in one launch: Adam on the FP32 masters and the bf16 weights of the
+// next products (ADAM), or the gradients alone in the layout of the parameters.
+constexpr int kMaxLayers = 8;
+struct ParamLayer {
+  float *W, *b, *gW, *gb, *mW, *vW, *mb, *vb;
+  unsigned char* w16;
+  const float *dw, *db;
+  int64_t first;  // this layer's first element of the launch
+  int in, out, ldi;
+};
+struct ParamArgs {
+  ParamLayer l[kMaxLayers];
+  int n;
+  int64_t total;
+  float lr, b1, b2, eps, c1, c2;
+};
+// (the moments' roundings written out: a bias or weight whose gradient is mostly rounding takes a
+// full step all the same, so another contraction of the same sums trains another network)
+__device__ __forceinline__ float adam_step(float w, float g, float* m, float* v, const ParamArgs& a) {
+  const float o1 = 1.f - a.b1, o2 = 1.f - a.b2;
+  const float mi = __fmaf_rn(o1, g, __fmul_rn(a.b1, *m));
+  const float vi = __fmaf_rn(__fmul_rn(o2, g), g, __fmul_rn(a.b2, *v));
+  *m = mi;
+  *v = vi;
+  return __fsub_rn(w, __fmul_rn(a.lr, mi / a.c1) / (sqrtf(vi / a.c2) + a.eps));
+}
+template <bool ADAM>
+__global__ void param_kernel(const __grid_constant__ ParamArgs a) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.total; i += (int64_t)gridDim.x * blockDim.x) {
+    int q = 0;
+    while (q + 1 < a.n && i >= a.l[q + 1].first) ++q;
+    const ParamLayer& L = a.l[q];
+    const int64_t k = i - L.first, nw = (int64_t)L.in * L.out;
+    if (k < nw) {
+      const int o = (int)(k / L.in), c = (int)(k - (int64_t)o * L.in);
+      const float g = L.dw[(int64_t)o * L.ldi + c];
+      if constexpr (ADAM) {
+        const float w = adam_step(L.W[k], g, L.mW + k, L.vW + k, a);
+        L.W[k] = w;
+        *reinterpret_cast<__nv_bfloat16*>(L.w16 + tiled(o, c, L.ldi)) = __float2bfloat16_rn(w);
+      } else {
+        L.gW[k] = g;
+      }
+    } else {
+      const int64_t o = k - nw;
+      const float g = L.db[o];
+      if constexpr (ADAM)
+        L.b[o] = adam_step(L.b[o], g, L.mb + o, L.vb + o, a);
+      else
+        L.gb[o] = g;
+    }
+  }
+}
+
+// bf16 weights of the products from the FP32 masters
+__global__ void weights_kernel(const float* W, int out, int in, unsigned char* w16, int ldi) {
+  const int64_t n = (int64_t)out * in;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int o = (int)(i / in), c = (int)(i - (int64_t)o * in);
+    *reinterpret_cast<__nv_bfloat16*>(w16 + tiled(o, c, ldi)) = __float2bfloat16_rn(W[i]);
+  }
 }
 
 unsigned grid_for(int64_t n) {
@@ -251,37 +455,81 @@ struct DBuf {
 struct Mlp {
   std::vector<int> w;  // widths: input, hidden..., output
   struct Layer {
-    int in, out;
+    int in, out, ldi, ldo;  // widths and their padded sizes
     DBuf<float> W, b, gW, gb, mW, vW, mb, vb;
-    DBuf<__nv_bfloat16> W16;
+    DBuf<unsigned char> w16;  // bf16 weights, tiled [out][in]
+    // per batch capacity
+    DBuf<float> act;                      // hidden layers: FP32 activation [batch][ldo]
+    DBuf<unsigned char> ahi, alo;         // ... and its bf16 parts
+    DBuf<unsigned char> dhi, dlo;         // bf16 parts of dZ [batch][ldo]
+    DBuf<float> dz;                       // dZ in FP32
+    DBuf<float> dw, db;
   };
   std::vector<std::unique_ptr<Layer>> layers;
-  std::vector<DBuf<float>> act, grad;  // per layer output (activations) and its gradient
-  DBuf<float> x, target;
-  DBuf<double> partial;
+  DBuf<float> x, target, y;
+  DBuf<unsigned char> xhi, xlo;
+  DBuf<double> loss_part, losses;
   DBuf<int> err;  // set by a tensor-core product whose bounded wait gave up
-  int cap = 0;
+  int cap = 0, loss_cap = 0;
   int64_t t = 0;  // Adam step
-  cudaStream_t s = nullptr;
+  cudaStream_t s = nullptr, side = nullptr;  // weight gradients run beside the chain of dX
+  cudaEvent_t ready = nullptr, joined = nullptr;
+  Mlp() = default;
+  Mlp(const Mlp&) = delete;
+  void open() {
+    check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
+    check(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking), "stream");
+    check(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming), "event");
+    check(cudaEventCreateWithFlags(&joined, cudaEventDisableTiming), "event");
+  }
+  ~Mlp() {
+    if (s) cudaStreamSynchronize(s);
+    if (side) cudaStreamSynchronize(side);
+    if (ready) cudaEventDestroy(ready);
+    if (joined) cudaEventDestroy(joined);
+    if (s) cudaStreamDestroy(s);
+    if (side) cudaStreamDestroy(side);
+  }
 
   void ensure(int batch) {
     if (batch <= cap) return;
     cap = batch;
+    const size_t bp = (size_t)padded(batch);
     x.alloc((size_t)batch * w[0]);
     target.alloc((size_t)batch * w.back());
-    act.resize(layers.size());
-    grad.resize(layers.size());
+    y.alloc((size_t)batch * w.back());
+    xhi.alloc(2 * bp * padded(w[0]));
+    xlo.alloc(2 * bp * padded(w[0]));
     for (size_t l = 0; l < layers.size(); ++l) {
-      act[l].alloc((size_t)batch * layers[l]->out);
-      grad[l].alloc((size_t)batch * layers[l]->out);
+      Layer& L = *layers[l];
+      const size_t e = bp * L.ldo;
+      if (l + 1 < layers.size()) {
+        L.act.alloc(e);
+        L.ahi.alloc(2 * e);
+        L.alo.alloc(2 * e);
+      }
+      L.dhi.alloc(2 * e);
+      L.dlo.alloc(2 * e);
+      L.dz.alloc(e);
+      L.dw.alloc((size_t)L.ldo * L.ldi);
+      L.db.alloc(L.ldo);
     }
-    partial.alloc(4096);
+    loss_part.alloc((bp / 128) * (layers.back()->ldo / 64));
     if (!err.p) err.alloc(1);
+    check(cudaStreamSynchronize(nullptr), "sync");  // the clears run on the default stream
+  }
+
+  void need_losses(int n) {
+    if (n <= loss_cap) return;
+    losses.alloc(n);
+    check(cudaStreamSynchronize(nullptr), "sync");
+    loss_cap = n;
   }
 
   // a bounded wait inside a tensor-core product gave up: report it (and clear the flag)
   void check_err() {
     int e = 0;
+    check(cudaGetLastError(), "launch");
     check(cudaMemcpyAsync(&e, err.p, sizeof(int), cudaMemcpyDeviceToHost, s), "copy");
     check(cudaStreamSynchronize(s), "sync");
     if (e) {
@@ -293,71 +541,131 @@ struct Mlp {
   void refresh_bf16() {
     for (auto& L : layers) {
       const int64_t n = (int64_t)L->in * L->out;
-      to_bf16_kernel<<<grid_for(n), 256, 0, s>>>(L->W.p, L->W16.p, n);
+      weights_kernel<<<grid_for(n), 256, 0, s>>>(L->W.p, L->out, L->in, L->w16.p, L->ldi);
       count_launch();
     }
   }
 
-  void forward(int batch) {
-    const float* in = x.p;
+  // bf16 parts of the inputs (once per call: they serve every step)
+  void load_inputs(int batch) {
+    split_kernel<<<grid_for((int64_t)padded(batch) * padded(w[0]) / 8), 256, 0, s>>>(x.p, batch, w[0], xhi.p, xlo.p,
+                                                                                     padded(w[0]));
+    count_launch();
+  }
+
+  Operand input_of(size_t l) const {
+    if (l == 0) return {xhi.p, xlo.p, padded(w[0])};
+    return {layers[l - 1]->ahi.p, layers[l - 1]->alo.p, layers[l - 1]->ldo};
+  }
+
+  // train: the output layer's epilogue turns into the loss and its gradient
+  void forward(int batch, bool train) {
+    const int bp = padded(batch);
     for (size_t l = 0; l < layers.size(); ++l) {
       Layer& L = *layers[l];
       // Z[b][o] = sum_i X[b][i] W[o][i]
-      tc_gemm(batch, L.out, L.in, GemmOperand{in, L.in, 1, 0}, GemmOperand{L.W16.p, L.in, 1, 1}, act[l].p, L.out,
-              err.p, s);
-      const int hidden = l + 1 < layers.size();
-      bias_act_kernel<<<grid_for((int64_t)batch * L.out), 256, 0, s>>>(act[l].p, L.b.p, batch, L.out, hidden);
-      count_launch();
-      in = act[l].p;
+      GemmArgs g{};
+      g.a = input_of(l);
+      g.b = Operand{L.w16.p, nullptr, L.ldi};
+      g.chunks = L.ldi / 64;
+      g.rows = batch;
+      g.cols = L.out;
+      g.ldc = L.ldo;
+      g.bias = L.b.p;
+      g.err = err.p;
+      const dim3 grid(L.ldo / 64, bp / 128);
+      if (l + 1 < layers.size()) {
+        g.c = L.act.p;
+        g.hi = L.ahi.p;
+        g.lo = L.alo.p;
+        launch_gemm<false, false, false, EPI_HIDDEN>(grid, g, s);
+      } else if (train) {
+        g.hi = L.dhi.p;
+        g.lo = L.dlo.p;
+        g.target = target.p;
+        g.scale = 2.0f / (float)((int64_t)batch * L.out);
+        g.loss = loss_part.p;
+        g.c = L.dz.p;
+        launch_gemm<false, false, false, EPI_LOSS>(grid, g, s);
+      } else {
+        g.c = y.p;
+        launch_gemm<false, false, false, EPI_OUT>(grid, g, s);
+      }
     }
   }
 
-  double backward(int batch) {
-    const int nl = (int)layers.size();
-    const int64_t nout = (int64_t)batch * w.back();
-    const unsigned gb = std::min<unsigned>(grid_for(nout), 4096);
-    mse_grad_kernel<<<gb, 256, 0, s>>>(act[nl - 1].p, target.p, grad[nl - 1].p, batch, w.back(), partial.p);
-    count_launch();
+  // the step's loss into *out (device), weight and bias gradients into the layers' partials
+  void backward(int batch, double* out) {
+    const int bp = padded(batch), nl = (int)layers.size();
+    const int tiles = (bp / 128) * (layers.back()->ldo / 64);
     for (int l = nl - 1; l >= 0; --l) {
       Layer& L = *layers[l];
-      if (l < nl - 1) {
-        tanh_back_kernel<<<grid_for((int64_t)batch * L.out), 256, 0, s>>>(grad[l].p, act[l].p,
-                                                                          (int64_t)batch * L.out);
+      // dW[o][i] = sum_b dZ[b][o] X[b][i]
+      GemmArgs g{};
+      g.a = Operand{L.dhi.p, L.dlo.p, L.ldo};
+      g.b = input_of(l);
+      g.chunks = bp / 64;
+      g.c = L.dw.p;
+      g.ldc = L.ldi;
+      g.err = err.p;
+      // (beside the chain of the gradient handed down)
+      check(cudaEventRecord(ready, s), "event");
+      check(cudaStreamWaitEvent(side, ready, 0), "event");
+      if (l == nl - 1) {
+        loss_kernel<<<1, 256, 0, side>>>(loss_part.p, tiles, 1.0 / ((double)batch * w.back()), out);
         count_launch();
       }
-      const float* in = l == 0 ? x.p : act[l - 1].p;
-      // dW[o][i] = sum_b dZ[b][o] X[b][i]
-      tc_gemm(L.out, L.in, batch, GemmOperand{grad[l].p, 1, L.out, 0}, GemmOperand{in, 1, L.in, 0}, L.gW.p, L.in,
-              err.p, s);
-      colsum_kernel<<<(L.out + 127) / 128, 128, 0, s>>>(grad[l].p, L.gb.p, batch, L.out);
+      launch_gemm<true, true, true, EPI_RAW>(dim3(L.ldi / 64, L.ldo / 128), g, side);
+      colsum_kernel<<<L.ldo / 32, 256, 0, side>>>(L.dz.p, L.db.p, batch, L.ldo);
       count_launch();
-      if (l > 0) {
-        // dX[b][i] = sum_o dZ[b][o] W[o][i]
-        tc_gemm(batch, L.in, L.out, GemmOperand{grad[l].p, L.out, 1, 0}, GemmOperand{L.W16.p, 1, L.in, 1},
-                grad[l - 1].p, L.in, err.p, s);
-      }
+      if (l == 0) continue;
+      // dX[b][i] = sum_o dZ[b][o] W[o][i], then the layer below's dZ
+      GemmArgs d{};
+      d.a = Operand{L.dhi.p, L.dlo.p, L.ldo};
+      d.b = Operand{L.w16.p, nullptr, L.ldi};
+      d.chunks = L.ldo / 64;
+      Layer& D = *layers[l - 1];
+      d.c = D.dz.p;
+      d.ldc = L.ldi;
+      d.err = err.p;
+      launch_gemm<false, true, false, EPI_RAW>(dim3(L.ldi / 64, bp / 128), d, s);
+      tanh_back_kernel<<<dim3(bp / 32, D.ldo / 64), 256, 0, s>>>(D.dz.p, D.act.p, D.dhi.p, D.dlo.p, D.ldo);
+      count_launch();
     }
-    std::vector<double> h(gb);
-    check(cudaMemcpyAsync(h.data(), partial.p, gb * sizeof(double), cudaMemcpyDeviceToHost, s), "copy");
-    check(cudaStreamSynchronize(s), "sync");
-    check_err();
-    double loss = 0.0;
-    for (double v : h) loss += v;
-    return loss / (double)nout;
+    check(cudaEventRecord(joined, side), "event");
+    check(cudaStreamWaitEvent(s, joined, 0), "event");
   }
 
-  void adam(float lr) {
-    ++t;
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    const float c1 = 1.f - std::pow(b1, (float)t), c2 = 1.f - std::pow(b2, (float)t);
-    for (auto& L : layers) {
-      const int64_t nw = (int64_t)L->in * L->out;
-      adam_kernel<<<grid_for(nw), 256, 0, s>>>(L->W.p, L->gW.p, L->mW.p, L->vW.p, nw, lr, b1, b2, eps, c1, c2);
-      adam_kernel<<<grid_for(L->out), 256, 0, s>>>(L->b.p, L->gb.p, L->mb.p, L->vb.p, L->out, lr, b1, b2, eps, c1,
-                                                   c2);
-      count_launch(2);
+  // the parameter kernel over every layer (kMaxLayers to a launch)
+  template <bool ADAM>
+  void params(int batch, ParamArgs a) {
+    const int nl = (int)layers.size();
+    for (int first = 0; first < nl; first += kMaxLayers) {
+      a.n = std::min(kMaxLayers, nl - first);
+      a.total = 0;
+      for (int q = 0; q < a.n; ++q) {
+        Layer& L = *layers[first + q];
+        a.l[q] = ParamLayer{L.W.p, L.b.p, L.gW.p, L.gb.p, L.mW.p, L.vW.p, L.mb.p, L.vb.p, L.w16.p, L.dw.p, L.db.p,
+                            a.total, L.in, L.out, L.ldi};
+        a.total += (int64_t)L.in * L.out + L.out;
+      }
+      param_kernel<ADAM><<<grid_for(a.total), 256, 0, s>>>(a);
+      count_launch();
     }
-    refresh_bf16();
+  }
+
+  void gradients(int batch) { params<false>(batch, ParamArgs{}); }
+
+  void adam(int batch, float lr) {
+    ++t;
+    ParamArgs a{};
+    a.lr = lr;
+    a.b1 = 0.9f;
+    a.b2 = 0.999f;
+    a.eps = 1e-8f;
+    a.c1 = 1.f - std::pow(a.b1, (float)t);
+    a.c2 = 1.f - std::pow(a.b2, (float)t);
+    params<true>(batch, a);
   }
 };
 
@@ -395,6 +703,7 @@ int so_mlp_new(const int* widths, size_t count, uint64_t seed, so_mlp* out) {
   return mlp_guard([&] {
     auto h = std::make_unique<so_mlp_t>();
     so::Mlp& m = h->m;
+    m.open();
     m.w.assign(widths, widths + count);
     std::mt19937_64 rng(seed);
     for (size_t l = 0; l + 1 < count; ++l) {
@@ -404,13 +713,17 @@ int so_mlp_new(const int* widths, size_t count, uint64_t seed, so_mlp* out) {
       const size_t nw = (size_t)L->in * L->out;
       for (auto* b : {&L->W, &L->gW, &L->mW, &L->vW}) b->alloc(nw);
       for (auto* b : {&L->b, &L->gb, &L->mb, &L->vb}) b->alloc(L->out);
-      L->W16.alloc(nw);
+      L->ldi = so::padded(L->in);
+      L->ldo = so::padded(L->out);
+      L->w16.alloc(2 * (size_t)L->ldi * L->ldo);  // zeros in the padding
+      so::check(cudaStreamSynchronize(nullptr), "sync");  // the clears run on the default stream
       // Glorot-uniform weights, zero biases
       std::uniform_real_distribution<float> u(-1.f, 1.f);
       const float lim = std::sqrt(6.f / (float)(L->in + L->out));
       std::vector<float> w(nw);
       for (float& v : w) v = lim * u(rng);
-      so::check(cudaMemcpy(L->W.p, w.data(), nw * sizeof(float), cudaMemcpyHostToDevice), "copy");
+      so::check(cudaMemcpyAsync(L->W.p, w.data(), nw * sizeof(float), cudaMemcpyHostToDevice, m.s), "copy");
+      so::check(cudaStreamSynchronize(m.s), "sync");  // (w goes out of scope)
       m.layers.push_back(std::move(L));
     }
     m.refresh_bf16();
@@ -444,9 +757,9 @@ int so_mlp_set_params(so_mlp h, const float* in) {
     size_t off = 0;
     for (auto& L : h->m.layers) {
       const size_t nw = (size_t)L->in * L->out;
-      so::check(cudaMemcpy(L->W.p, in + off, nw * 4, cudaMemcpyHostToDevice), "copy");
+      so::check(cudaMemcpyAsync(L->W.p, in + off, nw * 4, cudaMemcpyHostToDevice, h->m.s), "copy");
       off += nw;
-      so::check(cudaMemcpy(L->b.p, in + off, L->out * 4, cudaMemcpyHostToDevice), "copy");
+      so::check(cudaMemcpyAsync(L->b.p, in + off, L->out * 4, cudaMemcpyHostToDevice, h->m.s), "copy");
       off += L->out;
     }
     h->m.refresh_bf16();
@@ -459,10 +772,11 @@ int so_mlp_forward(so_mlp h, const float* x, size_t batch, float* y) {
   return mlp_guard([&] {
     so::Mlp& m = h->m;
     m.ensure((int)batch);
-    so::check(cudaMemcpy(m.x.p, x, batch * m.w[0] * 4, cudaMemcpyHostToDevice), "copy");
-    m.forward((int)batch);
+    so::check(cudaMemcpyAsync(m.x.p, x, batch * m.w[0] * 4, cudaMemcpyHostToDevice, m.s), "copy");
+    m.load_inputs((int)batch);
+    m.forward((int)batch, false);
     m.check_err();
-    so::check(cudaMemcpy(y, m.act.back().p, batch * m.w.back() * 4, cudaMemcpyDeviceToHost), "copy");
+    so::check(cudaMemcpy(y, m.y.p, batch * m.w.back() * 4, cudaMemcpyDeviceToHost), "copy");
   });
 }
 
@@ -471,10 +785,15 @@ int so_mlp_gradients(so_mlp h, const float* x, const float* target, size_t batch
   return mlp_guard([&] {
     so::Mlp& m = h->m;
     m.ensure((int)batch);
-    so::check(cudaMemcpy(m.x.p, x, batch * m.w[0] * 4, cudaMemcpyHostToDevice), "copy");
-    so::check(cudaMemcpy(m.target.p, target, batch * m.w.back() * 4, cudaMemcpyHostToDevice), "copy");
-    m.forward((int)batch);
-    *loss = m.backward((int)batch);
+    so::check(cudaMemcpyAsync(m.x.p, x, batch * m.w[0] * 4, cudaMemcpyHostToDevice, m.s), "copy");
+    so::check(cudaMemcpyAsync(m.target.p, target, batch * m.w.back() * 4, cudaMemcpyHostToDevice, m.s), "copy");
+    m.load_inputs((int)batch);
+    m.need_losses(1);
+    m.forward((int)batch, true);
+    m.backward((int)batch, m.losses.p);
+    m.gradients((int)batch);
+    so::check(cudaMemcpyAsync(loss, m.losses.p, sizeof(double), cudaMemcpyDeviceToHost, m.s), "copy");
+    m.check_err();
     size_t off = 0;
     for (auto& L : m.layers) {
       const size_t nw = (size_t)L->in * L->out;
@@ -492,15 +811,23 @@ int so_mlp_train(so_mlp h, const float* x, const float* target, size_t batch, si
   return mlp_guard([&] {
     so::Mlp& m = h->m;
     m.ensure((int)batch);
-    so::check(cudaMemcpy(m.x.p, x, batch * m.w[0] * 4, cudaMemcpyHostToDevice), "copy");
-    so::check(cudaMemcpy(m.target.p, target, batch * m.w.back() * 4, cudaMemcpyHostToDevice), "copy");
-    for (size_t i = 0; i < steps; ++i) {
-      m.forward((int)batch);
-      const double l = m.backward((int)batch);
-      if (losses) losses[i] = l;
-      m.adam(lr);
+    so::check(cudaMemcpyAsync(m.x.p, x, batch * m.w[0] * 4, cudaMemcpyHostToDevice, m.s), "copy");
+    so::check(cudaMemcpyAsync(m.target.p, target, batch * m.w.back() * 4, cudaMemcpyHostToDevice, m.s), "copy");
+    m.load_inputs((int)batch);
+    // the losses stay on the device until a run of steps is queued: no step waits for the host
+    constexpr size_t kRun = 1024;
+    m.need_losses((int)std::min(steps, kRun));
+    for (size_t i = 0; i < steps; i += kRun) {
+      const size_t n = std::min(steps - i, kRun);
+      for (size_t k = 0; k < n; ++k) {
+        m.forward((int)batch, true);
+        m.backward((int)batch, m.losses.p + k);
+        m.adam((int)batch, lr);
+      }
+      if (losses)
+        so::check(cudaMemcpyAsync(losses + i, m.losses.p, n * sizeof(double), cudaMemcpyDeviceToHost, m.s), "copy");
+      m.check_err();
     }
-    so::check(cudaDeviceSynchronize(), "sync");
   });
 }
 
