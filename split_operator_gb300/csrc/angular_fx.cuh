@@ -25,7 +25,7 @@
 //               NB neighbouring complex columns in every phase
 //   warp 16     streams the A digit images (8 KB per 128 rows x 32 K values) through a 64 KB
 //               ring by bulk TMA copies
-//   warp 17     issues tcgen05.mma kind::f16
+//   warp 17     issues tcgen05.mma kind::f16 (48 clocks a product: the reads of both operands)
 // B digits lie N-major in shared memory (eight real columns of one K row are 16 bytes), so a
 // thread writes its four complex columns of a digit with one 16-byte store.
 // Every mbarrier wait is bounded (2 s), as in angular_tc.cu.
@@ -265,8 +265,9 @@ __device__ __noinline__ void fx_producer(FxResolve resolve, int64_t total, uint3
   }
 }
 
-// Warp 17, lane 0: per matrix, once its B digits are written, the products of A digit i (chunk by
-// chunk) with the B digits j <= 6 - i into accumulator i + j.
+// Warp 17: per matrix, once its B digits are written, the products of A digit i (chunk by chunk)
+// with the B digits j <= 6 - i into accumulator i + j.  The warp stays converged and its elected
+// lane issues (elect_one).
 template <int N, int MH>
 __device__ __noinline__ void fx_issuer(FxResolve resolve, int64_t total, uint32_t ring, uint32_t b0, uint64_t* full,
                                        uint64_t* empty, uint64_t* dbar, uint64_t* bready, uint64_t* quiet,
@@ -276,6 +277,7 @@ __device__ __noinline__ void fx_issuer(FxResolve resolve, int64_t total, uint32_
   constexpr int ns = (int)(kRingBytes / bytes);
   constexpr uint32_t idesc = idesc_f16_nmajor(128, N);
   const uint64_t abits = smem_desc_bits(128, 512);
+  const uint32_t el = elect_one();
   int s = 0;
   uint32_t phase = 0, nready = 0;
   bool ok = true;
@@ -288,42 +290,39 @@ __device__ __noinline__ void fx_issuer(FxResolve resolve, int64_t total, uint32_
     const uint64_t bfirst = smem_desc_at(bbits, b0), bdig = (uint64_t)((2 * N * kp) >> 4);
     const int nmat = r.prm->nmat;
     for (int m = 0; m < nmat && ok; ++m) {
-      ok = mbar_poll(bready, nready & 1u, kFxWait);
+      ok = __all_sync(0xffffffffu, mbar_poll(bready, nready & 1u, kFxWait));
       ++nready;
       tc_fence_after();
-      for (int i = 0; i < kDigits && ok; ++i) {
+#pragma unroll
+      for (int i = 0; i < kDigits; ++i) {
         uint64_t bk = bfirst;
-        for (int q = 0; q < nk; ++q) {
-          ok = mbar_poll(&full[s], phase, kFxWait);
+        for (int q = 0; q < nk && ok; ++q) {
+          ok = __all_sync(0xffffffffu, mbar_poll(&full[s], phase, kFxWait));
           if (!ok) break;
           tc_fence_after();
-          uint64_t a = smem_desc_at(abits, ring + (uint32_t)s * bytes);
+          const uint64_t a = smem_desc_at(abits, ring + (uint32_t)s * bytes);
 #pragma unroll
-          for (int ks = 0; ks < 2; ++ks) {
-            for (int h = 0; h < MH; ++h) {
-              uint32_t d = tmem + (uint32_t)(i * MH * N + h * N);
-              uint64_t b = bk;
-              const uint32_t acc = (i | q | ks) != 0 ? 1u : 0u;
-              for (int j = 0; j < kDigits - i; ++j) {
-                mma_bf16(d, a + (uint64_t)(h * (kChunkRowBytes >> 4)), b, idesc, acc);  // types: idesc
-                d += MH * N;
-                b += bdig;
-              }
-            }
-            bk += 256 >> 4;
-            a += 256 >> 4;
-          }
-          mma_commit(&empty[s]);
+          for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+            for (int h = 0; h < MH; ++h)
+#pragma unroll
+              for (int j = 0; j < kDigits - i; ++j)
+                mma_f16_warp(tmem + (uint32_t)((i + j) * MH * N + h * N),
+                             a + (uint64_t)(ks * (256 >> 4) + h * (kChunkRowBytes >> 4)),
+                             bk + (uint64_t)(ks * (256 >> 4)) + (uint64_t)j * bdig, idesc,
+                             (i | ks) != 0 || q != 0 ? 1u : 0u, el);
+          bk += 512 >> 4;
+          if (el) mma_commit(&empty[s]);
           if (++s == ns) {
             s = 0;
             phase ^= 1u;
           }
         }
       }
-      if (ok) mma_commit(dbar);
+      if (ok && el) mma_commit(dbar);
     }
   }
-  if (!ok) {
+  if (!ok && el) {
     *fail = 1;
     // every MMA already issued completes before the tensor memory is released
     mma_commit(quiet);
@@ -514,8 +513,7 @@ __global__ void __launch_bounds__(kFxThreads, 1)
   if (warp == kFxWork / 32) {
     if (lane == 0) fx_producer<MH>(resolve, total, ring, full, empty, &s_fail);
   } else if (warp == kFxWork / 32 + 1) {
-    if (lane == 0)
-      fx_issuer<N, MH>(resolve, total, ring, ring + kRingBytes, full, empty, dbar, bready, quiet, tmem, &s_fail);
+    fx_issuer<N, MH>(resolve, total, ring, ring + kRingBytes, full, empty, dbar, bready, quiet, tmem, &s_fail);
   } else {
     const int quad = warp & 3, grp = warp >> 2;
     Work W;

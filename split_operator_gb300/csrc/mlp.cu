@@ -34,7 +34,10 @@ namespace {
 // K-major (rows = M or N, columns = K) and, transposed by the tensor core, as MN-major
 // operand (rows = K), so activations, gradients and weights are stored once and read by every
 // product they enter, by bulk TMA copies of whole blocks, half blocks or row groups.
-// Rows and columns are padded to multiples of 128 with zeros.
+// Rows and columns are padded to multiples of 128 with zeros.  The gradients dZ use blocks of 128
+// columns (32 KB, sixteen core matrices to a row group): both of their products then read
+// contiguous pieces of 16 KB and more (copies of one row group, 1 KB each, held a weight
+// gradient of 64 K values x 128 x 64 at 1.4 us a chunk).
 constexpr int kPadTo = 128;
 constexpr uint32_t kBlockBytes = 16384, kGroupBytes = 1024;  // 128 x 64 block; 8 rows x 64 columns
 
@@ -44,6 +47,12 @@ int padded(int n) { return (n + kPadTo - 1) / kPadTo * kPadTo; }
 __host__ __device__ __forceinline__ size_t tiled(int64_t r, int c, int cols) {
   return ((size_t)(r >> 7) * (size_t)(cols >> 6) + (size_t)(c >> 6)) * kBlockBytes + (size_t)((r & 127) >> 3) * kGroupBytes +
          (size_t)((c & 63) >> 3) * 128 + (size_t)(r & 7) * 16 + (size_t)(c & 7) * 2;
+}
+
+__host__ __device__ __forceinline__ size_t tiled_dz(int64_t r, int c, int cols) {
+  return ((size_t)(r >> 7) * (size_t)(cols >> 7) + (size_t)(c >> 7)) * (2 * kBlockBytes) +
+         (size_t)((r & 127) >> 3) * (2 * kGroupBytes) + (size_t)((c & 127) >> 3) * 128 + (size_t)(r & 7) * 16 +
+         (size_t)(c & 7) * 2;
 }
 
 // eight consecutive columns of one row as bf16 hi and lo parts (c a multiple of 8)
@@ -66,8 +75,11 @@ struct Operand {
   int cols;                      // padded columns
 };
 
-// ---- tensor-core product C[m][n] = sum_k A(m, k) B(n, k) on tiles of 128 x 64, K in chunks of 64
-// AMN / BMN: the operand's rows are K (MN-major) instead of M / N.  Warp 4 streams the chunks
+// ---- tensor-core product C[m][n] = sum_k A(m, k) B(n, k) on tiles of 128 x 64
+// FORM 0, forward: A = activations, B = weights, both K-major, K in chunks of 64.
+// FORM 1, dX: A = dZ, K-major; B = weights, MN-major (rows = K); K in chunks of 128.
+// FORM 2, dW: A = dZ and B = activations (split), both MN-major; K (rows) in chunks of 64.
+// Warp 4 streams the chunks
 // through shared-memory stages by bulk copies, warp 5 issues hi hi + lo hi (+ hi lo when B
 // is split; the lo lo term is 2^-16 of the result) per K step of 16 into one FP32 accumulator
 // (K is not split over CTAs: the tensor core truncates as it accumulates, so the order of the
@@ -84,7 +96,7 @@ enum Epilogue {
 };
 struct GemmArgs {
   Operand a, b;
-  int chunks;            // K / 64
+  int chunks;            // K / 64 (dX: K / 128)
   float* c;              // EPI_RAW: product; EPI_HIDDEN: activation; EPI_LOSS: gradient; EPI_OUT: output
   int rows, cols;        // valid extent of C (EPI_LOSS, EPI_OUT, EPI_HIDDEN)
   int ldc;               // padded columns of C
@@ -98,19 +110,20 @@ struct GemmArgs {
 constexpr uint64_t kGWait = 2000000000ull;  // 2 s
 constexpr int kGThreads = 192;
 
-// Shared-memory stages: two (and two CTAs per SM) where K is short and there are many tiles; the
-// products of the backward pass have few tiles and a long K, and hide a chunk's latency behind
-// the chunks after it (dX of the 4096-wide layer, 32 tiles of 64 chunks).
-__host__ __device__ constexpr int gemm_stages(bool bsplit, int epi) { return epi != EPI_RAW ? 2 : (bsplit ? 4 : 5); }
-__host__ __device__ constexpr uint32_t gemm_stage_bytes(bool bsplit) {
-  return 2 * kBlockBytes + (bsplit ? 2u : 1u) * (kBlockBytes / 2);
+// Shared-memory stages: two (and two CTAs per SM) in the forward products, where K is short and
+// there are many tiles; dW has few tiles and hides a chunk's latency behind the chunks after it.
+__host__ __device__ constexpr int gemm_stages(int form) { return form == 2 ? 4 : 2; }
+__host__ __device__ constexpr uint32_t gemm_a_bytes(int form) { return form == 1 ? 2 * kBlockBytes : kBlockBytes; }
+__host__ __device__ constexpr uint32_t gemm_b_bytes(int form) { return form == 1 ? kBlockBytes : kBlockBytes / 2; }
+__host__ __device__ constexpr uint32_t gemm_stage_bytes(int form) {  // A hi, A lo, B (hi, lo in dW)
+  return 2 * gemm_a_bytes(form) + (form == 2 ? 2u : 1u) * gemm_b_bytes(form);
 }
 
-template <bool AMN, bool BMN, bool BSPLIT, int EPI>
-__global__ void __launch_bounds__(kGThreads, EPI == EPI_RAW ? 1 : 2) gemm_kernel(const __grid_constant__ GemmArgs g) {
+template <int FORM, int EPI>
+__global__ void __launch_bounds__(kGThreads, FORM == 0 ? 2 : 1) gemm_kernel(const __grid_constant__ GemmArgs g) {
   using namespace tc;
-  constexpr uint32_t kB = BSPLIT ? 2 : 1, kStage = gemm_stage_bytes(BSPLIT);
-  constexpr int kNs = gemm_stages(BSPLIT, EPI);
+  constexpr uint32_t kA = gemm_a_bytes(FORM), kBb = gemm_b_bytes(FORM), kStage = gemm_stage_bytes(FORM);
+  constexpr int kNs = gemm_stages(FORM), kB = FORM == 2 ? 2 : 1, kSteps = FORM == 1 ? 8 : 4;
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t full[kNs], empty[kNs], done;
   __shared__ uint32_t tmem_s;
@@ -133,7 +146,6 @@ __global__ void __launch_bounds__(kGThreads, EPI == EPI_RAW ? 1 : 2) gemm_kernel
   const uint32_t tmem = tmem_s;
   bool ok = true;
   if (warp == 4) {
-    // the whole warp issues a chunk's copies: up to 32 row groups of A, the tiles of B
     int c = 0;
     for (; c < c1 && ok; ++c) {
       const int s = c % kNs, use = c / kNs;
@@ -143,55 +155,52 @@ __global__ void __launch_bounds__(kGThreads, EPI == EPI_RAW ? 1 : 2) gemm_kernel
       unsigned char* st = sm + (uint32_t)s * kStage;
       if (lane == 0) mbar_expect_tx(&full[s], kStage);
       __syncwarp();
-      if constexpr (!AMN) {
-        if (lane < 2)
-          bulk_g2s(st + (uint32_t)lane * kBlockBytes,
-                   (lane ? g.a.lo : g.a.hi) + ((size_t)mt * (g.a.cols >> 6) + c) * kBlockBytes, kBlockBytes, &full[s]);
-      } else {
-        // 64 rows (K) of two column blocks (M = 128), row group by row group side by side
-        const int q = lane >> 4, r = (lane >> 1) & 7, blk = lane & 1;
-        const unsigned char* src = (q ? g.a.lo : g.a.hi) +
-                                   ((size_t)(c >> 1) * (g.a.cols >> 6) + 2 * mt + blk) * kBlockBytes +
-                                   (size_t)((c & 1) * 8 + r) * kGroupBytes;
-        bulk_g2s(st + (uint32_t)q * kBlockBytes + r * 2048 + blk * 1024, src, kGroupBytes, &full[s]);
-      }
-      if (lane < (int)kB) {
-        const unsigned char* src = lane ? g.b.lo : g.b.hi;
-        const size_t blk = BMN ? (size_t)(c >> 1) * (g.b.cols >> 6) + nt : (size_t)(nt >> 1) * (g.b.cols >> 6) + c;
-        bulk_g2s(st + 2 * kBlockBytes + (uint32_t)lane * (kBlockBytes / 2),
-                 src + blk * kBlockBytes + (size_t)((BMN ? c : nt) & 1) * (kBlockBytes / 2), kBlockBytes / 2, &full[s]);
+      if (lane < 2) {
+        const unsigned char* src = lane ? g.a.lo : g.a.hi;
+        // FORM 0: block (mt, c); 1: 128-wide block (mt, c); 2: half of the 128-wide block (c / 2, mt)
+        const size_t at = FORM == 0 ? ((size_t)mt * (g.a.cols >> 6) + c) * kBlockBytes
+                          : FORM == 1 ? ((size_t)mt * (g.a.cols >> 7) + c) * (2 * kBlockBytes)
+                                      : ((size_t)(c >> 1) * (g.a.cols >> 7) + mt) * (2 * kBlockBytes) +
+                                            (size_t)(c & 1) * kBlockBytes;
+        bulk_g2s(st + (uint32_t)lane * kA, src + at, kA, &full[s]);
+      } else if (lane < 2 + kB) {
+        const int q = lane - 2;
+        const unsigned char* src = q ? g.b.lo : g.b.hi;
+        // FORM 0: half of block (nt / 2, c); 1: block (c, nt); 2: half of block (c / 2, nt)
+        const size_t at = FORM == 0 ? ((size_t)(nt >> 1) * (g.b.cols >> 6) + c) * kBlockBytes + (size_t)(nt & 1) * kBb
+                          : FORM == 1 ? ((size_t)c * (g.b.cols >> 6) + nt) * kBlockBytes
+                                      : ((size_t)(c >> 1) * (g.b.cols >> 6) + nt) * kBlockBytes + (size_t)(c & 1) * kBb;
+        bulk_g2s(st + 2 * kA + (uint32_t)q * kBb, src + at, kBb, &full[s]);
       }
     }
     if (!ok && lane == 0)  // let the copies in flight land before the CTA lets go of its shared memory
       for (int k = c < kNs ? 0 : c - kNs; k < c; ++k) mbar_poll(&full[k % kNs], (k / kNs) & 1u, kGWait);
   } else if (warp == 5) {
-    if (lane == 0) {
-      const uint32_t base = smem_u32(sm);
-      constexpr uint32_t idesc = idesc_bf16(128, 64) | (AMN ? 1u << 15 : 0u) | (BMN ? 1u << 16 : 0u);
-      // (K-group stride, M/N-group stride) of each form, and the step of 16 K values
-      const uint64_t abits = AMN ? smem_desc_bits(2048, 128) : smem_desc_bits(128, 1024);
-      const uint64_t bbits = BMN ? smem_desc_bits(1024, 128) : smem_desc_bits(128, 1024);
-      constexpr uint32_t astep = AMN ? 4096 : 256, bstep = BMN ? 2048 : 256;
-      for (int c = 0; c < c1 && ok; ++c) {
-        const int s = c % kNs, use = c / kNs;
-        ok = mbar_poll(&full[s], use & 1u, kGWait);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t st = base + (uint32_t)s * kStage;
+    const uint32_t base = smem_u32(sm), el = elect_one();
+    constexpr uint32_t idesc = idesc_bf16(128, 64) | (FORM == 2 ? 1u << 15 : 0u) | (FORM != 0 ? 1u << 16 : 0u);
+    // (K-group stride, M/N-group stride) of each form, and the step of 16 K values
+    const uint64_t abits = FORM == 0 ? smem_desc_bits(128, 1024) : (FORM == 1 ? smem_desc_bits(128, 2048)
+                                                                                : smem_desc_bits(2048, 128));
+    const uint64_t bbits = FORM == 0 ? smem_desc_bits(128, 1024) : smem_desc_bits(1024, 128);
+    constexpr uint32_t astep = FORM == 2 ? 4096 : 256, bstep = FORM == 0 ? 256 : 2048;
+    for (int c = 0; c < c1 && ok; ++c) {
+      const int s = c % kNs, use = c / kNs;
+      ok = __all_sync(0xffffffffu, mbar_poll(&full[s], use & 1u, kGWait));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t st = base + (uint32_t)s * kStage;
+      const uint64_t ah = smem_desc_at(abits, st), bh = smem_desc_at(bbits, st + 2 * kA);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint64_t ah = smem_desc_at(abits, st + k * astep), al = smem_desc_at(abits, st + kBlockBytes + k * astep);
-          const uint64_t bh = smem_desc_at(bbits, st + 2 * kBlockBytes + k * bstep);
-          mma_bf16(tmem, ah, bh, idesc, c > 0 || k > 0 ? 1u : 0u);
-          mma_bf16(tmem, al, bh, idesc, 1u);
-          if constexpr (BSPLIT)
-            mma_bf16(tmem, ah, smem_desc_at(bbits, st + 2 * kBlockBytes + kBlockBytes / 2 + k * bstep), idesc, 1u);
-        }
-        mma_commit(&empty[s]);
+      for (int k = 0; k < kSteps; ++k) {
+        const uint64_t ak = ah + (uint64_t)((k * astep) >> 4), bk = bh + (uint64_t)((k * bstep) >> 4);
+        mma_f16_warp(tmem, ak, bk, idesc, c > 0 || k > 0 ? 1u : 0u, el);
+        mma_f16_warp(tmem, ak + (kA >> 4), bk, idesc, 1u, el);
+        if constexpr (FORM == 2) mma_f16_warp(tmem, ak, bk + (kBb >> 4), idesc, 1u, el);
       }
-      mma_commit(&done);  // (after a failed wait: everything issued so far)
-      if (!ok) mbar_poll(&done, 0u, kGWait);
+      if (el) mma_commit(&empty[s]);
     }
+    if (el) mma_commit(&done);  // (after a failed wait: everything issued so far)
+    if (!ok) mbar_poll(&done, 0u, kGWait);
   } else {
     ok = mbar_wait(&done, 0u, kGWait);
     tc_fence_after();
@@ -261,7 +270,7 @@ __global__ void __launch_bounds__(kGThreads, EPI == EPI_RAW ? 1 : 2) gemm_kernel
         float* dst = g.c + row * g.ldc + n0 + k;
         *reinterpret_cast<float4*>(dst) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
         *reinterpret_cast<float4*>(dst + 4) = make_float4(v[k + 4], v[k + 5], v[k + 6], v[k + 7]);
-        store_split8(g.hi, g.lo, tiled(row, n0 + k, g.ldc), v + k);
+        store_split8(g.hi, g.lo, tiled_dz(row, n0 + k, g.ldc), v + k);
       }
       double l = (double)s + (double)e;
 #pragma unroll
@@ -277,11 +286,11 @@ __global__ void __launch_bounds__(kGThreads, EPI == EPI_RAW ? 1 : 2) gemm_kernel
   if (warp == 0) tmem_dealloc(tmem, 64);
 }
 
-template <bool AMN, bool BMN, bool BSPLIT, int EPI>
+template <int FORM, int EPI>
 void launch_gemm(dim3 grid, const GemmArgs& g, cudaStream_t s) {
-  constexpr size_t smem = (size_t)gemm_stages(BSPLIT, EPI) * gemm_stage_bytes(BSPLIT);
+  constexpr size_t smem = (size_t)gemm_stages(FORM) * gemm_stage_bytes(FORM);
   static bool done = false;
-  auto kern = gemm_kernel<AMN, BMN, BSPLIT, EPI>;
+  auto kern = gemm_kernel<FORM, EPI>;
   if (!done) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     done = true;
@@ -307,7 +316,7 @@ __global__ void __launch_bounds__(256) tanh_back_kernel(float* dx, const float* 
     v[k + 3] = q.w * (1.0f - y.w * y.w);
     *reinterpret_cast<float4*>(dx + at + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
   }
-  store_split8(hi, lo, tiled(row, c, ld), v);
+  store_split8(hi, lo, tiled_dz(row, c, ld), v);
 }
 
 // db[c] = sum_r dZ[r][c], rows in order: 256 threads bring 128 rows of 32 columns at a time into
@@ -472,8 +481,9 @@ struct Mlp {
   DBuf<int> err;  // set by a tensor-core product whose bounded wait gave up
   int cap = 0, loss_cap = 0;
   int64_t t = 0;  // Adam step
-  cudaStream_t s = nullptr, side = nullptr;  // weight gradients run beside the chain of dX
-  cudaEvent_t ready = nullptr, joined = nullptr;
+  // weight gradients and bias gradients run beside the chain of dX
+  cudaStream_t s = nullptr, side = nullptr, side2 = nullptr;
+  cudaEvent_t ready = nullptr, joined = nullptr, joined2 = nullptr;
   Mlp() = default;
   Mlp(const Mlp&) = delete;
   void open() {
@@ -481,14 +491,17 @@ struct Mlp {
     check(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking), "stream");
     check(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming), "event");
     check(cudaEventCreateWithFlags(&joined, cudaEventDisableTiming), "event");
+    check(cudaStreamCreateWithFlags(&side2, cudaStreamNonBlocking), "stream");
+    check(cudaEventCreateWithFlags(&joined2, cudaEventDisableTiming), "event");
   }
   ~Mlp() {
-    if (s) cudaStreamSynchronize(s);
-    if (side) cudaStreamSynchronize(side);
-    if (ready) cudaEventDestroy(ready);
-    if (joined) cudaEventDestroy(joined);
-    if (s) cudaStreamDestroy(s);
-    if (side) cudaStreamDestroy(side);
+    for (cudaStream_t q : {s, side, side2})
+      if (q) {
+        cudaStreamSynchronize(q);
+        cudaStreamDestroy(q);
+      }
+    for (cudaEvent_t e : {ready, joined, joined2})
+      if (e) cudaEventDestroy(e);
   }
 
   void ensure(int batch) {
@@ -578,7 +591,7 @@ struct Mlp {
         g.c = L.act.p;
         g.hi = L.ahi.p;
         g.lo = L.alo.p;
-        launch_gemm<false, false, false, EPI_HIDDEN>(grid, g, s);
+        launch_gemm<0, EPI_HIDDEN>(grid, g, s);
       } else if (train) {
         g.hi = L.dhi.p;
         g.lo = L.dlo.p;
@@ -586,10 +599,10 @@ struct Mlp {
         g.scale = 2.0f / (float)((int64_t)batch * L.out);
         g.loss = loss_part.p;
         g.c = L.dz.p;
-        launch_gemm<false, false, false, EPI_LOSS>(grid, g, s);
+        launch_gemm<0, EPI_LOSS>(grid, g, s);
       } else {
         g.c = y.p;
-        launch_gemm<false, false, false, EPI_OUT>(grid, g, s);
+        launch_gemm<0, EPI_OUT>(grid, g, s);
       }
     }
   }
@@ -611,29 +624,32 @@ struct Mlp {
       // (beside the chain of the gradient handed down)
       check(cudaEventRecord(ready, s), "event");
       check(cudaStreamWaitEvent(side, ready, 0), "event");
+      check(cudaStreamWaitEvent(side2, ready, 0), "event");
       if (l == nl - 1) {
-        loss_kernel<<<1, 256, 0, side>>>(loss_part.p, tiles, 1.0 / ((double)batch * w.back()), out);
+        loss_kernel<<<1, 256, 0, side2>>>(loss_part.p, tiles, 1.0 / ((double)batch * w.back()), out);
         count_launch();
       }
-      launch_gemm<true, true, true, EPI_RAW>(dim3(L.ldi / 64, L.ldo / 128), g, side);
-      colsum_kernel<<<L.ldo / 32, 256, 0, side>>>(L.dz.p, L.db.p, batch, L.ldo);
+      launch_gemm<2, EPI_RAW>(dim3(L.ldi / 64, L.ldo / 128), g, side);
+      colsum_kernel<<<L.ldo / 32, 256, 0, side2>>>(L.dz.p, L.db.p, batch, L.ldo);
       count_launch();
       if (l == 0) continue;
       // dX[b][i] = sum_o dZ[b][o] W[o][i], then the layer below's dZ
       GemmArgs d{};
       d.a = Operand{L.dhi.p, L.dlo.p, L.ldo};
       d.b = Operand{L.w16.p, nullptr, L.ldi};
-      d.chunks = L.ldo / 64;
+      d.chunks = L.ldo / 128;
       Layer& D = *layers[l - 1];
       d.c = D.dz.p;
       d.ldc = L.ldi;
       d.err = err.p;
-      launch_gemm<false, true, false, EPI_RAW>(dim3(L.ldi / 64, bp / 128), d, s);
+      launch_gemm<1, EPI_RAW>(dim3(L.ldi / 64, bp / 128), d, s);
       tanh_back_kernel<<<dim3(bp / 32, D.ldo / 64), 256, 0, s>>>(D.dz.p, D.act.p, D.dhi.p, D.dlo.p, D.ldo);
       count_launch();
     }
     check(cudaEventRecord(joined, side), "event");
     check(cudaStreamWaitEvent(s, joined, 0), "event");
+    check(cudaEventRecord(joined2, side2), "event");
+    check(cudaStreamWaitEvent(s, joined2, 0), "event");
   }
 
   // the parameter kernel over every layer (kMaxLayers to a launch)
