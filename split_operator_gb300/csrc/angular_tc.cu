@@ -23,7 +23,7 @@
 //              store, and fold the norms (named barrier 1 among themselves)
 //   warp 8     streams the A chunks (one MMA K step each) of every tile, in order,
 //              through 2-6 shared-memory stages by bulk TMA (it runs ahead across tiles)
-//   warp 9     issues tcgen05.mma (one lane) as chunks land and the B operand is ready
+//   warp 9     issues tcgen05.mma (its elected lane) as chunks land and the B operand is ready
 // The tensor core truncates its FP32 accumulation, so the A_hi B_hi products go to
 // three TMEM regions a couple of K steps each and the work warps drain the
 // regions into registers (round-to-nearest adds) every kFillSteps K steps; the
@@ -1020,7 +1020,8 @@ __device__ __noinline__ void tma_producer(Resolve resolve, int64_t total, const 
   }
 }
 
-// Warp 9, lane 0: for each tile and matrix (once its B operand is written) and each
+// Warp 9 (converged, its elected lane issues: elect_one): for each tile and matrix (once its B
+// operand is written) and each
 // fill, the K steps of the fill -- step t puts A_hi B_hi into main region
 // (t - t0) nused / span and both corrections into the correction region -- then a
 // commit of the fill to dbar.  Each chunk's MMAs are committed to its stage's empty
@@ -1048,18 +1049,20 @@ __device__ __noinline__ void mma_issuer(Resolve resolve, int64_t total, const Tc
   uint64_t ahi = 0;               // A_hi descriptor of the current K step (a chunk may span two fills)
   uint32_t nready = 0, nfree = 0;
   bool ok = true;
+  const uint32_t el = elect_one();
+  const auto all = [](bool v) { return __all_sync(0xffffffffu, v); };
   for (int64_t gt = blockIdx.x; gt < total && ok; gt += gridDim.x) {
     const TileRef tr = resolve(gt);
     const int nmat = tr.prm->nmat;
     unsigned long long* trace = tr.prm->trace ? tr.prm->trace + tr.tile * kTraceSlots : nullptr;
     const int64_t cc_tile = cc;  // first chunk of this tile
     for (int m = 0; m < nmat && ok; ++m) {
-      ok = mbar_poll(bready, nready & 1u, kWaitLimit);
+      ok = all(mbar_poll(bready, nready & 1u, kWaitLimit));
       ++nready;
       tc_fence_after();
       for (int f = 0; f < S.fills && ok; ++f) {
         if (f > 0) {
-          ok = mbar_poll(freebar, nfree & 1u, kWaitLimit);
+          ok = all(mbar_poll(freebar, nfree & 1u, kWaitLimit));
           ++nfree;
           tc_fence_after();
           if (!ok) break;
@@ -1078,9 +1081,9 @@ __device__ __noinline__ void mma_issuer(Resolve resolve, int64_t total, const Tc
         for (int t = fs.t0; t < fs.t1; ++t) {
           const int ks = t & (kpc - 1);  // kpc is 1 or 2
           if (ks == 0) {
-            ok = mbar_poll(&full[s], fphase, kWaitLimit);
+            ok = all(mbar_poll(&full[s], fphase, kWaitLimit));
             if (!ok) break;
-            if (trace && (int)(cc - cc_tile) < 8) trace[TR_FULL + (int)(cc - cc_tile)] = globaltimer_ns();
+            if (trace && el && (int)(cc - cc_tile) < 8) trace[TR_FULL + (int)(cc - cc_tile)] = globaltimer_ns();
             tc_fence_after();
             ahi = smem_desc_at(abits, sm0 + L.stage0 + (uint32_t)s * stage_bytes);
           }
@@ -1090,13 +1093,13 @@ __device__ __noinline__ void mma_issuer(Resolve resolve, int64_t total, const Tc
             const uint64_t ah = ahi + (uint64_t)(hh * S.a_half16);
             const uint64_t bo = (uint64_t)hh * bstep_half;  // parity split: each half its own B
             if constexpr (BF) {
-              mma_bf16(dm0 + (uint32_t)(hh * S.nc), ah, bh + bo, idesc, first_main);
-              mma_bf16(dc0 + (uint32_t)(hh * S.nc), ah, bl + bo, idesc, first_corr);
-              mma_bf16(dc0 + (uint32_t)(hh * S.nc), ah + (uint64_t)(S.chunk_bytes >> 4), bh + bo, idesc, 1u);
+              mma_f16_warp(dm0 + (uint32_t)(hh * S.nc), ah, bh + bo, idesc, first_main, el);
+              mma_f16_warp(dc0 + (uint32_t)(hh * S.nc), ah, bl + bo, idesc, first_corr, el);
+              mma_f16_warp(dc0 + (uint32_t)(hh * S.nc), ah + (uint64_t)(S.chunk_bytes >> 4), bh + bo, idesc, 1u, el);
             } else {
-              mma_tf32(dm0 + (uint32_t)(hh * S.nc), ah, bh + bo, idesc, first_main);
-              mma_tf32(dc0 + (uint32_t)(hh * S.nc), ah, bl + bo, idesc, first_corr);
-              mma_tf32(dc0 + (uint32_t)(hh * S.nc), ah + (uint64_t)(S.chunk_bytes >> 4), bh + bo, idesc, 1u);
+              mma_tf32_warp(dm0 + (uint32_t)(hh * S.nc), ah, bh + bo, idesc, first_main, el);
+              mma_tf32_warp(dc0 + (uint32_t)(hh * S.nc), ah, bl + bo, idesc, first_corr, el);
+              mma_tf32_warp(dc0 + (uint32_t)(hh * S.nc), ah + (uint64_t)(S.chunk_bytes >> 4), bh + bo, idesc, 1u, el);
             }
           }
           bh += (uint64_t)(2 * kLboB >> 4);
@@ -1110,8 +1113,8 @@ __device__ __noinline__ void mma_issuer(Resolve resolve, int64_t total, const Tc
             dm0 = tmem + (uint32_t)(rm * S.reg_cols);
           }
           if (ks == kpc - 1) {
-            mma_commit(&empty[s]);
-            if (trace && (int)(cc - cc_tile) < 8) trace[TR_MMA + (int)(cc - cc_tile)] = globaltimer_ns();
+            if (el) mma_commit(&empty[s]);
+            if (trace && el && (int)(cc - cc_tile) < 8) trace[TR_MMA + (int)(cc - cc_tile)] = globaltimer_ns();
             ++cc;
             if (++s == ns) {
               s = 0;
@@ -1119,11 +1122,11 @@ __device__ __noinline__ void mma_issuer(Resolve resolve, int64_t total, const Tc
             }
           }
         }
-        if (ok) mma_commit(dbar);
+        if (ok && el) mma_commit(dbar);
       }
     }
   }
-  if (!ok) {
+  if (!ok && el) {
     *fail = 1;
     // every MMA already issued completes before the tensor memory is released
     mma_commit(quiet);
@@ -1131,10 +1134,8 @@ __device__ __noinline__ void mma_issuer(Resolve resolve, int64_t total, const Tc
   }
 }
 
-// Warp 9, lane 0, split-BF16x6: the same schedule as mma_issuer with its invariants in
-// registers and the loops over the K steps of a chunk and the M halves unrolled (MH = 1:
-// chunks of two K steps; MH = 2: one), so the lane spends its time issuing products rather
-// than recomputing descriptors (a probe measured the product issue itself at ~51 cycles).
+// Warp 9, split-BF16x6: the same schedule as mma_issuer with the loops over the K steps of a
+// chunk and the M halves unrolled (MH = 1: chunks of two K steps; MH = 2: one).
 template <int MH, typename Resolve>
 __device__ __noinline__ void mma_issuer_oz(Resolve resolve, int64_t total, const TcShape S, uint32_t sm0,
                                            const TcSmemLayout L, uint32_t tmem, volatile int* fail) {
@@ -1160,20 +1161,22 @@ __device__ __noinline__ void mma_issuer_oz(Resolve resolve, int64_t total, const
   int s = 0;
   uint32_t fphase = 0, nready = 0;
   bool ok = true;
+  const uint32_t el = elect_one();
+  const auto all = [](bool v) { return __all_sync(0xffffffffu, v); };
   for (int64_t gt = blockIdx.x; gt < total && ok; gt += gridDim.x) {
     const TileRef tr = resolve(gt);
     const int nmat = tr.prm->nmat;
     unsigned long long* trace = tr.prm->trace ? tr.prm->trace + tr.tile * kTraceSlots : nullptr;
     const int64_t cc_tile = cc;
     for (int m = 0; m < nmat && ok; ++m) {
-      ok = mbar_poll(bready, nready & 1u, kWaitLimit);
+      ok = all(mbar_poll(bready, nready & 1u, kWaitLimit));
       ++nready;
       tc_fence_after();
       uint64_t bh = b0, bm = b1, bl = b2;
       for (int t = 0; t < ksteps && ok; t += KPC) {
-        ok = mbar_poll(&full[s], fphase, kWaitLimit);
+        ok = all(mbar_poll(&full[s], fphase, kWaitLimit));
         if (!ok) break;
-        if (trace && (int)(cc - cc_tile) < 8) trace[TR_FULL + (int)(cc - cc_tile)] = globaltimer_ns();
+        if (trace && el && (int)(cc - cc_tile) < 8) trace[TR_FULL + (int)(cc - cc_tile)] = globaltimer_ns();
         tc_fence_after();
         uint64_t a = a_first + (uint64_t)s * a_stage;
 #pragma unroll
@@ -1183,30 +1186,30 @@ __device__ __noinline__ void mma_issuer_oz(Resolve resolve, int64_t total, const
           for (int hh = 0; hh < MH; ++hh) {
             const uint64_t a0 = a + (uint64_t)hh * ahalf, bo = (uint64_t)hh * bhalf;
             const uint32_t r0 = tmem + (uint32_t)hh * nch;
-            mma_bf16(r0, a0, bh + bo, idesc, acc);
-            mma_bf16(r0 + rc, a0, bm + bo, idesc, acc);
-            mma_bf16(r0 + rc, a0 + slice, bh + bo, idesc, 1u);
-            mma_bf16(r0 + 2u * rc, a0, bl + bo, idesc, acc);
-            mma_bf16(r0 + 2u * rc, a0 + slice, bm + bo, idesc, 1u);
-            mma_bf16(r0 + 2u * rc, a0 + 2u * slice, bh + bo, idesc, 1u);
+            mma_f16_warp(r0, a0, bh + bo, idesc, acc, el);
+            mma_f16_warp(r0 + rc, a0, bm + bo, idesc, acc, el);
+            mma_f16_warp(r0 + rc, a0 + slice, bh + bo, idesc, 1u, el);
+            mma_f16_warp(r0 + 2u * rc, a0, bl + bo, idesc, acc, el);
+            mma_f16_warp(r0 + 2u * rc, a0 + slice, bm + bo, idesc, 1u, el);
+            mma_f16_warp(r0 + 2u * rc, a0 + 2u * slice, bh + bo, idesc, 1u, el);
           }
           bh += kBStep;
           bm += kBStep;
           bl += kBStep;
           a += kAStep;
         }
-        mma_commit(&empty[s]);
-        if (trace && (int)(cc - cc_tile) < 8) trace[TR_MMA + (int)(cc - cc_tile)] = globaltimer_ns();
+        if (el) mma_commit(&empty[s]);
+        if (trace && el && (int)(cc - cc_tile) < 8) trace[TR_MMA + (int)(cc - cc_tile)] = globaltimer_ns();
         ++cc;
         if (++s == ns) {
           s = 0;
           fphase ^= 1u;
         }
       }
-      if (ok) mma_commit(dbar);
+      if (ok && el) mma_commit(dbar);
     }
   }
-  if (!ok) {
+  if (!ok && el) {
     *fail = 1;
     // every MMA already issued completes before the tensor memory is released
     mma_commit(quiet);
@@ -1322,15 +1325,13 @@ __device__ __forceinline__ void tc_persistent(Resolve resolve, const int64_t tot
   if (warp == kWorkThreads / 32) {
     if (lane == 0) tma_producer(resolve, total, S, sm0, L, &s_fail);
   } else if (warp == kWorkThreads / 32 + 1) {
-    if (lane == 0) {
-      if constexpr (OZ) {
-        if (S.mh == 2)
-          mma_issuer_oz<2>(resolve, total, S, sm0, L, tmem, &s_fail);
-        else
-          mma_issuer_oz<1>(resolve, total, S, sm0, L, tmem, &s_fail);
-      } else {
-        mma_issuer<BF>(resolve, total, S, sm0, L, tmem, &s_fail);
-      }
+    if constexpr (OZ) {
+      if (S.mh == 2)
+        mma_issuer_oz<2>(resolve, total, S, sm0, L, tmem, &s_fail);
+      else
+        mma_issuer_oz<1>(resolve, total, S, sm0, L, tmem, &s_fail);
+    } else {
+      mma_issuer<BF>(resolve, total, S, sm0, L, tmem, &s_fail);
     }
   } else {
     // ================= work warps
