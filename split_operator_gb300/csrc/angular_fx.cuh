@@ -32,6 +32,7 @@
 #pragma once
 #include "common.cuh"
 #include "fx.cuh"
+#include "pass_end.cuh"
 #include "tc_common.cuh"
 
 namespace so {
@@ -60,10 +61,12 @@ constexpr uint32_t kChunkRowBytes = 8192;    // 128 rows x 32 K values of one di
 constexpr uint64_t kFxWait = 2000000000ull;  // 2 s per wait
 constexpr int kFxTabSlots = 4;               // DIAG1D ops on a non-lane axis per pass
 constexpr int kFxMaxCols = 32;
+constexpr int kNoTerm = 1 << 20;             // exponent of a zero weight: below every other
+constexpr int kFxPoison = 1 << 24;           // exponent of a column with a value that is not finite
 
 __host__ __device__ constexpr uint32_t fx_b_bytes(int cols, int kp) { return (uint32_t)(2 * cols * kp * 2); }
 __host__ __device__ constexpr uint32_t fx_tc_smem(int cols, int kp) {
-  return kRingBytes + kDigits * fx_b_bytes(cols, kp) + kMaxRed * kFxWork * 8;
+  return kRingBytes + kDigits * fx_b_bytes(cols, kp);
 }
 
 __device__ __forceinline__ void fx_work_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kFxWork) : "memory"); }
@@ -156,7 +159,9 @@ __device__ __forceinline__ double scale_pow2(double d, int k) {
 
 struct FxTabs {
   int4 colt[kFxTabSlots][kFxMaxCols];   // DIAG1D on a non-lane axis: its factor per tile column
-  double colw[kMaxRed][kFxMaxCols];     // NORM: product of the weights of every non-lane axis
+  // NORM: product of the weights of every non-lane axis, as a RowWeight's digits and exponent
+  int2 colwd[kMaxRed][kFxMaxCols];
+  int colwx[kMaxRed][kFxMaxCols];
   int scale_x[kMaxOps];                 // SCALE: factor = digits x 2^scale_x
   int2 scale_d[kMaxOps];
   int colx[kFxMaxCols];                 // exponent of the column's values (before row exponents)
@@ -165,6 +170,7 @@ struct FxTabs {
   int colb[kFxMaxCols];                 // exponent bound of the column's B operand
   int nonident[kFxTabSlots];            // the factors of this tile are not all 1
   int8_t slot[kMaxOps];
+  double red[kMaxRed][kFxWork / 32];    // norms: the warps' sums
 };
 
 __device__ __forceinline__ int64_t fx_coord(const Geometry& g, int a, int64_t o, int64_t i) {
@@ -179,25 +185,6 @@ __device__ __forceinline__ int64_t fx_coord(const Geometry& g, int a, int64_t o,
     v /= g.sshape[q];
   }
   return 0;
-}
-
-__device__ void fx_run_scalar(const PassParams& p, const DevOp& op, const double* totals) {
-  double* s = p.slots;
-  switch (op.kind) {
-    case OP_NORM: {
-      const double v = totals[op.red];
-      s[op.a] = v;
-      if (!isfinite(v) && p.nonfinite_slot >= 0) s[p.nonfinite_slot] = 1.0;
-      break;
-    }
-    case OP_COPY: s[op.a] = s[op.b]; break;
-    case OP_LOSS: s[op.a] += s[op.b] - s[op.c]; break;
-    case OP_SETC: s[op.a] = op.value; break;
-    case OP_RECORD:
-      if (p.record) p.record[op.count] = s[op.a];
-      break;
-    default: break;
-  }
 }
 
 // image block of matrix m for a tile (a state matrix: the one of the tile's coordinate)
@@ -330,6 +317,24 @@ __device__ __noinline__ void fx_issuer(FxResolve resolve, int64_t total, uint32_
   }
 }
 
+// a b 2^-64 (b: digits), rounded
+__device__ __forceinline__ i64 mulhi64(dig a, int2 b) {
+  return mw(a.h, b.y, mw(a.h, b.x, mw(a.l, b.y, 1ll << 31)) >> 32);
+}
+
+// w = m 2^x, m in [1/2, 1): digits {l, h} of m 2^62; x is kFxPoison if w is not finite
+struct RowWeight {
+  int2 d;
+  int x;
+  __device__ __forceinline__ void set(double w) {
+    int e = 0;
+    const double m = frexp(w, &e);
+    const dig q = split(isfinite(w) ? (i64)(m * 4611686018427387904.0) : 0);
+    d = {q.l, q.h};
+    x = isfinite(w) ? (w != 0.0 ? e : -kNoTerm) : kFxPoison;
+  }
+};
+
 // The work threads' view of a tile: row j, complex columns c0 .. c0 + NB - 1.
 template <int NB, bool FF>
 struct FxWork {
@@ -338,9 +343,11 @@ struct FxWork {
   int xs;      // exponent from SCALE ops, of the whole tile
   int j, c0, ncols;
   bool row_ok;
+  const double* roww_ptr;  // lane-axis weights of the pass's first norm, and this row's
+  RowWeight roww;
 
   // point-wise ops [ob, oe)
-  __device__ __forceinline__ void apply(const PassParams& p, FxTabs& T, int ob, int oe, int64_t ix0, double* acc) {
+  __device__ __forceinline__ void apply(const PassParams& p, FxTabs& T, int ob, int oe, int64_t ix0) {
     const Geometry& g = p.g;
     for (int oi = ob; oi < oe; ++oi) {
       const DevOp& op = p.ops[oi];
@@ -375,25 +382,47 @@ struct FxWork {
           break;
         }
         case OP_NORM: {
-          // squares of the values moved up to 61 bits, in units of 2^64
+          // Squares of the values moved up to 61 bits, in units of 2^64, times the column weights
+          // (digits of m 2^62 and an exponent) over the largest column factor of the thread, times
+          // the row's weight; the warp's sum over its largest row factor.  In integers throughout:
+          // the FP64 pipe takes 1.7 operations a clock, so weights and sums in FP64 (three
+          // operations a point, and their fold) took 5 us of a 32 x 128 tile.
           unsigned long long m = 0;
+          int top = -kPoison;
 #pragma unroll
-          for (int u = 0; u < NB; ++u)
+          for (int u = 0; u < NB; ++u) {
             m |= (unsigned long long)(w[u].x ^ (w[u].x >> 63)) | (unsigned long long)(w[u].y ^ (w[u].y >> 63));
+            top = max(top, T.colwx[op.red][c0 + u] + 2 * T.colx[c0 + u]);
+          }
           const int lz = __clzll((i64)m), s = lz > 3 ? (lz < 60 ? lz - 3 : 57) : 0;
-          double sum = 0.0;
+          i64 sum = 0;
 #pragma unroll
           for (int u = 0; u < NB; ++u) {
             const dig a = split(w[u].x << s), b = split(w[u].y << s);
             const i64 q = mw(a.h, a.h, (mw(a.h, a.l, 1ll << 30)) >> 31) + mw(b.h, b.h, (mw(b.h, b.l, 1ll << 30)) >> 31);
-            const int x = T.colx[c0 + u];
-            const double v = x == kPoison ? __longlong_as_double(0x7ff8000000000000ll)
-                                          : scale_pow2((double)q * T.colw[op.red][c0 + u], 2 * x);
-            sum += c0 + u < ncols ? v : 0.0;
+            const int2 cw = T.colwd[op.red][c0 + u];
+            sum += mulhi64(split(q << 2), cw) >> min(top - (T.colwx[op.red][c0 + u] + 2 * T.colx[c0 + u]), 63);
           }
-          if (row_ok)
-            acc[op.red * kFxWork + threadIdx.x] +=
-                scale_pow2(sum, 64 + 2 * (rowx + xs - s)) * __ldg(op.w[g.sweep_axis] + j);
+          RowWeight rw = roww;
+          if (op.w[g.sweep_axis] != roww_ptr) rw.set(row_ok ? __ldg(op.w[g.sweep_axis] + j) : 0.0);
+          const bool bad = row_ok && max(top, rw.x) >= kPoison / 2;
+          int e = -kPoison;  // the row's term is sum 2^e, |sum| < 2^60
+          if (row_ok && sum != 0) {
+            const int up = __clzll(sum ^ (sum >> 63)) - 2;  // |sum| <= 2^62
+            sum = up >= 0 ? sum << up : sum >> 1;
+            sum = mulhi64(split(sum), rw.d);
+            if (sum != 0) e = 66 + 2 * (rowx + xs - s) + top + rw.x - max(up, -1);
+          } else {
+            sum = 0;
+          }
+          const int et = __reduce_max_sync(0xffffffffu, e);
+          const bool any_bad = __any_sync(0xffffffffu, bad);
+          i64 t = ((sum >> min(et - e, 60)) + 4) >> 3;  // 32 of them stay below 2^63
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+          if ((threadIdx.x & 31) == 0)
+            T.red[op.red][threadIdx.x >> 5] =
+                any_bad ? __longlong_as_double(0x7ff8000000000000ll) : scale_pow2((double)t, et + 3);
           break;
         }
         case OP_ROUND: {
@@ -434,7 +463,7 @@ struct FxWork {
       }
     }
   }
-  static constexpr int kPoison = 1 << 24;  // colx of a column with a value that is not finite
+  static constexpr int kPoison = kFxPoison;
 
   // B digits of the values, K row j: v = value 2^(55 - colb) as seven digits
   __device__ __forceinline__ void write_operand(const FxTabs& T, unsigned char* B, int kp, uint32_t bbytes) {
@@ -486,7 +515,7 @@ __global__ void __launch_bounds__(kFxThreads, 1)
   __shared__ __align__(16) FxTabs T;
   __shared__ __align__(8) uint64_t bars[2 * 8 + 3];
   __shared__ uint32_t tmem_s;
-  __shared__ double totals[kMaxRed];
+  __shared__ double s_red[kMaxRed];
   __shared__ volatile int s_fail;
   __shared__ int s_bad;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -537,7 +566,6 @@ __global__ void __launch_bounds__(kFxThreads, 1)
       const uint32_t bbytes = fx_b_bytes(BN, kp);
       // products are drained with 2^-sh of their last bit: |product| <= 2^61
       const int sh = kp <= 32 ? 6 : (kp <= 64 ? 7 : (kp <= 128 ? 8 : 9));
-      double* acc = reinterpret_cast<double*>(sm + kRingBytes + kDigits * bbytes);
       const int64_t o = r.tile / g.tiles_per_outer;
       const int64_t i0 = (r.tile - o * g.tiles_per_outer) * BN;
       const int64_t left = g.inner - i0;
@@ -556,6 +584,10 @@ __global__ void __launch_bounds__(kFxThreads, 1)
         const longlong2 x = ok ? psi[u] : longlong2{0, 0};
         raw[u] = {x.x, x.y};
       }
+      W.roww_ptr = nullptr;
+      for (int oi = 0; oi < p.nops && W.roww_ptr == nullptr; ++oi)
+        if (p.ops[oi].kind == OP_NORM) W.roww_ptr = p.ops[oi].w[g.sweep_axis];
+      W.roww.set(W.roww_ptr && W.row_ok ? __ldg(W.roww_ptr + W.j) : 0.0);
       // per-tile tables
       if (tid < 2 * kFxMaxCols) T.cole[tid >> 5][tid & 31] = 0;
       if (tid < kFxTabSlots) T.nonident[tid] = 0;
@@ -576,7 +608,6 @@ __global__ void __launch_bounds__(kFxThreads, 1)
           if (!isfinite(f)) s_bad = 1;  // the whole tile becomes NaN
         }
       }
-      for (int k = 0; k < p.nred; ++k) acc[k * kFxWork + tid] = 0.0;
       fx_work_sync();
       for (int idx = tid; idx < p.nops * BN; idx += kFxWork) {
         const int oi = idx / BN, c = idx - oi * BN;
@@ -586,7 +617,10 @@ __global__ void __launch_bounds__(kFxThreads, 1)
           double wt = 1.0;
           for (int a = 0; a < g.ndim; ++a)
             if (a != g.sweep_axis) wt *= __ldg(op.w[a] + fx_coord(g, a, o, i));
-          T.colw[op.red][c] = wt;
+          RowWeight cw;
+          cw.set(wt);
+          T.colwd[op.red][c] = cw.d;
+          T.colwx[op.red][c] = cw.x;
         } else if (op.kind == OP_DIAG1D && op.axis != g.sweep_axis) {
           const int4 t = __ldg(reinterpret_cast<const int4*>(op.ptr) + fx_coord(g, op.axis, o, i));
           T.colt[T.slot[oi]][c] = t;
@@ -657,7 +691,7 @@ __global__ void __launch_bounds__(kFxThreads, 1)
         }
         const int ob = m < 0 ? 0 : tp.mat_op[m] + 1;
         const int oe = m + 1 < tp.nmat ? tp.mat_op[m + 1] : p.nops;
-        W.apply(p, T, ob, oe, ix0, acc);
+        W.apply(p, T, ob, oe, ix0);
         if (m + 1 < tp.nmat) {
           if (m >= 0 || oe > 0) {
             // the operand's column maxima
@@ -685,6 +719,31 @@ __global__ void __launch_bounds__(kFxThreads, 1)
         if (tid == 0) s_fail = 1;
         break;
       }
+      // norm partials and the pass ticket, drawn by warp 0 while the other warps store (a fence
+      // behind the stores would wait for them)
+      fx_work_sync();
+      if (warp < p.nred) {
+        double a = lane < kFxWork / 32 ? T.red[warp][lane] : 0.0;
+#pragma unroll
+        for (int o2 = kFxWork / 64; o2 > 0; o2 >>= 1) a += __shfl_down_sync(0xffffffffu, a, o2);
+        if (lane == 0) s_red[warp] = a;
+      }
+      fx_work_sync();
+      if (warp == 0) {
+        unsigned int last = 0;
+        EndOp end;
+        end.load(p);
+        if (lane == 0) {
+          for (int k = 0; k < p.nred; ++k) p.partials[(int64_t)k * g.tiles + r.tile] = s_red[k];
+          __threadfence();
+          last = atomicAdd(p.counter, 1u) == (unsigned int)(g.tiles - 1) ? 1u : 0u;
+        }
+        last = __shfl_sync(0xffffffffu, last, 0);
+        if (last) {
+          __threadfence();
+          finish_pass(p, end, p.partials, g.tiles);
+        }
+      }
       // store
 #pragma unroll
       for (int u = 0; u < NB; ++u) {
@@ -694,44 +753,6 @@ __global__ void __launch_bounds__(kFxThreads, 1)
         longlong2 v{fx_to_raw<FF>(W.w[u].x, e), fx_to_raw<FF>(W.w[u].y, e)};
         if (x == Work::kPoison) v = {raw_nan<FF>(), raw_nan<FF>()};
         psi[u] = v;
-      }
-      // norm partials and the pass ticket
-      fx_work_sync();
-      if (warp < p.nred) {
-        double a = 0.0;
-#pragma unroll
-        for (int k = 0; k < kFxWork / 32; ++k) a += acc[warp * kFxWork + lane + 32 * k];
-#pragma unroll
-        for (int o2 = 16; o2 > 0; o2 >>= 1) a += __shfl_down_sync(0xffffffffu, a, o2);
-        if (lane == 0) {
-          p.partials[(int64_t)warp * g.tiles + r.tile] = a;
-          __threadfence();
-        }
-      }
-      fx_work_sync();
-      if (warp == 0) {
-        unsigned int last = 0;
-        if (lane == 0) {
-          __threadfence();
-          last = atomicAdd(p.counter, 1u) == (unsigned int)(g.tiles - 1) ? 1u : 0u;
-        }
-        last = __shfl_sync(0xffffffffu, last, 0);
-        if (last) {
-          __threadfence();
-          for (int k = 0; k < p.nred; ++k) {
-            double a = 0.0;
-            for (int64_t b = lane; b < g.tiles; b += 32) a += __ldcg(p.partials + (int64_t)k * g.tiles + b);
-#pragma unroll
-            for (int o2 = 16; o2 > 0; o2 >>= 1) a += __shfl_down_sync(0xffffffffu, a, o2);
-            if (lane == 0) totals[k] = a;
-          }
-          __syncwarp();
-          if (lane == 0) {
-            for (int oi = 0; oi < p.nops; ++oi) fx_run_scalar(p, p.ops[oi], totals);
-            __threadfence();
-            *p.counter = 0u;
-          }
-        }
       }
       if (tid == 0) s_bad = 0;
       fx_work_sync();  // the tables and the pass copy are free for the next tile

@@ -36,6 +36,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "pass_end.cuh"
 #include "tc_common.cuh"
 
 namespace so {
@@ -895,25 +896,6 @@ __device__ __forceinline__ void stage_row(const float2 (&x)[NV], int c0, int j, 
         make_float4(x[u].x, x[u].y, x[u + 1].x, x[u + 1].y);
 }
 
-__device__ void run_scalar_tc(const PassParams& p, const DevOp& op, const double* totals) {
-  double* s = p.slots;
-  switch (op.kind) {
-    case OP_NORM: {
-      const double v = totals[op.red];
-      s[op.a] = v;
-      if (!isfinite(v) && p.nonfinite_slot >= 0) s[p.nonfinite_slot] = 1.0;
-      break;
-    }
-    case OP_COPY: s[op.a] = s[op.b]; break;
-    case OP_LOSS: s[op.a] += s[op.b] - s[op.c]; break;
-    case OP_SETC: s[op.a] = op.value; break;
-    case OP_RECORD:
-      if (p.record) p.record[op.count] = s[op.a];
-      break;
-    default: break;
-  }
-}
-
 }  // namespace
 
 struct TcParams {
@@ -1236,13 +1218,15 @@ struct PendTicket {
 
 // Warp 0 (all lanes): publish the pending partials; the CTA that draws a pass's last ticket
 // folds all of the pass's partials in FP64 in a fixed order and runs its scalar ops.
-__device__ __noinline__ void publish_pending(PendTicket& pd, double* totals, int lane) {
+__device__ __noinline__ void publish_pending(PendTicket& pd, int lane) {
   const TcParams* q = pd.prm;
   if (q == nullptr) return;
   double* const part = pd.partials;
   const int64_t tiles = pd.tiles;
   const int nred = pd.nred;
   unsigned int last = 0u;
+  EndOp end;
+  end.load(q->p);
   if (lane == 0) {
     for (int k = 0; k < nred; ++k) part[(int64_t)k * tiles + pd.tile] = pd.red[k];
     __threadfence();
@@ -1253,21 +1237,7 @@ __device__ __noinline__ void publish_pending(PendTicket& pd, double* totals, int
   if (lane == 0) pd.prm = nullptr;
   if (!last) return;
   __threadfence();
-  for (int k = 0; k < nred; ++k) {
-    double a = 0.0;
-    for (int64_t b = lane; b < tiles; b += 32) a += __ldcg(part + (int64_t)k * tiles + b);
-#pragma unroll
-    for (int o2 = 16; o2 > 0; o2 >>= 1) a += __shfl_down_sync(0xffffffffu, a, o2);
-    if (lane == 0) totals[k] = a;
-  }
-  __syncwarp();
-  if (lane == 0) {
-    const PassParams& p = q->p;
-    for (int oi = 0; oi < p.nops; ++oi) run_scalar_tc(p, p.ops[oi], totals);
-    __threadfence();
-    *p.counter = 0u;
-  }
-  __syncwarp();
+  finish_pass(q->p, end, part, tiles);
 }
 
 template <bool BF, bool OZ, int PK, typename Resolve>
@@ -1279,7 +1249,6 @@ __device__ __forceinline__ void tc_persistent(Resolve resolve, const int64_t tot
   __shared__ uint32_t tmem_base_s;
   __shared__ FF scratch[kMaxRed * (kWorkThreads / 32)];
   __shared__ double blk_red[kMaxRed];
-  __shared__ double totals[kMaxRed];
   __shared__ PendTicket s_pend;
   __shared__ volatile int s_fail;
   // split-BF16x6: column maxima of the two B operands of a tile (re and im of each column; a
@@ -1441,7 +1410,7 @@ __device__ __forceinline__ void tc_persistent(Resolve resolve, const int64_t tot
       }
 
       // the previous tile's partials and ticket, while this tile's first GEMM runs
-      if (warp == 0) publish_pending(s_pend, totals, lane);
+      if (warp == 0) publish_pending(s_pend, lane);
 
       bool ok = true;
       for (int m = 0; m < tp.nmat && ok; ++m) {
@@ -1649,7 +1618,7 @@ __device__ __forceinline__ void tc_persistent(Resolve resolve, const int64_t tot
     }
     // the last tile's partials (a CTA that stopped on a failed wait publishes nothing: the
     // pass has recorded its error)
-    if (warp == 0 && !s_fail) publish_pending(s_pend, totals, lane);
+    if (warp == 0 && !s_fail) publish_pending(s_pend, lane);
   }
   __syncthreads();
   if (tid == 0 && s_fail) {

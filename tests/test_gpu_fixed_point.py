@@ -186,6 +186,44 @@ def test_lane_matrices_match_long_double(so, precision, n, nr):
     assert err.max() < MAT_TOL[precision], err.max()
 
 
+# Every term of a norm is within a few 2^-55 of the largest of its warp's, a partial sum is rounded to
+# FP64 once per warp, tile and pass: 2^-50 of the sum of magnitudes holds all of it (float-float:
+# the mask is a table of 2^-48)
+@pytest.mark.parametrize("precision,tol", [("fp64", 2.0 ** -50), ("float_float", 2.0 ** -45)])
+@pytest.mark.parametrize("n,nr", [(16, 8), (33, 4100), (64, 31), (128, 33), (200, 130)])
+def test_norms_of_lane_matrix_passes(so, precision, tol, n, nr):
+    rng = np.random.default_rng(7 * n + nr)
+    t, tinv = _legendre(n)
+    # magnitudes from 1e-6 to 1e6 in both axes, weights of either sign and of zero
+    a = (rng.standard_normal((n, nr)) + 1j * rng.standard_normal((n, nr))) * 10.0 ** rng.uniform(-6, 6, (1, nr))
+    a = (a * 10.0 ** rng.uniform(-6, 6, (n, 1))).astype(np.complex64).astype(np.complex128)
+    wp, wr = rng.standard_normal(n), rng.uniform(0.5, 2.0, nr) * 10.0 ** rng.uniform(-3, 3, nr)
+    wp[n // 2] = 0.0
+    wr[nr // 3] = 0.0
+    pg = so.Grid.new_custom("p", np.arange(n, dtype=float), wp, 0)
+    rg = so.Grid.new_custom("r", np.arange(nr, dtype=float), wr, 1)
+    mask = rng.uniform(0.0, 1.0, nr)
+    mask[0] = 1.0
+    border = so.BorderDumping(mask.astype(np.complex128), rg)
+    border.add_loss_checker("border")
+    st = so.OperationStack()
+    st.add_control(border, so.FIRST_HALF)
+    mt = so.MatrixTransformation(pg, so.Grid.new_linear_countable("l", 0.0, n - 1.0, n, 0))
+    mt.set_diagonalization_matrix(t, tinv)
+    st.add_transformation(mt, so.NORMAL)
+    pd = so.NDimPropagator()
+    pd.set_operator(np.exp(1j * rng.uniform(0.0, 6.0, (n, nr))))
+    st.add_propagator(pd)
+    p = so.Propagation(so.WaveFunction(a, [pg, rg]), so.TimeGrid(0.01, 100), st, precision)
+    p.set_timing(True)
+    p.steps(1)
+    assert "tcfx" in " ".join(k[0] for k in p.kernel_times())
+    w = wp.astype(np.longdouble)[:, None] * wr.astype(np.longdouble)[None, :]
+    terms = w * (a.real.astype(np.longdouble) ** 2 + a.imag.astype(np.longdouble) ** 2)
+    loss = (terms * (1.0 - mask.astype(np.longdouble)[None, :] ** 2)).sum()
+    assert abs(p.all_losses()[0] - loss) < tol * np.abs(terms).sum()
+
+
 def test_columns_that_are_not_finite_stay_apart(so):
     rng = np.random.default_rng(3)
     n, nr = 64, 50
