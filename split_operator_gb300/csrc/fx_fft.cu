@@ -58,18 +58,20 @@ bool fx_pair_plan(PassParams& p, int real, const double* table_max) {
   int lg = 0;
   while ((int64_t)1 << lg < (pow2 ? g.n : 2 * g.n - 1)) ++lg;
   const int64_t m = (int64_t)1 << lg;
-  // 256 threads a CTA (512 for 8192 points), fewer while the tiles do not fill the SMs twice
-  int T = m >= 8192 ? 512 : 256;
-  const int least = m / kV > 32 ? (int)(m / kV) : 32;
-  while (T > least && (g.outer * m + (int64_t)kV * T - 1) / ((int64_t)kV * T) < 304) T /= 2;
-  const int64_t L = (int64_t)kV * T / m;
+  // 512 threads a CTA, fewer while the tiles do not fill the SMs twice
+  const int V = pair_vals(lg);
+  int T = kPairThreads;
+  const int least = m / V > 32 ? (int)(m / V) : 32;
+  while (T > least && (g.outer * m + (int64_t)V * T - 1) / ((int64_t)V * T) < 304) T /= 2;
+  const int64_t L = (int64_t)V * T / m;
   g.lanes_per_tile = (int32_t)L;
   g.tiles_per_outer = 1;
   g.tiles = (g.outer + L - 1) / L;
-  g.lane_stride = (int32_t)(m + m / 16 + 1);
+  g.vals = V;
+  g.lane_stride = (int32_t)(m + m / (V == 16 ? 16 : 8) + 1);
   p.fx_chirp = pow2 ? 0 : 1;
   p.fused = 1;
-  p.radix = 16;
+  p.radix = V;
   p.fx = lg;
   return true;
 }

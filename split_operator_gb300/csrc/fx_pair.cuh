@@ -3,13 +3,17 @@
 //
 // The FP64 form of this pass was bound by the FP64 pipe: about 90 FP64 operations per point
 // of a 4096-point lane at ~1.7 per clock and SM.  Here the butterflies are integer additions
-// and the products three 32 x 32 + 64 multiply-adds, ~690 issue slots per point at 128 per
-// clock.  The stage structure is that of the FP32 FFT-pair kernel: 16 values per thread in
-// registers, radix-16 stages in place in one shared buffer, the first stage from global
-// memory, the point-wise ops between the transforms in registers, the second transform in
-// reversed radix order so that its first stage needs no shared memory, the last stage to
-// global memory.  The unitary scaling sits in the products (w 2^62 times v is v w / 4, the
-// factor of a radix-16 stage) and in the exponent the lane leaves with.
+// and the products three 32 x 32 + 64 multiply-adds.  A thread holds 8 values: radix-8 stages in
+// place in one shared buffer, the first stage from global memory, the point-wise ops between the
+// transforms in registers, the second transform in reversed radix order so that its first stage
+// needs no shared memory, the last stage to global memory.  The unitary scaling sits in the
+// products and in the exponent the lane leaves with.
+//
+// What bounds it is fetching instructions and latency, not the pipes: the code is one loop over
+// the stages, one copy for both transforms (rolled_transform).  Unrolled, with 16 values per
+// thread, a lane ran 10,400 instructions in a row on 8 warps and 61 % of the stalls were for
+// instructions.  us per pass before / now: 128 lanes of 4096 points in float-float 37.1 / 29.1,
+// 64 of 2048 in FP64 28.9 / 18.3, 256 of 256 22.9 / 12.6, 45 of 1000 (through 2048) 53.7 / 28.7.
 #pragma once
 #include "fx_stage.cuh"
 
@@ -19,38 +23,31 @@ using namespace fx;
 
 namespace {
 
-constexpr int kV = 16;  // values per thread
-__host__ __device__ constexpr int pair_threads(int lgn) { return lgn >= 13 ? 512 : 256; }  // most threads of a CTA
+// values per thread: 8, and 16 where that would take more than 512 threads for a lane
+__host__ __device__ constexpr int pair_vals(int lgn) { return lgn >= 13 ? 16 : 8; }
+constexpr int kPairThreads = 512;  // most threads of a CTA
 
 // point-wise ops [ob, oe) on the outputs of a last stage of radix RS (span P = n / RS): value
-// j RS + q sits at lane b >> lg P, point k + q P; the first one scales by 2^-SC
-template <int LGN, int RS, int SC>
-__device__ __forceinline__ void pointwise(cx (&v)[kV], const PassParams& pp, int ob, int oe, int64_t lane0, int nl) {
+// j RS + q sits at lane b >> lg P, point k + q P
+template <int LGN, int KV, int RS>
+__device__ __forceinline__ void pointwise(cx (&v)[KV], const PassParams& pp, int ob, int oe, int64_t lane0, int nl) {
   constexpr int kN = 1 << LGN, kP = kN / RS, kLgP = LGN - lg2(RS);
   const int t = threadIdx.x, T = blockDim.x;
-  if constexpr (SC > 0) {
-    if (ob == oe) {
-#pragma unroll
-      for (int e = 0; e < kV; ++e) v[e] = shift_down<SC>(v[e]);
-    }
-  }
+#pragma unroll 1
   for (int oi = ob; oi < oe; ++oi) {
     const DevOp& op = pp.ops[oi];
     const bool nd = op.kind == OP_DIAGND;
     const int4* tab = reinterpret_cast<const int4*>(op.ptr) + (nd ? lane0 * kN : 0);
-    const bool first = SC > 0 && oi == ob;
 #pragma unroll
-    for (int j = 0; j < kV / RS; ++j) {
+    for (int j = 0; j < KV / RS; ++j) {
       const int b = t + j * T, l = b >> kLgP, k = b & (kP - 1);
       if (!nd || l < nl) {
         const int4* tr = tab + (nd ? l * kN : 0) + k;
-        if (first) {
+        int4 w[RS];
 #pragma unroll
-          for (int q = 0; q < RS; ++q) v[j * RS + q] = cmul<SC>(v[j * RS + q], __ldg(tr + q * kP));
-        } else {
+        for (int q = 0; q < RS; ++q) w[q] = __ldg(tr + q * kP);
 #pragma unroll
-          for (int q = 0; q < RS; ++q) v[j * RS + q] = cmul<0>(v[j * RS + q], __ldg(tr + q * kP));
-        }
+        for (int q = 0; q < RS; ++q) v[j * RS + q] = cmul<0>(v[j * RS + q], w[q]);
       }
     }
   }
@@ -58,8 +55,9 @@ __device__ __forceinline__ void pointwise(cx (&v)[kV], const PassParams& pp, int
 
 template <int LGN, bool FF>
 __device__ __forceinline__ void fx_pair_tile(const PassParams& pp, int64_t tile) {
+  constexpr int kV = pair_vals(LGN);
   using Sh = Shape<LGN, kV>;
-  constexpr int kN = Sh::kN, kNb = kN / 16, kLgNb = LGN - 4;
+  constexpr int kN = Sh::kN, kNb = kN / kV, kLgNb = LGN - Sh::kLgV;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ NormPart part[16];
   cx* buf = reinterpret_cast<cx*>(smem_raw);
@@ -71,36 +69,48 @@ __device__ __forceinline__ void fx_pair_tile(const PassParams& pp, int64_t tile)
   const int4* tw = reinterpret_cast<const int4*>(pp.twiddle);
   const int t = threadIdx.x;
   cx v[kV];
-  // the first stage's inputs straight from the lanes (points i + r n / 16; missing lanes: 0)
+  // the first stage's inputs straight from the lanes (points i + r n / kV; missing lanes: 0)
   const int l0 = t >> kLgNb, i0 = t & (kNb - 1);
   const bool ok0 = l0 < nl;
   {
     const longlong2* src = psi + l0 * kN + i0;
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
+    for (int r = 0; r < kV; ++r) {
       const longlong2 x = ok0 ? src[r * kNb] : longlong2{0, 0};
       v[r] = {x.x, x.y};
     }
   }
   const int e = lane_exponent<LGN, kV, FF>(v, part);
 #pragma unroll
-  for (int r = 0; r < 16; ++r) {
+  for (int r = 0; r < kV; ++r) {
     v[r].x = e == kNonFinite || e == kZero ? 0 : raw_to_fx<FF>(v[r].x, e);
     v[r].y = e == kNonFinite || e == kZero ? 0 : raw_to_fx<FF>(v[r].y, e);
   }
   int f1 = 1;
   while (f1 < pp.nops && pp.ops[f1].kind != OP_FFT) ++f1;
-  transform<LGN, kV, false, 0, -1>(v, buf, tw);
-  pointwise<LGN, Sh::kRl, Sh::kMid>(v, pp, 1, f1, lane0, nl);
-  transform<LGN, kV, true, 0, 1>(v, buf, tw);
-  pointwise<LGN, Sh::rs(true, Sh::kS - 1), 0>(v, pp, f1 + 1, pp.nops, lane0, nl);
-  // the last stage's outputs have the first stage's layout (radix 16, or the only stage):
-  // the same lane, points k + q n / 16
+  // one copy of the code for both transforms: the inverse one is conjugated
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+    if (half) conjugate(v);
+    rolled_transform<LGN, kV>(v, buf, tw, half != 0);
+    if (half) {
+      conjugate(v);
+    } else if (Sh::kMid > 0) {
+#pragma unroll
+      for (int r = 0; r < kV; ++r) v[r] = shift_down<Sh::kMid>(v[r]);
+    }
+    const int ob = half ? f1 + 1 : 1, oe = half ? pp.nops : f1;
+    if (Sh::kRl == kV || half)
+      pointwise<LGN, kV, kV>(v, pp, ob, oe, lane0, nl);
+    else
+      pointwise<LGN, kV, Sh::kRl>(v, pp, ob, oe, lane0, nl);
+  }
+  // the last stage's outputs have the first stage's layout: the same lane, points k + q n / kV
   if (ok0) {
     longlong2* dst = psi + l0 * kN + i0;
     const int x = e - Sh::kOut;
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
+    for (int q = 0; q < kV; ++q) {
       longlong2 o{fx_to_raw<FF>(v[q].x, x), fx_to_raw<FF>(v[q].y, x)};
       if (e == kNonFinite) o = {raw_nan<FF>(), raw_nan<FF>()};
       dst[q * kNb] = o;
@@ -118,8 +128,9 @@ __device__ __forceinline__ void fx_pair_tile(const PassParams& pp, int64_t tile)
 // pp.aux: the chirp w (n entries), then G 2^-pp.fx_g (M entries, natural order, magnitudes <= 1).
 template <int LGM, bool FF>
 __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile) {
+  constexpr int kV = pair_vals(LGM);
   using Sh = Shape<LGM, kV>;
-  constexpr int kM = Sh::kN, kNb = kM / 16, kLgNb = LGM - 4;
+  constexpr int kM = Sh::kN, kNb = kM / kV, kLgNb = LGM - Sh::kLgV;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ NormPart part[16];
   cx* buf = reinterpret_cast<cx*>(smem_raw);
@@ -134,18 +145,18 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
   const int4* gt = chirp + n;
   const int t = threadIdx.x, T = blockDim.x;
   cx v[kV];
-  // value r: point i0 + r M / 16 of lane l0 (the layout of the outer radix-16 stages)
+  // value r: point i0 + r M / kV of lane l0 (the layout of the outer stages)
   const int l0 = t >> kLgNb, i0 = t & (kNb - 1);
   const bool ok0 = l0 < nl;
 #pragma unroll
-  for (int r = 0; r < 16; ++r) {
+  for (int r = 0; r < kV; ++r) {
     const int j = i0 + r * kNb;
     const longlong2 x = ok0 && j < n ? psi[l0 * n + j] : longlong2{0, 0};
     v[r] = {x.x, x.y};
   }
   const int e = lane_exponent<LGM, kV, FF>(v, part);
 #pragma unroll
-  for (int r = 0; r < 16; ++r) {
+  for (int r = 0; r < kV; ++r) {
     const int j = i0 + r * kNb;
     v[r].x = e == kNonFinite || e == kZero ? 0 : raw_to_fx<FF>(v[r].x, e);
     v[r].y = e == kNonFinite || e == kZero ? 0 : raw_to_fx<FF>(v[r].y, e);
@@ -153,30 +164,36 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
   }
   int f1 = 1;
   while (f1 < pp.nops && pp.ops[f1].kind != OP_FFT) ++f1;
-  // (one copy of the transforms' code serves both halves)
+  // (one copy of the transforms' code serves all four)
 #pragma unroll 1
-  for (int half = 0; half < 2; ++half) {
-    transform<LGM, kV, false, 0, -1>(v, buf, tw);
-    // the filter on the outputs of the closing stage (value j RS + q: point k + q P)
-    constexpr int RS = Sh::kRl, kP = kM / RS;
+  for (int quarter = 0; quarter < 4; ++quarter) {
+    const int half = quarter >> 1;
+    const bool back = quarter & 1;
+    if (back) conjugate(v);
+    rolled_transform<LGM, kV>(v, buf, tw, back);
+    if (!back) {
+      // the filter on the outputs of the closing stage (value j RS + q: point k + q P)
+      constexpr int RS = Sh::kRl, kP = kM / RS;
 #pragma unroll
-    for (int j = 0; j < kV / RS; ++j) {
-      const int k = (t + j * T) & (kP - 1);
+      for (int j = 0; j < kV / RS; ++j) {
+        const int k = (t + j * T) & (kP - 1);
 #pragma unroll
-      for (int q = 0; q < RS; ++q) {
-        int4 w = __ldg(gt + k + q * kP);
-        if (half) {
-          w.z = -w.z;
-          w.w = -w.w;
+        for (int q = 0; q < RS; ++q) {
+          int4 w = __ldg(gt + k + q * kP);
+          if (half) {
+            w.z = -w.z;
+            w.w = -w.w;
+          }
+          v[j * RS + q] = cmul<Sh::kConvMid>(v[j * RS + q], w);
         }
-        v[j * RS + q] = cmul<Sh::kMid>(v[j * RS + q], w);
       }
+      continue;
     }
-    transform<LGM, kV, true, 0, 1>(v, buf, tw);
+    conjugate(v);
     // the n points of the transform, and the ops up to the next one
     const int ob = half ? f1 + 1 : 1, oe = half ? pp.nops : f1;
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
+    for (int r = 0; r < kV; ++r) {
       const int j = i0 + r * kNb;
       if (j >= n || !ok0) {
         v[r] = {0, 0};
@@ -196,9 +213,9 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
     }
   }
   if (ok0) {
-    const int x = e - (2 * Sh::kOut - 2 * pp.fx_g - 60);
+    const int x = e - (2 * Sh::kConvOut - 2 * pp.fx_g - 60);
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
+    for (int r = 0; r < kV; ++r) {
       const int j = i0 + r * kNb;
       if (j >= n) continue;
       longlong2 o{fx_to_raw<FF>(v[r].x, x), fx_to_raw<FF>(v[r].y, x)};
@@ -211,7 +228,7 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
 // one pass (params == nullptr: `one`), or many propagations' passes in one launch: block b
 // runs tile (b - offsets[i]) of params[i], offsets[i] <= b < offsets[i + 1]
 template <int LGN, bool FF, bool CHIRP>
-__global__ void __launch_bounds__(pair_threads(LGN), LGN >= 13 ? 1 : 2)
+__global__ void __launch_bounds__(kPairThreads, 1)
     fx_pair_kernel(const __grid_constant__ PassParams one, const PassParams* __restrict__ params,
                    const int64_t* __restrict__ offsets, int count) {
   if (params == nullptr) {
@@ -246,7 +263,7 @@ cudaError_t launch_lgn(const PassParams* one, const PassParams* params, const in
     if (e != cudaSuccess) return e;
     done = true;
   }
-  if (smem > 220 * 1024 || threads > pair_threads(LGN)) return cudaErrorInvalidValue;
+  if (smem > 220 * 1024 || threads > kPairThreads) return cudaErrorInvalidValue;
   static const PassParams none{};
   kern<<<(unsigned)blocks, threads, smem, s>>>(one ? *one : none, params, offsets, count);
   count_launch();

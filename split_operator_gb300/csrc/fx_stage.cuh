@@ -12,21 +12,36 @@ namespace {
 
 __host__ __device__ constexpr int lg2(int x) { return x <= 1 ? 0 : 1 + lg2(x / 2); }
 
-// A power-of-two transform of 2^LGN points with KV values per thread (16 or 4) and radix-KV stages.
+// A power-of-two transform of 2^LGN points with KV values per thread (16, 8 or 4) and radix-KV stages.
 // Values come in at 2^60 of the lane's norm bound or below; the first stage is unscaled, a stage
-// with twiddles scales by the square root of its radix or a little more in its products.
+// with twiddles scales by the square root of its radix or a little more in its products.  The norm
+// grows by the square root of a stage's radix and stays below 2^62.
 template <int LGN, int KV>
 struct Shape {
   static constexpr int kN = 1 << LGN, kLgV = lg2(KV);
   static constexpr int kS = (LGN + kLgV - 1) / kLgV;         // radix-KV stages, the last one kRl
   static constexpr int kLgRl = LGN - kLgV * (kS - 1);        // closing radix (2 .. KV)
   static constexpr int kRl = 1 << kLgRl;
-  static constexpr int kSc = kLgV / 2;                       // scaling of a full stage: 2^-kSc
+  static constexpr int kSc = (kLgV + 1) / 2;                 // scaling of a full stage: 2^-kSc
   static constexpr int kSh = (kLgRl + 1) / 2;                // of the closing stage of the forward order
-  static constexpr int kMid = kLgRl / 2;                     // of the factors between a pair's transforms
+  static constexpr int kSumF = kS > 1 ? (kS - 2) * kSc + kSh : 0, kSumR = (kS - 1) * kSc;
+  // of the factors between a pair's transforms: brings the norm back to 2^60, or (radix 8, whose
+  // stages scale by more than they need) just keeps it below 2^62 after the next unscaled stage
+  static constexpr int kTop = 120 + LGN - 2 * kSumF + kLgRl;  // half bits of the norm there
+  static constexpr int kMid = KV != 8 ? kLgRl / 2 : (kTop > 124 ? (kTop - 123) / 2 : 0);
+  // ... of the filter between the transforms of a convolution (a unitary one times 2^-g, g >= 2,
+  // magnitudes <= 1): the norm below 2^62 after the next stage, and 2^60.5 or less behind it
+  static constexpr int conv_mid() {
+    if (KV != 8) return kMid;
+    int m = kMid;
+    while (kTop - 2 * (m - 1) <= 124 && 120 + 2 * LGN - 2 * kSumF - 2 * (m - 1) - 2 * kSumR <= 121 + 4) --m;
+    return m;
+  }
+  static constexpr int kConvMid = conv_mid();
   static constexpr int kPad = KV == 16 ? 4 : 3;              // one padding element every 2^kPad
   static constexpr int kLs = kN + (kN >> kPad) + 1;          // padded lane stride
-  static constexpr int kOut = 60 + kSc;                      // exponent after a pair: x 2^(kOut - e)
+  static constexpr int kOut = 60 + LGN - kSumF - kMid - kSumR;  // exponent after a pair: x 2^(kOut - e)
+  static constexpr int kConvOut = kOut + kMid - kConvMid;       // ... after a convolution
   __host__ __device__ static constexpr int rs(bool rev, int s) {
     return rev ? (s == 0 ? kRl : KV) : (s + 1 < kS ? KV : kRl);
   }
@@ -100,6 +115,66 @@ __device__ __forceinline__ void transform(cx (&v)[KV], cx* buf, const int4* tw) 
   constexpr int sc = (!REV && S + 1 == Sh::kS) ? Sh::kSh : Sh::kSc;
   stage<LGN, KV, rs, p, Sh::twoff(REV, S), (S > 0), (S + 1 < Sh::kS), DIR, sc>(v, buf, tw);
   if constexpr (S + 1 < Sh::kS) transform<LGN, KV, REV, S + 1, DIR>(v, buf, tw);
+}
+
+// A transform whose full stages are one loop: forward order (REV false), or the reversed radix order
+// with its own twiddles.  The direction is forward in both (conjugate around it for the inverse).
+// Unrolled, a pair of 4096-point transforms was 10,400 instructions in a row, each executed once
+// by a warp, and most of its time went into fetching them (61 % of the stalls).
+// Values come and leave in registers: point i + r nb of the first stage, k + q P of the last.
+template <int LGN, int KV>
+__device__ __forceinline__ void rolled_transform(cx (&v)[KV], cx* buf, const int4* __restrict__ tw, bool rev) {
+  using Sh = Shape<LGN, KV>;
+  constexpr int kN = Sh::kN, kNb = kN / KV, kLgNb = LGN - Sh::kLgV, kLs = Sh::kLs, kPad = Sh::kPad;
+  constexpr bool kEven = Sh::kRl == KV;  // every stage is a full one: both orders are the same
+  const int t = threadIdx.x, l = t >> kLgNb, i = t & (kNb - 1);
+  cx* const mine = buf + l * kLs;
+  if constexpr (!kEven) {
+    if (rev) stage<LGN, KV, Sh::kRl, 1, 0, false, true, -1, 0>(v, buf, tw);
+  }
+  int lgp = !kEven && rev ? Sh::kLgRl : 0;
+  const int4* w = tw + (!kEven && rev ? kN : 0);
+  constexpr int kFull = kEven ? Sh::kS : Sh::kS - 1;
+#pragma unroll 1
+  for (int s = 0; s < kFull; ++s) {
+    const int k = i & ((1 << lgp) - 1);
+    if (lgp > 0) {
+      const int4* wk = w + k;
+      int4 wv[KV];
+#pragma unroll
+      for (int r = 1; r < KV; ++r) wv[r] = __ldg(wk + ((r - 1) << lgp));
+#pragma unroll
+      for (int r = 0; r < KV; ++r)
+        v[r] = kNb % (1 << kPad) == 0 ? mine[i + (i >> kPad) + r * kNb + ((r * kNb) >> kPad)]
+                                      : mine[i + r * kNb + ((i + r * kNb) >> kPad)];
+      __syncthreads();  // every read of the stage before any write (in place)
+      v[0] = shift_down<Sh::kSc>(v[0]);
+#pragma unroll
+      for (int r = 1; r < KV; ++r) v[r] = cmul<Sh::kSc>(v[r], wv[r]);
+      w += (KV - 1) << lgp;
+    }
+    dft_r<KV, -1>(v);
+    if (s + 1 < kFull || (!kEven && !rev)) {
+      const int base = ((i - k) << Sh::kLgV) + k;
+#pragma unroll
+      for (int q = 0; q < KV; ++q) {
+        const int x = base + (q << lgp);
+        mine[x + (x >> kPad)] = v[q];
+      }
+      __syncthreads();
+    }
+    lgp += Sh::kLgV;
+  }
+  if constexpr (!kEven) {
+    if (!rev)
+      stage<LGN, KV, Sh::kRl, Sh::span(false, Sh::kS - 1), Sh::twoff(false, Sh::kS - 1), true, false, -1, Sh::kSh>(v, buf, tw);
+  }
+}
+
+template <int KV>
+__device__ __forceinline__ void conjugate(cx (&v)[KV]) {
+#pragma unroll
+  for (int r = 0; r < KV; ++r) v[r].y = -v[r].y;
 }
 
 // Lane norm bounds.  A thread's KV values lie in one lane (lane = t >> lg(n / KV)).  Returns e

@@ -1302,7 +1302,7 @@ static cudaError_t launch_pair_batched_ct_any(int lgn, const PassParams* params_
 int fft_pair_threads(const Geometry& g) { return g.n >= 8192 ? 512 : 256; }
 
 int fft_pair_block(const PassParams& p) {
-  return (int)((int64_t)p.g.lanes_per_tile * (p.fx ? (int64_t)1 << p.fx : p.g.n) / kPairV);
+  return (int)((int64_t)p.g.lanes_per_tile * (p.fx ? (int64_t)1 << p.fx : p.g.n) / (p.fx ? p.g.vals : kPairV));
 }
 
 bool fft_pair_plan(PassParams& p, int real, bool resident) {

@@ -935,7 +935,7 @@ bool Engine::try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p, bo
   if (!(resident ? fx_line_plan(p, real, mx) : fx_pair_plan(p, real, mx))) return false;
   for (size_t i = 0; i < ops.size(); ++i)
     if (tab[i]) p.ops[i].ptr = fx_table(*tab[i]);
-  p.twiddle = fx_twiddle((size_t)1 << p.fx, resident ? 4 : 16);
+  p.twiddle = fx_twiddle((size_t)1 << p.fx, resident ? 4 : p.radix);
   if (p.fx_chirp) {
     const FxFactors& f = fx_chirp((size_t)p.g.n, p.fx);
     p.aux = f.buf.ptr;
