@@ -143,6 +143,7 @@ void fx_angular_params(const PassParams& p, const int* mat_op, int nmat, const u
   FxTcParams t{};
   t.p = p;
   t.nmat = nmat;
+  t.handover = pass_handover(p, mat_op, nmat);
   t.kp = fx_kp((int)p.g.n);
   t.error_slot = error_slot;
   const Geometry& g = p.g;

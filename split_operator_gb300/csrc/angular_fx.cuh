@@ -32,6 +32,7 @@
 #pragma once
 #include "common.cuh"
 #include "fx.cuh"
+#include "overlap.cuh"
 #include "pass_end.cuh"
 #include "tc_common.cuh"
 
@@ -43,6 +44,7 @@ struct FxTcParams {
   PassParams p;
   int32_t mat_op[2];  // op indices of the (one or two) lane matrices
   int32_t nmat;
+  int32_t handover;   // see pass_handover
   int32_t kp;         // lane extent rounded up to 32: K of the products
   int32_t error_slot;
   int32_t slice_axis[2];      // state matrix: the logical axis whose coordinate picks the image (-1: one)
@@ -170,7 +172,7 @@ struct FxTabs {
   int colb[kFxMaxCols];                 // exponent bound of the column's B operand
   int nonident[kFxTabSlots];            // the factors of this tile are not all 1
   int8_t slot[kMaxOps];
-  double red[kMaxRed][kFxWork / 32];    // norms: the warps' sums
+  double red[2][kMaxRed][kFxWork / 32];  // norms: the warps' sums (of every second tile)
 };
 
 __device__ __forceinline__ int64_t fx_coord(const Geometry& g, int a, int64_t o, int64_t i) {
@@ -252,13 +254,30 @@ __device__ __noinline__ void fx_producer(FxResolve resolve, int64_t total, uint3
   }
 }
 
+// One whole warp: lane k < nred gets the sum of reduction k's warp sums (a fixed tree).
+__device__ __forceinline__ double fx_tile_sum(const double (&red)[kMaxRed][kFxWork / 32], int nred) {
+  static_assert(kFxWork / 32 == 16, "two reductions per warp-wide add");
+  const int lane = threadIdx.x & 31;
+  double v = 0.0;
+#pragma unroll 1
+  for (int k = 0; k < nred; k += 2) {
+    double a = red[k + (lane >> 4)][lane & 15];
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+    const double a0 = __shfl_sync(0xffffffffu, a, 0), a1 = __shfl_sync(0xffffffffu, a, 16);
+    if (lane == k) v = a0;
+    if (lane == k + 1) v = a1;
+  }
+  return v;
+}
+
 // Warp 17: per matrix, once its B digits are written, the products of A digit i (chunk by chunk)
 // with the B digits j <= 6 - i into accumulator i + j.  The warp stays converged and its elected
 // lane issues (elect_one).
 template <int N, int MH>
 __device__ __noinline__ void fx_issuer(FxResolve resolve, int64_t total, uint32_t ring, uint32_t b0, uint64_t* full,
                                        uint64_t* empty, uint64_t* dbar, uint64_t* bready, uint64_t* quiet,
-                                       uint32_t tmem, volatile int* fail) {
+                                       uint32_t tmem, volatile int* fail, const FxTabs* T, volatile int* handed) {
   using namespace tc;
   constexpr uint32_t bytes = kChunkRowBytes * MH;
   constexpr int ns = (int)(kRingBytes / bytes);
@@ -268,22 +287,25 @@ __device__ __noinline__ void fx_issuer(FxResolve resolve, int64_t total, uint32_
   int s = 0;
   uint32_t phase = 0, nready = 0;
   bool ok = true;
-  for (int64_t gt = blockIdx.x; gt < total && ok; gt += gridDim.x) {
+  int ntile = 0, need = 0;  // tiles of this CTA, warps that have handed over by then
+  for (int64_t gt = blockIdx.x; gt < total && ok; gt += gridDim.x, ++ntile) {
     const FxTile r = resolve(gt);
     const int kp = r.prm->kp, nk = kp / 32;
     // B: K rows of 16 bytes (eight columns), K groups of 8 rows 128 bytes apart, column groups
     // 16 kp apart, digits 2 N kp apart
     const uint64_t bbits = smem_desc_bits(128, (uint32_t)(16 * kp));
     const uint64_t bfirst = smem_desc_at(bbits, b0), bdig = (uint64_t)((2 * N * kp) >> 4);
-    const int nmat = r.prm->nmat;
-    for (int m = 0; m < nmat && ok; ++m) {
-      ok = __all_sync(0xffffffffu, mbar_poll(bready, nready & 1u, kFxWait));
-      ++nready;
-      tc_fence_after();
+    const int nmat = r.prm->nmat, handover = r.prm->handover;
+    for (int m = 0; m <= nmat && ok; ++m) {
+      if (m < nmat) {
+        ok = __all_sync(0xffffffffu, mbar_poll(bready, nready & 1u, kFxWait));
+        ++nready;
+        tc_fence_after();
+      }
 #pragma unroll
       for (int i = 0; i < kDigits; ++i) {
         uint64_t bk = bfirst;
-        for (int q = 0; q < nk && ok; ++q) {
+        for (int q = 0; q < nk && ok && m < nmat; ++q) {
           ok = __all_sync(0xffffffffu, mbar_poll(&full[s], phase, kFxWait));
           if (!ok) break;
           tc_fence_after();
@@ -306,7 +328,12 @@ __device__ __noinline__ void fx_issuer(FxResolve resolve, int64_t total, uint32_
           }
         }
       }
-      if (ok && el) mma_commit(dbar);
+      if (ok && el && m < nmat) mma_commit(dbar);
+      if (ok && m == handover) {
+        // the tile's norms, while the matrix just issued runs (m == nmat: after the tile)
+        ok = await_handover(handed, need += kFxWork / 32, fail, kFxWait);
+        if (ok) publish_tile(r.prm->p, r.tile, fx_tile_sum(T->red[ntile & 1], r.prm->p.nred));
+      }
     }
   }
   if (!ok && el) {
@@ -342,6 +369,7 @@ struct FxWork {
   int rowx;    // exponent of this row's values on top of their column's
   int xs;      // exponent from SCALE ops, of the whole tile
   int j, c0, ncols;
+  int par;     // of the CTA's tiles: 0, 1, 0, ...
   bool row_ok;
   const double* roww_ptr;  // lane-axis weights of the pass's first norm, and this row's
   RowWeight roww;
@@ -421,7 +449,7 @@ struct FxWork {
 #pragma unroll
           for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
           if ((threadIdx.x & 31) == 0)
-            T.red[op.red][threadIdx.x >> 5] =
+            T.red[par][op.red][threadIdx.x >> 5] =
                 any_bad ? __longlong_as_double(0x7ff8000000000000ll) : scale_pow2((double)t, et + 3);
           break;
         }
@@ -515,11 +543,13 @@ __global__ void __launch_bounds__(kFxThreads, 1)
   __shared__ __align__(16) FxTabs T;
   __shared__ __align__(8) uint64_t bars[2 * 8 + 3];
   __shared__ uint32_t tmem_s;
-  __shared__ double s_red[kMaxRed];
-  __shared__ volatile int s_fail;
+  __shared__ volatile int s_fail, s_handed;
   __shared__ int s_bad;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (blockIdx.x >= total) return;
+  if (blockIdx.x >= total) {
+    wait_for_previous();
+    return;
+  }
   const FxResolve resolve{&one, params, owners};
   uint64_t *full = bars, *empty = bars + kRing, *dbar = bars + 2 * kRing, *bready = dbar + 1, *quiet = dbar + 2;
   if (tid == 0) {
@@ -529,20 +559,26 @@ __global__ void __launch_bounds__(kFxThreads, 1)
     mbar_init(quiet, 1);
     fence_mbar_init();
     s_fail = 0;
+    s_handed = 0;
     s_bad = 0;
   }
   if (warp == 0) tmem_alloc(&tmem_s, 512);
+  // (ahead of the wait below: the parameters are no memory of the kernel before)
+  if (params == nullptr)
+    for (int k = tid; k < (int)(sizeof(FxTcParams) / 4); k += kFxThreads)
+      reinterpret_cast<uint32_t*>(&tp)[k] = reinterpret_cast<const uint32_t*>(&one)[k];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_s;
+  wait_for_previous();
   const uint32_t ring = smem_u32(sm);
   unsigned char* B = sm + kRingBytes;
 
   if (warp == kFxWork / 32) {
     if (lane == 0) fx_producer<MH>(resolve, total, ring, full, empty, &s_fail);
   } else if (warp == kFxWork / 32 + 1) {
-    fx_issuer<N, MH>(resolve, total, ring, ring + kRingBytes, full, empty, dbar, bready, quiet, tmem, &s_fail);
+    fx_issuer<N, MH>(resolve, total, ring, ring + kRingBytes, full, empty, dbar, bready, quiet, tmem, &s_fail, &T, &s_handed);
   } else {
     const int quad = warp & 3, grp = warp >> 2;
     Work W;
@@ -551,8 +587,10 @@ __global__ void __launch_bounds__(kFxThreads, 1)
     // this thread's accumulator columns: half (MH = 2) grp >> 1, real columns 2 c0 ..
     const uint32_t tcol = tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)((MH == 2 ? (grp >> 1) * N : 0) + 2 * W.c0);
     uint32_t drains = 0;
-    const FxTcParams* cur = nullptr;
+    const FxTcParams* cur = params == nullptr ? &one : nullptr;
+    W.par = 1;
     for (int64_t gt = blockIdx.x; gt < total; gt += gridDim.x) {
+      W.par ^= 1;
       const FxTile r = resolve(gt);
       if (r.prm != cur) {
         for (int k = tid; k < (int)(sizeof(FxTcParams) / 4); k += kFxWork)
@@ -714,35 +752,12 @@ __global__ void __launch_bounds__(kFxThreads, 1)
           fence_proxy_async();
           mbar_arrive(bready);
         }
+        // the tile's norms are complete: the issuing warp publishes them
+        if (m + 1 == tp.handover && lane == 0) hand_over(&s_handed);
       }
       if (!ok) {
         if (tid == 0) s_fail = 1;
         break;
-      }
-      // norm partials and the pass ticket, drawn by warp 0 while the other warps store (a fence
-      // behind the stores would wait for them)
-      fx_work_sync();
-      if (warp < p.nred) {
-        double a = lane < kFxWork / 32 ? T.red[warp][lane] : 0.0;
-#pragma unroll
-        for (int o2 = kFxWork / 64; o2 > 0; o2 >>= 1) a += __shfl_down_sync(0xffffffffu, a, o2);
-        if (lane == 0) s_red[warp] = a;
-      }
-      fx_work_sync();
-      if (warp == 0) {
-        unsigned int last = 0;
-        EndOp end;
-        end.load(p);
-        if (lane == 0) {
-          for (int k = 0; k < p.nred; ++k) p.partials[(int64_t)k * g.tiles + r.tile] = s_red[k];
-          __threadfence();
-          last = atomicAdd(p.counter, 1u) == (unsigned int)(g.tiles - 1) ? 1u : 0u;
-        }
-        last = __shfl_sync(0xffffffffu, last, 0);
-        if (last) {
-          __threadfence();
-          finish_pass(p, end, p.partials, g.tiles);
-        }
       }
       // store
 #pragma unroll

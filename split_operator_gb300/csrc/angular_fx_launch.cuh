@@ -18,17 +18,16 @@ cudaError_t fx_angular_one(int kp, const void* one, const FxTcParams* params, co
   static bool done = false;
   auto kern = fx_angular_kernel<NB, MH, FF>;
   if (!done) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 180 * 1024);
     if (e != cudaSuccess) return e;
     done = true;
   }
   const uint32_t smem = fx_tc_smem(NB * (MH == 1 ? 4 : 2), kp);
-  if (smem > 216 * 1024) return cudaErrorInvalidValue;
+  if (smem > 180 * 1024) return cudaErrorInvalidValue;
   FxTcParams p{};
   if (one) std::memcpy(&p, one, sizeof(p));
-  kern<<<grid, kFxThreads, smem, s>>>(p, params, owners, tiles);
   count_launch();
-  return cudaGetLastError();
+  return launch_overlapped(kern, grid, kFxThreads, smem, s, p, params, owners, tiles);
 }
 
 template <bool FF>

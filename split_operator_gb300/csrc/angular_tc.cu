@@ -36,6 +36,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "overlap.cuh"
 #include "pass_end.cuh"
 #include "tc_common.cuh"
 
@@ -189,12 +190,9 @@ __device__ __forceinline__ bool work_all(bool v) {
   return r != 0;
 }
 
-// fixed-order sum of one float per work thread, in float-float; valid in thread 0
-// The tile's nred float-float block sums together (fixed order): each warp reduces every
-// value by the same shuffle tree, lane 0 stores them, one barrier; thread k adds reduction
-// k's warp partials 0 .. 7 in order and stores its FP64 value in out[k]; a second barrier
-// publishes them.  scratch: kMaxRed x (kWorkThreads / 32) entries.
-__device__ __forceinline__ void block_sums(const float (&acc)[kMaxRed], int nred, FF* scratch, double* out) {
+// The tile's nred float-float sums together (fixed order): each warp reduces every value by the
+// same shuffle tree and its lane 0 stores them.  scratch: kMaxRed x (kWorkThreads / 32) entries.
+__device__ __forceinline__ void warp_sums(const float (&acc)[kMaxRed], int nred, FF* scratch) {
   constexpr int kW = kWorkThreads / 32;
 #pragma unroll
   for (int k = 0; k < kMaxRed; ++k) {
@@ -207,13 +205,14 @@ __device__ __forceinline__ void block_sums(const float (&acc)[kMaxRed], int nred
     }
     if ((threadIdx.x & 31) == 0) scratch[k * kW + (threadIdx.x >> 5)] = a;
   }
-  work_sync();
-  if ((int)threadIdx.x < nred) {
-    FF r{0.0f, 0.0f};
-    for (int w = 0; w < kW; ++w) r = ff_add(r, scratch[threadIdx.x * kW + w]);
-    out[threadIdx.x] = (double)r.hi + (double)r.lo;
-  }
-  work_sync();
+}
+// The issuing warp: lane k < nred adds reduction k's warp sums 0 .. 7 in order.
+__device__ __forceinline__ double tile_sum(const FF* scratch, int nred, int lane) {
+  constexpr int kW = kWorkThreads / 32;
+  FF r{0.0f, 0.0f};
+  if (lane < nred)
+    for (int w = 0; w < kW; ++w) r = ff_add(r, scratch[lane * kW + w]);
+  return (double)r.hi + (double)r.lo;
 }
 
 // logical coordinate of axis `a` for element (outer o, inner i) (a != sweep axis)
@@ -902,6 +901,7 @@ struct TcParams {
   PassParams p;
   int32_t mat_op[2];      // op indices of the (one or two) lane matrices
   int32_t nmat;
+  int32_t handover;       // see pass_handover
   const float* images[2]; // A chunk images per matrix: nk x slices x chunk_bytes
   int32_t error_slot;
   int32_t parity[2];          // per matrix: 0 plain; 1 sum / difference rows; 2 even / odd columns
@@ -1011,7 +1011,8 @@ __device__ __noinline__ void tma_producer(Resolve resolve, int64_t total, const 
 // own issuer, mma_issuer_oz.)
 template <bool BF, typename Resolve>
 __device__ __noinline__ void mma_issuer(Resolve resolve, int64_t total, const TcShape S, uint32_t sm0,
-                                        const TcSmemLayout L, uint32_t tmem, volatile int* fail) {
+                                        const TcSmemLayout L, uint32_t tmem, volatile int* fail, const FF* sums,
+                                        volatile int* handed) {
   using namespace tc;
   uint64_t* full = reinterpret_cast<uint64_t*>(sm_ptr(sm0 + L.bars));
   const int ns = S.stages;
@@ -1031,18 +1032,21 @@ __device__ __noinline__ void mma_issuer(Resolve resolve, int64_t total, const Tc
   uint64_t ahi = 0;               // A_hi descriptor of the current K step (a chunk may span two fills)
   uint32_t nready = 0, nfree = 0;
   bool ok = true;
+  int ntile = 0, need = 0;  // tiles of this CTA, warps that have handed over by then
   const uint32_t el = elect_one();
   const auto all = [](bool v) { return __all_sync(0xffffffffu, v); };
-  for (int64_t gt = blockIdx.x; gt < total && ok; gt += gridDim.x) {
+  for (int64_t gt = blockIdx.x; gt < total && ok; gt += gridDim.x, ++ntile) {
     const TileRef tr = resolve(gt);
-    const int nmat = tr.prm->nmat;
+    const int nmat = tr.prm->nmat, handover = tr.prm->handover;
     unsigned long long* trace = tr.prm->trace ? tr.prm->trace + tr.tile * kTraceSlots : nullptr;
     const int64_t cc_tile = cc;  // first chunk of this tile
-    for (int m = 0; m < nmat && ok; ++m) {
-      ok = all(mbar_poll(bready, nready & 1u, kWaitLimit));
-      ++nready;
-      tc_fence_after();
-      for (int f = 0; f < S.fills && ok; ++f) {
+    for (int m = 0; m <= nmat && ok; ++m) {
+      if (m < nmat) {
+        ok = all(mbar_poll(bready, nready & 1u, kWaitLimit));
+        ++nready;
+        tc_fence_after();
+      }
+      for (int f = 0; f < S.fills && ok && m < nmat; ++f) {
         if (f > 0) {
           ok = all(mbar_poll(freebar, nfree & 1u, kWaitLimit));
           ++nfree;
@@ -1106,6 +1110,12 @@ __device__ __noinline__ void mma_issuer(Resolve resolve, int64_t total, const Tc
         }
         if (ok && el) mma_commit(dbar);
       }
+      if (ok && m == handover) {
+        // the tile's norms, while the matrix just issued runs (m == nmat: after the tile)
+        ok = await_handover(handed, need += kWorkThreads / 32, fail, kWaitLimit);
+        const FF* mine = sums + (ntile & 1) * (kMaxRed * kWorkThreads / 32);
+        if (ok) publish_tile(tr.prm->p, tr.tile, tile_sum(mine, tr.prm->p.nred, threadIdx.x & 31));
+      }
     }
   }
   if (!ok && el) {
@@ -1120,7 +1130,8 @@ __device__ __noinline__ void mma_issuer(Resolve resolve, int64_t total, const Tc
 // chunk and the M halves unrolled (MH = 1: chunks of two K steps; MH = 2: one).
 template <int MH, typename Resolve>
 __device__ __noinline__ void mma_issuer_oz(Resolve resolve, int64_t total, const TcShape S, uint32_t sm0,
-                                           const TcSmemLayout L, uint32_t tmem, volatile int* fail) {
+                                           const TcSmemLayout L, uint32_t tmem, volatile int* fail, const FF* sums,
+                                           volatile int* handed) {
   using namespace tc;
   constexpr int KPC = MH == 1 ? 2 : 1;  // K steps per chunk
   uint64_t* full = reinterpret_cast<uint64_t*>(sm_ptr(sm0 + L.bars));
@@ -1143,19 +1154,22 @@ __device__ __noinline__ void mma_issuer_oz(Resolve resolve, int64_t total, const
   int s = 0;
   uint32_t fphase = 0, nready = 0;
   bool ok = true;
+  int ntile = 0, need = 0;
   const uint32_t el = elect_one();
   const auto all = [](bool v) { return __all_sync(0xffffffffu, v); };
-  for (int64_t gt = blockIdx.x; gt < total && ok; gt += gridDim.x) {
+  for (int64_t gt = blockIdx.x; gt < total && ok; gt += gridDim.x, ++ntile) {
     const TileRef tr = resolve(gt);
-    const int nmat = tr.prm->nmat;
+    const int nmat = tr.prm->nmat, handover = tr.prm->handover;
     unsigned long long* trace = tr.prm->trace ? tr.prm->trace + tr.tile * kTraceSlots : nullptr;
     const int64_t cc_tile = cc;
-    for (int m = 0; m < nmat && ok; ++m) {
-      ok = all(mbar_poll(bready, nready & 1u, kWaitLimit));
-      ++nready;
-      tc_fence_after();
+    for (int m = 0; m <= nmat && ok; ++m) {
+      if (m < nmat) {
+        ok = all(mbar_poll(bready, nready & 1u, kWaitLimit));
+        ++nready;
+        tc_fence_after();
+      }
       uint64_t bh = b0, bm = b1, bl = b2;
-      for (int t = 0; t < ksteps && ok; t += KPC) {
+      for (int t = 0; t < ksteps && ok && m < nmat; t += KPC) {
         ok = all(mbar_poll(&full[s], fphase, kWaitLimit));
         if (!ok) break;
         if (trace && el && (int)(cc - cc_tile) < 8) trace[TR_FULL + (int)(cc - cc_tile)] = globaltimer_ns();
@@ -1188,7 +1202,13 @@ __device__ __noinline__ void mma_issuer_oz(Resolve resolve, int64_t total, const
           fphase ^= 1u;
         }
       }
-      if (ok && el) mma_commit(dbar);
+      if (ok && el && m < nmat) mma_commit(dbar);
+      if (ok && m == handover) {
+        // the tile's norms, while the matrix just issued runs (m == nmat: after the tile)
+        ok = await_handover(handed, need += kWorkThreads / 32, fail, kWaitLimit);
+        const FF* mine = sums + (ntile & 1) * (kMaxRed * kWorkThreads / 32);
+        if (ok) publish_tile(tr.prm->p, tr.tile, tile_sum(mine, tr.prm->p.nred, threadIdx.x & 31));
+      }
     }
   }
   if (!ok && el) {
@@ -1204,53 +1224,16 @@ __device__ __noinline__ void mma_issuer_oz(Resolve resolve, int64_t total, const
 // PK > 1: packed tiles of lane extent 128 / PK (see tab_w): the tensor core sees one
 // 128-row tile whose row R is lane row R % nl of column group R / nl, with the lane matrix
 // block-diagonal (PK copies), so no accumulator row and no epilogue thread is idle.
-// A finished tile's norm partials, waiting to be published: the work warps of the next tile
-// write them and draw the pass ticket while that tile's first GEMM runs (or after the CTA's
-// last tile), so the ticket's fence and atomic round trip stay off the tile chain.
-struct PendTicket {
-  const TcParams* prm;  // nullptr: nothing pending
-  double* partials;
-  unsigned int* counter;
-  int64_t tiles, tile;
-  int nred;
-  double red[kMaxRed];
-};
-
-// Warp 0 (all lanes): publish the pending partials; the CTA that draws a pass's last ticket
-// folds all of the pass's partials in FP64 in a fixed order and runs its scalar ops.
-__device__ __noinline__ void publish_pending(PendTicket& pd, int lane) {
-  const TcParams* q = pd.prm;
-  if (q == nullptr) return;
-  double* const part = pd.partials;
-  const int64_t tiles = pd.tiles;
-  const int nred = pd.nred;
-  unsigned int last = 0u;
-  EndOp end;
-  end.load(q->p);
-  if (lane == 0) {
-    for (int k = 0; k < nred; ++k) part[(int64_t)k * tiles + pd.tile] = pd.red[k];
-    __threadfence();
-    last = atomicAdd(pd.counter, 1u) == (unsigned int)(tiles - 1) ? 1u : 0u;
-  }
-  last = __shfl_sync(0xffffffffu, last, 0);
-  __syncwarp();
-  if (lane == 0) pd.prm = nullptr;
-  if (!last) return;
-  __threadfence();
-  finish_pass(q->p, end, part, tiles);
-}
-
-template <bool BF, bool OZ, int PK, typename Resolve>
+// ONE: a single pass, whose parameters are the kernel's.
+template <bool BF, bool OZ, int PK, bool ONE, typename Resolve>
 __device__ __forceinline__ void tc_persistent(Resolve resolve, const int64_t total) {
   using namespace tc;
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(16) TcParams tp;  // the pass of the work warps' current tile
   __shared__ TileTabs tabs;
   __shared__ uint32_t tmem_base_s;
-  __shared__ FF scratch[kMaxRed * (kWorkThreads / 32)];
-  __shared__ double blk_red[kMaxRed];
-  __shared__ PendTicket s_pend;
-  __shared__ volatile int s_fail;
+  __shared__ FF sums[2][kMaxRed * (kWorkThreads / 32)];  // norms of a tile, per work warp
+  __shared__ volatile int s_fail, s_handed;
   // split-BF16x6: column maxima of the two B operands of a tile (re and im of each column; a
   // packed tile keeps one set per column group: its block-diagonal matrix only sums products
   // within a group, so each group's columns carry their own quanta)
@@ -1258,7 +1241,10 @@ __device__ __forceinline__ void tc_persistent(Resolve resolve, const int64_t tot
   __shared__ uint32_t s_colmax[2][kCm];
   static_assert(sizeof(TcParams) % 4 == 0, "TcParams is copied as 32-bit words");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (blockIdx.x >= total) return;
+  if (blockIdx.x >= total) {
+    wait_for_previous();
+    return;
+  }
   const TcParams* first = resolve(blockIdx.x).prm;  // every tile of a launch shares n and parity mode
   const int nl = (int)first->p.g.n;  // the lane extent; n: the tile's rows (nl PK)
   const int n = nl * PK;
@@ -1282,13 +1268,18 @@ __device__ __forceinline__ void tc_persistent(Resolve resolve, const int64_t tot
     mbar_init(dbar + 3, 1);  // quiet
     fence_mbar_init();
     s_fail = 0;
-    s_pend.prm = nullptr;
+    s_handed = 0;
   }
   if (warp == 0) tmem_alloc(&tmem_base_s, kTmemCols);
+  // (ahead of the wait below: the parameters are no memory of the kernel before)
+  if constexpr (ONE)
+    for (int k = tid; k < (int)(sizeof(TcParams) / 4); k += kThreads)
+      reinterpret_cast<uint32_t*>(&tp)[k] = reinterpret_cast<const uint32_t*>(first)[k];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
+  wait_for_previous();
   const uint32_t sm0 = smem_u32(sm);
 
   if (warp == kWorkThreads / 32) {
@@ -1296,11 +1287,11 @@ __device__ __forceinline__ void tc_persistent(Resolve resolve, const int64_t tot
   } else if (warp == kWorkThreads / 32 + 1) {
     if constexpr (OZ) {
       if (S.mh == 2)
-        mma_issuer_oz<2>(resolve, total, S, sm0, L, tmem, &s_fail);
+        mma_issuer_oz<2>(resolve, total, S, sm0, L, tmem, &s_fail, sums[0], &s_handed);
       else
-        mma_issuer_oz<1>(resolve, total, S, sm0, L, tmem, &s_fail);
+        mma_issuer_oz<1>(resolve, total, S, sm0, L, tmem, &s_fail, sums[0], &s_handed);
     } else {
-      mma_issuer<BF>(resolve, total, S, sm0, L, tmem, &s_fail);
+      mma_issuer<BF>(resolve, total, S, sm0, L, tmem, &s_fail, sums[0], &s_handed);
     }
   } else {
     // ================= work warps
@@ -1318,8 +1309,9 @@ __device__ __forceinline__ void tc_persistent(Resolve resolve, const int64_t tot
     const uint32_t bhb2 = L.bhalf;  // bytes between the two B halves
     float* stg = bhi;  // output staging reuses the B_hi area once the last GEMM is done
     uint32_t drains = 0;
-    const TcParams* cur = nullptr;
-    for (int64_t gt = blockIdx.x; gt < total; gt += gridDim.x) {
+    const TcParams* cur = ONE ? first : nullptr;
+    int ntile = 0;
+    for (int64_t gt = blockIdx.x; gt < total; gt += gridDim.x, ++ntile) {
       const TileRef r = resolve(gt);
       if (r.prm != cur) {
         for (int k = tid; k < (int)(sizeof(TcParams) / 4); k += kWorkThreads)
@@ -1409,11 +1401,14 @@ __device__ __forceinline__ void tc_persistent(Resolve resolve, const int64_t tot
         }
       }
 
-      // the previous tile's partials and ticket, while this tile's first GEMM runs
-      if (warp == 0) publish_pending(s_pend, lane);
-
       bool ok = true;
-      for (int m = 0; m < tp.nmat && ok; ++m) {
+      for (int m = 0; m <= tp.nmat; ++m) {
+        if (m == tp.handover) {
+          // the tile's norms are complete: the issuing warp publishes them
+          warp_sums(acc, p.nred, sums[ntile & 1]);
+          if (lane == 0) hand_over(&s_handed);
+        }
+        if (m == tp.nmat) break;
         const int kind = tp.parity[m];
         const bool last = m + 1 == tp.nmat;
         const int next = last ? -1 : tp.parity[m + 1];
@@ -1585,20 +1580,6 @@ __device__ __forceinline__ void tc_persistent(Resolve resolve, const int64_t tot
       }
       work_sync();  // staging complete
 
-      // norm partials of this tile (float-float, fixed order) and the pass ticket first, so
-      // the fence waits for no state store and the ticket's round trip overlaps the store
-      block_sums(acc, p.nred, scratch, blk_red);
-      if (tid == 0) {
-        // published by the next tile (or after the last one): see PendTicket
-        s_pend.partials = p.partials;
-        s_pend.counter = p.counter;
-        s_pend.tiles = g.tiles;
-        s_pend.tile = tile;
-        s_pend.nred = p.nred;
-        for (int k = 0; k < p.nred; ++k) s_pend.red[k] = blk_red[k];
-        s_pend.prm = r.prm;
-      }
-
       // coalesced store of the staged tile: thread = complex column
       {
         const int c = tid % S.bn, h = tid / S.bn, G = S.groups;
@@ -1616,9 +1597,6 @@ __device__ __forceinline__ void tc_persistent(Resolve resolve, const int64_t tot
       work_sync();  // the staging and the pass copy are free for the next tile
       if (tid == 0) trace_mark(tp, tile, TR_END);
     }
-    // the last tile's partials (a CTA that stopped on a failed wait publishes nothing: the
-    // pass has recorded its error)
-    if (warp == 0 && !s_fail) publish_pending(s_pend, lane);
   }
   __syncthreads();
   if (tid == 0 && s_fail) {
@@ -1636,7 +1614,7 @@ __device__ __forceinline__ void tc_persistent(Resolve resolve, const int64_t tot
 template <int OPM, int PK = 1>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) angular_tc_kernel(const __grid_constant__ TcParams tp) {
   const TcParams* prm = &tp;
-  tc_persistent<OPM != 0, OPM == 2, PK>([prm](int64_t t) { return TileRef{prm, t}; }, tp.p.g.tiles);
+  tc_persistent<OPM != 0, OPM == 2, PK, true>([prm](int64_t t) { return TileRef{prm, t}; }, tp.p.g.tiles);
 }
 
 // Many propagations' lane-matrix passes in one launch (all with the same lane extent):
@@ -1653,7 +1631,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) angular_tc_kernel_batche
     const uint2 o = __ldg(owners + b);
     return TileRef{params + o.x, (int64_t)o.y};
   };
-  tc_persistent<OPM != 0, OPM == 2, PK>(resolve, total);
+  tc_persistent<OPM != 0, OPM == 2, PK, false>(resolve, total);
 }
 
 // ------------------------------------------------------------------ host side
@@ -1697,6 +1675,7 @@ void make_tc_params(const PassParams& p, const int* mat_op, int nmat, const floa
       tp.slice_stride[i] = slice_stride[i];
     }
   }
+  tp.handover = pass_handover(p, mat_op, nmat);
   tp.error_slot = error_slot;
   // the distinct full-size tables after the first matrix (the kernel prefetches their tile rows)
   for (int oi = nmat > 0 ? mat_op[0] + 1 : p.nops; oi < p.nops && tp.npre < 4; ++oi) {
@@ -1727,7 +1706,8 @@ static size_t tc_max_dynamic_smem() {
 // persistent CTAs with the whole shared-memory carveout
 static bool configure_once(const void* kern, bool& flag) {
   if (flag) return true;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_max_dynamic_smem()) !=
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)std::max(tc_max_dynamic_smem(), kHalfSmem)) !=
       cudaSuccess)
     return false;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) !=
@@ -2026,15 +2006,16 @@ cudaError_t launch_angular_tc(const PassParams& p, const int* mat_op, int nmat, 
   if (!configure_once(kerns[v], configured[v])) return cudaGetLastError();
   if (smem > tc_max_dynamic_smem()) return cudaErrorInvalidValue;
   const unsigned grid = persistent_grid(p.g.tiles, ctas_per_sm);
+  cudaError_t e;
   switch (v) {
-    case 4: angular_tc_kernel<2, 4><<<grid, kThreads, smem, s>>>(tp); break;
-    case 3: angular_tc_kernel<2, 2><<<grid, kThreads, smem, s>>>(tp); break;
-    case 2: angular_tc_kernel<2><<<grid, kThreads, smem, s>>>(tp); break;
-    case 1: angular_tc_kernel<1><<<grid, kThreads, smem, s>>>(tp); break;
-    default: angular_tc_kernel<0><<<grid, kThreads, smem, s>>>(tp); break;
+    case 4: e = launch_overlapped(angular_tc_kernel<2, 4>, grid, kThreads, one_block_per_sm(grid, smem), s, tp); break;
+    case 3: e = launch_overlapped(angular_tc_kernel<2, 2>, grid, kThreads, one_block_per_sm(grid, smem), s, tp); break;
+    case 2: e = launch_overlapped(angular_tc_kernel<2>, grid, kThreads, one_block_per_sm(grid, smem), s, tp); break;
+    case 1: e = launch_overlapped(angular_tc_kernel<1>, grid, kThreads, one_block_per_sm(grid, smem), s, tp); break;
+    default: e = launch_overlapped(angular_tc_kernel<0>, grid, kThreads, one_block_per_sm(grid, smem), s, tp); break;
   }
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace so

@@ -16,6 +16,7 @@
 // 64 of 2048 in FP64 28.9 / 18.3, 256 of 256 22.9 / 12.6, 45 of 1000 (through 2048) 53.7 / 28.7.
 #pragma once
 #include "fx_stage.cuh"
+#include "overlap.cuh"
 
 namespace so {
 
@@ -231,6 +232,7 @@ template <int LGN, bool FF, bool CHIRP>
 __global__ void __launch_bounds__(kPairThreads, 1)
     fx_pair_kernel(const __grid_constant__ PassParams one, const PassParams* __restrict__ params,
                    const int64_t* __restrict__ offsets, int count) {
+  wait_for_previous();
   if (params == nullptr) {
     if constexpr (CHIRP)
       fx_chirp_tile<LGN, FF>(one, blockIdx.x);
@@ -265,9 +267,8 @@ cudaError_t launch_lgn(const PassParams* one, const PassParams* params, const in
   }
   if (smem > 220 * 1024 || threads > kPairThreads) return cudaErrorInvalidValue;
   static const PassParams none{};
-  kern<<<(unsigned)blocks, threads, smem, s>>>(one ? *one : none, params, offsets, count);
   count_launch();
-  return cudaGetLastError();
+  return launch_overlapped(kern, (unsigned)blocks, threads, one_block_per_sm(blocks, smem), s, one ? *one : none, params, offsets, count);
 }
 
 // lgn: log2 of the lane length (CHIRP: of M)

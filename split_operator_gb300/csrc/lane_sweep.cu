@@ -27,6 +27,7 @@
 
 #include "common.cuh"
 #include "ff.cuh"
+#include "overlap.cuh"
 
 namespace so {
 
@@ -1210,6 +1211,7 @@ __device__ __forceinline__ void fft_pair_tile_ct(const PassParams& pp, int64_t t
 
 template <int LGN>
 __global__ void __launch_bounds__(512, 2) fft_pair_kernel_ct(const __grid_constant__ PassParams p) {
+  wait_for_previous();
   fft_pair_tile_ct<LGN>(p, blockIdx.x);
 }
 
@@ -1262,8 +1264,8 @@ static cudaError_t launch_pair_ct(const PassParams& p, cudaStream_t s) {
   static bool done = false;
   cudaError_t e = configure_once(fft_pair_kernel_ct<LGN>, done);
   if (e != cudaSuccess) return e;
-  fft_pair_kernel_ct<LGN><<<(unsigned)p.g.tiles, fft_pair_block(p), fft_pair_smem(p.g, false), s>>>(p);
-  return cudaGetLastError();
+  return launch_overlapped(fft_pair_kernel_ct<LGN>, (unsigned)p.g.tiles, fft_pair_block(p),
+                           one_block_per_sm(p.g.tiles, fft_pair_smem(p.g, false)), s, p);
 }
 
 template <int LGN>

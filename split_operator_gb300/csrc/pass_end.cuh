@@ -10,6 +10,19 @@
 #include "common.cuh"
 
 namespace so {
+
+// The first lane matrix (0 .. nmat; nmat: the end of the tile) by whose product a tile's norms are
+// complete and its factors from slots taken: there the tile hands its partials over, and the
+// chain below runs beside the rest of the tile.
+inline int pass_handover(const PassParams& p, const int* mat_op, int nmat) {
+  int last = -1;
+  for (int i = 0; i < p.nops; ++i)
+    if (p.ops[i].kind == OP_NORM || p.ops[i].kind == OP_SCALE) last = i;
+  int m = 0;
+  while (m < nmat && last > mat_op[m]) ++m;
+  return m;
+}
+
 namespace {
 
 static_assert(kMaxOps <= 32 && kMaxRed == 8, "one lane per op; three halving levels");
@@ -133,6 +146,48 @@ __device__ __forceinline__ void finish_pass(const PassParams& p, EndOp& op, cons
     __syncwarp();  // stores of one slot by two lanes stay in program order
   }
   if (lane == 0) *counter = 0u;
+}
+
+// The tensor-core kernels' warps that issue products are idle between two of them, and take a
+// tile's partials from there: the work warps leave their warp sums in shared memory, count
+// themselves in, and go on with the tile.  On the work warps' own path the ticket took 3 us of
+// every pass, and the last CTA's fold another 5.
+__device__ __forceinline__ void hand_over(volatile int* handed) {  // lane 0 of a work warp
+  __threadfence_block();
+  atomicAdd(const_cast<int*>(handed), 1);
+}
+// One whole warp: waits until `need` warps have handed over (false after limit_ns, or on *fail).
+__device__ __forceinline__ bool await_handover(volatile int* handed, int need, volatile int* fail,
+                                               unsigned long long limit_ns) {
+  unsigned long long t0, t1;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+  while (__any_sync(0xffffffffu, *handed < need)) {
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+    if (__any_sync(0xffffffffu, *fail != 0 || t1 - t0 > limit_ns)) return false;
+    __nanosleep(40);
+  }
+  __threadfence_block();
+  return true;
+}
+// One whole warp: the tile's partials (lane k: reduction k) and its ticket; the last one finishes
+// the pass.  p may lie in any memory.
+__device__ __noinline__ void publish_tile(const PassParams& p, int64_t tile, double v) {
+  const int lane = threadIdx.x & 31;
+  double* const part = p.partials;
+  const int64_t tiles = p.g.tiles;
+  EndOp end;
+  end.load(p);
+  if (lane < p.nred) part[(int64_t)lane * tiles + tile] = v;
+  __syncwarp();
+  unsigned int last = 0u;
+  if (lane == 0) {
+    __threadfence();
+    last = atomicAdd(p.counter, 1u) == (unsigned int)(tiles - 1) ? 1u : 0u;
+  }
+  last = __shfl_sync(0xffffffffu, last, 0);
+  if (!last) return;
+  __threadfence();
+  finish_pass(p, end, part, tiles);
 }
 
 }  // namespace
