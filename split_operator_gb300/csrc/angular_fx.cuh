@@ -215,7 +215,9 @@ struct FxResolve {
   }
 };
 
-// Warp 16, lane 0: the digit images of every tile's matrices, digit by digit, through the ring.
+// Warp 16, lane 0: the digit images of every tile's matrices through the ring, all digits of 32 K
+// values, then the next 32: the last digits of a chunk take few products, and in this order the
+// copies keep an even pace.
 template <int MH>
 __device__ __noinline__ void fx_producer(FxResolve resolve, int64_t total, uint32_t ring, uint64_t* full,
                                          uint64_t* empty, volatile int* fail) {
@@ -228,16 +230,17 @@ __device__ __noinline__ void fx_producer(FxResolve resolve, int64_t total, uint3
   bool ok = true;
   for (int64_t gt = blockIdx.x; gt < total && ok && !*fail; gt += gridDim.x) {
     const FxTile r = resolve(gt);
-    const int chunks = kDigits * (r.prm->kp / 32);
+    const int nk = r.prm->kp / 32;
     for (int m = 0; m < r.prm->nmat && ok; ++m) {
       const unsigned char* img = fx_image(*r.prm, m, r.tile);
-      for (int q = 0; q < chunks; ++q) {
+      for (int q = 0; q < kDigits * nk; ++q) {
+        const int part = (q % kDigits) * nk + q / kDigits;  // stored digit by digit
         if (use > 0 && !mbar_poll(&empty[s], (use - 1) & 1u, kFxWait)) {
           ok = false;
           break;
         }
         mbar_expect_tx(&full[s], bytes);
-        bulk_g2s(sm_ptr(ring + (uint32_t)s * bytes), img + (size_t)q * bytes, bytes, &full[s]);
+        bulk_g2s(sm_ptr(ring + (uint32_t)s * bytes), img + (size_t)part * bytes, bytes, &full[s]);
         ++cc;
         if (++s == ns) {
           s = 0;
@@ -271,9 +274,9 @@ __device__ __forceinline__ double fx_tile_sum(const double (&red)[kMaxRed][kFxWo
   return v;
 }
 
-// Warp 17: per matrix, once its B digits are written, the products of A digit i (chunk by chunk)
-// with the B digits j <= 6 - i into accumulator i + j.  The warp stays converged and its elected
-// lane issues (elect_one).
+// Warp 17: per matrix, once its B digits are written, the products of A digit i with the B digits
+// j <= 6 - i into accumulator i + j, for 32 K values after the other.  The warp stays converged and
+// its elected lane issues (elect_one).
 template <int N, int MH>
 __device__ __noinline__ void fx_issuer(FxResolve resolve, int64_t total, uint32_t ring, uint32_t b0, uint64_t* full,
                                        uint64_t* empty, uint64_t* dbar, uint64_t* bready, uint64_t* quiet,
@@ -301,34 +304,34 @@ __device__ __noinline__ void fx_issuer(FxResolve resolve, int64_t total, uint32_
         ok = __all_sync(0xffffffffu, mbar_poll(bready, nready & 1u, kFxWait));
         ++nready;
         tc_fence_after();
-      }
-#pragma unroll
-      for (int i = 0; i < kDigits; ++i) {
         uint64_t bk = bfirst;
-        for (int q = 0; q < nk && ok && m < nmat; ++q) {
-          ok = __all_sync(0xffffffffu, mbar_poll(&full[s], phase, kFxWait));
-          if (!ok) break;
-          tc_fence_after();
-          const uint64_t a = smem_desc_at(abits, ring + (uint32_t)s * bytes);
+        for (int q = 0; q < nk && ok; ++q) {
 #pragma unroll
-          for (int ks = 0; ks < 2; ++ks)
+          for (int i = 0; i < kDigits; ++i) {
+            if (ok) ok = __all_sync(0xffffffffu, mbar_poll(&full[s], phase, kFxWait));
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t a = smem_desc_at(abits, ring + (uint32_t)s * bytes);
 #pragma unroll
-            for (int h = 0; h < MH; ++h)
+            for (int ks = 0; ks < 2; ++ks)
 #pragma unroll
-              for (int j = 0; j < kDigits - i; ++j)
-                mma_f16_warp(tmem + (uint32_t)((i + j) * MH * N + h * N),
-                             a + (uint64_t)(ks * (256 >> 4) + h * (kChunkRowBytes >> 4)),
-                             bk + (uint64_t)(ks * (256 >> 4)) + (uint64_t)j * bdig, idesc,
-                             (i | ks) != 0 || q != 0 ? 1u : 0u, el);
-          bk += 512 >> 4;
-          if (el) mma_commit(&empty[s]);
-          if (++s == ns) {
-            s = 0;
-            phase ^= 1u;
+              for (int h = 0; h < MH; ++h)
+#pragma unroll
+                for (int j = 0; j < kDigits - i; ++j)
+                  mma_f16_warp(tmem + (uint32_t)((i + j) * MH * N + h * N),
+                               a + (uint64_t)(ks * (256 >> 4) + h * (kChunkRowBytes >> 4)),
+                               bk + (uint64_t)(ks * (256 >> 4)) + (uint64_t)j * bdig, idesc,
+                               (i | ks) != 0 || q != 0 ? 1u : 0u, el);
+            if (el) mma_commit(&empty[s]);
+            if (++s == ns) {
+              s = 0;
+              phase ^= 1u;
+            }
           }
+          bk += 512 >> 4;
         }
+        if (ok && el) mma_commit(dbar);
       }
-      if (ok && el && m < nmat) mma_commit(dbar);
       if (ok && m == handover) {
         // the tile's norms, while the matrix just issued runs (m == nmat: after the tile)
         ok = await_handover(handed, need += kFxWork / 32, fail, kFxWait);
