@@ -207,6 +207,35 @@ cudaError_t launch_import(void* dst, int dst_real, const double* src, const Geom
   return e;
 }
 
+// the largest |v|^2 of n complex values as the bits of a double (infinity when one is not finite
+// or above 1e300); out: zero at the launch
+__global__ void table_max_kernel(unsigned long long* out, const double2* src, int64_t n) {
+  double m = 0.0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const double2 v = src[i];
+    const double a = __dadd_rn(__dmul_rn(v.x, v.x), __dmul_rn(v.y, v.y));
+    if (!(a <= 1e300))
+      m = __longlong_as_double(0x7ff0000000000000ll);
+    else if (a > m)
+      m = a;
+  }
+  // non-negative doubles order like their bits
+  unsigned long long b = (unsigned long long)__double_as_longlong(m);
+  for (int off = 16; off > 0; off >>= 1) {
+    const unsigned long long o = __shfl_xor_sync(0xffffffffu, b, off);
+    b = o > b ? o : b;
+  }
+  if ((threadIdx.x & 31) == 0) atomicMax(out, b);
+}
+
+cudaError_t launch_table_max(unsigned long long* out, const double* src, int64_t n, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(out, 0, sizeof(*out), st);
+  if (e != cudaSuccess) return e;
+  table_max_kernel<<<blocks_for(n), 256, 0, st>>>(out, (const double2*)src, n);
+  count_launch();
+  return cudaGetLastError();
+}
+
 cudaError_t launch_export(double* dst, const void* src, int src_real, const Geometry& g, cudaStream_t st) {
   const int64_t total = total_of(g);
   if (layout_is_transpose2(g)) {

@@ -268,6 +268,8 @@ cudaError_t launch_scalar_program(const PassParams& p, cudaStream_t s);
 // real: the state precision of the device side (kRealF32, kRealF64, kRealFF)
 // dst (storage order, precision of dst) <- src (logical row-major complex128)
 cudaError_t launch_import(void* dst, int dst_real, const double* src, const Geometry& g, cudaStream_t s);
+// *out (device) <- the largest |v|^2 of n complex128 values, as the bits of a double
+cudaError_t launch_table_max(unsigned long long* out, const double* src, int64_t n, cudaStream_t s);
 // storage order is the logical order / the transpose of a two-axis logical order (the
 // layouts whose import and export stay coalesced on both sides)
 bool layout_is_identity(const Geometry& g);

@@ -287,32 +287,36 @@ const void* Engine::table_1d(const void* key, uint64_t version, const std::vecto
   return c.buf.ptr;
 }
 
+static Geometry flat_geometry(const Engine& e) {
+  Geometry g{};
+  g.ndim = (int)e.shape.size();
+  for (int q = 0; q < g.ndim; ++q) {
+    g.perm[q] = e.perm[q];
+    g.sshape[q] = (int64_t)e.shape[e.perm[q]];
+  }
+  return g;
+}
+
 const void* Engine::table_nd(const void* key, uint64_t version, const std::vector<cplx>& t) {
   auto& c = tables_[{key, 1}];
   if (c.buf.ptr && c.version == version) return c.buf.ptr;
   if (c.buf.ptr) flush();
-  // logical row-major -> storage order
-  const int nd = (int)shape.size();
-  std::vector<cplx> st(t.size());
-  std::vector<size_t> lstride(nd);
-  size_t acc = 1;
-  for (int a = nd - 1; a >= 0; --a) {
-    lstride[a] = acc;
-    acc *= shape[a];
+  // logical row-major -> storage order and precision, on the device (a host loop over the strides
+  // took 6 ms of the first pass for 524,288 points); the last 8 bytes of raw: the largest magnitude
+  const size_t b = t.size() * sizeof(cplx);
+  DeviceBuffer raw(b + sizeof(unsigned long long));
+  unsigned long long* const top = reinterpret_cast<unsigned long long*>(raw.as<unsigned char>() + b);
+  cuda_check(cudaMemcpyAsync(raw.ptr, t.data(), b, cudaMemcpyHostToDevice, stream), "table upload");
+  if (c.buf.bytes != t.size() * elem_bytes()) c.buf = DeviceBuffer(t.size() * elem_bytes());
+  cuda_check(launch_import(c.buf.ptr, real, raw.as<double>(), flat_geometry(*this), stream), "table import");
+  double max2 = 0.0;
+  if (fx) {
+    cuda_check(launch_table_max(top, raw.as<double>(), (int64_t)t.size(), stream), "table maximum");
+    cuda_check(cudaMemcpyAsync(&max2, top, sizeof(max2), cudaMemcpyDeviceToHost, stream), "table maximum");
   }
-  std::vector<size_t> idx(nd, 0);
-  for (size_t s = 0; s < t.size(); ++s) {
-    size_t li = 0, r = s;
-    for (int q = nd - 1; q >= 0; --q) {
-      const size_t ext = shape[perm[q]];
-      li += (r % ext) * lstride[perm[q]];
-      r /= ext;
-    }
-    st[s] = t[li];
-  }
-  upload_complex(c.buf, st, real, stream);
+  cuda_check(cudaStreamSynchronize(stream), "table upload sync");
+  if (fx) c.max_abs = std::sqrt(max2);
   c.fx = DeviceBuffer();
-  if (fx) c.max_abs = table_max(t);
   c.version = version;
   return c.buf.ptr;
 }
@@ -1168,16 +1172,6 @@ void Engine::check_nonfinite() {
     write_slot(nonfinite_slot, 0.0);
     throw Error(SO_ERR_NONFINITE, "a norm of the wave function is not finite");
   }
-}
-
-static Geometry flat_geometry(const Engine& e) {
-  Geometry g{};
-  g.ndim = (int)e.shape.size();
-  for (int q = 0; q < g.ndim; ++q) {
-    g.perm[q] = e.perm[q];
-    g.sshape[q] = (int64_t)e.shape[e.perm[q]];
-  }
-  return g;
 }
 
 static bool identity_perm(const std::vector<int>& p) {
