@@ -58,7 +58,6 @@ namespace {
 constexpr int kFxWork = 512;                 // work threads (warps 0-15)
 constexpr int kFxThreads = kFxWork + 64;     // + warp 16 (TMA) + warp 17 (MMA)
 constexpr int kDigits = 7;
-constexpr uint32_t kRingBytes = 65536;
 constexpr uint32_t kChunkRowBytes = 8192;    // 128 rows x 32 K values of one digit
 constexpr uint64_t kFxWait = 2000000000ull;  // 2 s per wait
 constexpr int kFxTabSlots = 4;               // DIAG1D ops on a non-lane axis per pass
@@ -67,6 +66,7 @@ constexpr int kNoTerm = 1 << 20;             // exponent of a zero weight: below
 constexpr int kFxPoison = 1 << 24;           // exponent of a column with a value that is not finite
 
 __host__ __device__ constexpr uint32_t fx_b_bytes(int cols, int kp) { return (uint32_t)(2 * cols * kp * 2); }
+constexpr uint32_t kRingBytes = 65536;
 __host__ __device__ constexpr uint32_t fx_tc_smem(int cols, int kp) {
   return kRingBytes + kDigits * fx_b_bytes(cols, kp);
 }
@@ -170,7 +170,7 @@ struct FxTabs {
   int cole[2][kFxMaxCols];              // column maxima: biased exponents
   int coler[kFxMaxCols];                // the same at a ROUND
   int colb[kFxMaxCols];                 // exponent bound of the column's B operand
-  int nonident[kFxTabSlots];            // the factors of this tile are not all 1
+  int nonident[kFxTabSlots];            // the factors of this tile: 0 all are 1, 1 all real, else complex
   int8_t slot[kMaxOps];
   double red[2][kMaxRed][kFxWork / 32];  // norms: the warps' sums (of every second tile)
 };
@@ -365,6 +365,29 @@ struct RowWeight {
   }
 };
 
+// v 2^e rounded as a store in FP64 would (fx_to_f64), in place; E: the biased exponent of the stored
+// value (0: it is zero, and so is the result; 2047: infinite).
+__device__ __forceinline__ i64 round_f64(i64 v, int e, int& E) {
+  const i64 s = v >> 63;
+  unsigned long long a = (unsigned long long)((v ^ s) - s);
+  const int lz = __clzll((i64)a), drop = 11 - lz;
+  const int before = 63 - lz + e + 1023;
+  if (drop > 0) a = ((a >> drop) + ((a >> (drop - 1)) & 1ull)) << drop;
+  const int after = 63 - __clzll((i64)a) + e + 1023;  // one more after a carry
+  if (a == 0 || before < 1) a = 0;
+  E = a == 0 ? 0 : min(after, 2047);
+  return ((i64)a ^ s) - s;
+}
+// ... and as the load of that value would scale it (raw_to_fx): v 2^-k
+__device__ __forceinline__ i64 rescale_f64(i64 v, int k) {
+  if (k <= 0) return v << (k < -63 ? 63 : -k);
+  const i64 s = v >> 63;
+  const unsigned long long a = (unsigned long long)((v ^ s) - s);
+  unsigned long long r = k > 62 ? 0ull : ((a >> (k - 1)) + 1ull) >> 1;
+  if (r == 0 && a != 0) r = 1;  // shr_round keeps a unit of what is not zero
+  return ((i64)r ^ s) - s;
+}
+
 // The work threads' view of a tile: row j, complex columns c0 .. c0 + NB - 1.
 template <int NB, bool FF>
 struct FxWork {
@@ -399,9 +422,17 @@ struct FxWork {
 #pragma unroll
               for (int u = 0; u < NB; ++u) w[u] = cmul<0>(w[u], t);
             }
-          } else if (T.nonident[T.slot[oi]]) {
+          } else if (const int kind = T.nonident[T.slot[oi]]) {
+            if (kind & 2) {
 #pragma unroll
-            for (int u = 0; u < NB; ++u) w[u] = cmul<0>(w[u], T.colt[T.slot[oi]][c0 + u]);
+              for (int u = 0; u < NB; ++u) w[u] = cmul<0>(w[u], T.colt[T.slot[oi]][c0 + u]);
+            } else {  // real factors (a mask)
+#pragma unroll
+              for (int u = 0; u < NB; ++u) {
+                const int4 t = T.colt[T.slot[oi]][c0 + u];
+                w[u] = cmul<0>(w[u], int4{t.x, t.y, 0, 0});
+              }
+            }
           }
           break;
         }
@@ -464,10 +495,23 @@ struct FxWork {
             const int x = T.colx[c0 + u];
             const bool ok = row_ok && c0 + u < ncols && x != kPoison;
             const int e = x + rowx + xs;
-            raw[u] = {ok ? fx_to_raw<FF>(w[u].x, e) : 0, ok ? fx_to_raw<FF>(w[u].y, e) : 0};
-            mx[u] = __reduce_max_sync(0xffffffffu, max(raw_exp<FF>(raw[u].x), raw_exp<FF>(raw[u].y)));
+            int m;
+            if constexpr (FF) {
+              raw[u] = {ok ? fx_to_raw<FF>(w[u].x, e) : 0, ok ? fx_to_raw<FF>(w[u].y, e) : 0};
+              m = max(raw_exp<FF>(raw[u].x), raw_exp<FF>(raw[u].y));
+            } else {
+              // FP64: rounded in place (packing and unpacking would only move the bits)
+              const i64 re = ok ? w[u].x : 0, im = ok ? w[u].y : 0;
+              int ex, ey;
+              w[u] = {round_f64(re, e, ex), round_f64(im, e, ey)};
+              m = max(ex, ey);
+            }
+            mx[u] = __reduce_max_sync(0xffffffffu, m);
           }
           if (threadIdx.x < 4 * NB) T.coler[threadIdx.x] = 0;
+          int unit[NB];
+#pragma unroll
+          for (int u = 0; u < NB; ++u) unit[u] = T.colx[c0 + u] + rowx + xs;
           fx_work_sync();
 #pragma unroll
           for (int u = 0; u < NB; ++u)
@@ -482,7 +526,12 @@ struct FxWork {
           for (int u = 0; u < NB; ++u) {
             const int e = T.coler[c0 + u];
             const bool live = e != 2047 && e != 0;
-            w[u] = {live ? raw_to_fx<FF>(raw[u].x, e - 1022) : 0, live ? raw_to_fx<FF>(raw[u].y, e - 1022) : 0};
+            if constexpr (FF) {
+              w[u] = {live ? raw_to_fx<FF>(raw[u].x, e - 1022) : 0, live ? raw_to_fx<FF>(raw[u].y, e - 1022) : 0};
+            } else {
+              const int k = e - 1082 - unit[u];
+              w[u] = {live ? rescale_f64(w[u].x, k) : 0, live ? rescale_f64(w[u].y, k) : 0};
+            }
           }
           rowx = 0;
           xs = 0;
@@ -665,7 +714,8 @@ __global__ void __launch_bounds__(kFxThreads, 1)
         } else if (op.kind == OP_DIAG1D && op.axis != g.sweep_axis) {
           const int4 t = __ldg(reinterpret_cast<const int4*>(op.ptr) + fx_coord(g, op.axis, o, i));
           T.colt[T.slot[oi]][c] = t;
-          if (t.x != 0 || t.y != (1 << 30) || t.z != 0 || t.w != 0) T.nonident[T.slot[oi]] = 1;
+          const int kind = (t.x != 0 || t.y != (1 << 30) ? 1 : 0) | (t.z != 0 || t.w != 0 ? 3 : 0);
+          if (kind) atomicOr(&T.nonident[T.slot[oi]], kind);
         }
       }
       // column exponents
