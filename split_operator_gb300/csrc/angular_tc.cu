@@ -329,7 +329,18 @@ __device__ __forceinline__ void apply_row(const PassParams& p, const TileTabs& T
       }
       case OP_DIAGND: {
         const float2* t = reinterpret_cast<const float2*>(op.ptr) + ix0;
-        if ((reinterpret_cast<uintptr_t>(t) & 15u) == 0) {
+        if (NB % 4 == 0 && (reinterpret_cast<uintptr_t>(t) & 31u) == 0) {
+          // 32 bytes an access: the lanes' rows lie apart, so each access then takes whole sectors
+          float2 tv[NB];
+#pragma unroll
+          for (int q = 0; q < NB; q += 4)
+            asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                : "=f"(tv[q].x), "=f"(tv[q].y), "=f"(tv[q + 1].x), "=f"(tv[q + 1].y), "=f"(tv[q + 2].x),
+                  "=f"(tv[q + 2].y), "=f"(tv[q + 3].x), "=f"(tv[q + 3].y)
+                : "l"(t + q));
+#pragma unroll
+          for (int u = 0; u < NB; ++u) v[u] = cmulf(v[u], tv[u]);
+        } else if ((reinterpret_cast<uintptr_t>(t) & 15u) == 0) {
           float4 tv[NB / 2];
 #pragma unroll
           for (int q = 0; q < NB / 2; ++q) tv[q] = __ldg(reinterpret_cast<const float4*>(t) + q);
@@ -877,13 +888,16 @@ __device__ __forceinline__ void write_b_row_oz(const float2 (&x)[NV], int c0, in
 template <int NV>
 __device__ __forceinline__ void colmax_rows(const float2 (&x)[NV], int c0, uint32_t* cm) {
   const int lane = threadIdx.x & 31;
+  static_assert(NV <= 16, "a lane per value");
+  uint32_t mine = 0u;
 #pragma unroll
   for (int u = 0; u < NV; ++u) {
     const uint32_t mr = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(x[u].x)));
     const uint32_t mi = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(x[u].y)));
-    if (lane == (2 * u) % 32) atomicMax(cm + 2 * (c0 + u), mr);
-    if (lane == (2 * u + 1) % 32) atomicMax(cm + 2 * (c0 + u) + 1, mi);
+    if (lane == 2 * u) mine = mr;
+    if (lane == 2 * u + 1) mine = mi;
   }
+  if (lane < 2 * NV) atomicMax(cm + 2 * c0 + lane, mine);
 }
 
 // NV complex values of row j, columns c0 .., into the output staging
