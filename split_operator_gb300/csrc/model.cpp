@@ -304,18 +304,45 @@ const void* Engine::table_nd(const void* key, uint64_t version, const std::vecto
   // logical row-major -> storage order and precision, on the device (a host loop over the strides
   // took 6 ms of the first pass for 524,288 points); the last 8 bytes of raw: the largest magnitude
   const size_t b = t.size() * sizeof(cplx);
-  DeviceBuffer raw(b + sizeof(unsigned long long));
-  unsigned long long* const top = reinterpret_cast<unsigned long long*>(raw.as<unsigned char>() + b);
-  cuda_check(cudaMemcpyAsync(raw.ptr, t.data(), b, cudaMemcpyHostToDevice, stream), "table upload");
-  if (c.buf.bytes != t.size() * elem_bytes()) c.buf = DeviceBuffer(t.size() * elem_bytes());
-  cuda_check(launch_import(c.buf.ptr, real, raw.as<double>(), flat_geometry(*this), stream), "table import");
-  double max2 = 0.0;
-  if (fx) {
-    cuda_check(launch_table_max(top, raw.as<double>(), (int64_t)t.size(), stream), "table maximum");
-    cuda_check(cudaMemcpyAsync(&max2, top, sizeof(max2), cudaMemcpyDeviceToHost, stream), "table maximum");
+  DeviceBuffer raw;
+  try {
+    raw = DeviceBuffer(b + sizeof(unsigned long long));
+  } catch (const Error&) {
+    cudaGetLastError();  // no room beside the table: the host's order below
   }
-  cuda_check(cudaStreamSynchronize(stream), "table upload sync");
-  if (fx) c.max_abs = std::sqrt(max2);
+  if (raw.ptr) {
+    unsigned long long* const top = reinterpret_cast<unsigned long long*>(raw.as<unsigned char>() + b);
+    cuda_check(cudaMemcpyAsync(raw.ptr, t.data(), b, cudaMemcpyHostToDevice, stream), "table upload");
+    if (c.buf.bytes != t.size() * elem_bytes()) c.buf = DeviceBuffer(t.size() * elem_bytes());
+    cuda_check(launch_import(c.buf.ptr, real, raw.as<double>(), flat_geometry(*this), stream), "table import");
+    double max2 = 0.0;
+    if (fx) {
+      cuda_check(launch_table_max(top, raw.as<double>(), (int64_t)t.size(), stream), "table maximum");
+      cuda_check(cudaMemcpyAsync(&max2, top, sizeof(max2), cudaMemcpyDeviceToHost, stream), "table maximum");
+    }
+    cuda_check(cudaStreamSynchronize(stream), "table upload sync");
+    if (fx) c.max_abs = std::sqrt(max2);
+  } else {
+    const int nd = (int)shape.size();
+    std::vector<cplx> st(t.size());
+    std::vector<size_t> lstride(nd);
+    size_t acc = 1;
+    for (int a = nd - 1; a >= 0; --a) {
+      lstride[a] = acc;
+      acc *= shape[a];
+    }
+    for (size_t s = 0; s < t.size(); ++s) {
+      size_t li = 0, r = s;
+      for (int q = nd - 1; q >= 0; --q) {
+        const size_t ext = shape[perm[q]];
+        li += (r % ext) * lstride[perm[q]];
+        r /= ext;
+      }
+      st[s] = t[li];
+    }
+    upload_complex(c.buf, st, real, stream);
+    if (fx) c.max_abs = table_max(t);
+  }
   c.fx = DeviceBuffer();
   c.version = version;
   return c.buf.ptr;
