@@ -404,6 +404,39 @@ __device__ __forceinline__ i64 rescale_f64(i64 v, int k) {
   return ((i64)r ^ s) - s;
 }
 
+// The tile's tables of weights and factors (all but SCALE's); clears the column maxima.  All work threads.
+__device__ __forceinline__ void fx_tables(FxTabs& T, const PassParams& p, int64_t o, int64_t i0, int ncols, int bn) {
+  const Geometry& g = p.g;
+  const int tid = threadIdx.x;
+  if (tid < 2 * kFxMaxCols) T.cole[tid >> 5][tid & 31] = 0;
+  if (tid < kFxTabSlots) T.nonident[tid] = 0;
+  if (tid < p.nops) {
+    int k = 0;
+    for (int q = 0; q < tid; ++q) k += p.ops[q].kind == OP_DIAG1D && p.ops[q].axis != g.sweep_axis;
+    T.slot[tid] = (int8_t)k;
+  }
+  fx_work_sync();
+  for (int idx = tid; idx < p.nops * bn; idx += kFxWork) {
+    const int oi = idx / bn, c = idx - oi * bn;
+    const DevOp& op = p.ops[oi];
+    const int64_t i = i0 + (c < ncols ? c : 0);
+    if (op.kind == OP_NORM) {
+      double wt = 1.0;
+      for (int a = 0; a < g.ndim; ++a)
+        if (a != g.sweep_axis) wt *= __ldg(op.w[a] + fx_coord(g, a, o, i));
+      RowWeight cw;
+      cw.set(wt);
+      T.colwd[op.red][c] = cw.d;
+      T.colwx[op.red][c] = cw.x;
+    } else if (op.kind == OP_DIAG1D && op.axis != g.sweep_axis) {
+      const int4 t = __ldg(reinterpret_cast<const int4*>(op.ptr) + fx_coord(g, op.axis, o, i));
+      T.colt[T.slot[oi]][c] = t;
+      const int kind = (t.x != 0 || t.y != (1 << 30) ? 1 : 0) | (t.z != 0 || t.w != 0 ? 3 : 0);
+      if (kind) atomicOr(&T.nonident[T.slot[oi]], kind);
+    }
+  }
+}
+
 // The work threads' view of a tile: row j, complex columns c0 .. c0 + NB - 1.
 template <int NB, bool FF>
 struct FxWork {
@@ -415,6 +448,15 @@ struct FxWork {
   bool row_ok;
   const double* roww_ptr;  // lane-axis weights of the pass's first norm, and this row's
   RowWeight roww;
+
+  // this row's weight of the pass's first norm
+  __device__ __forceinline__ void load_roww(const PassParams& p) {
+    const int axis = p.g.sweep_axis;
+    roww_ptr = nullptr;
+    for (int oi = 0; oi < p.nops && roww_ptr == nullptr; ++oi)
+      if (p.ops[oi].kind == OP_NORM) roww_ptr = p.ops[oi].w[axis];
+    roww.set(roww_ptr && row_ok ? __ldg(roww_ptr + j) : 0.0);
+  }
 
   // point-wise ops [ob, oe)
   __device__ __forceinline__ void apply(const PassParams& p, FxTabs& T, int ob, int oe, int64_t ix0) {
@@ -647,14 +689,16 @@ __global__ void __launch_bounds__(kFxThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_s;
-  wait_for_previous();
   const uint32_t ring = smem_u32(sm);
   unsigned char* B = sm + kRingBytes;
 
   if (warp == kFxWork / 32) {
+    wait_for_previous();
     if (lane == 0) fx_producer<MH>(resolve, total, ring, full, empty, &s_fail);
   } else if (warp == kFxWork / 32 + 1) {
-    fx_issuer<N, MH>(resolve, total, ring, ring + kRingBytes, full, empty, dbar, bready, quiet, tmem, &s_fail, &T, &s_handed);
+    wait_for_previous();
+    fx_issuer<N, MH>(resolve, total, ring, ring + kRingBytes, full, empty, dbar, bready, quiet, tmem, &s_fail, &T,
+                     &s_handed);
   } else {
     const int quad = warp & 3, grp = warp >> 2;
     Work W;
@@ -665,6 +709,22 @@ __global__ void __launch_bounds__(kFxThreads, 1)
     uint32_t drains = 0;
     const FxTcParams* cur = params == nullptr ? &one : nullptr;
     W.par = 1;
+    // A single pass makes its first tile's tables while the launch ahead drains: they are constants,
+    // complete before this launch was made (the host waits for every upload of one).  That takes a
+    // block that fits beside the launch ahead (half of an SM's shared memory, one_block_per_sm); one
+    // that starts behind it overlaps them with the loads of the tile instead.  us per step, tables
+    // with the loads / ahead: 2048 x 64 61.2 / 59.3, state matrix 256 x 64 x 4 33.5 / 31.8 (both fit),
+    // 4096 x 128 83.5 / 85.8 (does not).
+    // (The widest tiles, 8 columns a thread, fit for 32 rows alone and always take the second way.)
+    bool tabled = NB < 8 && params == nullptr && fx_tc_smem(BN, tp.kp) <= 100 * 1024;
+    if (tabled) {
+      const Geometry& g = tp.p.g;
+      const int64_t o = blockIdx.x / g.tiles_per_outer, i0 = (blockIdx.x - o * g.tiles_per_outer) * BN;
+      W.row_ok = W.j < (int)g.n;
+      W.load_roww(tp.p);
+      fx_tables(T, tp.p, o, i0, (int)min((int64_t)BN, g.inner - i0), BN);
+    }
+    wait_for_previous();
     for (int64_t gt = blockIdx.x; gt < total; gt += gridDim.x) {
       W.par ^= 1;
       const FxTile r = resolve(gt);
@@ -706,49 +766,20 @@ __global__ void __launch_bounds__(kFxThreads, 1)
             raw[u] = {x.x, x.y};
           }
       }
-      W.roww_ptr = nullptr;
-      for (int oi = 0; oi < p.nops && W.roww_ptr == nullptr; ++oi)
-        if (p.ops[oi].kind == OP_NORM) W.roww_ptr = p.ops[oi].w[g.sweep_axis];
-      W.roww.set(W.roww_ptr && W.row_ok ? __ldg(W.roww_ptr + W.j) : 0.0);
-      // per-tile tables
-      if (tid < 2 * kFxMaxCols) T.cole[tid >> 5][tid & 31] = 0;
-      if (tid < kFxTabSlots) T.nonident[tid] = 0;
-      if (tid < p.nops) {
-        int k = 0;
-        for (int q = 0; q < tid; ++q) k += p.ops[q].kind == OP_DIAG1D && p.ops[q].axis != g.sweep_axis;
-        T.slot[tid] = (int8_t)k;
-        if (p.ops[tid].kind == OP_SCALE) {
-          // sqrt(target / norm) = m 2^x, m in [1/2, 1): digits of m 2^62
-          const double f = sqrt(__ldcg(p.slots + p.ops[tid].b) / __ldcg(p.slots + p.ops[tid].c));
-          int x = 0;
-          const double m = frexp(f, &x);
-          i64 v = isfinite(f) ? __double2ll_rn(ldexp(m, 62)) : 0;
-          if ((int)v == (int)0x80000000) ++v;
-          const dig d = split(v);
-          T.scale_d[tid] = {d.l, d.h};
-          T.scale_x[tid] = x;
-          if (!isfinite(f)) s_bad = 1;  // the whole tile becomes NaN
-        }
-      }
-      fx_work_sync();
-      for (int idx = tid; idx < p.nops * BN; idx += kFxWork) {
-        const int oi = idx / BN, c = idx - oi * BN;
-        const DevOp& op = p.ops[oi];
-        const int64_t i = i0 + (c < W.ncols ? c : 0);
-        if (op.kind == OP_NORM) {
-          double wt = 1.0;
-          for (int a = 0; a < g.ndim; ++a)
-            if (a != g.sweep_axis) wt *= __ldg(op.w[a] + fx_coord(g, a, o, i));
-          RowWeight cw;
-          cw.set(wt);
-          T.colwd[op.red][c] = cw.d;
-          T.colwx[op.red][c] = cw.x;
-        } else if (op.kind == OP_DIAG1D && op.axis != g.sweep_axis) {
-          const int4 t = __ldg(reinterpret_cast<const int4*>(op.ptr) + fx_coord(g, op.axis, o, i));
-          T.colt[T.slot[oi]][c] = t;
-          const int kind = (t.x != 0 || t.y != (1 << 30) ? 1 : 0) | (t.z != 0 || t.w != 0 ? 3 : 0);
-          if (kind) atomicOr(&T.nonident[T.slot[oi]], kind);
-        }
+      if (!tabled) W.load_roww(p);
+      if (!tabled) fx_tables(T, p, o, i0, W.ncols, BN);
+      tabled = false;
+      if (tid < p.nops && p.ops[tid].kind == OP_SCALE) {
+        // sqrt(target / norm) = m 2^x, m in [1/2, 1): digits of m 2^62
+        const double f = sqrt(__ldcg(p.slots + p.ops[tid].b) / __ldcg(p.slots + p.ops[tid].c));
+        int x = 0;
+        const double m = frexp(f, &x);
+        i64 v = isfinite(f) ? __double2ll_rn(ldexp(m, 62)) : 0;
+        if ((int)v == (int)0x80000000) ++v;
+        const dig d = split(v);
+        T.scale_d[tid] = {d.l, d.h};
+        T.scale_x[tid] = x;
+        if (!isfinite(f)) s_bad = 1;  // the whole tile becomes NaN
       }
       // column exponents
 #pragma unroll
