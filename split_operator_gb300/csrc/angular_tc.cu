@@ -20,10 +20,11 @@
 // Persistent CTAs, two per SM, each walking its share of the tiles of the launch:
 //   warps 0-7  load the tile, run the point-wise ops, split it into the B operand,
 //              drain the accumulators, run the ops between / after the matrices,
-//              store, and fold the norms (named barrier 1 among themselves)
+//              store, and sum the norms per warp (named barrier 1 among themselves)
 //   warp 8     streams the A chunks (one MMA K step each) of every tile, in order,
 //              through 2-6 shared-memory stages by bulk TMA (it runs ahead across tiles)
-//   warp 9     issues tcgen05.mma (its elected lane) as chunks land and the B operand is ready
+//   warp 9     issues tcgen05.mma (its elected lane) as chunks land and the B operand is ready, and
+//              publishes a tile's norms and ticket while a product runs (pass_end.cuh)
 // The tensor core truncates its FP32 accumulation, so the A_hi B_hi products go to
 // three TMEM regions a couple of K steps each and the work warps drain the
 // regions into registers (round-to-nearest adds) every kFillSteps K steps; the
