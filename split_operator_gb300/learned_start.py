@@ -189,6 +189,10 @@ class RadialBasis:
         self.xi = np.linspace(-xi_max, xi_max, nxi)
         if u is not None:  # a saved basis
             self.u = np.asarray(u, dtype=np.float64)
+            try:  # loaded here: the first prediction would wait 0.2 s for it, a fifth of a relaxation
+                import scipy.interpolate  # noqa: F401
+            except ImportError:
+                pass
             return
         psil = np.stack([self.to_xi(g.to_l(s.astype(np.float64)), p) for s, p in zip(states, params)])
         self.u = np.empty((g.nth, nxi, modes))
