@@ -224,6 +224,51 @@ def test_norms_of_lane_matrix_passes(so, precision, tol, n, nr):
     assert abs(p.all_losses()[0] - loss) < tol * np.abs(terms).sum()
 
 
+# Two masks with loss checkers on both halves: the pass that closes one step and opens the next folds
+# five reductions over its tiles.  Two steps of numpy's FP64 and of exact
+# digit products differ by some 1e-14 of the norm; split-BF16x6 by 2.2e-7 a step and FP32 sums
+# of 16 terms with masks of three roundings (2e-6).
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-13), ("float_float", 1e-12), ("fp32_bf16x6", 5e-6)])
+@pytest.mark.parametrize("n,nr", [(128, 4096), (64, 4096)])
+def test_many_reductions_in_a_pass(so, precision, tol, n, nr):
+    from oracle import split_operator_oracle as O
+    rng = np.random.default_rng(n)
+    t, tinv = _legendre(n)
+    wp = np.polynomial.legendre.leggauss(n)[1]
+    wr = rng.uniform(0.5, 2.0, nr)
+    a = rng.standard_normal((n, nr)) + 1j * rng.standard_normal((n, nr))
+    a /= np.sqrt((np.abs(a) ** 2 * wp[:, None] * wr[None, :]).sum())
+    masks = rng.uniform(0.5, 1.0, (2, nr))
+    masks[:, 0] = 1.0
+    ph = np.exp(1j * rng.uniform(0.0, 6.0, (n, nr)))
+
+    def build(lib):
+        pg = lib.Grid.new_custom("p", np.arange(n, dtype=float), wp, 0)
+        rg = lib.Grid.new_custom("r", np.arange(nr, dtype=float), wr, 1)
+        st = lib.OperationStack()
+        for k, m in enumerate(masks):
+            b = lib.BorderDumping(m.astype(np.complex128), rg)
+            b.add_loss_checker(f"border {k}" if lib is so else lib.LossChecker(f"border {k}"))
+            st.add_control(b, lib.FIRST_HALF | lib.SECOND_HALF)
+        mt = lib.MatrixTransformation(pg, lib.Grid.new_linear_countable("l", 0.0, n - 1.0, n, 0))
+        mt.set_diagonalization_matrix(t, tinv)
+        st.add_transformation(mt, lib.NORMAL)
+        pd = lib.NDimPropagator()
+        pd.set_operator(ph)
+        st.add_propagator(pd)
+        return lib.WaveFunction(a, [pg, rg]), lib.TimeGrid(0.01, 100), st
+
+    p = so.Propagation(*build(so), precision)
+    q = O.Propagation(*build(O))
+    p.set_timing(True)
+    p.steps(3)
+    q.propagate(3)
+    assert "tc" in " ".join(k[0] for k in p.kernel_times())
+    assert np.abs(np.array(p.all_losses()) - np.array([v for _, v in q.all_losses()])).max() < tol
+    assert abs(p.norm() - q.wave_function.norm()) < tol
+    assert np.linalg.norm(p.get_array() - q.wave_function.array) < 10 * tol * np.linalg.norm(q.wave_function.array)
+
+
 def test_columns_that_are_not_finite_stay_apart(so):
     rng = np.random.default_rng(3)
     n, nr = 64, 50
