@@ -43,7 +43,7 @@ enum OpKind : int32_t {
   OP_RECORD = 11,    // record[count] = slot[a]
   OP_DOT = 12,       // slot[a] + i slot[b] = sum psi conj(other) prod w  (other = ptr, same layout)
   OP_ROUND = 13      // end of a step inside a pass: psi as it would be stored and loaded again (fixed-point
-                     // passes of FP64 states, so that a run split here gives the same bits; else nothing)
+                     // passes, so that a run split here gives the same bits; else nothing)
 };
 
 struct DevOp {

@@ -1121,7 +1121,7 @@ std::string Engine::collect_timing() {
 }
 
 void Engine::step_end() {
-  if (!fx || real != kRealF64 || cur_.empty() || cur_.back().kind == OP_ROUND) return;
+  if (!fx || real == kRealF32 || cur_.empty() || cur_.back().kind == OP_ROUND) return;
   if ((int)cur_.size() >= kMaxOps) {
     flush();
     return;

@@ -269,6 +269,18 @@ def test_many_reductions_in_a_pass(so, precision, tol, n, nr):
     assert np.linalg.norm(p.get_array() - q.wave_function.array) < 10 * tol * np.linalg.norm(q.wave_function.array)
 
 
+@pytest.mark.parametrize("precision", ["fp64", "float_float"])
+@pytest.mark.parametrize("nr,nth", [(256, 64), (300, 45)])
+def test_plane_steps_do_not_depend_on_the_split(so, precision, nr, nth):
+    from split_operator_gb300 import workloads
+    whole, _ = workloads.radial_angular_2d(nr=nr, nth=nth, precision=precision)
+    whole.steps(6)
+    parts, _ = workloads.radial_angular_2d(nr=nr, nth=nth, precision=precision)
+    for k in (1, 3, 2):
+        parts.steps(k)
+    np.testing.assert_array_equal(parts.get_array(), whole.get_array())
+
+
 def test_columns_that_are_not_finite_stay_apart(so):
     rng = np.random.default_rng(3)
     n, nr = 64, 50
