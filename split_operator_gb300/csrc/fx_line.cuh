@@ -239,7 +239,11 @@ __global__ void __launch_bounds__((1 << LG) / kLineV, 1) fx_line_kernel(const __
               tot = ldexp((double)a, 62 + wx + 2 * ex);
             } else {
               for (int i = 0; i < kWarps; ++i) tot += __longlong_as_double(S.red[par][i]);
-              tot = ldexp(tot, 62 + 2 * ex);
+              // between the transforms of a power of two, ex still stands for the values ahead of the
+              // forward one: the unitary transform is v 2^(ex + kSumF + kMid - LG / 2), without kMid
+              // while that shift has not been made (CHIRP transforms are unitary, ex is theirs)
+              const int mid = !CHIRP && between ? 2 * Sh::kSumF - LG + (shift ? 0 : 2 * Sh::kMid) : 0;
+              tot = ldexp(tot, 62 + 2 * ex + mid);
             }
             if (bad) tot = __longlong_as_double(0x7ff8000000000000ll);
             S.slots[op.a] = tot;
