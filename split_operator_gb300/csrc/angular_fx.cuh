@@ -402,8 +402,7 @@ __device__ __forceinline__ i64 rescale_f64(i64 v, int k) {
   if (k <= 0) return v << (k < -63 ? 63 : -k);
   const i64 s = v >> 63;
   const unsigned long long a = (unsigned long long)((v ^ s) - s);
-  unsigned long long r = k > 62 ? 0ull : ((a >> (k - 1)) + 1ull) >> 1;
-  if (r == 0 && a != 0) r = 1;  // shr_round keeps a unit of what is not zero
+  const unsigned long long r = ((a >> (k > 64 ? 63 : k - 1)) + 1ull) >> 1;
   return ((i64)r ^ s) - s;
 }
 

@@ -226,9 +226,10 @@ __device__ __forceinline__ float raw_rel(i64 r, int ref) {
     return b >= (1 << 23) && d > 0 ? __int_as_float(d) : 0.0f;
   }
 }
-// a significand with its top bit at 62, moved right by r >= 1 bits, rounded to nearest
+// a significand with its top bit at 62, moved right by r >= 1 bits, rounded to nearest (from 64
+// bits on it is below half a unit: zero)
 __device__ __forceinline__ i64 shr_round(unsigned long long m, int r) {
-  r = r > 63 ? 63 : (r < 1 ? 1 : r);
+  r = r > 64 ? 64 : (r < 1 ? 1 : r);
   return (i64)(((m >> (r - 1)) + 1ull) >> 1);
 }
 __device__ __forceinline__ i64 apply_sign(i64 v, int s) { return (v ^ (i64)s) - (i64)s; }  // s: 0 or -1
