@@ -42,8 +42,8 @@ enum OpKind : int32_t {
   OP_SETC = 10,      // slot[a] = value
   OP_RECORD = 11,    // record[count] = slot[a]
   OP_DOT = 12,       // slot[a] + i slot[b] = sum psi conj(other) prod w  (other = ptr, same layout)
-  OP_ROUND = 13      // end of a step inside a pass: psi as it would be stored and loaded again (fixed-point
-                     // passes, so that a run split here gives the same bits; else nothing)
+  OP_ROUND = 13      // end of a step inside a pass: psi as it would be stored and loaded again, so that a
+                     // run split here gives the same bits (fixed-point lane-matrix passes only)
 };
 
 struct DevOp {

@@ -985,7 +985,8 @@ void Engine::grow_partials(PassParams& p) {
   p.partials = partials_.as<double>();
 }
 
-void Engine::launch(const std::vector<DevOp>& ops, int axis, bool resident, int repeat) {
+void Engine::launch(const std::vector<DevOp>& all, int axis, bool resident, int repeat) {
+  std::vector<DevOp> ops = all;
   PassParams p{};
   const char* name_tag = "";
   p.g = geometry(axis, resident);
@@ -1011,6 +1012,12 @@ void Engine::launch(const std::vector<DevOp>& ops, int axis, bool resident, int 
   pass_choose_buffers(p, fp64);
   if (!fp64 && tc_mode() >= 0 && !resident && try_launch_tc(ops, axis, p)) return;
   if (fx && !resident && try_launch_fx_tc(ops, axis, p)) return;
+  // step ends inside the pass concern that kernel alone (the others' plans know no such op)
+  ops.erase(std::remove_if(ops.begin(), ops.end(), [](const DevOp& o) { return o.kind == OP_ROUND; }), ops.end());
+  if ((int)ops.size() != p.nops) {
+    std::fill(std::copy(ops.begin(), ops.end(), p.ops), p.ops + kMaxOps, DevOp{});
+    p.nops = (int)ops.size();
+  }
   if (fx && !(resident && recording) && try_launch_fx_pair(ops, p, resident)) {
     name_tag = resident ? " fx" : " fftpair fx";
   } else if ((fft_pair || (fp64 && p.g.n > 4096)) && fft_pair_plan(p, real, resident)) {
@@ -1122,6 +1129,9 @@ std::string Engine::collect_timing() {
 
 void Engine::step_end() {
   if (!fx || real == kRealF32 || cur_.empty() || cur_.back().kind == OP_ROUND) return;
+  // the fixed-point lane-matrix pass alone rounds there, and it takes none of these
+  for (const DevOp& o : cur_)
+    if (o.kind == OP_FFT || o.kind == OP_MAT_LANE) return;
   if ((int)cur_.size() >= kMaxOps) {
     flush();
     return;

@@ -202,7 +202,7 @@ class Engine {
   std::string collect_timing();  // "name\tlaunches\ttotal_ms\tbytes\n" lines; synchronizes and resets
 
  private:
-  void launch(const std::vector<DevOp>& ops, int axis, bool resident, int repeat);
+  void launch(const std::vector<DevOp>& all, int axis, bool resident, int repeat);
   struct TimedLaunch {
     std::string name;
     cudaEvent_t a, b;
