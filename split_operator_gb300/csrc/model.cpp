@@ -26,6 +26,18 @@ void cuda_check(cudaError_t e, const char* what) {
 DeviceBuffer::DeviceBuffer(size_t b) : bytes(b) {
   if (b) cuda_check(cudaMalloc(&ptr, b), "cudaMalloc");
 }
+DeviceBuffer DeviceBuffer::if_room(size_t b) {
+  DeviceBuffer r;
+  const cudaError_t e = cudaMalloc(&r.ptr, b);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    r.ptr = nullptr;
+    return r;
+  }
+  cuda_check(e, "cudaMalloc");
+  r.bytes = b;
+  return r;
+}
 DeviceBuffer& DeviceBuffer::operator=(DeviceBuffer&& o) noexcept {
   if (this != &o) {
     if (ptr) cudaFree(ptr);
@@ -282,6 +294,7 @@ const void* Engine::table_1d(const void* key, uint64_t version, const std::vecto
   if (c.buf.ptr) flush();  // replacing a table the open pass may reference (a first upload needs no flush)
   upload_complex(c.buf, t, real, stream);
   c.fx = DeviceBuffer();
+  c.fx_denied = false;
   if (fx) c.max_abs = table_max(t);
   c.version = version;
   return c.buf.ptr;
@@ -301,19 +314,17 @@ const void* Engine::table_nd(const void* key, uint64_t version, const std::vecto
   auto& c = tables_[{key, 1}];
   if (c.buf.ptr && c.version == version) return c.buf.ptr;
   if (c.buf.ptr) flush();
+  c.fx = DeviceBuffer();
+  c.fx_denied = false;
   // logical row-major -> storage order and precision, on the device (a host loop over the strides
-  // took 6 ms of the first pass for 524,288 points); the last 8 bytes of raw: the largest magnitude
+  // took 6 ms of the first pass for 524,288 points); the last 8 bytes of raw: the largest magnitude.
+  // The table itself first; without room for the scratch copy beside it, the host's order below.
   const size_t b = t.size() * sizeof(cplx);
-  DeviceBuffer raw;
-  try {
-    raw = DeviceBuffer(b + sizeof(unsigned long long));
-  } catch (const Error&) {
-    cudaGetLastError();  // no room beside the table: the host's order below
-  }
+  if (c.buf.bytes != t.size() * elem_bytes()) c.buf = DeviceBuffer(t.size() * elem_bytes());
+  const DeviceBuffer raw = DeviceBuffer::if_room(b + sizeof(unsigned long long));
   if (raw.ptr) {
     unsigned long long* const top = reinterpret_cast<unsigned long long*>(raw.as<unsigned char>() + b);
     cuda_check(cudaMemcpyAsync(raw.ptr, t.data(), b, cudaMemcpyHostToDevice, stream), "table upload");
-    if (c.buf.bytes != t.size() * elem_bytes()) c.buf = DeviceBuffer(t.size() * elem_bytes());
     cuda_check(launch_import(c.buf.ptr, real, raw.as<double>(), flat_geometry(*this), stream), "table import");
     double max2 = 0.0;
     if (fx) {
@@ -343,7 +354,6 @@ const void* Engine::table_nd(const void* key, uint64_t version, const std::vecto
     upload_complex(c.buf, st, real, stream);
     if (fx) c.max_abs = table_max(t);
   }
-  c.fx = DeviceBuffer();
   c.version = version;
   return c.buf.ptr;
 }
@@ -354,13 +364,24 @@ Engine::Cached* Engine::phase_table(const void* device_ptr) {
   return nullptr;
 }
 
+// nullptr: no room, the passes with this table stay in floating point.  The copy of a large table (16 MB
+// and more) leaves as much again free: what a program allocates later (the copy of the state that an
+// energy takes, a staging buffer) found its room when there was no second copy.
 const void* Engine::fx_table(Cached& c) {
-  if (c.fx.ptr) return c.fx.ptr;
-  DeviceBuffer b(c.buf.bytes);
+  if (c.fx.ptr || c.fx_denied) return c.fx.ptr;
+  c.fx_denied = true;
+  if (c.buf.bytes >= (size_t)1 << 24) {
+    size_t free_bytes = 0, total = 0;
+    cuda_check(cudaMemGetInfo(&free_bytes, &total), "cudaMemGetInfo");
+    if (free_bytes / 2 < c.buf.bytes) return nullptr;
+  }
+  DeviceBuffer b = DeviceBuffer::if_room(c.buf.bytes);
+  if (!b.ptr) return nullptr;
   cuda_check(launch_fx_table(b.ptr, c.buf.ptr, real, (int64_t)(c.buf.bytes / 16), stream), "fixed-point table");
   // as the uploads: complete before any stream of the engine uses it
   cuda_check(cudaStreamSynchronize(stream), "fixed-point table sync");
   c.fx = std::move(b);
+  c.fx_denied = false;
   return c.fx.ptr;
 }
 
@@ -401,7 +422,7 @@ int64_t fx_of(long double v) { return (int64_t)llroundl(ldexpl(v, 62)); }
 }  // namespace
 
 // Factors the fixed-point FFT pairs share, one copy per device, kind and length for the process
-// (held weakly, by the engines that use them).
+// (held weakly, by the engines that use them); nullptr without room for them.
 std::shared_ptr<FxFactors> Engine::fx_shared(int kind, size_t n, const std::function<FxHost()>& make) {
   static std::mutex mu;
   static std::map<std::tuple<int, int, size_t>, std::weak_ptr<FxFactors>> cache;
@@ -415,6 +436,8 @@ std::shared_ptr<FxFactors> Engine::fx_shared(int kind, size_t n, const std::func
   if (mine) return mine;
   const FxHost h = make();
   auto f = std::make_shared<FxFactors>();
+  f->buf = DeviceBuffer::if_room(h.words.size() * sizeof(int32_t));
+  if (!f->buf.ptr) return nullptr;
   upload(f->buf, h.words, stream);
   f->g = h.g;
   slot = mine = f;
@@ -423,7 +446,7 @@ std::shared_ptr<FxFactors> Engine::fx_shared(int kind, size_t n, const std::func
 
 // Twiddles, stage-major (forward order, then reversed order).
 const void* Engine::fx_twiddle(size_t n, int radix) {
-  return fx_shared(radix, n, [n, radix] {
+  const auto f = fx_shared(radix, n, [n, radix] {
     const Circle circ(n);
     FxHost h;
     h.words.assign(8 * n, 0);
@@ -433,13 +456,14 @@ const void* Engine::fx_twiddle(size_t n, int radix) {
       fx_put(fx_of(-w.second), &h.words[4 * e + 2]);  // exp(-2 pi i m / n)
     }
     return h;
-  })->buf.ptr;
+  });
+  return f ? f->buf.ptr : nullptr;
 }
 
 // Chirp w_j = exp(-i pi j^2 / n) and the spectrum of the filter conj w (length M, times 2^-g and
 // 1 / sqrt n: a unitary transform) of lanes whose length is no power of two.
-const FxFactors& Engine::fx_chirp(size_t n, int lgm) {
-  return *fx_shared(1, n, [n, lgm] {
+const FxFactors* Engine::fx_chirp(size_t n, int lgm) {
+  const auto f = fx_shared(1, n, [n, lgm] {
     using C = std::complex<long double>;
     const size_t M = (size_t)1 << lgm;
     const Circle circ(8 * n);  // pi j^2 / n = 2 pi (4 j^2) / (8 n)
@@ -487,6 +511,7 @@ const FxFactors& Engine::fx_chirp(size_t n, int lgm) {
     }
     return h;
   });
+  return f.get();  // (this engine holds it)
 }
 
 // Parity structure of a real n x n matrix (logical M[a][b] = m[a n + b]) within tol of its
@@ -874,7 +899,7 @@ void Engine::submit(const Action& a) {
 
 // Digit images of `count` real n x n matrices for the fixed-point lane-matrix pass, one copy per
 // value for the process (entries are held weakly by the engines that use them, like the FP32
-// images above).  Sparse matrices and ones with a value that is not finite get none.
+// images above).  Sparse matrices, ones with a value that is not finite and ones without room get none.
 void Engine::fx_images(const void* matrix, const std::vector<cplx>& m, size_t n, size_t count) {
   struct Entry {
     int device;
@@ -900,7 +925,8 @@ void Engine::fx_images(const void* matrix, const std::vector<cplx>& m, size_t n,
   std::vector<unsigned char> h(b * count);
   for (size_t i = 0; i < count; ++i)
     if (!fx_angular_image(md.data() + i * n * n, (int)n, h.data() + i * b)) return;
-  auto img = std::make_shared<DeviceBuffer>();
+  auto img = std::make_shared<DeviceBuffer>(DeviceBuffer::if_room(h.size()));
+  if (!img->ptr) return;
   upload(*img, h, stream);
   fx_images_[matrix] = img;
   cache.push_back(Entry{dev, n, std::move(md), img});
@@ -928,9 +954,9 @@ bool Engine::try_launch_fx_tc(const std::vector<DevOp>& ops, int axis, PassParam
   int cols = 0;
   PassParams q = p;
   if (nmat == 0 || !fx_angular_plan(q, ops.data(), (int)ops.size(), mx, &cols)) return false;
-  p = q;
   for (size_t i = 0; i < ops.size(); ++i)
-    if (tab[i]) p.ops[i].ptr = fx_table(*tab[i]);
+    if (tab[i] && !(q.ops[i].ptr = fx_table(*tab[i]))) return false;
+  p = q;
   grow_partials(p);
   const Geometry& g = p.g;
   std::string name = std::string(real == kRealFF ? "ff" : "f64") + " tcfx axis" + std::to_string(axis) + ":";
@@ -963,15 +989,18 @@ bool Engine::try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p, bo
       if (!tab[i]) return false;
       mx[i] = tab[i]->max_abs;
     }
-  if (!(resident ? fx_line_plan(p, real, mx) : fx_pair_plan(p, real, mx))) return false;
+  PassParams q = p;
+  if (!(resident ? fx_line_plan(q, real, mx) : fx_pair_plan(q, real, mx))) return false;
   for (size_t i = 0; i < ops.size(); ++i)
-    if (tab[i]) p.ops[i].ptr = fx_table(*tab[i]);
-  p.twiddle = fx_twiddle((size_t)1 << p.fx, resident ? 4 : p.radix);
-  if (p.fx_chirp) {
-    const FxFactors& f = fx_chirp((size_t)p.g.n, p.fx);
-    p.aux = f.buf.ptr;
-    p.fx_g = f.g;
+    if (tab[i] && !(q.ops[i].ptr = fx_table(*tab[i]))) return false;
+  if (!(q.twiddle = fx_twiddle((size_t)1 << q.fx, resident ? 4 : q.radix))) return false;
+  if (q.fx_chirp) {
+    const FxFactors* f = fx_chirp((size_t)q.g.n, q.fx);
+    if (!f) return false;
+    q.aux = f->buf.ptr;
+    q.fx_g = f->g;
   }
+  p = q;
   return true;
 }
 

@@ -66,6 +66,7 @@ struct DeviceBuffer {
   size_t bytes = 0;
   DeviceBuffer() = default;
   explicit DeviceBuffer(size_t b);
+  static DeviceBuffer if_room(size_t b);  // empty when the device has no room
   DeviceBuffer(const DeviceBuffer&) = delete;
   DeviceBuffer& operator=(const DeviceBuffer&) = delete;
   DeviceBuffer(DeviceBuffer&& o) noexcept : ptr(o.ptr), bytes(o.bytes) { o.ptr = nullptr; o.bytes = 0; }
@@ -224,6 +225,7 @@ class Engine {
     bool real;
     double max_abs = 0.0;  // phase tables: the largest magnitude (infinity when one is not finite)
     DeviceBuffer fx;       // phase tables: fixed-point copy, made at its first use
+    bool fx_denied = false;  // ... no room for it
     int parity = 0;     // float-float: kind of the parity structure, half matrix in half_buf
     DeviceBuffer half_buf;
     // A-operand chunk images of the tensor-core passes, and the same for the parity-split
@@ -246,11 +248,11 @@ class Engine {
   void fx_images(const void* matrix, const std::vector<cplx>& m, size_t n, size_t count);
   std::map<const void*, std::shared_ptr<DeviceBuffer>> fx_images_;  // digit images by device matrix
   Cached* phase_table(const void* device_ptr);           // the cache entry of a phase table
-  const void* fx_table(Cached& c);                       // its fixed-point copy
+  const void* fx_table(Cached& c);                       // its fixed-point copy (nullptr: no room)
   // fixed-point factors shared by the process: twiddles of n points, chirp and filter of n points
   std::shared_ptr<FxFactors> fx_shared(int kind, size_t n, const std::function<FxHost()>& make);
   const void* fx_twiddle(size_t n, int radix);
-  const FxFactors& fx_chirp(size_t n, int lgm);
+  const FxFactors* fx_chirp(size_t n, int lgm);
   std::map<std::pair<int, size_t>, std::shared_ptr<FxFactors>> fx_factors_;
   std::map<uint64_t, DeviceBuffer> weights_;
   std::map<std::pair<size_t, int>, DeviceBuffer> twiddles_;  // by (n, stage radix)
