@@ -20,7 +20,9 @@
 namespace so {
 
 void cuda_check(cudaError_t e, const char* what) {
-  if (e != cudaSuccess) throw Error(SO_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+  if (e == cudaSuccess) return;
+  cudaGetLastError();  // an error that the context survives ends with this call, not at the next launch
+  throw Error(SO_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
 DeviceBuffer::DeviceBuffer(size_t b) : bytes(b) {

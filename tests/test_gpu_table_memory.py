@@ -73,3 +73,26 @@ def test_tables_without_room_for_their_copies(beside):
     assert "tcfx" in " ".join(k[0] for k in r.kernel_times())
     got = p.get_array()
     assert np.linalg.norm(r.get_array() - got) < 2e-14 * np.linalg.norm(got)
+
+
+def test_an_out_of_memory_error_ends_with_its_call():
+    ensure_built()
+    import torch
+
+    import split_operator_gb300 as so
+    p, wf, step = _build(so, 64, 2, 64)
+    p.steps(1)
+    torch.cuda.empty_cache()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (1 << 28), dtype=torch.uint8, device="cuda")
+    try:
+        with pytest.raises(Exception, match="out of memory"):
+            so.WaveFunction(np.zeros((1 << 15, 1 << 10), dtype=np.complex128),  # 512 MB
+                            [so.Grid.new_linear_countable("a", 0.0, 1.0, 1 << 15, 0),
+                             so.Grid.new_linear_countable("b", 0.0, 1.0, 1 << 10, 1)])
+        p.steps(1)
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    q, *_ = _build(so, 64, 2, 64)
+    q.steps(2)
+    np.testing.assert_array_equal(p.get_array(), q.get_array())
