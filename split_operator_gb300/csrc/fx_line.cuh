@@ -71,7 +71,8 @@ __global__ void __launch_bounds__((1 << LG) / kLineV, 1) fx_line_kernel(const __
     const longlong2 x = j < n ? psi[j] : longlong2{0, 0};
     v[r] = {x.x, x.y};
   }
-  // weights of the program's first norm as digits (position grid), scaled by their largest exponent
+  // weights of the program's first norm as digits (position grid), scaled by their largest exponent:
+  // weights within 2^8 of each other keep all of their bits so, others take the general sum below
   const double* w0 = nullptr;
   int2 wd[kLineV];
   int wx = 0;
@@ -79,21 +80,27 @@ __global__ void __launch_bounds__((1 << LG) / kLineV, 1) fx_line_kernel(const __
     if (p.ops[oi].kind == OP_NORM) w0 = p.ops[oi].w[0];
   if (w0) {
     double w[kLineV];
-    int m = 1;
+    int m = 1, least = 2047;
 #pragma unroll
     for (int r = 0; r < kLineV; ++r) {
       const int j = t + r * kT;
       w[r] = j < n ? __ldg(w0 + j) : 0.0;
-      m = max(m, (int)((__double_as_longlong(w[r]) >> 52) & 0x7ff));
+      const int e = (int)((__double_as_longlong(w[r]) >> 52) & 0x7ff);
+      m = max(m, e);
+      if (w[r] != 0.0) least = min(least, e);
     }
     m = __reduce_max_sync(kMask, m);
-    if (lane == 0) S.part[warp].ref = m;
+    least = __reduce_min_sync(kMask, least);
+    if (lane == 0) S.part[warp] = {m, (uint32_t)least};
     __syncthreads();
-    for (int i = 0; i < kWarps; ++i) m = max(m, S.part[i].ref);
+    for (int i = 0; i < kWarps; ++i) {
+      m = max(m, S.part[i].ref);
+      least = min(least, (int)S.part[i].sum);
+    }
     wx = m - 1022;  // |w| < 2^wx
 #pragma unroll
     for (int r = 0; r < kLineV; ++r) wd[r] = real_digits(w[r], wx);
-    if (m == 2047) w0 = nullptr;  // weights that are not finite: the general sum below
+    if (m == 2047 || least < m - 8) w0 = nullptr;
   }
   __syncthreads();
   bool bad = false;  // a value was not finite: the state is NaN from here on
@@ -206,19 +213,21 @@ __global__ void __launch_bounds__((1 << LG) / kLineV, 1) fx_line_kernel(const __
           break;
         }
         case OP_NORM: {
-          // sum w |v|^2: squares in units of 2^62 (their sum stays below 2^62), weighted digits
+          // sum w |v|^2: squares in units of 2^62 (their sum stays below 2^62) and weighted digits, or
+          // (weights of many decades, the momentum grid's) in FP64
           i64 s = 0;
           double sd = 0.0;
           const bool quick = w0 != nullptr && op.w[0] == w0 && !between;
 #pragma unroll
           for (int r = 0; r < kLineV; ++r) {
-            const dig a = split(v[r].x), b = split(v[r].y);
-            const i64 q = (mw(b.h, b.h, mw(a.h, a.h, 0)) << 2) + (mw(b.h, b.l, mw(a.h, a.l, 1ll << 28)) >> 29);
             if (quick) {
+              const dig a = split(v[r].x), b = split(v[r].y);
+              const i64 q = (mw(b.h, b.h, mw(a.h, a.h, 0)) << 2) + (mw(b.h, b.l, mw(a.h, a.l, 1ll << 28)) >> 29);
               s += rmul(q, wd[r]);
             } else {
               const int j = point(r, between);
-              if (j < n) sd += (double)q * __ldg(op.w[0] + j);
+              const double x = (double)v[r].x, y = (double)v[r].y;
+              if (j < n) sd = fma(fma(x, x, y * y), __ldg(op.w[0] + j), sd);
             }
           }
           if (quick) {
@@ -243,7 +252,7 @@ __global__ void __launch_bounds__((1 << LG) / kLineV, 1) fx_line_kernel(const __
               // forward one: the unitary transform is v 2^(ex + kSumF + kMid - LG / 2), without kMid
               // while that shift has not been made (CHIRP transforms are unitary, ex is theirs)
               const int mid = !CHIRP && between ? 2 * Sh::kSumF - LG + (shift ? 0 : 2 * Sh::kMid) : 0;
-              tot = ldexp(tot, 62 + 2 * ex + mid);
+              tot = ldexp(tot, 2 * ex + mid);
             }
             if (bad) tot = __longlong_as_double(0x7ff8000000000000ll);
             S.slots[op.a] = tot;
