@@ -160,13 +160,17 @@ __global__ void __launch_bounds__((1 << LG) / kLineV, 1) fx_line_kernel(const __
               }
             }
             transform<LG, kLineV, true, 0, 1>(v, buf, tw);
-            ex += p.fx_g - Sh::kSc;
+            // (the first convolution's bits are moved back up, see fx_pair.cuh)
+            const int up = p.fx_g - Sh::kSc;
+            if (!fwd) ex += up;
 #pragma unroll
             for (int r = 0; r < kLineV; ++r) {
               const int j = t + r * kT;
               if (j >= n) {
                 v[r] = {0, 0};
-              } else if (!fwd) {
+              } else if (fwd) {
+                v[r] = {v[r].x << up, v[r].y << up};
+              } else {
                 int4 w = __ldg(chirp + j);
                 w.z = -w.z;
                 w.w = -w.w;

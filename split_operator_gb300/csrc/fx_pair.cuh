@@ -191,8 +191,13 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
       continue;
     }
     conjugate(v);
-    // the n points of the transform, and the ops up to the next one
+    // the n points of the transform, and the ops up to the next one.  A convolution leaves them at
+    // 2^(kConvOut - g) of the norm bound; the first one's go back up to 2^60, or the second would round at
+    // 2^-56 of it (error of a packet of 1000 points through the pair 1.35e-15 / 4.6e-16 without / with
+    // it, 8.0e-16 by the sum in FP64).
     const int ob = half ? f1 + 1 : 1, oe = half ? pp.nops : f1;
+    const int up = half ? 0 : 60 - Sh::kConvOut + pp.fx_g;
+    static_assert(Sh::kConvOut <= 62, "g is at least 2: up is not negative");
 #pragma unroll
     for (int r = 0; r < kV; ++r) {
       const int j = i0 + r * kNb;
@@ -200,6 +205,7 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
         v[r] = {0, 0};
         continue;
       }
+      v[r] = {v[r].x << up, v[r].y << up};
       if (half) {
         int4 w = __ldg(chirp + j);
         w.z = -w.z;
@@ -214,7 +220,7 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
     }
   }
   if (ok0) {
-    const int x = e - (2 * Sh::kConvOut - 2 * pp.fx_g - 60);
+    const int x = e - (Sh::kConvOut - pp.fx_g);
 #pragma unroll
     for (int r = 0; r < kV; ++r) {
       const int j = i0 + r * kNb;
