@@ -173,13 +173,14 @@ void fx_angular_params(const PassParams& p, const int* mat_op, int nmat, const u
   std::memcpy(out, &t, sizeof(t));
 }
 
-cudaError_t launch_fx_angular(int real, int n, int cols, const void* one, const void* params_dev, const void* owners_dev,
-                              int64_t tiles, cudaStream_t s) {
+cudaError_t launch_fx_angular(int real, int n, int cols, bool exps, const void* one, const void* params_dev,
+                              const void* owners_dev, int64_t tiles, cudaStream_t s) {
   const unsigned grid = (unsigned)(tiles < fx_sms() ? tiles : fx_sms());
   const FxTcParams* prm = reinterpret_cast<const FxTcParams*>(params_dev);
   const uint2* own = reinterpret_cast<const uint2*>(owners_dev);
-  return real == kRealFF ? launch_fx_angular_ff(fx_halves(n), fx_kp(n), cols, one, prm, own, tiles, grid, s)
-                         : fx_angular_launch<false>(fx_halves(n), fx_kp(n), cols, one, prm, own, tiles, grid, s);
+  FxAngularLaunch* const launch = real == kRealFF ? (exps ? launch_fx_angular_ff_exps : launch_fx_angular_ff)
+                                                  : (exps ? launch_fx_angular_exps : fx_angular_launch<false, false>);
+  return launch(fx_halves(n), fx_kp(n), cols, one, prm, own, tiles, grid, s);
 }
 
 int64_t fx_angular_grid(int64_t tiles) { return tiles < fx_sms() ? tiles : fx_sms(); }

@@ -190,6 +190,8 @@ struct FxTabs {
   int coler[kFxMaxCols];                // the same at a ROUND
   int colb[kFxMaxCols];                 // exponent bound of the column's B operand
   int nonident[kFxTabSlots];            // the factors of this tile: 0 all are 1, 1 all real, else complex
+  int16_t opk[kMaxOps][kFxMaxCols];     // tables with exponents: of the op's factors per column
+  uint32_t kany;                        // bit i: op i has one in this tile
   int8_t slot[kMaxOps];
   double red[2][kMaxRed][kFxWork / 32];  // norms: the warps' sums (of every second tile)
 };
@@ -407,11 +409,13 @@ __device__ __forceinline__ i64 rescale_f64(i64 v, int k) {
 }
 
 // The tile's tables of weights and factors (all but SCALE's); clears the column maxima.  All work threads.
+template <bool EXPS>
 __device__ __forceinline__ void fx_tables(FxTabs& T, const PassParams& p, int64_t o, int64_t i0, int ncols, int bn) {
   const Geometry& g = p.g;
   const int tid = threadIdx.x;
   if (tid < 2 * kFxMaxCols) T.cole[tid >> 5][tid & 31] = 0;
   if (tid < kFxTabSlots) T.nonident[tid] = 0;
+  if (EXPS && tid == kFxWork - 1) T.kany = 0u;
   if (tid < p.nops) {
     int k = 0;
     for (int q = 0; q < tid; ++q) k += p.ops[q].kind == OP_DIAG1D && p.ops[q].axis != g.sweep_axis;
@@ -436,11 +440,23 @@ __device__ __forceinline__ void fx_tables(FxTabs& T, const PassParams& p, int64_
       const int kind = (t.x != 0 || t.y != (1 << 30) ? 1 : 0) | (t.z != 0 || t.w != 0 ? 3 : 0);
       if (kind) atomicOr(&T.nonident[T.slot[oi]], kind);
     }
+    if (EXPS && (op.kind == OP_DIAGND || op.kind == OP_DIAG1D) && op.exps) {
+      const int16_t k = c >= ncols ? 0 : __ldg(op.exps + (op.kind == OP_DIAGND ? o * g.inner + i : fx_coord(g, op.axis, o, i)));
+      T.opk[oi][c] = k;
+      if (k) atomicOr(&T.kany, 1u << oi);
+    }
   }
 }
 
+// Op oi's factors are 2^opk too large: the columns' exponents go down.  All work threads.
+__device__ __forceinline__ void lower_columns(FxTabs& T, int oi, int bn) {
+  fx_work_sync();
+  if ((int)threadIdx.x < bn && T.colx[threadIdx.x] != kFxPoison) T.colx[threadIdx.x] -= T.opk[oi][threadIdx.x];
+  fx_work_sync();
+}
+
 // The work threads' view of a tile: row j, complex columns c0 .. c0 + NB - 1.
-template <int NB, bool FF>
+template <int NB, bool FF, bool EXPS>
 struct FxWork {
   cx w[NB];
   int rowx;    // exponent of this row's values on top of their column's
@@ -461,7 +477,7 @@ struct FxWork {
   }
 
   // point-wise ops [ob, oe)
-  __device__ __forceinline__ void apply(const PassParams& p, FxTabs& T, int ob, int oe, int64_t ix0) {
+  __device__ __forceinline__ void apply(const PassParams& p, FxTabs& T, int ob, int oe, int64_t ix0, int bn) {
     const Geometry& g = p.g;
     for (int oi = ob; oi < oe; ++oi) {
       const DevOp& op = p.ops[oi];
@@ -481,6 +497,7 @@ struct FxWork {
             for (int u = 0; u < NB; ++u)
               if (c0 + u < ncols) w[u] = cmul<0>(w[u], __ldg(t + u));
           }
+          if (EXPS && ((T.kany >> oi) & 1u)) lower_columns(T, oi, bn);
           break;
         }
         case OP_DIAG1D: {
@@ -502,6 +519,7 @@ struct FxWork {
               }
             }
           }
+          if (EXPS && ((T.kany >> oi) & 1u)) lower_columns(T, oi, bn);
           break;
         }
         case OP_SCALE: {
@@ -649,7 +667,9 @@ struct FxWork {
   }
 };
 
-template <int NB, int MH, bool FF>
+// EXPS: tables with an exponent per column (Engine::fx_table).  A kernel of its own: asking every op
+// whether it has them took 1 us of a 25 us pass (256 x 64 points with a matrix per Omega).
+template <int NB, int MH, bool FF, bool EXPS>
 __global__ void __launch_bounds__(kFxThreads, 1)
     fx_angular_kernel(const __grid_constant__ FxTcParams one, const FxTcParams* __restrict__ params,
                       const uint2* __restrict__ owners, const int64_t total) {
@@ -657,7 +677,7 @@ __global__ void __launch_bounds__(kFxThreads, 1)
   constexpr int kGroups = MH == 1 ? 4 : 2;     // column groups of the work warps
   constexpr int BN = NB * kGroups, N = 2 * BN;
   constexpr int kRing = (int)(kRingBytes / (kChunkRowBytes * MH));
-  using Work = FxWork<NB, FF>;
+  using Work = FxWork<NB, FF, EXPS>;
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(16) FxTcParams tp;
   __shared__ __align__(16) FxTabs T;
@@ -724,7 +744,7 @@ __global__ void __launch_bounds__(kFxThreads, 1)
       const int64_t o = blockIdx.x / g.tiles_per_outer, i0 = (blockIdx.x - o * g.tiles_per_outer) * BN;
       W.row_ok = W.j < (int)g.n;
       W.load_roww(tp.p);
-      fx_tables(T, tp.p, o, i0, (int)min((int64_t)BN, g.inner - i0), BN);
+      fx_tables<EXPS>(T, tp.p, o, i0, (int)min((int64_t)BN, g.inner - i0), BN);
     }
     wait_for_previous();
     for (int64_t gt = blockIdx.x; gt < total; gt += gridDim.x) {
@@ -769,7 +789,7 @@ __global__ void __launch_bounds__(kFxThreads, 1)
           }
       }
       if (!tabled) W.load_roww(p);
-      if (!tabled) fx_tables(T, p, o, i0, W.ncols, BN);
+      if (!tabled) fx_tables<EXPS>(T, p, o, i0, W.ncols, BN);
       tabled = false;
       if (tid < p.nops && p.ops[tid].kind == OP_SCALE) {
         // sqrt(target / norm) = m 2^x, m in [1/2, 1): digits of m 2^62
@@ -847,7 +867,7 @@ __global__ void __launch_bounds__(kFxThreads, 1)
         }
         const int ob = m < 0 ? 0 : tp.mat_op[m] + 1;
         const int oe = m + 1 < tp.nmat ? tp.mat_op[m + 1] : p.nops;
-        W.apply(p, T, ob, oe, ix0);
+        W.apply(p, T, ob, oe, ix0, BN);
         if (m + 1 < tp.nmat) {
           if (m >= 0 || oe > 0) {
             // the operand's column maxima

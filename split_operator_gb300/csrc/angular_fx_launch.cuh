@@ -6,17 +6,18 @@
 
 namespace so {
 
-// angular_fx_ff.cu
-cudaError_t launch_fx_angular_ff(int halves, int kp, int cols, const void* one, const FxTcParams* params,
-                                 const uint2* owners, int64_t tiles, unsigned grid, cudaStream_t s);
+// angular_fx_ff.cu, angular_fx_exps.cu, angular_fx_ff_exps.cu
+using FxAngularLaunch = cudaError_t(int halves, int kp, int cols, const void* one, const FxTcParams* params,
+                                    const uint2* owners, int64_t tiles, unsigned grid, cudaStream_t s);
+FxAngularLaunch launch_fx_angular_ff, launch_fx_angular_exps, launch_fx_angular_ff_exps;
 
 namespace {
 
-template <int NB, int MH, bool FF>
+template <int NB, int MH, bool FF, bool EXPS>
 cudaError_t fx_angular_one(int kp, const void* one, const FxTcParams* params, const uint2* owners, int64_t tiles,
                            unsigned grid, cudaStream_t s) {
   static bool done = false;
-  auto kern = fx_angular_kernel<NB, MH, FF>;
+  auto kern = fx_angular_kernel<NB, MH, FF, EXPS>;
   if (!done) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 180 * 1024);
     if (e != cudaSuccess) return e;
@@ -30,14 +31,14 @@ cudaError_t fx_angular_one(int kp, const void* one, const FxTcParams* params, co
   return launch_overlapped(kern, grid, kFxThreads, smem, s, p, params, owners, tiles);
 }
 
-template <bool FF>
+template <bool FF, bool EXPS>
 cudaError_t fx_angular_launch(int halves, int kp, int cols, const void* one, const FxTcParams* params,
                               const uint2* owners, int64_t tiles, unsigned grid, cudaStream_t s) {
-  if (halves == 1 && cols == 32) return fx_angular_one<8, 1, FF>(kp, one, params, owners, tiles, grid, s);
-  if (halves == 1 && cols == 16) return fx_angular_one<4, 1, FF>(kp, one, params, owners, tiles, grid, s);
-  if (halves == 1 && cols == 8) return fx_angular_one<2, 1, FF>(kp, one, params, owners, tiles, grid, s);
-  if (halves == 2 && cols == 16) return fx_angular_one<8, 2, FF>(kp, one, params, owners, tiles, grid, s);
-  if (halves == 2 && cols == 8) return fx_angular_one<4, 2, FF>(kp, one, params, owners, tiles, grid, s);
+  if (halves == 1 && cols == 32) return fx_angular_one<8, 1, FF, EXPS>(kp, one, params, owners, tiles, grid, s);
+  if (halves == 1 && cols == 16) return fx_angular_one<4, 1, FF, EXPS>(kp, one, params, owners, tiles, grid, s);
+  if (halves == 1 && cols == 8) return fx_angular_one<2, 1, FF, EXPS>(kp, one, params, owners, tiles, grid, s);
+  if (halves == 2 && cols == 16) return fx_angular_one<8, 2, FF, EXPS>(kp, one, params, owners, tiles, grid, s);
+  if (halves == 2 && cols == 8) return fx_angular_one<4, 2, FF, EXPS>(kp, one, params, owners, tiles, grid, s);
   return cudaErrorInvalidValue;
 }
 

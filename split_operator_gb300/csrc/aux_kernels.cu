@@ -208,12 +208,14 @@ cudaError_t launch_import(void* dst, int dst_real, const double* src, const Geom
 }
 
 // the largest |v|^2 of n complex values as the bits of a double (infinity when one is not finite
-// or above 1e300); out: zero at the launch
+// or above 1e300), and whether one that is not zero is below 1/4; out: zeros at the launch
 __global__ void table_max_kernel(unsigned long long* out, const double2* src, int64_t n) {
   double m = 0.0;
+  bool small = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const double2 v = src[i];
     const double a = __dadd_rn(__dmul_rn(v.x, v.x), __dmul_rn(v.y, v.y));
+    small = small || (a < 0.0625 && (v.x != 0.0 || v.y != 0.0));
     if (!(a <= 1e300))
       m = __longlong_as_double(0x7ff0000000000000ll);
     else if (a > m)
@@ -226,10 +228,11 @@ __global__ void table_max_kernel(unsigned long long* out, const double2* src, in
     b = o > b ? o : b;
   }
   if ((threadIdx.x & 31) == 0) atomicMax(out, b);
+  if (small) out[1] = 1ull;
 }
 
 cudaError_t launch_table_max(unsigned long long* out, const double* src, int64_t n, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(out, 0, sizeof(*out), st);
+  cudaError_t e = cudaMemsetAsync(out, 0, 2 * sizeof(*out), st);
   if (e != cudaSuccess) return e;
   table_max_kernel<<<blocks_for(n), 256, 0, st>>>(out, (const double2*)src, n);
   count_launch();

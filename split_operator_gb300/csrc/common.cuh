@@ -56,7 +56,10 @@ struct DevOp {
   int64_t count;  // matrices available (MAT_LANE / MAT_SLICE), record index (RECORD)
   double value;   // SETC
   const void* ptr;               // table / matrix base / other wave function
-  const double* w[kMaxDims];     // NORM / DOT weights per logical axis
+  union {
+    const double* w[kMaxDims];   // NORM / DOT weights per logical axis
+    const int16_t* exps;         // fixed-point DIAG1D / DIAGND: the table holds value 2^exps[lane] (nullptr: 0)
+  };
   const float* wf[kMaxDims];     // the same weights rounded to FP32 (FP32 passes)
 };
 
@@ -98,6 +101,7 @@ struct PassParams {
   int32_t fx;                   // fused FP64 / float-float: log2 n of the fixed-point kernel (0: floating point)
   int32_t fx_chirp, fx_g;       // ... lengths that are no power of two: fx is log2 of the inner transforms'
                                 // length M, and the filter in aux is scaled by 2^-fx_g
+  int32_t fx_exps;              // ... 1: an op has exps
   const void* aux;              // ... chirp (n factors) and filter spectrum (M factors)
   DevOp ops[kMaxOps];
 };
@@ -192,8 +196,13 @@ cudaError_t launch_fx_pair(int real, bool chirp, int lgn, const PassParams* one,
 // per repetition.  Sets p.fx and p.fx_chirp; tables and twiddles (radix 4) are then fixed point.
 bool fx_line_plan(PassParams& p, int real, const double* table_max);
 cudaError_t launch_fx_line(int real, const PassParams& p, cudaStream_t s);
-// a device table in the state precision as fixed-point factors (16 bytes a value as well)
-cudaError_t launch_fx_table(void* dst, const void* src, int real, int64_t n, cudaStream_t s);
+// a device table in the state precision as fixed-point factors (16 bytes a value as well); exps: the
+// exponents of its lanes of lane_n values, inner apart (nullptr: all 0)
+cudaError_t launch_fx_table(void* dst, const void* src, int real, int64_t n, const int16_t* exps, int64_t lane_n,
+                            int64_t inner, cudaStream_t s);
+// those exponents (one per lane), and whether one is not 0
+cudaError_t launch_fx_exponents(int16_t* exps, int* any, const void* src, int real, int64_t lanes, int64_t lane_n,
+                                int64_t inner, cudaStream_t s);
 
 // Lane-matrix passes of FP64 and float-float states on the tensor cores (angular_fx.cu): real
 // matrices of 16 to 256 points, at most two per pass.  The plan sets the tiling (*cols complex
@@ -204,9 +213,9 @@ bool fx_angular_image(const double* m, int n, unsigned char* out);  // false: no
 size_t fx_angular_params_bytes();
 void fx_angular_params(const PassParams& p, const int* mat_op, int nmat, const unsigned char* const* images,
                        const int* slice_axis, int error_slot, void* out);
-// one: the parameters of a single pass (host); or the batched form (params_dev, owners_dev)
-cudaError_t launch_fx_angular(int real, int n, int cols, const void* one, const void* params_dev, const void* owners_dev,
-                              int64_t tiles, cudaStream_t s);
+// one: the parameters of a single pass (host); or the batched form (params_dev, owners_dev).  exps: p.fx_exps
+cudaError_t launch_fx_angular(int real, int n, int cols, bool exps, const void* one, const void* params_dev,
+                              const void* owners_dev, int64_t tiles, cudaStream_t s);
 int64_t fx_angular_grid(int64_t tiles);  // persistent CTAs of a launch
 
 // Host launchers (lane_sweep.cu)
@@ -268,7 +277,8 @@ cudaError_t launch_scalar_program(const PassParams& p, cudaStream_t s);
 // real: the state precision of the device side (kRealF32, kRealF64, kRealFF)
 // dst (storage order, precision of dst) <- src (logical row-major complex128)
 cudaError_t launch_import(void* dst, int dst_real, const double* src, const Geometry& g, cudaStream_t s);
-// *out (device) <- the largest |v|^2 of n complex128 values, as the bits of a double
+// out[0] (device) <- the largest |v|^2 of n complex128 values, as the bits of a double; out[1] <- 1 when a
+// value that is not zero is below 1/4 in magnitude
 cudaError_t launch_table_max(unsigned long long* out, const double* src, int64_t n, cudaStream_t s);
 // storage order is the logical order / the transpose of a two-axis logical order (the
 // layouts whose import and export stay coalesced on both sides)

@@ -13,12 +13,49 @@ cudaError_t launch_fx_chirp_ff(int lgn, const PassParams* one, const PassParams*
 
 namespace {
 
-// a table's values as digits of w 2^62
+// 2 log2 |v| of a table's value, to 2^-9 (zero: far below every other)
 template <bool FF>
-__global__ void fx_table_kernel(int4* dst, const longlong2* src, int64_t n) {
+__device__ __forceinline__ float log_square(longlong2 v) {
+  const int e = max(raw_exp<FF>(v.x), raw_exp<FF>(v.y));
+  const float x = raw_rel<FF>(v.x, e), y = raw_rel<FF>(v.y, e);
+  return e == 0 ? -1e6f : 2.0f * (float)(e - 1023) + log2f(fmaf(x, x, y * y));
+}
+
+// Exponents of a table's lanes (`lanes` = outer x inner lanes of n values, `inner` apart): k with the
+// largest |value| 2^k in [1/2, 1] where that value is below 1/4, else 0.  A warp per contiguous lane,
+// a thread per lane of strided ones.  *any: set when an exponent is not 0.
+template <bool FF>
+__global__ void fx_exponent_kernel(int16_t* exps, int* any, const longlong2* src, int64_t n, int64_t inner, int64_t lanes) {
+  const int per = inner == 1 ? 32 : 1, sub = threadIdx.x % per;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x / per;
+  // (whole warps stay in the loop together)
+  for (int64_t l0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / per; l0 - (threadIdx.x & 31) / per < lanes; l0 += step) {
+    float m = -1e6f;
+    if (l0 < lanes) {
+      const int64_t o = l0 / inner, i = l0 - o * inner;
+      const longlong2* at = src + o * n * inner + i;
+#pragma unroll 8
+      for (int64_t j = sub; j < n; j += per) m = fmaxf(m, log_square<FF>(__ldg(at + j * inner)));
+    }
+    if (per == 32)
+      for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+    if (l0 < lanes && sub == 0) {
+      // (a lane of zeros has no exponent)
+      const int k = m < -4.0f && m > -1e5f ? (int)floorf(-0.5f * m) : 0;
+      if (k) *any = 1;
+      exps[l0] = (int16_t)k;
+    }
+  }
+}
+
+// a table's values as digits of w 2^62, of w 2^(62 + k) with the exponents of its lanes
+template <bool FF>
+__global__ void fx_table_kernel(int4* dst, const longlong2* src, int64_t n, const int16_t* exps, int64_t lane_n,
+                                int64_t inner) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const longlong2 v = src[i];
-    i64 d[2] = {raw_to_fx<FF>(v.x, -1), raw_to_fx<FF>(v.y, -1)};  // x 2^61, |x| < 2
+    const int e = -1 - (exps ? exps[i / (lane_n * inner) * inner + i % inner] : 0);
+    i64 d[2] = {raw_to_fx<FF>(v.x, e), raw_to_fx<FF>(v.y, e)};  // x 2^(61 + k), |x| 2^k < 2
     int4 o;
     int* w = &o.x;
     for (int k = 0; k < 2; ++k) {
@@ -86,12 +123,27 @@ cudaError_t launch_fx_pair(int real, bool chirp, int lgn, const PassParams* one,
                          : launch_any<false, false>(lgn, one, params_dev, offsets_dev, count, blocks, threads, smem, s);
 }
 
-cudaError_t launch_fx_table(void* dst, const void* src, int real, int64_t n, cudaStream_t s) {
+cudaError_t launch_fx_exponents(int16_t* exps, int* any, const void* src, int real, int64_t lanes, int64_t lane_n,
+                                int64_t inner, cudaStream_t s) {
+  const cudaError_t e = cudaMemsetAsync(any, 0, sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  const int64_t threads = lanes * (inner == 1 ? 32 : 1);
+  const unsigned blocks = (unsigned)(threads + 255 < 256 * 1216 ? (threads + 255) / 256 : 1216);
+  if (real == kRealFF)
+    fx_exponent_kernel<true><<<blocks, 256, 0, s>>>(exps, any, (const longlong2*)src, lane_n, inner, lanes);
+  else
+    fx_exponent_kernel<false><<<blocks, 256, 0, s>>>(exps, any, (const longlong2*)src, lane_n, inner, lanes);
+  count_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fx_table(void* dst, const void* src, int real, int64_t n, const int16_t* exps, int64_t lane_n,
+                            int64_t inner, cudaStream_t s) {
   const unsigned blocks = (unsigned)(n + 255 < 256 * 1216 ? (n + 255) / 256 : 1216);
   if (real == kRealFF)
-    fx_table_kernel<true><<<blocks, 256, 0, s>>>((int4*)dst, (const longlong2*)src, n);
+    fx_table_kernel<true><<<blocks, 256, 0, s>>>((int4*)dst, (const longlong2*)src, n, exps, lane_n, inner);
   else
-    fx_table_kernel<false><<<blocks, 256, 0, s>>>((int4*)dst, (const longlong2*)src, n);
+    fx_table_kernel<false><<<blocks, 256, 0, s>>>((int4*)dst, (const longlong2*)src, n, exps, lane_n, inner);
   count_launch();
   return cudaGetLastError();
 }

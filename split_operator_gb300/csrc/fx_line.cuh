@@ -35,6 +35,12 @@ __device__ __forceinline__ i64 rmul(i64 v, int2 f) {
   return (mw(a.h, f.y, 0) << 2) + (t >> 30);
 }
 
+// s + w |v|^2 (out of line: the steps' usual norms do not fetch it)
+__device__ __noinline__ double norm_term(cx v, double w, double s) {
+  const double x = (double)v.x, y = (double)v.y;
+  return fma(fma(x, x, y * y), w, s);
+}
+
 // digits of d 2^(62 - x), |d| < 2^(x + 1/2)
 __device__ __forceinline__ int2 real_digits(double d, int x) {
   i64 v = __double2ll_rn(ldexp(d, 62 - x));
@@ -230,8 +236,7 @@ __global__ void __launch_bounds__((1 << LG) / kLineV, 1) fx_line_kernel(const __
               s += rmul(q, wd[r]);
             } else {
               const int j = point(r, between);
-              const double x = (double)v[r].x, y = (double)v[r].y;
-              if (j < n) sd = fma(fma(x, x, y * y), __ldg(op.w[0] + j), sd);
+              if (j < n) sd = norm_term(v[r], __ldg(op.w[0] + j), sd);
             }
           }
           if (quick) {

@@ -54,6 +54,14 @@ __device__ __forceinline__ void pointwise(cx (&v)[KV], const PassParams& pp, int
   }
 }
 
+// exponent of a lane's factors together (out of line: few passes have them)
+__device__ __noinline__ int table_exponent(const PassParams& pp, int64_t lane) {
+  int k = 0;
+  for (int oi = 0; oi < pp.nops; ++oi)
+    if (pp.ops[oi].kind == OP_DIAGND && pp.ops[oi].exps) k += __ldg(pp.ops[oi].exps + lane);
+  return k;
+}
+
 template <int LGN, bool FF>
 __device__ __forceinline__ void fx_pair_tile(const PassParams& pp, int64_t tile) {
   constexpr int kV = pair_vals(LGN);
@@ -109,7 +117,7 @@ __device__ __forceinline__ void fx_pair_tile(const PassParams& pp, int64_t tile)
   // the last stage's outputs have the first stage's layout: the same lane, points k + q n / kV
   if (ok0) {
     longlong2* dst = psi + l0 * kN + i0;
-    const int x = e - Sh::kOut;
+    const int x = e - Sh::kOut - (pp.fx_exps ? table_exponent(pp, lane0 + l0) : 0);
 #pragma unroll
     for (int q = 0; q < kV; ++q) {
       longlong2 o{fx_to_raw<FF>(v[q].x, x), fx_to_raw<FF>(v[q].y, x)};
@@ -196,7 +204,6 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
     // 2^-56 of it (error of a packet of 1000 points through the pair 1.35e-15 / 4.6e-16 without / with
     // it, 8.0e-16 by the sum in FP64).
     const int ob = half ? f1 + 1 : 1, oe = half ? pp.nops : f1;
-    const int up = half ? 0 : 60 - Sh::kConvOut + pp.fx_g;
     static_assert(Sh::kConvOut <= 62, "g is at least 2: up is not negative");
 #pragma unroll
     for (int r = 0; r < kV; ++r) {
@@ -205,12 +212,14 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
         v[r] = {0, 0};
         continue;
       }
-      v[r] = {v[r].x << up, v[r].y << up};
       if (half) {
         int4 w = __ldg(chirp + j);
         w.z = -w.z;
         w.w = -w.w;
         v[r] = cmul<0>(v[r], w);
+      } else {
+        const int up = 60 - Sh::kConvOut + pp.fx_g;
+        v[r] = {v[r].x << up, v[r].y << up};
       }
       for (int oi = ob; oi < oe; ++oi) {
         const DevOp& op = pp.ops[oi];
@@ -220,7 +229,7 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
     }
   }
   if (ok0) {
-    const int x = e - (Sh::kConvOut - pp.fx_g);
+    const int x = e - (Sh::kConvOut - pp.fx_g) - (pp.fx_exps ? table_exponent(pp, lane0 + l0) : 0);
 #pragma unroll
     for (int r = 0; r < kV; ++r) {
       const int j = i0 + r * kNb;

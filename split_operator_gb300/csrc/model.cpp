@@ -278,13 +278,16 @@ static void upload_complex(DeviceBuffer& buf, const std::vector<cplx>& t, int re
   }
 }
 
-// largest magnitude of a table (infinity when a value is not finite)
-static double table_max(const std::vector<cplx>& t) {
+// largest magnitude of a table (infinity when a value is not finite); small: one that is not zero is
+// below 1/4
+static double table_max(const std::vector<cplx>& t, bool& small) {
   double m = 0.0;
   bool ok = true;
+  small = false;
   for (const cplx& v : t) {
     const double a = v.real() * v.real() + v.imag() * v.imag();
     ok = ok && a <= 1e300;  // false for NaN
+    small = small || (a < 0.0625 && v != cplx(0.0, 0.0));
     m = a > m ? a : m;
   }
   return ok ? std::sqrt(m) : HUGE_VAL;
@@ -295,9 +298,8 @@ const void* Engine::table_1d(const void* key, uint64_t version, const std::vecto
   if (c.buf.ptr && c.version == version) return c.buf.ptr;
   if (c.buf.ptr) flush();  // replacing a table the open pass may reference (a first upload needs no flush)
   upload_complex(c.buf, t, real, stream);
-  c.fx = DeviceBuffer();
-  c.fx_denied = false;
-  if (fx) c.max_abs = table_max(t);
+  c.fx.clear();
+  if (fx) c.max_abs = table_max(t, c.small);
   c.version = version;
   return c.buf.ptr;
 }
@@ -316,25 +318,31 @@ const void* Engine::table_nd(const void* key, uint64_t version, const std::vecto
   auto& c = tables_[{key, 1}];
   if (c.buf.ptr && c.version == version) return c.buf.ptr;
   if (c.buf.ptr) flush();
-  c.fx = DeviceBuffer();
-  c.fx_denied = false;
+  c.fx.clear();
   // logical row-major -> storage order and precision, on the device (a host loop over the strides
-  // took 6 ms of the first pass for 524,288 points); the last 8 bytes of raw: the largest magnitude.
-  // The table itself first; without room for the scratch copy beside it, the host's order below.
-  const size_t b = t.size() * sizeof(cplx);
-  if (c.buf.bytes != t.size() * elem_bytes()) c.buf = DeviceBuffer(t.size() * elem_bytes());
-  const DeviceBuffer raw = DeviceBuffer::if_room(b + sizeof(unsigned long long));
+  // took 6 ms of the first pass for 524,288 points); the last 16 bytes of raw: launch_table_max's.
+  // Without room for the scratch copy beside the table, the host's order below.
+  const size_t b = t.size() * sizeof(cplx), have = t.size() * elem_bytes();
+  DeviceBuffer raw = DeviceBuffer::if_room(b + 2 * sizeof(unsigned long long));
+  if (c.buf.bytes != have) c.buf = DeviceBuffer::if_room(have);
+  if (!c.buf.ptr) {
+    raw = DeviceBuffer();
+    c.buf = DeviceBuffer(have);
+  }
   if (raw.ptr) {
     unsigned long long* const top = reinterpret_cast<unsigned long long*>(raw.as<unsigned char>() + b);
     cuda_check(cudaMemcpyAsync(raw.ptr, t.data(), b, cudaMemcpyHostToDevice, stream), "table upload");
     cuda_check(launch_import(c.buf.ptr, real, raw.as<double>(), flat_geometry(*this), stream), "table import");
-    double max2 = 0.0;
+    unsigned long long found[2] = {0, 0};
     if (fx) {
       cuda_check(launch_table_max(top, raw.as<double>(), (int64_t)t.size(), stream), "table maximum");
-      cuda_check(cudaMemcpyAsync(&max2, top, sizeof(max2), cudaMemcpyDeviceToHost, stream), "table maximum");
+      cuda_check(cudaMemcpyAsync(found, top, sizeof(found), cudaMemcpyDeviceToHost, stream), "table maximum");
     }
     cuda_check(cudaStreamSynchronize(stream), "table upload sync");
-    if (fx) c.max_abs = std::sqrt(max2);
+    double max2;
+    std::memcpy(&max2, found, sizeof(max2));
+    c.max_abs = std::sqrt(max2);
+    c.small = found[1] != 0;
   } else {
     const int nd = (int)shape.size();
     std::vector<cplx> st(t.size());
@@ -354,7 +362,7 @@ const void* Engine::table_nd(const void* key, uint64_t version, const std::vecto
       st[s] = t[li];
     }
     upload_complex(c.buf, st, real, stream);
-    if (fx) c.max_abs = table_max(t);
+    if (fx) c.max_abs = table_max(t, c.small);
   }
   c.version = version;
   return c.buf.ptr;
@@ -366,25 +374,65 @@ Engine::Cached* Engine::phase_table(const void* device_ptr) {
   return nullptr;
 }
 
-// nullptr: no room, the passes with this table stay in floating point.  The copy of a large table (16 MB
+// false: no room, the passes with this table stay in floating point.  The copy of a large table (16 MB
 // and more) leaves as much again free: what a program allocates later (the copy of the state that an
 // energy takes, a staging buffer) found its room when there was no second copy.
-const void* Engine::fx_table(Cached& c) {
-  if (c.fx.ptr || c.fx_denied) return c.fx.ptr;
-  c.fx_denied = true;
-  if (c.buf.bytes >= (size_t)1 << 24) {
-    size_t free_bytes = 0, total = 0;
-    cuda_check(cudaMemGetInfo(&free_bytes, &total), "cudaMemGetInfo");
-    if (free_bytes / 2 < c.buf.bytes) return nullptr;
+//
+// A factor has 62 bits below the point, so one of 2^-30 (imaginary time, a wall of the potential) would
+// keep 32 of them, and a column it multiplies as many: every lane of the table (the values that multiply
+// one lane of the pass) whose factors are all below 1/4 has an exponent of its own.
+bool Engine::fx_table(Cached& c, int64_t n, int64_t inner, DevOp& op) {
+  if (!c.small) n = inner = 0;
+  Cached::Fx* f = &c.fx[{n, inner}];
+  if (f->denied) return false;
+  if (f->plain) f = &c.fx[{0, 0}];
+  if (!f->digits.ptr && !f->denied) {
+    const int64_t count = (int64_t)(c.buf.bytes / 16), lanes = n > 0 ? count / n : 0;
+    Cached::Fx made;
+    made.denied = true;  // until all of it has found room
+    auto give_up = [&] {
+      *f = std::move(made);
+      return false;
+    };
+    if (c.buf.bytes >= (size_t)1 << 24) {
+      size_t free_bytes = 0, total = 0;
+      cuda_check(cudaMemGetInfo(&free_bytes, &total), "cudaMemGetInfo");
+      if (free_bytes / 2 < c.buf.bytes) return give_up();
+    }
+    const size_t exp_bytes = ((size_t)lanes * sizeof(int16_t) + 15) / 16 * 16;
+    if (n > 0) {
+      // (the flag lies behind the exponents)
+      if (fx_scratch_.bytes < exp_bytes + sizeof(int)) fx_scratch_ = DeviceBuffer::if_room(exp_bytes + sizeof(int));
+      if (!fx_scratch_.ptr) return give_up();
+      int any = 0;
+      int* const flag = reinterpret_cast<int*>(fx_scratch_.as<unsigned char>() + exp_bytes);
+      cuda_check(launch_fx_exponents(fx_scratch_.as<int16_t>(), flag, c.buf.ptr, real, lanes, n, inner, stream),
+                 "table exponents");
+      cuda_check(cudaMemcpyAsync(&any, flag, sizeof(any), cudaMemcpyDeviceToHost, stream), "table exponents");
+      cuda_check(cudaStreamSynchronize(stream), "table exponents sync");
+      if (!any) {
+        f->plain = true;
+        return fx_table(c, 0, 0, op);
+      }
+    }
+    DeviceBuffer b = DeviceBuffer::if_room(c.buf.bytes + exp_bytes);
+    if (!b.ptr) return give_up();
+    if (n > 0) {
+      made.exps = reinterpret_cast<int16_t*>(b.as<unsigned char>() + c.buf.bytes);
+      cuda_check(cudaMemcpyAsync(b.as<unsigned char>() + c.buf.bytes, fx_scratch_.ptr, exp_bytes, cudaMemcpyDeviceToDevice,
+                                 stream), "table exponents");
+    }
+    cuda_check(launch_fx_table(b.ptr, c.buf.ptr, real, count, made.exps, n, inner, stream), "fixed-point table");
+    // as the uploads: complete before any stream of the engine uses it
+    cuda_check(cudaStreamSynchronize(stream), "fixed-point table sync");
+    made.digits = std::move(b);
+    made.denied = false;
+    *f = std::move(made);
   }
-  DeviceBuffer b = DeviceBuffer::if_room(c.buf.bytes);
-  if (!b.ptr) return nullptr;
-  cuda_check(launch_fx_table(b.ptr, c.buf.ptr, real, (int64_t)(c.buf.bytes / 16), stream), "fixed-point table");
-  // as the uploads: complete before any stream of the engine uses it
-  cuda_check(cudaStreamSynchronize(stream), "fixed-point table sync");
-  c.fx = std::move(b);
-  c.fx_denied = false;
-  return c.fx.ptr;
+  if (f->denied) return false;
+  op.ptr = f->digits.ptr;
+  op.exps = f->exps;
+  return true;
 }
 
 // Factor w 2^62 in two signed digits (fx.cuh).
@@ -956,8 +1004,13 @@ bool Engine::try_launch_fx_tc(const std::vector<DevOp>& ops, int axis, PassParam
   int cols = 0;
   PassParams q = p;
   if (nmat == 0 || !fx_angular_plan(q, ops.data(), (int)ops.size(), mx, &cols)) return false;
-  for (size_t i = 0; i < ops.size(); ++i)
-    if (tab[i] && !(q.ops[i].ptr = fx_table(*tab[i]))) return false;
+  for (size_t i = 0; i < ops.size(); ++i) {
+    if (!tab[i]) continue;
+    // exponents: of every column, or of every entry of a table along another axis
+    const bool nd = ops[i].kind == OP_DIAGND, along = !nd && ops[i].axis == q.g.sweep_axis;
+    if (!fx_table(*tab[i], along ? 0 : (nd ? q.g.n : 1), along ? 0 : (nd ? q.g.inner : 1), q.ops[i])) return false;
+    if (q.ops[i].exps) q.fx_exps = 1;
+  }
   p = q;
   grow_partials(p);
   const Geometry& g = p.g;
@@ -966,16 +1019,16 @@ bool Engine::try_launch_fx_tc(const std::vector<DevOp>& ops, int axis, PassParam
   std::vector<unsigned char> prm(fx_angular_params_bytes());
   fx_angular_params(p, mats, nmat, images, slices, timeout_slot, prm.data());
   if (recording) {
-    // threads: the lane extent and the tile's columns (one batched launch serves one of each)
-    recording->push_back(RecordedPass{RecordedPass::TensorCore, real, p, std::move(prm), (int)g.n | (cols << 16), 0,
-                                      name, pass_bytes(ops, g)});
+    // threads: the lane extent, the tile's columns and the tables' form (one batched launch serves one of each)
+    recording->push_back(RecordedPass{RecordedPass::TensorCore, real, p, std::move(prm),
+                                      (int)g.n | (cols << 16) | (p.fx_exps << 24), 0, name, pass_bytes(ops, g)});
     return true;
   }
   if (timing) {
     timed_begin(name);
     timed_.back().bytes = pass_bytes(ops, g);
   }
-  cuda_check(launch_fx_angular(real, (int)g.n, cols, prm.data(), nullptr, nullptr, g.tiles, stream),
+  cuda_check(launch_fx_angular(real, (int)g.n, cols, p.fx_exps != 0, prm.data(), nullptr, nullptr, g.tiles, stream),
              "lane-matrix pass launch");
   if (timing) timed_end();
   return true;
@@ -993,8 +1046,12 @@ bool Engine::try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p, bo
     }
   PassParams q = p;
   if (!(resident ? fx_line_plan(q, real, mx) : fx_pair_plan(q, real, mx))) return false;
-  for (size_t i = 0; i < ops.size(); ++i)
-    if (tab[i] && !(q.ops[i].ptr = fx_table(*tab[i]))) return false;
+  for (size_t i = 0; i < ops.size(); ++i) {
+    if (!tab[i]) continue;
+    const bool lanes = !resident && ops[i].kind == OP_DIAGND;
+    if (!fx_table(*tab[i], lanes ? q.g.n : 0, lanes ? 1 : 0, q.ops[i])) return false;
+    if (q.ops[i].exps) q.fx_exps = 1;
+  }
   if (!(q.twiddle = fx_twiddle((size_t)1 << q.fx, resident ? 4 : q.radix))) return false;
   if (q.fx_chirp) {
     const FxFactors* f = fx_chirp((size_t)q.g.n, q.fx);
@@ -2337,8 +2394,8 @@ void Batch::run_groups(std::vector<Group>& gs, bool concurrent) {
       cuda_check(cudaEventRecord(t.a, stream_), "event record");
     }
     if (g.kind == RecordedPass::TensorCore && g.real != kRealF32)
-      cuda_check(launch_fx_angular(g.real, g.threads & 0xffff, g.threads >> 16, nullptr, g.params.ptr, g.owners.ptr,
-                                   g.blocks, st),
+      cuda_check(launch_fx_angular(g.real, g.threads & 0xffff, (g.threads >> 16) & 0xff, (g.threads >> 24) & 1, nullptr,
+                                   g.params.ptr, g.owners.ptr, g.blocks, st),
                  "batched lane-matrix pass");
     else if (g.kind == RecordedPass::TensorCore)
       cuda_check(launch_angular_tc_batched(g.params.ptr, g.owners.ptr, g.blocks, g.smem, (g.threads >> 17) & 3,

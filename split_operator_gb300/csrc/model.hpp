@@ -224,8 +224,15 @@ class Engine {
     DeviceBuffer buf;
     bool real;
     double max_abs = 0.0;  // phase tables: the largest magnitude (infinity when one is not finite)
-    DeviceBuffer fx;       // phase tables: fixed-point copy, made at its first use
-    bool fx_denied = false;  // ... no room for it
+    bool small = false;    // ... and whether one that is not zero is below 1/4
+    // fixed-point copies, made at their first use: by the (extent, stride) of the lanes that have an
+    // exponent each, {0, 0} for the one without exponents
+    struct Fx {
+      DeviceBuffer digits;
+      const int16_t* exps = nullptr;       // behind the digits
+      bool plain = false, denied = false;  // no lane needs an exponent; no room for the copy
+    };
+    std::map<std::pair<int64_t, int64_t>, Fx> fx;
     int parity = 0;     // float-float: kind of the parity structure, half matrix in half_buf
     DeviceBuffer half_buf;
     // A-operand chunk images of the tensor-core passes, and the same for the parity-split
@@ -245,10 +252,12 @@ class Engine {
                                std::shared_ptr<DeviceBuffer>& img, std::shared_ptr<DeviceBuffer>& par, int& kind);
   bool try_launch_fx_pair(const std::vector<DevOp>& ops, PassParams& p, bool resident);
   bool try_launch_fx_tc(const std::vector<DevOp>& ops, int axis, PassParams& p);
+  DeviceBuffer fx_scratch_;  // exponents of a table being converted
   void fx_images(const void* matrix, const std::vector<cplx>& m, size_t n, size_t count);
   std::map<const void*, std::shared_ptr<DeviceBuffer>> fx_images_;  // digit images by device matrix
   Cached* phase_table(const void* device_ptr);           // the cache entry of a phase table
-  const void* fx_table(Cached& c);                       // its fixed-point copy (nullptr: no room)
+  // puts its fixed-point copy into op (lanes of n values, inner apart; n = 0: no exponents); false: no room
+  bool fx_table(Cached& c, int64_t n, int64_t inner, DevOp& op);
   // fixed-point factors shared by the process: twiddles of n points, chirp and filter of n points
   std::shared_ptr<FxFactors> fx_shared(int kind, size_t n, const std::function<FxHost()>& make);
   const void* fx_twiddle(size_t n, int radix);
