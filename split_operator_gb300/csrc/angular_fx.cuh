@@ -152,12 +152,13 @@ __device__ __forceinline__ int bits_of(i64 x, i64 y) {  // |x|, |y| <= 2^bits (0
   return a == 0 ? ((x | y) != 0 ? 1 : 0) : 64 - __clzll((i64)a);
 }
 
-// d 2^k (d >= 0 or NaN), flushing to zero and saturating to infinity
+// d 2^k (d >= 0 or NaN), saturating to infinity
 __device__ __forceinline__ double scale_pow2(double d, int k) {
   const i64 b = __double_as_longlong(d);
   const int e = (int)(b >> 52) & 0x7ff;
   if (e == 0 || e == 0x7ff) return d;
-  if (e + k <= 0) return 0.0;
+  if (e + k <= 0)  // subnormal
+    return e + k < -60 ? 0.0 : __longlong_as_double(b + ((i64)(k + 64) << 52)) * 0x1p-64;
   if (e + k >= 0x7ff) return __longlong_as_double(0x7ff0000000000000ll);
   return __longlong_as_double(b + ((i64)k << 52));
 }
@@ -387,15 +388,14 @@ struct RowWeight {
 };
 
 // v 2^e rounded as a store in FP64 would (fx_to_f64), in place; E: the biased exponent of the stored
-// value (0: it is zero, and so is the result; 2047: infinite).
+// value (0 or less: zero or subnormal; 2047: infinite).  Subnormal values keep their 53 bits here: the check
+// for them took 1 % of the pass, so among them a run in parts may differ by one unit of 2^-1074.
 __device__ __forceinline__ i64 round_f64(i64 v, int e, int& E) {
   const i64 s = v >> 63;
   unsigned long long a = (unsigned long long)((v ^ s) - s);
-  const int lz = __clzll((i64)a), drop = 11 - lz;
-  const int before = 63 - lz + e + 1023;
+  const int drop = 11 - __clzll((i64)a);
   if (drop > 0) a = ((a >> drop) + ((a >> (drop - 1)) & 1ull)) << drop;
   const int after = 63 - __clzll((i64)a) + e + 1023;  // one more after a carry
-  if (a == 0 || before < 1) a = 0;
   E = a == 0 ? 0 : min(after, 2047);
   return ((i64)a ^ s) - s;
 }
@@ -407,6 +407,9 @@ __device__ __forceinline__ i64 rescale_f64(i64 v, int k) {
   const unsigned long long r = ((a >> (k > 64 ? 63 : k - 1)) + 1ull) >> 1;
   return ((i64)r ^ s) - s;
 }
+
+// (out of line: columns below 2^-962)
+__device__ __noinline__ i64 cold_to_f64(i64 v, int e) { return fx_to_f64<true>(v, e); }
 
 // The tile's tables of weights and factors (all but SCALE's); clears the column maxima.  All work threads.
 template <bool EXPS>
@@ -606,12 +609,12 @@ struct FxWork {
           if (threadIdx.x < 4 * NB) {
             const int e = T.coler[threadIdx.x];
             if (e == 2047) T.colx[threadIdx.x] = kPoison;
-            if (T.colx[threadIdx.x] != kPoison) T.colx[threadIdx.x] = max(e, 1) - 1022 - 60;
+            if (T.colx[threadIdx.x] != kPoison) T.colx[threadIdx.x] = max(e, kMinExp<FF>) - 1022 - 60;
           }
 #pragma unroll
           for (int u = 0; u < NB; ++u) {
-            const int e = T.coler[c0 + u];
-            const bool live = e != 2047 && e != 0;
+            const int e = max(T.coler[c0 + u], kMinExp<FF>);
+            const bool live = e != 2047;
             if constexpr (FF) {
               w[u] = {live ? raw_to_fx<FF>(raw[u].x, e - 1022) : 0, live ? raw_to_fx<FF>(raw[u].y, e - 1022) : 0};
             } else {
@@ -812,13 +815,13 @@ __global__ void __launch_bounds__(kFxThreads, 1)
       fx_work_sync();
       if (tid < BN) {
         const int e = T.cole[0][tid];
-        T.colx[tid] = e == 2047 || s_bad ? Work::kPoison : max(e, 1) - 1022 - 60;
-        T.colb[tid] = max(e, 1) - 1022;
+        T.colx[tid] = e == 2047 || s_bad ? Work::kPoison : max(e, kMinExp<FF>) - 1022 - 60;
+        T.colb[tid] = max(e, kMinExp<FF>) - 1022;
       }
 #pragma unroll
       for (int u = 0; u < NB; ++u) {
-        const int e = T.cole[0][W.c0 + u];
-        const bool live = e != 2047 && e != 0 && !s_bad;
+        const int e = max(T.cole[0][W.c0 + u], kMinExp<FF>);
+        const bool live = e != 2047 && !s_bad;
         W.w[u] = {live ? raw_to_fx<FF>(raw[u].x, e - 1022) : 0, live ? raw_to_fx<FF>(raw[u].y, e - 1022) : 0};
       }
       fx_work_sync();  // the exponents and tables are complete
@@ -898,13 +901,23 @@ __global__ void __launch_bounds__(kFxThreads, 1)
         break;
       }
       // store
+      bool low = false;
+      if constexpr (!FF) {
 #pragma unroll
-      for (int u = 0; u < NB; ++u) {
-        const int x = T.colx[W.c0 + u];
-        const int e = x + W.rowx + W.xs;
-        W.w[u] = {fx_to_raw<FF>(W.w[u].x, e), fx_to_raw<FF>(W.w[u].y, e)};
-        if (x == Work::kPoison) W.w[u] = {raw_nan<FF>(), raw_nan<FF>()};
+        for (int u = 0; u < NB; ++u) low = low || T.colx[W.c0 + u] + W.rowx + W.xs < kLowExp;
       }
+      auto packed = [&](auto&& f) {
+#pragma unroll
+        for (int u = 0; u < NB; ++u) {
+          const int x = T.colx[W.c0 + u], e = x + W.rowx + W.xs;
+          W.w[u] = {f(W.w[u].x, e), f(W.w[u].y, e)};
+          if (x == Work::kPoison) W.w[u] = {raw_nan<FF>(), raw_nan<FF>()};
+        }
+      };
+      if (!FF && __builtin_expect(low, 0))
+        packed([](i64 v, int e) { return cold_to_f64(v, e); });
+      else
+        packed([](i64 v, int e) { return fx_to_raw<FF, false>(v, e); });
       if (whole) {
 #pragma unroll
         for (int u = 0; u < NB; u += 2) store_pair(psi + u, W.w[u], W.w[u + 1]);

@@ -205,6 +205,9 @@ __device__ __forceinline__ cx shift_down(cx v) {
 
 // ---- conversions.  The state's element: FP64 pairs, or hi + lo FP32 pairs (FF); a raw
 // element is its two 8-byte halves.  Exponents are FP64's biased ones in both cases.
+// the least biased exponent of a normal number; subnormal ones are below 2^(kMinExp - 1023)
+template <bool FF>
+constexpr int kMinExp = FF ? 897 : 1;
 // biased exponent of a raw real (0 for zero and subnormals; 2047 when it is not finite)
 template <bool FF>
 __device__ __forceinline__ int raw_exp(i64 r) {
@@ -225,6 +228,20 @@ __device__ __forceinline__ float raw_rel(i64 r, int ref) {
     const int d = b - (ref - 896 - 127) * (1 << 23);
     return b >= (1 << 23) && d > 0 ? __int_as_float(d) : 0.0f;
   }
+}
+// the bits of |x|, of hi and lo together for a pair: below kMinExp, |x| < 2^(their length - kSubnormal)
+template <bool FF>
+__device__ __forceinline__ unsigned long long raw_bits(i64 r) {
+  if constexpr (!FF) return (unsigned long long)(r & 0x7fffffffffffffffll);
+  return (uint32_t)(r | (r >> 32)) & 0x7fffffffu;
+}
+template <bool FF>
+constexpr int kSubnormal = FF ? 149 : 1074;
+// raw_rel at ref = kMinExp of a value that is not above that exponent, subnormal ones as well
+template <bool FF>
+__device__ __forceinline__ float raw_rel_least(i64 r) {
+  if constexpr (!FF) return (float)(r & 0x1fffffffffffffll) * 0x1p-52f;
+  return (float)((uint32_t)r & 0xffffffu) * 0x1p-23f;
 }
 // a significand with its top bit at 62, moved right by r >= 1 bits, rounded to nearest (from 64
 // bits on it is below half a unit: zero)
@@ -257,17 +274,26 @@ __device__ __forceinline__ i64 raw_to_fx(i64 r, int e) {
     return v;
   }
 }
-// v 2^x -> FP64 bits, rounded to nearest (subnormal results become zero)
+// |d| 2^(x + 1022), x < -1022 (out of line: lanes below 2^-962 come here)
+static __device__ __noinline__ unsigned long long lower_f64(unsigned long long b, int x) {
+  if (x < -2022) return 0ull;
+  return (unsigned long long)__double_as_longlong(__longlong_as_double((i64)b) * __longlong_as_double((i64)(x + 2045) << 52));
+}
+// v 2^x -> FP64 bits, rounded to nearest.  From x = kLowExp on no result is subnormal; below (LOW), it is
+// made at kLowExp and brought down by a multiplication.
+constexpr int kLowExp = -1022;
+template <bool LOW>
 __device__ __forceinline__ i64 fx_to_f64(i64 v, int x) {
   const int s = (int)(v >> 63);
   const unsigned long long a = (unsigned long long)apply_sign(v, s);
   const int lz = __clzll((i64)a);
   const unsigned long long n = a << (lz & 63);               // top bit at 63
   const unsigned long long m = (n >> 11) + ((n >> 10) & 1);  // 53 bits (2^53 after a carry)
-  const int E = 63 - lz + x + 1023;
+  const int E = 63 - lz + (LOW ? max(x, kLowExp) : x) + 1023;
   unsigned long long b = m + ((unsigned long long)(E - 1) << 52);  // the hidden bit adds 1 to E - 1
   if (E > 2046) b = 0x7ffull << 52;
-  if (a == 0 || E < 1) b = 0;
+  if (a == 0) b = 0;
+  if (LOW && __builtin_expect(x < kLowExp, 0)) b = lower_f64(b, x);
   return (i64)(b | ((unsigned long long)(uint32_t)s << 63));
 }
 // v 2^x -> the hi + lo FP32 pair as a raw half
@@ -292,10 +318,10 @@ __device__ __forceinline__ i64 fx_to_ff(i64 v0, int x) {
   fl = fl * f1 * f2;
   return (i64)(((unsigned long long)__float_as_uint(fl) << 32) | __float_as_uint(fh));
 }
-template <bool FF>
+template <bool FF, bool LOW = true>
 __device__ __forceinline__ i64 fx_to_raw(i64 v, int x) {
   if constexpr (FF) return fx_to_ff(v, x);
-  return fx_to_f64(v, x);
+  return fx_to_f64<LOW>(v, x);
 }
 template <bool FF>
 __device__ __forceinline__ i64 raw_nan() {

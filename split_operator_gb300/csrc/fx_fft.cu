@@ -16,9 +16,12 @@ namespace {
 // 2 log2 |v| of a table's value, to 2^-9 (zero: far below every other)
 template <bool FF>
 __device__ __forceinline__ float log_square(longlong2 v) {
-  const int e = max(raw_exp<FF>(v.x), raw_exp<FF>(v.y));
-  const float x = raw_rel<FF>(v.x, e), y = raw_rel<FF>(v.y, e);
-  return e == 0 ? -1e6f : 2.0f * (float)(e - 1023) + log2f(fmaf(x, x, y * y));
+  const int e = max(max(raw_exp<FF>(v.x), raw_exp<FF>(v.y)), kMinExp<FF>);
+  const bool least = e == kMinExp<FF>;
+  const float x = least ? raw_rel_least<FF>(v.x) : raw_rel<FF>(v.x, e);
+  const float y = least ? raw_rel_least<FF>(v.y) : raw_rel<FF>(v.y, e);
+  const float s = fmaf(x, x, y * y);
+  return s > 0.0f ? 2.0f * (float)(e - 1023) + log2f(s) : -1e6f;
 }
 
 // Exponents of a table's lanes (`lanes` = outer x inner lanes of n values, `inner` apart): k with the
@@ -41,7 +44,7 @@ __global__ void fx_exponent_kernel(int16_t* exps, int* any, const longlong2* src
       for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
     if (l0 < lanes && sub == 0) {
       // (a lane of zeros has no exponent)
-      const int k = m < -4.0f && m > -1e5f ? (int)floorf(-0.5f * m) : 0;
+      const int k = m < -4.0f && m > -1e5f ? min((int)floorf(-0.5f * m), 1024 - kMinExp<FF> - 1) : 0;
       if (k) *any = 1;
       exps[l0] = (int16_t)k;
     }

@@ -287,9 +287,12 @@ __global__ void __launch_bounds__((1 << LG) / kLineV, 1) fx_line_kernel(const __
       }
     }
     // the step's result in the state's precision
+    by_exponent<FF>(ex, [&](auto low) {
+      constexpr bool L = decltype(low)::value;
 #pragma unroll
-    for (int r = 0; r < kLineV; ++r)
-      v[r] = {bad ? raw_nan<FF>() : fx_to_raw<FF>(v[r].x, ex), bad ? raw_nan<FF>() : fx_to_raw<FF>(v[r].y, ex)};
+      for (int r = 0; r < kLineV; ++r)
+        v[r] = {bad ? raw_nan<FF>() : fx_to_raw<FF, L>(v[r].x, ex), bad ? raw_nan<FF>() : fx_to_raw<FF, L>(v[r].y, ex)};
+    });
     if (CHIRP) {
 #pragma unroll
       for (int r = 0; r < kLineV; ++r)

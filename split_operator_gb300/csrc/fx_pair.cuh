@@ -118,12 +118,15 @@ __device__ __forceinline__ void fx_pair_tile(const PassParams& pp, int64_t tile)
   if (ok0) {
     longlong2* dst = psi + l0 * kN + i0;
     const int x = e - Sh::kOut - (pp.fx_exps ? table_exponent(pp, lane0 + l0) : 0);
+    auto store = [&](auto low) {
 #pragma unroll
-    for (int q = 0; q < kV; ++q) {
-      longlong2 o{fx_to_raw<FF>(v[q].x, x), fx_to_raw<FF>(v[q].y, x)};
-      if (e == kNonFinite) o = {raw_nan<FF>(), raw_nan<FF>()};
-      dst[q * kNb] = o;
-    }
+      for (int q = 0; q < kV; ++q) {
+        longlong2 o{fx_to_raw<FF, decltype(low)::value>(v[q].x, x), fx_to_raw<FF, decltype(low)::value>(v[q].y, x)};
+        if (e == kNonFinite) o = {raw_nan<FF>(), raw_nan<FF>()};
+        dst[q * kNb] = o;
+      }
+    };
+    by_exponent<FF>(x, store);
   }
 }
 
@@ -230,14 +233,17 @@ __device__ __forceinline__ void fx_chirp_tile(const PassParams& pp, int64_t tile
   }
   if (ok0) {
     const int x = e - (Sh::kConvOut - pp.fx_g) - (pp.fx_exps ? table_exponent(pp, lane0 + l0) : 0);
+    auto store = [&](auto low) {
 #pragma unroll
-    for (int r = 0; r < kV; ++r) {
-      const int j = i0 + r * kNb;
-      if (j >= n) continue;
-      longlong2 o{fx_to_raw<FF>(v[r].x, x), fx_to_raw<FF>(v[r].y, x)};
-      if (e == kNonFinite) o = {raw_nan<FF>(), raw_nan<FF>()};
-      psi[l0 * n + j] = o;
-    }
+      for (int r = 0; r < kV; ++r) {
+        const int j = i0 + r * kNb;
+        if (j >= n) continue;
+        longlong2 o{fx_to_raw<FF, decltype(low)::value>(v[r].x, x), fx_to_raw<FF, decltype(low)::value>(v[r].y, x)};
+        if (e == kNonFinite) o = {raw_nan<FF>(), raw_nan<FF>()};
+        psi[l0 * n + j] = o;
+      }
+    };
+    by_exponent<FF>(x, store);
   }
 }
 

@@ -1,6 +1,8 @@
 // Fixed-point transforms (fx.cuh) of power-of-two lanes held in registers, KV values per thread,
 // exchanged in place in one shared buffer; and the norm bound a lane is scaled by.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 #include "fx.cuh"
 
@@ -177,14 +179,24 @@ __device__ __forceinline__ void conjugate(cx (&v)[KV]) {
   for (int r = 0; r < KV; ++r) v[r].y = -v[r].y;
 }
 
+// store(true) for a lane whose results may be subnormal, else store(false): the check once, out of the
+// conversions (in each of them it took 2 % of a resident step)
+template <bool FF, class F>
+__device__ __forceinline__ void by_exponent(int x, F&& store) {
+  if (!FF && __builtin_expect(x < kLowExp, 0))
+    store(std::integral_constant<bool, true>{});
+  else
+    store(std::integral_constant<bool, false>{});
+}
+
 // Lane norm bounds.  A thread's KV values lie in one lane (lane = t >> lg(n / KV)).  Returns e
 // with |lane|_2 <= 2^e, kNonFinite for a lane with a value that is not finite, kZero for one of
-// zeros and subnormals (which becomes zero).  part: one entry per warp.
+// zeros.  part: one entry per warp.
 struct NormPart {
   int ref;
   uint32_t sum;  // sum |x|^2 2^(2 (1023 - ref)) in units of 2^-12, rounded up
 };
-constexpr int kNonFinite = 1 << 20, kZero = -(1 << 20);
+constexpr int kNonFinite = 1 << 20, kZero = -(1 << 20), kNone = -4096;
 template <int LGN, int KV, bool FF>
 __device__ __forceinline__ int lane_exponent(const cx (&raw)[KV], NormPart* part) {
   constexpr int kTpl = (1 << LGN) / KV;  // threads per lane
@@ -192,6 +204,13 @@ __device__ __forceinline__ int lane_exponent(const cx (&raw)[KV], NormPart* part
   int m = 0;
 #pragma unroll
   for (int e = 0; e < KV; ++e) m = max(m, max(raw_exp<FF>(raw[e].x), raw_exp<FF>(raw[e].y)));
+  if (__builtin_expect(m == 0, 0)) {
+    // zeros and subnormal values: the exponent these stand for
+    unsigned long long any = 0;
+#pragma unroll
+    for (int e = 0; e < KV; ++e) any |= raw_bits<FF>(raw[e].x) | raw_bits<FF>(raw[e].y);
+    m = any ? 64 - __clzll((i64)any) - kSubnormal<FF> + 1022 : kNone;
+  }
   constexpr int kG = kTpl < 32 ? kTpl : 32;
   const unsigned mask = kG == 32 ? 0xffffffffu : ((1u << (kG & 31)) - 1u) << (lane & ~(kG - 1));
   m = __reduce_max_sync(mask, m);
@@ -210,7 +229,7 @@ __device__ __forceinline__ int lane_exponent(const cx (&raw)[KV], NormPart* part
     const int w = t >> 5, w0 = w & ~(kW - 1);
     if (lane == 0) part[w] = {m, q};
     __syncthreads();
-    m = 0;
+    m = kNone;
 #pragma unroll
     for (int i = 0; i < kW; ++i) m = max(m, part[w0 + i].ref);
     ref = max(m, 1);
@@ -223,10 +242,13 @@ __device__ __forceinline__ int lane_exponent(const cx (&raw)[KV], NormPart* part
     tot += 1.0f;  // the terms cut off above, in units of 2^-12 of the largest value's square
   }
   if (m == 2047) return kNonFinite;
-  if (m == 0) return kZero;
+  // subnormal values alone: by their number; beside larger ones they are covered by a least exponent
+  // (four times what they come to)
+  constexpr int kCount = (LGN + 2) / 2, kLeast = kMinExp<FF> - 1023;
+  if (__builtin_expect(m < kMinExp<FF>, 0)) return m == kNone ? kZero : max(m - 1022 + kCount, kLeast);
   // |lane|^2 <= tot (1 + 2^-15) 2^-12 2^(2 (ref - 1023)): e = the least integer with 4^e above
   const int ex = (__float_as_int(fmaf(tot, 0x1p-15f, tot)) >> 23) - 127 - 12;  // tot < 2^(ex + 1)
-  return (ref - 1023) + ((ex + 2) >> 1);
+  return max((ref - 1023) + ((ex + 2) >> 1), kLeast + kCount + 2);
 }
 
 }  // namespace
