@@ -78,7 +78,7 @@ __global__ void __launch_bounds__((1 << LG) / kLineV, 1) fx_line_kernel(const __
     v[r] = {x.x, x.y};
   }
   // weights of the program's first norm as digits (position grid), scaled by their largest exponent:
-  // weights within 2^8 of each other keep all of their bits so, others take the general sum below
+  // weights within a factor of 4 leave the sum its bits, others take the general sum below
   const double* w0 = nullptr;
   int2 wd[kLineV];
   int wx = 0;
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__((1 << LG) / kLineV, 1) fx_line_kernel(const __
     wx = m - 1022;  // |w| < 2^wx
 #pragma unroll
     for (int r = 0; r < kLineV; ++r) wd[r] = real_digits(w[r], wx);
-    if (m == 2047 || least < m - 8) w0 = nullptr;
+    if (m == 2047 || least < m - 2) w0 = nullptr;
   }
   __syncthreads();
   bool bad = false;  // a value was not finite: the state is NaN from here on
@@ -166,17 +166,16 @@ __global__ void __launch_bounds__((1 << LG) / kLineV, 1) fx_line_kernel(const __
               }
             }
             transform<LG, kLineV, true, 0, 1>(v, buf, tw);
-            // (the first convolution's bits are moved back up, see fx_pair.cuh)
+            // a convolution leaves the points 2^up below the scale that ex stands for: moved back up, or
+            // the second one and the norms would round at that
             const int up = p.fx_g - Sh::kSc;
-            if (!fwd) ex += up;
 #pragma unroll
             for (int r = 0; r < kLineV; ++r) {
               const int j = t + r * kT;
+              v[r] = {v[r].x << up, v[r].y << up};
               if (j >= n) {
                 v[r] = {0, 0};
-              } else if (fwd) {
-                v[r] = {v[r].x << up, v[r].y << up};
-              } else {
+              } else if (!fwd) {
                 int4 w = __ldg(chirp + j);
                 w.z = -w.z;
                 w.w = -w.w;
@@ -232,7 +231,11 @@ __global__ void __launch_bounds__((1 << LG) / kLineV, 1) fx_line_kernel(const __
           for (int r = 0; r < kLineV; ++r) {
             if (quick) {
               const dig a = split(v[r].x), b = split(v[r].y);
-              const i64 q = (mw(b.h, b.h, mw(a.h, a.h, 0)) << 2) + (mw(b.h, b.l, mw(a.h, a.l, 1ll << 28)) >> 29);
+              // (with the low digits' squares, from their upper halves: the thirds of a unit that they come
+              // to were 4e-14 of the norm of 500 points)
+              const int al = a.l >> 16, bl = b.l >> 16;
+              const uint32_t low = ((uint32_t)(al * al) + (uint32_t)(bl * bl) + (1u << 29)) >> 1;
+              const i64 q = (mw(b.h, b.h, mw(a.h, a.h, 0)) << 2) + (mw(b.h, b.l, mw(a.h, a.l, (i64)low)) >> 29);
               s += rmul(q, wd[r]);
             } else {
               const int j = point(r, between);
