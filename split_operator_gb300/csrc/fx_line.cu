@@ -10,7 +10,7 @@ bool fx_line_plan(PassParams& p, int real, const double* table_max) {
   const Geometry& g = p.g;
   const bool pow2 = (g.n & (g.n - 1)) == 0;
   if (real == kRealF32 || g.ndim != 1 || !p.resident || g.n < 16 || g.n > (pow2 ? 4096 : 2048)) return false;
-  int ffts = 0;
+  int ffts = 0, scales = 0;
   double prod = 1.0;
   for (int i = 0; i < p.nops; ++i) {
     switch (p.ops[i].kind) {
@@ -22,7 +22,9 @@ bool fx_line_plan(PassParams& p, int real, const double* table_max) {
         if (!(table_max[i] >= kMinTable && table_max[i] <= kMaxTable)) return false;
         prod *= table_max[i] > 1.0 ? table_max[i] : 1.0;
         break;
-      case OP_NORM: case OP_COPY: case OP_LOSS: case OP_SETC: case OP_RECORD: case OP_SCALE: break;
+      // the headroom of the values holds two factors of up to 1.25: the ones after them stay below 1
+      case OP_SCALE: p.ops[i].a = ++scales > 2 ? 1 : 0; break;
+      case OP_NORM: case OP_COPY: case OP_LOSS: case OP_SETC: case OP_RECORD: break;
       default: return false;
     }
   }

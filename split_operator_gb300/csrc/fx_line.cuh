@@ -204,7 +204,8 @@ __global__ void __launch_bounds__((1 << LG) / kLineV, 1) fx_line_kernel(const __
             const double f = sqrt(S.slots[op.b] / S.slots[op.c]);
             int x = 0;
             double m = frexp(f, &x);
-            if (m < 0.625) {  // factors about 1, and below 1.25
+            // factors about 1, and below 1.25, or (op.a, from the third of a step on) below 1
+            if (m < 0.625 && op.a == 0) {
               m *= 2.0;
               x -= 1;
             }
