@@ -361,6 +361,8 @@ int so_mlp_gradients(so_mlp m, const float* x, const float* target, size_t batch
 /* `steps` full-batch Adam steps; losses[i] (may be NULL) = loss before step i */
 int so_mlp_train(so_mlp m, const float* x, const float* target, size_t batch, size_t steps, float lr,
                  double* losses);
+/* self-test: the next call's products report that a bounded wait gave up */
+int so_selftest_mlp_give_up(so_mlp m);
 void so_mlp_free(so_mlp m);
 
 /* ---- Allocation-free lane FFT + norm (no counterpart in the reference) ----

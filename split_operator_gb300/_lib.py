@@ -152,6 +152,7 @@ SIGNATURES = {
     "so_mlp_set_params": [_P, C.POINTER(C.c_float)],
     "so_mlp_forward": [_P, C.POINTER(C.c_float), _S, C.POINTER(C.c_float)],
     "so_mlp_gradients": [_P, C.POINTER(C.c_float), C.POINTER(C.c_float), _S, _DP, C.POINTER(C.c_float)],
+    "so_selftest_mlp_give_up": [_P],
     "so_mlp_train": [_P, C.POINTER(C.c_float), C.POINTER(C.c_float), _S, _S, C.c_float, _DP],
 }
 VOID = {

@@ -809,6 +809,11 @@ def selftest_bounded_wait(limit_ns: int):
     return bool(out[0]), bool(out[1]), int(out[2])
 
 
+def selftest_mlp_give_up(net: Mlp):
+    """The next call's products of the network report that a bounded wait gave up."""
+    call("so_selftest_mlp_give_up", net._h)
+
+
 def launch_count() -> int:
     v = C.c_uint64()
     call("so_launch_count", C.byref(v))

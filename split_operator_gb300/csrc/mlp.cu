@@ -383,22 +383,31 @@ struct ParamLayer {
 };
 struct ParamArgs {
   ParamLayer l[kMaxLayers];
+  const int* err;  // set: a product of this step or of one before it gave up, and the parameters stay
+  int* steps;      // ADAM: the steps applied so far (nullptr: not counted by this launch)
   int n;
   int64_t total;
   float lr, b1, b2, eps, c1, c2;
 };
 // (the moments' roundings written out: a bias or weight whose gradient is mostly rounding takes a
 // full step all the same, so another contraction of the same sums trains another network)
-__device__ __forceinline__ float adam_step(float w, float g, float* m, float* v, const ParamArgs& a) {
+// (stop: nothing is stored; the flag's load runs beside the others)
+__device__ __forceinline__ float adam_step(float w, float g, float* m, float* v, const ParamArgs& a, int stop) {
   const float o1 = 1.f - a.b1, o2 = 1.f - a.b2;
   const float mi = __fmaf_rn(o1, g, __fmul_rn(a.b1, *m));
   const float vi = __fmaf_rn(__fmul_rn(o2, g), g, __fmul_rn(a.b2, *v));
+  if (stop) return w;
   *m = mi;
   *v = vi;
   return __fsub_rn(w, __fmul_rn(a.lr, mi / a.c1) / (sqrtf(vi / a.c2) + a.eps));
 }
 template <bool ADAM>
 __global__ void param_kernel(const __grid_constant__ ParamArgs a) {
+  int stop = 0;
+  if constexpr (ADAM) {
+    stop = *a.err;
+    if (a.steps && blockIdx.x == 0 && threadIdx.x == 0 && !stop) ++*a.steps;
+  }
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.total; i += (int64_t)gridDim.x * blockDim.x) {
     int q = 0;
     while (q + 1 < a.n && i >= a.l[q + 1].first) ++q;
@@ -408,7 +417,7 @@ __global__ void param_kernel(const __grid_constant__ ParamArgs a) {
       const int o = (int)(k / L.in), c = (int)(k - (int64_t)o * L.in);
       const float g = L.dw[(int64_t)o * L.ldi + c];
       if constexpr (ADAM) {
-        const float w = adam_step(L.W[k], g, L.mW + k, L.vW + k, a);
+        const float w = adam_step(L.W[k], g, L.mW + k, L.vW + k, a, stop);
         L.W[k] = w;
         *reinterpret_cast<__nv_bfloat16*>(L.w16 + tiled(o, c, L.ldi)) = __float2bfloat16_rn(w);
       } else {
@@ -418,7 +427,7 @@ __global__ void param_kernel(const __grid_constant__ ParamArgs a) {
       const int64_t o = k - nw;
       const float g = L.db[o];
       if constexpr (ADAM)
-        L.b[o] = adam_step(L.b[o], g, L.mb + o, L.vb + o, a);
+        L.b[o] = adam_step(L.b[o], g, L.mb + o, L.vb + o, a, stop);
       else
         L.gb[o] = g;
     }
@@ -478,7 +487,7 @@ struct Mlp {
   DBuf<float> x, target, y;
   DBuf<unsigned char> xhi, xlo;
   DBuf<double> loss_part, losses;
-  DBuf<int> err;  // set by a tensor-core product whose bounded wait gave up
+  DBuf<int> err;  // [0] set by a tensor-core product whose bounded wait gave up; [1] Adam steps applied
   int cap = 0, loss_cap = 0;
   int64_t t = 0;  // Adam step
   // weight gradients and bias gradients run beside the chain of dX
@@ -528,7 +537,7 @@ struct Mlp {
       L.db.alloc(L.ldo);
     }
     loss_part.alloc((bp / 128) * (layers.back()->ldo / 64));
-    if (!err.p) err.alloc(1);
+    if (!err.p) err.alloc(2);
     check(cudaStreamSynchronize(nullptr), "sync");  // the clears run on the default stream
   }
 
@@ -539,13 +548,15 @@ struct Mlp {
     loss_cap = n;
   }
 
-  // a bounded wait inside a tensor-core product gave up: report it (and clear the flag)
+  // a bounded wait inside a tensor-core product gave up: report it (and clear the flag).  No step took
+  // part of it (param_kernel), so the optimiser is where the steps applied have brought it.
   void check_err() {
-    int e = 0;
+    int e[2] = {0, 0};
     check(cudaGetLastError(), "launch");
-    check(cudaMemcpyAsync(&e, err.p, sizeof(int), cudaMemcpyDeviceToHost, s), "copy");
+    check(cudaMemcpyAsync(e, err.p, sizeof(e), cudaMemcpyDeviceToHost, s), "copy");
     check(cudaStreamSynchronize(s), "sync");
-    if (e) {
+    if (e[0]) {
+      t = e[1];
       check(cudaMemsetAsync(err.p, 0, sizeof(int), s), "memset");
       throw std::runtime_error("a tensor-core product's bounded wait gave up");
     }
@@ -665,6 +676,8 @@ struct Mlp {
                             a.total, L.in, L.out, L.ldi};
         a.total += (int64_t)L.in * L.out + L.out;
       }
+      a.err = err.p;
+      a.steps = first == 0 ? err.p + 1 : nullptr;
       param_kernel<ADAM><<<grid_for(a.total), 256, 0, s>>>(a);
       count_launch();
     }
@@ -844,6 +857,17 @@ int so_mlp_train(so_mlp h, const float* x, const float* target, size_t batch, si
         so::check(cudaMemcpyAsync(losses + i, m.losses.p, n * sizeof(double), cudaMemcpyDeviceToHost, m.s), "copy");
       m.check_err();
     }
+  });
+}
+
+// Self-test: the next product's error flag is set as if its bounded wait had given up.
+int so_selftest_mlp_give_up(so_mlp h) {
+  if (!h) return SO_ERR_INVALID;
+  return mlp_guard([&] {
+    h->m.ensure(1);
+    const int one = 1;
+    so::check(cudaMemcpyAsync(h->m.err.p, &one, sizeof(int), cudaMemcpyHostToDevice, h->m.s), "copy");
+    so::check(cudaStreamSynchronize(h->m.s), "sync");
   });
 }
 
