@@ -450,7 +450,9 @@ unsigned grid_for(int64_t n) {
 }
 
 void check(cudaError_t e, const char* w) {
-  if (e != cudaSuccess) throw std::runtime_error(std::string(w) + ": " + cudaGetErrorString(e));
+  if (e == cudaSuccess) return;
+  cudaGetLastError();  // an error that the context survives ends with this call
+  throw std::runtime_error(std::string(w) + ": " + cudaGetErrorString(e));
 }
 
 template <typename T>
@@ -459,6 +461,7 @@ struct DBuf {
   size_t n = 0;
   void alloc(size_t count) {
     if (p) cudaFree(p);
+    p = nullptr;
     n = count;
     check(cudaMalloc(&p, std::max<size_t>(1, count) * sizeof(T)), "cudaMalloc");
     check(cudaMemset(p, 0, std::max<size_t>(1, count) * sizeof(T)), "cudaMemset");
@@ -515,7 +518,7 @@ struct Mlp {
 
   void ensure(int batch) {
     if (batch <= cap) return;
-    cap = batch;
+    cap = 0;  // until every buffer has its new size
     const size_t bp = (size_t)padded(batch);
     x.alloc((size_t)batch * w[0]);
     target.alloc((size_t)batch * w.back());
@@ -539,10 +542,12 @@ struct Mlp {
     loss_part.alloc((bp / 128) * (layers.back()->ldo / 64));
     if (!err.p) err.alloc(2);
     check(cudaStreamSynchronize(nullptr), "sync");  // the clears run on the default stream
+    cap = batch;
   }
 
   void need_losses(int n) {
     if (n <= loss_cap) return;
+    loss_cap = 0;
     losses.alloc(n);
     check(cudaStreamSynchronize(nullptr), "sync");
     loss_cap = n;

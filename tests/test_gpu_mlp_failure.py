@@ -31,3 +31,18 @@ def test_no_step_is_taken_on_a_product_that_gave_up():
     net.train(x, t, steps=5, lr=1e-2)
     other.train(x, t, steps=5, lr=1e-2)
     np.testing.assert_array_equal(net.get_params(), other.get_params())
+
+
+def test_a_batch_without_room_leaves_the_network_usable():
+    """The activations of 2^23 rows x 16384 do not fit; what the failed call had already freed is not used
+    by the next one."""
+    ensure_built()
+    import split_operator_gb300 as so
+    net = so.Mlp([1, 16384, 1], seed=5)
+    x = np.linspace(-1, 1, 10, dtype=np.float32)[:, None]
+    first = net.forward(x)
+    with pytest.raises(Exception, match="out of memory"):
+        net.forward(np.zeros((1 << 23, 1), dtype=np.float32))
+    np.testing.assert_array_equal(net.forward(x), first)
+    loss, g = net.gradients(x, first)
+    assert loss == 0.0 and np.all(np.isfinite(g))
