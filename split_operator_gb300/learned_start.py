@@ -179,6 +179,48 @@ def well_frame(prm):
     return re, math.sqrt(a * math.sqrt(2.0 * d * mass))
 
 
+def _recurrence(s, a):
+    """s[i] += a[i] s[i - 1] for i = 1, 2, ..., in place, by doubling: 64 terms each, beyond which the
+    products of the spline's factors (2 - 3^(1/2) and nearly that) are below 1e-36."""
+    a = a.copy()
+    for j in (1, 2, 4, 8, 16, 32):
+        if j >= len(s):
+            break
+        s[j:] += a[j:, None] * s[:-j]
+        a[j:] = a[j:] * a[:-j]
+
+
+def uniform_spline(x, y, at):
+    """Values at `at` of the cubic splines through the columns of y at the uniform points x, with
+    not-a-knot ends (the third derivative is continuous at the second and the last but one point).  In
+    numpy: the first prediction of a process would wait 0.2 s for scipy.interpolate, a fifth of a
+    relaxation."""
+    n, h = len(x), (x[-1] - x[0]) / (len(x) - 1.0)
+    if n < 4:  # the polynomial through them
+        return sum(y[j] * np.prod([(at - x[i]) / (x[j] - x[i]) for i in range(n) if i != j], axis=0)[:, None]
+                   for j in range(n))
+    # slopes s: s[i-1] + 4 s[i] + s[i+1] = 3 (y[i+1] - y[i-1]) / h inside; the end conditions
+    # combined with their neighbours: s[0] + 2 s[1] = (-5 y[0] + 4 y[1] + y[2]) / (2 h), and the mirror image
+    s = np.empty_like(y)
+    s[1:-1] = (y[2:] - y[:-2]) * (3.0 / h)
+    s[0] = (-5.0 * y[0] + 4.0 * y[1] + y[2]) / (2.0 * h)
+    s[-1] = (5.0 * y[-1] - 4.0 * y[-2] - y[-3]) / (2.0 * h)
+    # tridiagonal elimination (diagonal 1, 4, ..., 4, 1; beside it 2 at the ends and 1)
+    c = np.empty(n)
+    c[0] = 2.0
+    for i in range(1, n - 1):
+        c[i] = 1.0 / (4.0 - c[i - 1])
+    s[1:-1] *= c[1:-1, None]
+    _recurrence(s[:-1], np.concatenate([[0.0], -c[1:-1]]))
+    s[-1] = (s[-1] - 2.0 * s[-2]) / (1.0 - 2.0 * c[n - 2])
+    _recurrence(s[::-1], np.concatenate([[0.0], -c[n - 2::-1]]))
+    k = np.clip(((at - x[0]) / h).astype(np.int64), 0, n - 2)
+    t = ((at - x[k]) / h)[:, None]
+    d = y[k + 1] - y[k]
+    a, b = h * s[k] - d, d - h * s[k + 1]
+    return y[k] + t * (d + (1.0 - t) * ((1.0 - t) * a + t * b))
+
+
 class RadialBasis:
     """Per l: the leading `modes` left singular vectors of the training radial functions,
     sampled in the well's scaled coordinate xi (well_frame) on a fixed grid, so that the
@@ -189,10 +231,6 @@ class RadialBasis:
         self.xi = np.linspace(-xi_max, xi_max, nxi)
         if u is not None:  # a saved basis
             self.u = np.asarray(u, dtype=np.float64)
-            try:  # loaded here: the first prediction would wait 0.2 s for it, a fifth of a relaxation
-                import scipy.interpolate  # noqa: F401
-            except ImportError:
-                pass
             return
         psil = np.stack([self.to_xi(g.to_l(s.astype(np.float64)), p) for s, p in zip(states, params)])
         self.u = np.empty((g.nth, nxi, modes))
@@ -210,11 +248,11 @@ class RadialBasis:
         return out
 
     def from_xi(self, psixi, prm):  # [nxi, nl] -> [nr, nl]
-        from scipy.interpolate import CubicSpline
         re, sc = well_frame(prm)
         xi = (self.g.r - re) * sc
-        out = CubicSpline(self.xi, psixi, axis=0)(np.clip(xi, self.xi[0], self.xi[-1]))
-        out[(xi < self.xi[0]) | (xi > self.xi[-1])] = 0.0
+        inside = (xi >= self.xi[0]) & (xi <= self.xi[-1])
+        out = np.zeros((len(xi), psixi.shape[1]))
+        out[inside] = uniform_spline(self.xi, psixi, xi[inside])
         return out
 
     def coefficients(self, state, prm):
