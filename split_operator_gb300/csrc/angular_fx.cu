@@ -79,17 +79,6 @@ static int fx_columns(const Geometry& g, int64_t stride, int sms) {
   return best;
 }
 
-static int fx_sms() {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sms = 1;
-  }
-  return sms;
-}
-
 bool fx_angular_plan(PassParams& p, const DevOp* ops, int nops, const double* table_max, int* cols) {
   Geometry& g = p.g;
   if (g.n < 16 || g.n > 256) return false;
@@ -126,7 +115,7 @@ bool fx_angular_plan(PassParams& p, const DevOp* ops, int nops, const double* ta
     }
   }
   if (mats < 1 || mats > 2 || across > kFxTabSlots || !(prod <= kMaxProduct)) return false;
-  const int bn = fx_columns(g, stride, fx_sms());
+  const int bn = fx_columns(g, stride, sm_count());
   if (bn == 0) return false;
   g.lanes_per_tile = bn;
   g.tiles_per_outer = (int32_t)((g.inner + bn - 1) / bn);
@@ -175,7 +164,7 @@ void fx_angular_params(const PassParams& p, const int* mat_op, int nmat, const u
 
 cudaError_t launch_fx_angular(int real, int n, int cols, bool exps, const void* one, const void* params_dev,
                               const void* owners_dev, int64_t tiles, cudaStream_t s) {
-  const unsigned grid = (unsigned)(tiles < fx_sms() ? tiles : fx_sms());
+  const unsigned grid = (unsigned)(tiles < sm_count() ? tiles : sm_count());
   const FxTcParams* prm = reinterpret_cast<const FxTcParams*>(params_dev);
   const uint2* own = reinterpret_cast<const uint2*>(owners_dev);
   FxAngularLaunch* const launch = real == kRealFF ? (exps ? launch_fx_angular_ff_exps : launch_fx_angular_ff)
@@ -183,6 +172,6 @@ cudaError_t launch_fx_angular(int real, int n, int cols, bool exps, const void* 
   return launch(fx_halves(n), fx_kp(n), cols, one, prm, own, tiles, grid, s);
 }
 
-int64_t fx_angular_grid(int64_t tiles) { return tiles < fx_sms() ? tiles : fx_sms(); }
+int64_t fx_angular_grid(int64_t tiles) { return tiles < sm_count() ? tiles : sm_count(); }
 
 }  // namespace so

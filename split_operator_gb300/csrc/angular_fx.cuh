@@ -14,9 +14,12 @@
 // likewise; both are cut into seven signed 8-bit digits, held as FP16 integers of magnitude
 // <= 128.  The digit products of one order r = i + j (A digit i, B digit j) share a weight, so
 // they sum in one FP32 accumulator: (r + 1) K 2^14 <= 2^24 for K = 128 and every r <= 6, so
-// the sums are exact (K = 256: r <= 3; the other orders weigh less than 2^-48).  The 28
-// products of orders 0 .. 6 give the matrix product to 2^-54 of (row maximum x column
-// maximum), a rounding error of FP64's size at the largest terms.
+// the sums are exact (K = 256: r <= 3; the other orders weigh less than 2^-48).  The products of
+// orders 7 .. 12 are left out: at most 2^-51 of (row maximum x column maximum) for random rows and
+// columns of K = 128, 2^-47 for constant ones, whose sum is 2^7 times as large (2^-45.5 and 2^8 for K =
+// 256).  Error of [T, phase, T^-1], relative L2 per column, against the same in FP64: Legendre pairs of
+// 16 to 256 points 1.0e-16 - 5.2e-16 / 1.6e-16 - 9.4e-16 (columns random, constant, of few or the highest
+// l, of one point), random orthogonal ones of 16 points 2.3e-16 / 2.1e-16, from 32 on below FP64's.
 //
 // A tile is BN complex columns of the inner axis for all n rows (n <= 256), N = 2 BN real
 // columns.  One persistent CTA per SM (seven accumulators of 64 columns fill its tensor memory):

@@ -184,9 +184,9 @@ int fft_pair_threads(const Geometry& g);  // the default threads per CTA
 int fft_pair_block(const PassParams& p);  // threads per CTA of a planned pass (lanes per tile x n / 16)
 
 // The same pass of FP64 and float-float states in 64-bit fixed point (fx_fft.cu), powers of two
-// from 16 to 8192 and other lengths from 17 to 4096 (p.fx_chirp): a forward transform, then an inverse one, with tables whose largest magnitudes (table_max,
-// per op) fx.cuh's bounds allow.  Sets the tiling and p.fx; the ops' tables and p.twiddle are
-// then the fixed-point ones.
+// from 16 to 8192 and other lengths from 17 to 4096 (p.fx_chirp): a forward transform, then an
+// inverse one, with tables whose largest magnitudes (table_max, per op) fx.cuh's bounds allow.  Sets
+// the tiling and p.fx; the ops' tables and p.twiddle are then the fixed-point ones.
 bool fx_pair_plan(PassParams& p, int real, const double* table_max);
 // one pass (one != nullptr) or a batched launch
 cudaError_t launch_fx_pair(int real, bool chirp, int lgn, const PassParams* one, const PassParams* params_dev,

@@ -102,7 +102,7 @@ bool fx_pair_plan(PassParams& p, int real, const double* table_max) {
   const int V = pair_vals(lg);
   int T = kPairThreads;
   const int least = m / V > 32 ? (int)(m / V) : 32;
-  while (T > least && (g.outer * m + (int64_t)V * T - 1) / ((int64_t)V * T) < 304) T /= 2;
+  while (T > least && (g.outer * m + (int64_t)V * T - 1) / ((int64_t)V * T) < 2 * sm_count()) T /= 2;
   const int64_t L = (int64_t)V * T / m;
   g.lanes_per_tile = (int32_t)L;
   g.tiles_per_outer = 1;

@@ -5,10 +5,11 @@
 // FP64 a single SM's FP64 pipe set the pace (about 100 operations per point and step at 1.7 per
 // clock: 51 us a step of 1024 points).  Here a thread holds 4 values (radix-4 stages: n / 4
 // threads keep every scheduler of the SM busy from 512 points on, where 16 values per thread
-// would leave one warp to a scheduler), the norms are integer sums and the scalar slots live in
-// shared memory during the launch (a dependent access to the slots in global memory costs more
-// than a stage).  At the end of every step the state is rounded to its storage precision, as a
-// store and load would, so a run of steps gives the same bits however it is split into launches.
+// would leave one warp to a scheduler), the norms are integer sums (units of 2^62, sums of 2^56 and
+// more; weights of many decades and momentum grids: FP64) and the scalar slots live in shared
+// memory during the launch (a dependent access to the slots in global memory costs more than a
+// stage).  At the end of every step the state is rounded to its storage precision, as a store and
+// load would, so a run of steps gives the same bits however it is split into launches.
 // Lengths that are no power of two go through transforms of M >= 2 n - 1 points (fx_pair.cuh).
 #pragma once
 #include "fx_stage.cuh"

@@ -24,18 +24,23 @@ __device__ __forceinline__ void wait_for_previous() {
 }
 #endif
 
+// SMs of the current device at the first call (1 if it cannot be asked)
+inline int sm_count() {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      n = 1;
+    return n;
+  }();
+  return sms;
+}
+
 // Dynamic shared memory of an overlapped launch: where its blocks do not outnumber the SMs, enough
 // that an SM holds only one.  Blocks that begin while the kernel ahead still runs would otherwise
 // crowd on the SMs that it left idle (measured: 41.5 us a step instead of 39.2, and 71.7 instead of
 // 61.0 for 45 x 1000 points in FP64).
 inline size_t one_block_per_sm(int64_t blocks, size_t smem) {
-  static const int sms = [] {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      n = 0;
-    return n;
-  }();
-  return blocks <= sms && smem < kHalfSmem ? kHalfSmem : smem;
+  return blocks <= sm_count() && smem < kHalfSmem ? kHalfSmem : smem;
 }
 
 template <typename... P, typename... A>
